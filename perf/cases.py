@@ -282,3 +282,136 @@ def tolerance(c):
     if c["dtype"] == "fp16":
         return {"rel": 1.7e-3 if paged else 1.25e-3, "max": 0.04}
     return {"rel": 1.3e-2 if paged else 1e-2, "max": 0.5 if c.get("grad") else 0.1}
+
+
+# ---------------------------------------------------------------------------
+# the same in 64 bits
+# ---------------------------------------------------------------------------
+def _attend64(q, k, v, scale, causal, window=-1, softcap=0.0, mask=None, do=None):
+    """Attention of one head in float64, [N, D] against [S, D]; with ``do`` also the gradients of q, k and v."""
+    N, S, D = q.shape[0], k.shape[0], q.shape[1]
+    out, lse = torch.zeros_like(q), torch.full((N,), -math.inf, dtype=torch.float64, device=q.device)
+    dq, dk, dv = (torch.zeros_like(x) for x in (q, k, v)) if do is not None else (None, None, None)
+    step = max(64, (1 << 26) // max(S, 1))
+    if window >= 0:
+        step = min(step, 2048)
+    for i in range(0, N, step):
+        n = min(step, N - i)
+        hi = min(S, i + n + S - N) if causal else S
+        lo = max(0, i + S - N - window) if window >= 0 else 0
+        if hi <= lo:
+            continue
+        raw = q[i:i + n] @ k[lo:hi].T
+        raw *= scale
+        s = softcap * torch.tanh(raw / softcap) if softcap > 0 else raw
+        qpos = torch.arange(i, i + n, device=q.device)[:, None] + (S - N)
+        kpos = torch.arange(lo, hi, device=q.device)[None, :]
+        off = torch.zeros((n, hi - lo), dtype=torch.bool, device=q.device)
+        if causal:
+            off |= kpos > qpos
+        if window >= 0:
+            off |= kpos < qpos - window
+        if mask is not None:
+            off |= ~mask(i, i + n, lo, hi)
+        s = s.masked_fill(off, -math.inf)
+        m = s.amax(1, keepdim=True)
+        m[m == -math.inf] = 0.0
+        p = torch.exp(s - m)
+        total = p.sum(1, keepdim=True)
+        lse[i:i + n] = (m + torch.log(total))[:, 0] / math.log(2.0)
+        p /= torch.where(total > 0, total, torch.ones_like(total))
+        out[i:i + n] = p @ v[lo:hi]
+        if do is not None:
+            g = do[i:i + n]
+            dv[lo:hi] += p.T @ g
+            ds = p * (g @ v[lo:hi].T - (g * out[i:i + n]).sum(1, keepdim=True))
+            if softcap > 0:
+                ds *= 1 - torch.tanh(raw / softcap) ** 2
+            dq[i:i + n] = ds @ k[lo:hi] * scale
+            dk[lo:hi] += ds.T @ q[i:i + n] * scale
+    return out, lse, dq, dk, dv
+
+
+def _rotated64(x, s):
+    half = x.shape[-1] // 2
+    pos = torch.tensor(s["pos"], device=x.device)
+    cos, sin = s["cos"][pos].double()[:, None, None], s["sin"][pos].double()[:, None, None]
+    a, b = x[..., :half].double(), x[..., half:].double()
+    return torch.cat([a * cos - b * sin, a * sin + b * cos], -1)
+
+
+def exact(c, seed):
+    """What ``run`` returns for these inputs, in float64.  The bytes of an 8-bit pool have no such value."""
+    s = prepare(c, seed)
+    D, scale = c["D"], 1.0 / math.sqrt(c["D"])
+    if c["kind"] in ("paged", "serve"):
+        q, pools = s["q"].double(), []
+        for pool, sc in ((s["kp"], s["ks"]), (s["vp"], s["vs"])):
+            pools.append((pool.view(-1, c["Hkv"], D), None if sc is None else sc.view(-1, c["Hkv"])))
+        new = None
+        if c["kind"] == "serve":
+            q, new = _rotated64(s["q"], s), (_rotated64(s["k"], s)[:, :, 0], s["v"][:, :, 0].double())
+            if c["kv"] in ("int8", "e4m3"):     # the stored row: one float16 scale, values rounded to the pool's type
+                top, rounded = (127.0, []) if c["kv"] == "int8" else (448.0, [])
+                for x in new:
+                    one = (x.abs().amax(-1, keepdim=True) / top).half().double()
+                    y = (x / one).clamp(-top, top)
+                    rounded.append((y.round() if c["kv"] == "int8" else y.float().to(torch.float8_e4m3fn).double()) * one)
+                new = rounded
+        out = torch.zeros_like(q)
+        group, lens = c["Hq"] // c["Hkv"], s["lens"].tolist()
+        for b, n in enumerate(lens):
+            pages = s["table"][b, :-(-n // c["page"])].long()
+            at = (pages[:, None] * c["page"] + torch.arange(c["page"], device=pages.device)).reshape(-1)[:n]
+            kv = []
+            for i, (pool, sc) in enumerate(pools):
+                x = pool[at].double()
+                if sc is not None:
+                    x *= sc[at].double().unsqueeze(-1)
+                if new is not None:
+                    x[n - 1] = new[i][b]
+                kv.append(x)
+            for h in range(c["Hkv"]):
+                for g in range(h * group, (h + 1) * group):
+                    out[b, g] = _attend64(q[b, g], kv[0][:, h], kv[1][:, h], scale, True)[0]
+        if c["kind"] == "paged":
+            return out
+        if c["kv"] in ("int8", "e4m3"):
+            return [out, None, None, None, None]
+        full = []
+        for i, pool in enumerate((s["kp"], s["vp"])):
+            x = pool.double()
+            x.view(-1, c["Hkv"], D)[s["slots"]] = new[i]
+            full.append(x)
+        return [out, full[0], full[1], None, None]
+    q, k, v = (s[n].detach().double() for n in "qkv")
+    do = s["do"].double() if c.get("grad") else None
+    mask = None
+    if c["kind"] == "sparse":
+        rows, cols = 32, 32 if D <= 64 else 16
+        cells = s["mask"].bool()
+
+        def mask(i0, i1, j0, j1):
+            r, t = torch.arange(i0, i1, device=cells.device) // rows, torch.arange(j0, j1, device=cells.device) // cols
+            return cells[r[:, None], t[None, :]]
+    spans = [(0, q.shape[2], 0, k.shape[2])]
+    if c["kind"] == "varlen":
+        cu = s["cu"].tolist()
+        spans = [(a, b, a, b) for a, b in zip(cu, cu[1:])]
+    out, lse = torch.zeros_like(q), torch.zeros(q.shape[:3], dtype=torch.float64, device=q.device)
+    dq, dk, dv = (torch.zeros_like(x) for x in (q, k, v))
+    group = q.shape[1] // k.shape[1]
+    for b in range(q.shape[0]):
+        for h in range(q.shape[1]):
+            for i0, i1, j0, j1 in spans:
+                r = _attend64(q[b, h, i0:i1], k[b, h // group, j0:j1], v[b, h // group, j0:j1], scale, c["causal"],
+                              c.get("window", -1) if c["kind"] == "dense" else -1, c.get("softcap", 0.0), mask,
+                              None if do is None else do[b, h, i0:i1])
+                out[b, h, i0:i1], lse[b, h, i0:i1] = r[0], r[1]
+                if do is not None:
+                    dq[b, h, i0:i1] = r[2]
+                    dk[b, h // group, j0:j1] += r[3]
+                    dv[b, h // group, j0:j1] += r[4]
+    if do is not None:
+        return [out, dq, dk, dv]
+    return (out, lse) if c.get("lse") else out

@@ -46,13 +46,18 @@ namespace {
 
 constexpr int kBS = 16;           // tokens per unit (one TMA box, one consumer step); a page is 1, 2, 4, ... units
 constexpr int kMaxStages = 8;
+// Up to this many sequences every CTA makes the page prefix sums itself, in shared memory (at most 4 KB): one read of
+// seq_lens and a scan, ~1 us, where a planning kernel in front and a binary search through its result in global memory
+// cost ~6 us before the first page was requested.  Beyond it decode_plan_kernel scans once for all.
+constexpr int kSmemSeqs = 1024;
 
 enum KvKind { KV_F16 = 0, KV_BF16 = 1, KV_I8 = 2, KV_E4M3 = 3 };
 
 struct DecodeLayout {          // workspace carve-up, in bytes from the workspace base
   size_t err;                  // int[4]: [0] error word
-  size_t counters;             // int[B * HG]
-  size_t page_start;           // int[B + 1]
+  size_t counters;             // int[B * HG]: parts (or groups of parts) of a sequence that have arrived
+  size_t group_counters;       // int[slots * HG]: parts of a group that have arrived, by the group's first slot
+  size_t page_start;           // int[B + 1], only when B > kSmemSeqs
   size_t part_lse;             // float[slots * Hq * Nq]
   size_t part_o;               // float[slots * Hq * Nq * D]
   size_t total;
@@ -65,9 +70,10 @@ __host__ __device__ inline DecodeLayout make_layout(int B, int Hq, int Nq, int H
   DecodeLayout L;
   L.err = 0;
   L.counters = 16;
-  L.page_start = align_up(L.counters + sizeof(int) * static_cast<size_t>(B) * HG, 16);
   L.slots = G + B;
-  L.part_lse = align_up(L.page_start + sizeof(int) * (static_cast<size_t>(B) + 1), 16);
+  L.group_counters = L.counters + sizeof(int) * static_cast<size_t>(B) * HG;
+  L.page_start = align_up(L.group_counters + sizeof(int) * static_cast<size_t>(L.slots) * HG, 16);
+  L.part_lse = align_up(L.page_start + (B > kSmemSeqs ? sizeof(int) * (static_cast<size_t>(B) + 1) : 0), 16);
   L.part_o = align_up(L.part_lse + sizeof(float) * static_cast<size_t>(L.slots) * Hq * Nq, 16);
   L.total = align_up(L.part_o + sizeof(float) * static_cast<size_t>(L.slots) * Hq * Nq * kD, 16);
   return L;
@@ -89,28 +95,37 @@ struct KernelArgs {
 };
 
 // ---------------------------------------------------------------------------
-// plan: page prefix sums, counters and error word reset
+// plan: counters and error word reset; page prefix sums when there are more than kSmemSeqs sequences
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch: the main kernel may start as soon as this one has, and waits (pdl_wait) before it
+// touches anything that is written here.  Up to kSmemSeqs sequences that is only the counters, which it needs last, so
+// this launch costs no time of its own; it starts after everything earlier in the stream has completed, so whatever
+// the main kernel reads before its wait (pools, table, lengths, queries) is in place.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+__device__ __forceinline__ int units_of(const int32_t* seq_lens, int i, int max_kv_len) {
+  int len = seq_lens != nullptr ? seq_lens[i] : max_kv_len;
+  len = len < 0 ? 0 : (len > max_kv_len ? max_kv_len : len);
+  return (len + kBS - 1) / kBS;
+}
+
 __global__ void __launch_bounds__(1024) decode_plan_kernel(const int32_t* __restrict__ seq_lens, int B,
                                                            int max_kv_len, int n_counters,
                                                            int* __restrict__ err, int* __restrict__ counters,
                                                            int* __restrict__ page_start) {
+  pdl_launch_dependents();
   __shared__ int warp_sums[32];
   __shared__ int carry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) { carry = 0; page_start[0] = 0; }
   if (tid < 4) err[tid] = 0;
   for (int i = tid; i < n_counters; i += blockDim.x) counters[i] = 0;
+  if (page_start == nullptr) return;
+  if (tid == 0) { carry = 0; page_start[0] = 0; }
   __syncthreads();
   for (int base = 0; base < B; base += blockDim.x) {
     const int i = base + tid;
-    int val = 0;
-    if (i < B) {
-      int len = seq_lens != nullptr ? seq_lens[i] : max_kv_len;
-      len = len < 0 ? 0 : (len > max_kv_len ? max_kv_len : len);
-      val = (len + kBS - 1) / kBS;
-    }
-    int x = val;
+    int x = i < B ? units_of(seq_lens, i, max_kv_len) : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -194,6 +209,56 @@ __device__ __forceinline__ int cta_of_unit(long long u, int G, long long U) {
 }
 
 // ---------------------------------------------------------------------------
+// combine of partials
+// ---------------------------------------------------------------------------
+// One warp merges n partials of one query row: L = log2 sum_i 2^lse_i, O = sum_i 2^(lse_i - L) O_i
+// (csrc/mfa_steel_fwd.cpp:2066-2101).  lse / o point at the first partial's row, stride slots apart in units of
+// lse_step / o_step floats; lane l carries head-dim values [4l, 4l + 4).  What bounds it is the latency of L2: the
+// lanes fetch 32 log-sum-exps at once and the rows are read 16 at a time, all in flight together (one after the other,
+// the 148 partials of one 262144-token sequence took longer than half of its keys: 198 us in all).
+template <int kD>
+__device__ __forceinline__ float combine_row(const float* lse, size_t lse_step, const float* o, size_t o_step, int n,
+                                             int lane, float4& out) {
+  float m = -INFINITY, wsum = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool live = lane * 4 < kD;                  // head_dim 64: the first 16 lanes carry the row
+  for (int base = 0; base < n; base += 32) {
+    const int cn = min(32, n - base);
+    const float lv = lane < cn ? __ldcg(lse + (base + lane) * lse_step) : -INFINITY;
+    float mx = lv;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+    const float m_new = fmaxf(m, mx);
+    const float ms = (m_new == -INFINITY) ? 0.f : m_new;
+    const float corr = exp2f(m - ms);               // 0 from -inf
+    acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
+    const float w = exp2f(lv - ms);
+    float ws = w;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, s);
+    wsum = fmaf(wsum, corr, ws);
+    m = m_new;
+    for (int i0 = 0; i0 < cn; i0 += 16) {
+      float4 v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live && i0 + k < cn) v[k] = __ldcg(reinterpret_cast<const float4*>(o + (base + i0 + k) * o_step + lane * 4));
+      }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float wk = __shfl_sync(0xffffffffu, w, (i0 + k) & 31);
+        acc.x = fmaf(wk, v[k].x, acc.x); acc.y = fmaf(wk, v[k].y, acc.y);
+        acc.z = fmaf(wk, v[k].z, acc.z); acc.w = fmaf(wk, v[k].w, acc.w);
+      }
+    }
+  }
+  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
+  out = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+  return wsum > 0.f ? m + log2f(wsum) : -INFINITY;
+}
+
+// ---------------------------------------------------------------------------
 // main kernel
 // ---------------------------------------------------------------------------
 // CAP: soft cap on.  A template parameter so that the common launch without one carries no tanh code in its unrolled
@@ -223,6 +288,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   int* s_page = reinterpret_cast<int*>(bars + 2 * kMaxStages);
   volatile int* s_abort = s_page + kMaxStages;
   int* s_last = const_cast<int*>(s_abort) + 1;
+  int* s_page_start = s_last + 2;                       // int[B + 1] when B <= kSmemSeqs
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -232,12 +298,49 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
   int* err = reinterpret_cast<int*>(ws + a.lay.err);
   int* counters = reinterpret_cast<int*>(ws + a.lay.counters);
-  const int* page_start = reinterpret_cast<const int*>(ws + a.lay.page_start);
+  int* group_counters = reinterpret_cast<int*>(ws + a.lay.group_counters);
   float* part_lse = reinterpret_cast<float*>(ws + a.lay.part_lse);
   float* part_o = reinterpret_cast<float*>(ws + a.lay.part_o);
 
   const int rows = a.rows;
   const int HqNq = p.Hq * p.Nq;
+
+  if (tid == 0) {
+    prefetch_tmap(&tmK);
+    prefetch_tmap(&tmV);
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(smem_u32(&bars[i]), 1);                 // full: producer arrive (+ tx bytes)
+      mbar_init(smem_u32(&bars[kMaxStages + i]), HPC);  // empty: one arrive per consumer warp
+    }
+    *s_abort = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  // page prefix sums
+  const int* page_start = s_page_start;
+  if (p.B <= kSmemSeqs) {
+    for (int i = tid; i < p.B; i += blockDim.x) s_page_start[i + 1] = units_of(p.seq_lens, i, p.max_kv_len);
+    __syncthreads();
+    if (warp == 0) {
+      // lane l owns the entries [l * per, (l + 1) * per)
+      const int per = (p.B + 31) >> 5, i0 = lane * per, i1 = min(p.B, i0 + per);
+      int sum = 0;
+      for (int i = i0; i < i1; ++i) sum += s_page_start[i + 1];
+      int x = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      x -= sum;
+      for (int i = i0; i < i1; ++i) { x += s_page_start[i + 1]; s_page_start[i + 1] = x; }
+      if (lane == 0) s_page_start[0] = 0;
+    }
+  } else {
+    pdl_wait();
+    page_start = reinterpret_cast<const int*>(ws + a.lay.page_start);
+  }
+  __syncthreads();
 
   // Sequences of length zero have no unit: CTA 0 of each head group zero-fills them.
   if (c == 0) {
@@ -267,22 +370,12 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   // CTAs sharing a sequence are always consecutive.
   const long long U = page_start[p.B];
   const int G = U < static_cast<long long>(gridDim.x) ? static_cast<int>(U) : static_cast<int>(gridDim.x);
-  if (c >= G) return;
-  const long long lo = static_cast<long long>(c) * U / G;
-  const long long hi = static_cast<long long>(c + 1) * U / G;
-  if (lo >= hi) return;
-
-  if (tid == 0) {
-    for (int i = 0; i < NS; ++i) {
-      mbar_init(smem_u32(&bars[i]), 1);                 // full: producer arrive (+ tx bytes)
-      mbar_init(smem_u32(&bars[kMaxStages + i]), HPC);  // empty: one arrive per consumer warp
-    }
-    *s_abort = 0;
-    *s_last = 0;
-    fence_barrier_init();
-    fence_proxy_async();
+  const long long lo = c < G ? static_cast<long long>(c) * U / G : 0;
+  const long long hi = c < G ? static_cast<long long>(c + 1) * U / G : 0;
+  if (lo >= hi) {
+    pdl_wait();               // the launch completes only after the plan kernel has
+    return;
   }
-  __syncthreads();
 
   // first sequence: largest b with page_start[b] <= lo
   int b_first;
@@ -304,6 +397,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     long long u = lo;
     int b = b_first;
     bool ok = true;
+    int bad = 0;                // error bits; the error word is the plan kernel's to clear, so they go there at the end
     while (u < hi && ok) {
       const int s0 = page_start[b], s1 = page_start[b + 1];
       if (s1 <= u) { ++b; continue; }
@@ -320,7 +414,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             my_tok = jj * kBS;
           } else {
             const int pg_id = row[jj / a.upp];
-            if (pg_id >= p.num_pages) atomicOr(err, 2);              // table entry beyond the pool
+            if (pg_id >= p.num_pages) bad = 2;                       // table entry beyond the pool
             else if (pg_id >= 0) my_tok = pg_id * p.block_size + (jj % a.upp) * kBS;
           }
         }
@@ -354,7 +448,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       u = s0 + j_hi;
       if (u >= s1) ++b;
     }
-    if (!ok && lane == 0) atomicOr(err, 1);
+    if (!ok) bad |= 1;
+    pdl_wait();
+    if (bad != 0) atomicOr(err, bad);
     return;
   }
 
@@ -734,63 +830,72 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     }
 
     if (!direct) {
-      __threadfence();
-      named_bar_sync(1, HPC * 32);
-      if (tid == 0) {
-        const int old = atomicAdd(&counters[b * a.HG + hg], 1);
-        *s_last = (old == n_parts - 1) ? 1 : 0;
-      }
-      named_bar_sync(1, HPC * 32);
-      const bool last = *s_last != 0;
-      if (last) {
-        __threadfence();
-        // combine: L = log2 sum_i 2^lse_i ; O = sum_i 2^(lse_i - L) O_i  (csrc/mfa_steel_fwd.cpp:2066-2101)
+      // The part that arrives last combines.  Up to 32 parts at once; more in two steps, so that the work of a sequence
+      // spread over many CTAs is shared out: the last part of each group of 16 (64 from 512 parts on) merges its group
+      // into the group's first slot, the last group merges those.  Parts of a sequence are consecutive CTAs and their
+      // slots consecutive, so every split is the same whoever arrives last: results do not depend on the order.
+      // 262144 tokens x 8 heads over 148 CTAs: 198 us with one warp reading 148 partials a row at a time.
+      const int gsz = n_parts <= 32 ? 32 : (n_parts <= 512 ? 16 : 64);
+      const int grp = (c - c_first) / gsz, n_grp = (n_parts + gsz - 1) / gsz;
+      const int slot0 = c_first + b;                                  // the sequence's first slot
+      const int gslot = slot0 + grp * gsz;                            // the group's first slot
+      const int gn = min(gsz, n_parts - grp * gsz);
+      auto merge = [&](int first, int step, int n, bool final_out) {
         for (int r = 0; r < rows; ++r) {
           const int hq = kvh * a.group + r % a.group;
           const int qi = r / a.group;
           const size_t rowi = static_cast<size_t>(hq) * p.Nq + qi;
-          float mmax = -INFINITY;
-          for (int i = 0; i < n_parts; ++i)
-            mmax = fmaxf(mmax, __ldcg(&part_lse[static_cast<size_t>(c_first + i + b) * HqNq + rowi]));
-          const float msb = (mmax == -INFINITY) ? 0.f : mmax;
-          float wsum = 0.f;
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          const bool col_live = lane * 4 < kD;            // head_dim 64: the first 16 lanes carry the row
-          for (int i = 0; i < n_parts; ++i) {
-            const size_t sl = static_cast<size_t>(c_first + i + b);
-            const float w = exp2f(__ldcg(&part_lse[sl * HqNq + rowi]) - msb);
-            wsum += w;
-            if (!col_live) continue;
-            const float4 v4 = __ldcg(reinterpret_cast<const float4*>(&part_o[(sl * HqNq + rowi) * kD + lane * 4]));
-            acc.x = fmaf(w, v4.x, acc.x); acc.y = fmaf(w, v4.y, acc.y);
-            acc.z = fmaf(w, v4.z, acc.z); acc.w = fmaf(w, v4.w, acc.w);
+          const size_t row0 = static_cast<size_t>(first) * HqNq + rowi;
+          float4 v;
+          const float lse = combine_row<kD>(part_lse + row0, static_cast<size_t>(step) * HqNq, part_o + row0 * kD,
+                                            static_cast<size_t>(step) * HqNq * kD, n, lane, v);
+          const bool col_live = lane * 4 < kD;
+          if (!final_out) {
+            // in place: only this warp reads these rows, and it has
+            __syncwarp();
+            if (col_live) __stcg(reinterpret_cast<float4*>(part_o + row0 * kD + lane * 4), v);
+            if (lane == 0) __stcg(part_lse + row0, lse);
+            continue;
           }
-          const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
           const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
           const size_t o = orow * kD + lane * 4;
           if (p.packed_f32) {
             float* pk = reinterpret_cast<float*>(p.out) + orow * (kD + 4);
-            if (col_live) *reinterpret_cast<float4*>(pk + lane * 4) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-            if (lane == 0) pk[kD] = wsum > 0.f ? mmax + log2f(wsum) : -INFINITY;
-          } else if (!col_live) {
-          } else if (p.q_dtype == 0) {
-            __half2 h0 = __floats2half2_rn(acc.x * inv, acc.y * inv), h1 = __floats2half2_rn(acc.z * inv, acc.w * inv);
-            uint2 pk = make_uint2(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1));
-            *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.out) + o) = pk;
+            if (col_live) *reinterpret_cast<float4*>(pk + lane * 4) = v;
+            if (lane == 0) pk[kD] = lse;
           } else {
-            __nv_bfloat162 h0 = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), h1 = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
-            uint2 pk = make_uint2(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1));
-            *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + o) = pk;
+            if (col_live) {
+              const uint2 pk = p.q_dtype == 0 ? make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w))
+                                              : make_uint2(pack_bf2(v.x, v.y), pack_bf2(v.z, v.w));
+              *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out) + o) = pk;
+            }
+            if (p.lse != nullptr && lane == 0) p.lse[orow] = lse;
           }
-          if (!p.packed_f32 && p.lse != nullptr && lane == 0) p.lse[orow] = wsum > 0.f ? mmax + log2f(wsum) : -INFINITY;
         }
+      };
+      // true in every consumer thread of the CTA that brings `counter` to n
+      auto arrive_last = [&](int* counter, int n, int* flag) -> bool {
+        __threadfence();
+        named_bar_sync(1, HPC * 32);
+        if (tid == 0) *flag = atomicAdd(counter, 1) == n - 1 ? 1 : 0;
+        named_bar_sync(1, HPC * 32);
+        const bool last = *flag != 0;
+        if (last) __threadfence();
+        return last;
+      };
+      pdl_wait();                                                     // the counters are the plan kernel's to clear
+      if (arrive_last(&group_counters[static_cast<size_t>(gslot) * a.HG + hg], gn, s_last)) {
+        merge(gslot, 1, gn, n_grp == 1);
+        if (n_grp > 1 && arrive_last(&counters[static_cast<size_t>(b) * a.HG + hg], n_grp, s_last + 1))
+          merge(slot0, gsz, n_grp, true);
       }
-      named_bar_sync(1, HPC * 32);   // s_last is reused by the next sequence
+      named_bar_sync(1, HPC * 32);   // the flags are reused by the next sequence
     }
 
     u = static_cast<long long>(s0) + j_hi;
     if (u >= s1) ++b;
   }
+  pdl_wait();
   if (!ok && lane == 0) atomicOr(err, 1);
 }
 
@@ -867,8 +972,17 @@ cudaError_t launch_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const Kerne
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    kern<<<grid, (HPC + 1) * 32, smem, stream>>>(tmK, tmV, a);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((HPC + 1) * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, tmK, tmV, a);
   };
   return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true>) : go(decode_paged_kernel<KV, HPC, D, false>);
 }
@@ -940,7 +1054,8 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.q_prescale = sc;
   a.cap_log2 = p.softcap * kLog2e;
   a.inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
-  const size_t smem = 1024 + static_cast<size_t>(stages) * per_stage + 2 * kMaxStages * 8 + kMaxStages * 4 + 64;
+  const size_t smem = 1024 + static_cast<size_t>(stages) * per_stage + 2 * kMaxStages * 8 + kMaxStages * 4 + 64 +
+                      (p.B <= kSmemSeqs ? sizeof(int) * (static_cast<size_t>(p.B) + 1) : 0);
 
   // tensor maps, in bytes: (128 B, tokens, 128-byte halves of a row, heads, batch).  A pool is one "batch" of
   // num_pages * block_size tokens with the heads of a token side by side; a dense cache has its own strides.
@@ -976,10 +1091,10 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   }
 
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
-  decode_plan_kernel<<<1, 1024, 0, stream>>>(p.seq_lens, p.B, p.max_kv_len, p.B * HG,
+  decode_plan_kernel<<<1, 1024, 0, stream>>>(p.seq_lens, p.B, p.max_kv_len, (p.B + a.lay.slots) * HG,
                                              reinterpret_cast<int*>(ws + a.lay.err),
                                              reinterpret_cast<int*>(ws + a.lay.counters),
-                                             reinterpret_cast<int*>(ws + a.lay.page_start));
+                                             p.B > kSmemSeqs ? reinterpret_cast<int*>(ws + a.lay.page_start) : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   switch (p.kv_dtype) {

@@ -50,6 +50,9 @@ constexpr int kMaxStages = 8;
 // seq_lens and a scan, ~1 us, where a planning kernel in front and a binary search through its result in global memory
 // cost ~6 us before the first page was requested.  Beyond it decode_plan_kernel scans once for all.
 constexpr int kSmemSeqs = 1024;
+// CTAs that share an SM when a CTA holds few heads: as many as make 8 consumer warps (6 CTAs of one, whose registers
+// would otherwise not fit).  The grid counts on all of them being resident at once, hence the launch bounds.
+__host__ __device__ constexpr int ctas_per_sm(int warps) { return warps >= 8 ? 1 : (warps >= 4 ? 2 : (warps >= 2 ? 4 : 6)); }
 
 enum KvKind { KV_F16 = 0, KV_BF16 = 1, KV_I8 = 2, KV_E4M3 = 3 };
 
@@ -84,12 +87,14 @@ struct KernelArgs {
   DecodeLayout lay;
   int HG;            // head groups = Hkv / HPC
   int group;         // Hq / Hkv
-  int rows;          // group * Nq (<= 8)
+  int rows;          // group * Nq
+  int hpc;           // kv heads per CTA
+  int row_groups;    // consumer warps per kv head (1 up to 16 rows)
   int stages;
   int upp;              // 16-token units per page = block_size / 16
   int stage_kv_bytes;   // bytes of one K (or V) stage tile = HPC * kBS * row_bytes
   int scale_bytes;      // bytes of one scale page = kBS * Hkv * 2 (0 when not quantized)
-  float q_prescale;     // folded into Q (8-bit pools) or applied to the scores (16-bit)
+  float q_prescale;     // folded into Q (8-bit pools) or applied to the scores (16-bit pools)
   float cap_log2;       // softcap * log2(e)
   float inv_cap;        // 1 / softcap
 };
@@ -159,11 +164,6 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
   return d;
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(addr));
-  return v;
-}
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -180,11 +180,6 @@ __device__ __forceinline__ uint32_t i8pair_to_h2(uint32_t biased, uint32_t sel) 
   __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&magic), __floats2half2_rn(1152.f, 1152.f));
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// the same without the subtraction: half2 of 1024 + (x + 128) = x + 1152.  Used for K, where the constant offset
-// becomes 1152 * sum(q) in each score and is taken out of the fp32 accumulator after the eight MMAs of a tile.
-__device__ __forceinline__ uint32_t i8pair_to_h2_biased(uint32_t biased, uint32_t sel) {
-  return prmt(biased, 0x64646464u, sel);
-}
 __device__ __forceinline__ uint32_t e4m3pair_to_h2(uint32_t two_bytes) {
   __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(two_bytes & 0xffffu), __NV_E4M3);
   __half2 h = r;
@@ -200,6 +195,14 @@ __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
 }
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+// D (16 x 8, int32) += A (16 x 32, int8) B (32 x 8, int8).  8.3 clk per instruction and scheduler, what the f16
+// m16n8k16 takes (8.4), for twice the depth.
+__device__ __forceinline__ void mma16832_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ float clamp_h(float x) { return fminf(fmaxf(x, -65504.f), 65504.f); }
 
@@ -263,15 +266,17 @@ __device__ __forceinline__ float combine_row(const float* lse, size_t lse_step, 
 // ---------------------------------------------------------------------------
 // CAP: soft cap on.  A template parameter so that the common launch without one carries no tanh code in its unrolled
 // inner loops (with it compiled in, config 4 -- which has no soft cap -- ran 4 % slower).
-template <int KV, int HPC, int kD, bool CAP>
-__global__ void __launch_bounds__((HPC + 1) * 32, 1)
+// RT: tiles of 8 query rows (of the group's heads x query tokens) per consumer warp.  RT = 1: up to 8 rows, one warp per
+// kv head, HPC heads per CTA.  RT = 2 (HPC = 0: a.hpc heads, known at run time): up to 16 rows per warp, which fills the
+// 16 rows of the MMA, and a.row_groups warps per head share a page when there are more.
+template <int KV, int HPC, int kD, bool CAP, int RT>
+__global__ void __launch_bounds__(((HPC > 0 ? HPC : 8) + 1) * 32, HPC > 0 ? ctas_per_sm(HPC) : 1)
 decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const KernelArgs a) {
   constexpr bool kQuant = (KV == KV_I8 || KV == KV_E4M3);
   static_assert(kD == 128 || (kD == 64 && !kQuant), "head_dim 64 is built for 16-bit pools only");
   constexpr int kKS = kD / 16;                         // k-steps of S = Q.K^T, m-tiles of O^T
   constexpr int kRowBytes = kQuant ? kD : 2 * kD;      // bytes of one (token, head) row
-  constexpr int kHalves = kRowBytes / 128;
   constexpr int kHeadBytes = kBS * kRowBytes;          // one head of one page in shared memory
   using MmaT = typename std::conditional<KV == KV_BF16, __nv_bfloat16, __half>::type;
 
@@ -294,6 +299,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int g = lane >> 2, t = lane & 3;
   const int hg = blockIdx.y;
   const int c = blockIdx.x;
+  const int hpc = HPC > 0 ? HPC : a.hpc;
+  const int n_cons = HPC > 0 ? HPC : a.hpc * a.row_groups;       // consumer warps; the next one is the producer
 
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
   int* err = reinterpret_cast<int*>(ws + a.lay.err);
@@ -310,7 +317,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     prefetch_tmap(&tmV);
     for (int i = 0; i < NS; ++i) {
       mbar_init(smem_u32(&bars[i]), 1);                 // full: producer arrive (+ tx bytes)
-      mbar_init(smem_u32(&bars[kMaxStages + i]), HPC);  // empty: one arrive per consumer warp
+      mbar_init(smem_u32(&bars[kMaxStages + i]), n_cons);  // empty: one arrive per consumer warp
     }
     *s_abort = 0;
     fence_barrier_init();
@@ -346,11 +353,11 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   if (c == 0) {
     for (int b = 0; b < p.B; ++b) {
       if (page_start[b + 1] != page_start[b]) continue;
-      for (int i = tid; i < HPC * a.group * p.Nq * kD; i += blockDim.x) {
+      for (int i = tid; i < hpc * a.group * p.Nq * kD; i += blockDim.x) {
         const int d = i % kD;
         const int r = i / kD;                       // (head in cta, group, qi)
         const int qi = r % p.Nq;
-        const int hq = (hg * HPC) * a.group + r / p.Nq;
+        const int hq = (hg * hpc) * a.group + r / p.Nq;
         const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
         const size_t o = orow * kD + d;
         if (p.packed_f32) {
@@ -390,7 +397,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
   const uint32_t tx_bytes = 2u * a.stage_kv_bytes + 2u * a.scale_bytes;
 
-  if (warp == HPC) {
+  if (warp == n_cons) {
     // ======================= producer warp =======================
     int stage = 0;
     uint32_t phase = 0;
@@ -428,8 +435,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             if (page >= 0) {
               mbar_arrive_expect_tx(full, tx_bytes);
               const int batch_coord = p.dense ? b : 0;
-              tma_load_5d(smem_u32(sK + static_cast<size_t>(stage) * a.stage_kv_bytes), &tmK, full, 0, page, 0, hg * HPC, batch_coord);
-              tma_load_5d(smem_u32(sV + static_cast<size_t>(stage) * a.stage_kv_bytes), &tmV, full, 0, page, 0, hg * HPC, batch_coord);
+              tma_load_5d(smem_u32(sK + static_cast<size_t>(stage) * a.stage_kv_bytes), &tmK, full, 0, page, 0, hg * hpc, batch_coord);
+              tma_load_5d(smem_u32(sV + static_cast<size_t>(stage) * a.stage_kv_bytes), &tmV, full, 0, page, 0, hg * hpc, batch_coord);
               if (kQuant) {
                 const size_t soff = static_cast<size_t>(page / kBS) * a.scale_bytes;
                 bulk_load(smem_u32(sKs + static_cast<size_t>(stage) * a.scale_bytes),
@@ -455,10 +462,18 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   }
 
   // ======================= consumer warps =======================
-  const int kvh = hg * HPC + warp;
-  const int qi_row = g / a.group;                // query token of fragment row g
-  const int hq_row = kvh * a.group + g % a.group;
-  const bool row_valid = g < rows;
+  const int wh = RT == 1 ? warp : warp / a.row_groups;          // kv head of this warp within the CTA
+  const int rbase = RT == 1 ? 0 : (warp % a.row_groups) * (8 * RT);
+  const int kvh = hg * hpc + wh;
+  // fragment row g of row tile rt is query row rbase + 8 rt + g = (query token, head of the group)
+  int row_of[RT], qi_row[RT], hq_row[RT];
+#pragma unroll
+  for (int rt = 0; rt < RT; ++rt) {
+    row_of[rt] = rbase + 8 * rt + g;
+    qi_row[rt] = row_of[rt] / a.group;
+    hq_row[rt] = kvh * a.group + row_of[rt] % a.group;
+  }
+  const int my_rows = min(8 * RT, rows - rbase);                // may be <= 0: the warp then only keeps step
   int stage = 0;
   uint32_t phase = 0;
   long long u = lo;
@@ -476,81 +491,108 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     const int c_last = cta_of_unit(static_cast<long long>(s1) - 1, G, U);
     const int n_parts = c_last - c_first + 1;
 
-    // ---- Q fragments (A operand rows 0..7; rows 8..15 are zero padding) ----
-    uint32_t qa[8][2];                 // kKS k-steps are used
-    float q_bias = 0.f;          // int8 pools: 1152 * sum of the row's query values (see i8pair_to_h2_biased)
-    {
-      const size_t qoff = ((static_cast<size_t>(b) * p.Hq + hq_row) * p.Nq + qi_row) * kD;
-      if constexpr (kQuant) {
-        // lane t owns d in [32t, 32t+32): k-step s uses d = 32t + 4s + {0,1 | 2,3}
-        float f[32];
-        if (row_valid) {
-          if (p.q_dtype == 0) {
-            const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.q) + qoff + 32 * t);
+    // ---- Q fragments (A operand) ----
+    // 16-bit and e4m3 pools: qa[s][0 | 1] = row tile 0 (k low, k high), [2 | 3] = row tile 1; kKS k-steps.
+    // int8 pools: the products run on the integer tensor cores, K as it is stored.  A row of Q is fixed point with 16
+    // bits below its largest value, q = qscale * (256 hi + lo), two signed bytes; 256 * hi.k + lo.k is exact in 32 bits
+    // (|.| <= 128 * 32639 * 128).  The step is max|q| / 32639, against a relative 2^-12 per value in f16; the widening
+    // of K to f16 (3 operations per two values) and half of the MMAs fall away.  One row tile: hi in rows 0..7, lo in
+    // rows 8..15 of one MMA; two row tiles: an MMA each.
+    constexpr bool kI8 = KV == KV_I8;
+    constexpr int kQA = kI8 ? 4 * RT : kKS;
+    constexpr int kQR = kI8 ? 4 : 2 * RT;
+    uint32_t qa[kQA][kQR];
+    float qscale[RT];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint4 w = src[i];
-              const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    for (int rt = 0; rt < RT; ++rt) {
+      const bool row_valid = row_of[rt] < rows;
+      const size_t qoff = row_valid ? ((static_cast<size_t>(b) * p.Hq + hq_row[rt]) * p.Nq + qi_row[rt]) * kD : 0;
+      qscale[rt] = 1.f;
+      if constexpr (kQuant) {
+        // lane t owns d in [32t, 32t+32)
+        float f[32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 w = row_valid ? reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q) + qoff + 32 * t)[i]
+                                    : make_uint4(0u, 0u, 0u, 0u);
+          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 v2 = p.q_dtype == 0 ? __half22float2(*reinterpret_cast<const __half2*>(&ww[e]))
+                                             : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww[e]));
+            f[i * 8 + e * 2] = clamp_h(v2.x * a.q_prescale);
+            f[i * 8 + e * 2 + 1] = clamp_h(v2.y * a.q_prescale);
+          }
+        }
+        if constexpr (kI8) {
+          float mx = 0.f;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fabsf(f[i]));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          // below 2^-100 the reciprocal would leave the float range; such a row scores zero, as its f16 values did
+          const float inv = mx > 7.9e-31f ? 32639.f / mx : 0.f;
+          qscale[rt] = mx * (1.f / 32639.f);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            uint32_t hi4[2], lo4[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              hi4[h] = lo4[h] = 0u;
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                float2 v2 = __half22float2(*reinterpret_cast<const __half2*>(&ww[e]));
-                f[i * 8 + e * 2] = v2.x; f[i * 8 + e * 2 + 1] = v2.y;
+                const int qi = __float2int_rn(f[8 * s + 4 * h + e] * inv);
+                const int hb = (qi + 128) >> 8, lb = qi - (hb << 8);
+                hi4[h] |= (static_cast<uint32_t>(hb) & 0xffu) << (8 * e);
+                lo4[h] |= (static_cast<uint32_t>(lb) & 0xffu) << (8 * e);
               }
             }
-          } else {
-            const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + qoff + 32 * t);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint4 w = src[i];
-              const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float2 v2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww[e]));
-                f[i * 8 + e * 2] = v2.x; f[i * 8 + e * 2 + 1] = v2.y;
-              }
+            if constexpr (RT == 1) {
+              qa[s][0] = hi4[0]; qa[s][1] = lo4[0]; qa[s][2] = hi4[1]; qa[s][3] = lo4[1];
+            } else {
+              qa[s][rt] = hi4[0]; qa[s][2 + rt] = hi4[1];
+              qa[4 + s][rt] = lo4[0]; qa[4 + s][2 + rt] = lo4[1];
             }
           }
         } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) f[i] = 0.f;
-        }
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          qa[s][0] = pack_h2(clamp_h(f[4 * s] * a.q_prescale), clamp_h(f[4 * s + 1] * a.q_prescale));
-          qa[s][1] = pack_h2(clamp_h(f[4 * s + 2] * a.q_prescale), clamp_h(f[4 * s + 3] * a.q_prescale));
-        }
-        if (KV == KV_I8) {
-          // 1152 * (sum over the head dim of this row's f16 query values): the part of every score that comes from
-          // the +1152 offset left inside the widened K values
-          float qs = 0.f;
+          // k-step s uses d = 32t + 4s + {0,1 | 2,3}
 #pragma unroll
           for (int s = 0; s < 8; ++s) {
-            const float2 u = __half22float2(*reinterpret_cast<const __half2*>(&qa[s][0]));
-            const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&qa[s][1]));
-            qs += (u.x + u.y) + (w.x + w.y);
+            qa[s][2 * rt] = pack_h2(f[4 * s], f[4 * s + 1]);
+            qa[s][2 * rt + 1] = pack_h2(f[4 * s + 2], f[4 * s + 3]);
           }
-          qs += __shfl_xor_sync(0xffffffffu, qs, 1);
-          qs += __shfl_xor_sync(0xffffffffu, qs, 2);
-          q_bias = 1152.f * qs;
         }
       } else {
         // natural order: a0 = Q[g][16s + 2t, +1], a2 = Q[g][16s + 8 + 2t, +1]
         const uint32_t* src = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.q) + qoff);
 #pragma unroll
         for (int s = 0; s < kKS; ++s) {
-          qa[s][0] = row_valid ? src[8 * s + t] : 0u;
-          qa[s][1] = row_valid ? src[8 * s + 4 + t] : 0u;
+          qa[s][2 * rt] = row_valid ? src[8 * s + t] : 0u;
+          qa[s][2 * rt + 1] = row_valid ? src[8 * s + 4 + t] : 0u;
         }
       }
     }
 
-    float oacc[8][4];
+    float oacc[RT][kKS][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f; }
-    float m_run = -INFINITY, l_run = 0.f;
-    float vnorm = 1.f, vunnorm = 1.f;             // power-of-two normalisation of v_scale inside P
+    for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+      for (int i = 0; i < kKS; ++i) { oacc[rt][i][0] = oacc[rt][i][1] = oacc[rt][i][2] = oacc[rt][i][3] = 0.f; }
+    float m_run[RT], l_run[RT];
+    int causal_lim[RT];                           // last visible token of the row
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt) {
+      m_run[rt] = -INFINITY;
+      l_run[rt] = 0.f;
+      causal_lim[rt] = p.causal ? (qi_row[rt] + len - p.Nq) : 0x7fffffff;
+    }
+    // Tokens before this one are visible to every row and inside the sequence: steps that end before it need no masks.
+    const int open_end = p.causal ? min(len, len - p.Nq + 1) : len;
+    // Quantised pools: P goes into its 16-bit operand multiplied by v_scale.  Every exponent is shifted by vexp, minus
+    // the exponent of the part's first v scale, so that the product stays inside f16's normal range; the row sum
+    // carries the same power of two and it cancels.
+    float vexp = 0.f;
     bool first_page = true;
-    const int causal_lim = p.causal ? (qi_row + len - p.Nq) : 0x7fffffff;   // last visible token of row g
 
     // Two pages per iteration: their loads, conversions and MMAs are independent, which gives the
     // scheduler twice the instruction-level parallelism, and one online-softmax step covers 32 tokens.
@@ -571,130 +613,186 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
         if (!okw) { ok = false; break; }
       }
-      uint32_t kbase[2], vbase[2], ksb[2], vsb[2];
+      uint32_t kbase[2], vbase[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         pg[q] = q < np ? s_page[stg[q]] : -2;       // -1: hole in the table, -2: no second page
-        kbase[q] = smem_u32(sK + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + warp * kHeadBytes;
-        vbase[q] = smem_u32(sV + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + warp * kHeadBytes;
-        ksb[q] = smem_u32(sKs + static_cast<size_t>(stg[q]) * a.scale_bytes) + kvh * 2;
-        vsb[q] = smem_u32(sVs + static_cast<size_t>(stg[q]) * a.scale_bytes) + kvh * 2;
+        kbase[q] = smem_u32(sK + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + wh * kHeadBytes;
+        vbase[q] = smem_u32(sV + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + wh * kHeadBytes;
       }
-      const int scale_stride = p.Hkv * 2;          // bytes between tokens in a scale page
+      // warp-uniform: two pages of visible tokens -- everything below that deals with edges is skipped
+      const bool full = (pg[0] | pg[1]) >= 0 && (j + 2) * kBS <= open_end;
 
-      // ---- S = Q K^T : rows = query rows (8 real), cols = 16 tokens (two n-tiles) per page ----
-      float sacc[2][2][4];
+      // ---- scales: lane l fetches those of token l & 15 of page l >> 4; shuffles hand them round ----
+      float ksl = 1.f, vsl = 1.f;
+      if constexpr (kQuant) {
+        const int q = lane >> 4;
+        if (full || (q == 0 ? pg[0] : pg[1]) >= 0) {
+          const uint32_t off = static_cast<uint32_t>(q == 0 ? stg[0] : stg[1]) * a.scale_bytes +
+                               static_cast<uint32_t>(((lane & 15) * p.Hkv + kvh) * 2);
+          ksl = lds_half(smem_u32(sKs) + off);
+          vsl = lds_half(smem_u32(sVs) + off);
+        }
+        if (first_page) {
+          const float v0 = __shfl_sync(0xffffffffu, vsl, 0);
+          const uint32_t bits = __float_as_uint(v0) & 0x7f800000u;
+          vexp = (bits == 0u || bits == 0x7f800000u) ? 0.f : 127.f - static_cast<float>(bits >> 23);
+          first_page = false;
+        }
+        // whatever the scale of a slot beyond the sequence holds (it may be a NaN pattern)
+        if (!full && (j + q) * kBS + (lane & 15) >= len) vsl = 0.f;
+      }
+
+      // ---- S = Q K^T : per page this lane gets tokens {2t, 2t+1, 8+2t, 9+2t} of its rows ----
+      float sc[RT][2][4];
+      if constexpr (kI8) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) { sacc[q][i][0] = sacc[q][i][1] = sacc[q][i][2] = sacc[q][i][3] = 0.f; }
+          for (int jn = 0; jn < 2; ++jn) {
+            int acc[RT][4];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (pg[q] >= 0) {
-          if constexpr (kQuant) {
-#pragma unroll
-            for (int jn = 0; jn < 2; ++jn) {
-              const int tok = 8 * jn + g;                     // tok & 7 == g
-              const uint32_t rowa = kbase[q] + tok * 128;
+            for (int rt = 0; rt < RT; ++rt) { acc[rt][0] = acc[rt][1] = acc[rt][2] = acc[rt][3] = 0; }
+            if (pg[q] >= 0) {
+              const uint32_t rowa = kbase[q] + (8 * jn + g) * 128;           // token 8 jn + g
               const uint4 w0 = lds128(rowa + (((2 * t) ^ g) << 4));
               const uint4 w1 = lds128(rowa + (((2 * t + 1) ^ g) << 4));
               const uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-              for (int s = 0; s < 8; ++s) {
-                uint32_t b0, b1;
-                if (KV == KV_I8) {
-                  const uint32_t x = words[s] ^ 0x80808080u;
-                  b0 = i8pair_to_h2_biased(x, 0x4140u);
-                  b1 = i8pair_to_h2_biased(x, 0x4342u);
-                } else {
-                  b0 = e4m3pair_to_h2(words[s]);
-                  b1 = e4m3pair_to_h2(words[s] >> 16);
-                }
-                const uint32_t afrag[4] = {qa[s][0], 0u, qa[s][1], 0u};
-                mma16816<MmaT>(sacc[q][jn], afrag, b0, b1);
+              for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int h = 0; h < RT; ++h)                                  // RT == 2: acc[0] = hi, acc[1] = lo
+                  mma16832_s8(acc[h], qa[4 * h + s], words[2 * s], words[2 * s + 1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if constexpr (RT == 1) {
+                sc[0][q][2 * jn + e] = __int2float_rn((acc[0][e] << 8) + acc[0][2 + e]) * qscale[0];
+              } else {
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt)
+                  sc[rt][q][2 * jn + e] = __int2float_rn((acc[0][2 * rt + e] << 8) + acc[1][2 * rt + e]) * qscale[rt];
               }
             }
-          } else {
+          }
+      } else {
+        float sacc[2][2][4];
 #pragma unroll
-            for (int s = 0; s < kKS; ++s) {
-              uint32_t bfr[4];
-              const int tok = (lane & 7) + ((lane >> 4) << 3);
-              const int dcol = 16 * s + (((lane >> 3) & 1) << 3);
-              const uint32_t addr = kbase[q] + (dcol >> 6) * (kBS * 128) + tok * 128 + ((((dcol & 63) >> 3) ^ (tok & 7)) << 4);
-              ldmatrix_x4(bfr, addr);
-              const uint32_t afrag[4] = {qa[s][0], 0u, qa[s][1], 0u};
-              mma16816<MmaT>(sacc[q][0], afrag, bfr[0], bfr[1]);
-              mma16816<MmaT>(sacc[q][1], afrag, bfr[2], bfr[3]);
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) { sacc[q][i][0] = sacc[q][i][1] = sacc[q][i][2] = sacc[q][i][3] = 0.f; }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (pg[q] >= 0) {
+            if constexpr (kQuant) {
+#pragma unroll
+              for (int jn = 0; jn < 2; ++jn) {
+                const uint32_t rowa = kbase[q] + (8 * jn + g) * 128;
+                const uint4 w0 = lds128(rowa + (((2 * t) ^ g) << 4));
+                const uint4 w1 = lds128(rowa + (((2 * t + 1) ^ g) << 4));
+                const uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                  const uint32_t afrag[4] = {qa[s][0], RT == 2 ? qa[s][2 * (RT - 1)] : 0u, qa[s][1], RT == 2 ? qa[s][2 * (RT - 1) + 1] : 0u};
+                  mma16816<MmaT>(sacc[q][jn], afrag, e4m3pair_to_h2(words[s]), e4m3pair_to_h2(words[s] >> 16));
+                }
+              }
+            } else {
+#pragma unroll
+              for (int s = 0; s < kKS; ++s) {
+                uint32_t bfr[4];
+                const int tok = (lane & 7) + ((lane >> 4) << 3);
+                const int dcol = 16 * s + (((lane >> 3) & 1) << 3);
+                const uint32_t addr = kbase[q] + (dcol >> 6) * (kBS * 128) + tok * 128 + ((((dcol & 63) >> 3) ^ (tok & 7)) << 4);
+                ldmatrix_x4(bfr, addr);
+                const uint32_t afrag[4] = {qa[s][0], RT == 2 ? qa[s][2 * (RT - 1)] : 0u, qa[s][1], RT == 2 ? qa[s][2 * (RT - 1) + 1] : 0u};
+                mma16816<MmaT>(sacc[q][0], afrag, bfr[0], bfr[1]);
+                mma16816<MmaT>(sacc[q][1], afrag, bfr[2], bfr[3]);
+              }
             }
           }
         }
-      }
-
-      // ---- scale / softcap / masks: per page this lane holds tokens {2t, 2t+1, 8+2t, 9+2t} of row g ----
-      float sc[2][4], vsc[2][4];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int tok0 = (j + q) * kBS;
+        for (int rt = 0; rt < RT; ++rt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int tok = ((e >> 1) << 3) + 2 * t + (e & 1);
-          float s = sacc[q][e >> 1][e & 1];
-          vsc[q][e] = 1.f;
-          if (kQuant) {
-            float ksv = 1.f;
-            if (pg[q] >= 0) {
-              ksv = lds_half(ksb[q] + tok * scale_stride);
-              vsc[q][e] = lds_half(vsb[q] + tok * scale_stride);
-              if (KV == KV_I8) s -= q_bias;                 // the K values went into the MMA as x + 1152
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float s = sacc[q][e >> 1][2 * rt + (e & 1)];
+              sc[rt][q][e] = kQuant ? s : s * a.q_prescale;
             }
-            s *= ksv;
-          } else {
-            s *= a.q_prescale;
-          }
-          if constexpr (CAP) s = a.cap_log2 * cap_tanh(s * a.inv_cap, a.inv_cap * kPreciseTanhMinCap <= 1.f);
-          const int tg = tok0 + tok;
-          sc[q][e] = (pg[q] != -2 && tg < len && tg <= causal_lim) ? s : -INFINITY;
-          if (tg >= len) vsc[q][e] = 0.f;               // whatever the slot's scale holds (it may be a NaN pattern)
-        }
-      }
-      if (kQuant && first_page) {
-        // power of two near the first token's v scale keeps p * v_scale inside f16's normal range
-        float v0 = (pg[0] >= 0) ? lds_half(vsb[0]) : 1.f;
-        v0 = __shfl_sync(0xffffffffu, v0, 0);
-        uint32_t bits = __float_as_uint(v0) & 0x7f800000u;
-        if (bits == 0u || bits == 0x7f800000u) bits = 0x3f800000u;
-        vunnorm = __uint_as_float(bits);
-        vnorm = 1.f / vunnorm;
-        first_page = false;
       }
 
-      // ---- online softmax over the (up to) 32 tokens ----
-      float mx = fmaxf(fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[0][2], sc[0][3])),
-                       fmaxf(fmaxf(sc[1][0], sc[1][1]), fmaxf(sc[1][2], sc[1][3])));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const float m_new = fmaxf(m_run, mx);
-      const float msub = (m_new == -INFINITY) ? 0.f : m_new;
-      const bool grew = m_new > m_run;
-      if (__any_sync(0xffffffffu, grew)) {
-        const float corr = fast_exp2(m_run - msub);       // 1 when unchanged, 0 from -inf
-        l_run *= corr;
-        const float c0 = __shfl_sync(0xffffffffu, corr, (2 * t) * 4);
-        const float c1 = __shfl_sync(0xffffffffu, corr, (2 * t + 1) * 4);
-#pragma unroll
-        for (int i = 0; i < kKS; ++i) {
-          oacc[i][0] *= c0; oacc[i][1] *= c1; oacc[i][2] *= c0; oacc[i][3] *= c1;
-        }
-        m_run = m_new;
-      }
-      float pr[2][4];
+      // ---- scale / softcap / masks ----
+      float vsc[2][4];
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          pr[q][e] = fast_exp2(sc[q][e] - msub);
-          l_run += pr[q][e];
+          const int tok = ((e >> 1) << 3) + 2 * t + (e & 1);
+          if constexpr (kQuant) {
+            const float ksv = __shfl_sync(0xffffffffu, ksl, 16 * q + tok);
+            vsc[q][e] = __shfl_sync(0xffffffffu, vsl, 16 * q + tok);
+#pragma unroll
+            for (int rt = 0; rt < RT; ++rt) sc[rt][q][e] *= ksv;
+          }
+          if constexpr (CAP) {
+#pragma unroll
+            for (int rt = 0; rt < RT; ++rt)
+              sc[rt][q][e] = a.cap_log2 * cap_tanh(sc[rt][q][e] * a.inv_cap, a.inv_cap * kPreciseTanhMinCap <= 1.f);
+          }
+          if (!full) {
+            const int tg = (j + q) * kBS + tok;
+#pragma unroll
+            for (int rt = 0; rt < RT; ++rt)
+              if (!(pg[q] != -2 && tg < len && tg <= causal_lim[rt])) sc[rt][q][e] = -INFINITY;
+          }
         }
+
+      // ---- online softmax over the (up to) 32 tokens ----
+      float m_new[RT], msub[RT];
+      bool grew = false;
+#pragma unroll
+      for (int rt = 0; rt < RT; ++rt) {
+        float mx = fmaxf(fmaxf(fmaxf(sc[rt][0][0], sc[rt][0][1]), fmaxf(sc[rt][0][2], sc[rt][0][3])),
+                         fmaxf(fmaxf(sc[rt][1][0], sc[rt][1][1]), fmaxf(sc[rt][1][2], sc[rt][1][3])));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        m_new[rt] = fmaxf(m_run[rt], mx);
+        msub[rt] = (m_new[rt] == -INFINITY) ? 0.f : m_new[rt];
+        grew = grew || m_new[rt] > m_run[rt];
+      }
+      if (__any_sync(0xffffffffu, grew)) {
+#pragma unroll
+        for (int rt = 0; rt < RT; ++rt) {
+          const float corr = fast_exp2(m_run[rt] - msub[rt]);       // 1 when unchanged, 0 from -inf
+          l_run[rt] *= corr;
+          const float c0 = __shfl_sync(0xffffffffu, corr, (2 * t) * 4);
+          const float c1 = __shfl_sync(0xffffffffu, corr, (2 * t + 1) * 4);
+#pragma unroll
+          for (int i = 0; i < kKS; ++i) {
+            oacc[rt][i][0] *= c0; oacc[rt][i][1] *= c1; oacc[rt][i][2] *= c0; oacc[rt][i][3] *= c1;
+          }
+          m_run[rt] = m_new[rt];
+        }
+      }
+      uint32_t pb[RT][2][2];
+#pragma unroll
+      for (int rt = 0; rt < RT; ++rt) {
+        const float sub = kQuant ? msub[rt] - vexp : msub[rt];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float pr[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            pr[e] = fast_exp2(sc[rt][q][e] - sub);
+            l_run[rt] += pr[e];
+            if (kQuant) pr[e] *= vsc[q][e];
+          }
+          pb[rt][q][0] = KV == KV_BF16 ? pack_bf2(pr[0], pr[1]) : pack_h2(pr[0], pr[1]);
+          pb[rt][q][1] = KV == KV_BF16 ? pack_bf2(pr[2], pr[3]) : pack_h2(pr[2], pr[3]);
+        }
+      }
 
       // ---- O^T += V^T P^T : rows = 16 head-dim values per m-tile, cols = query rows ----
 #pragma unroll
@@ -704,43 +802,31 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
           // zero, but 0 * NaN (or 0 * inf) would still poison the row, so their V values are cleared as they are
           // loaded.  amask[h]: tokens (2t, 2t+1) for h = 0, (2t+8, 2t+9) for h = 1, one 16-bit lane per token.
           const int tail_from = len - (j + q) * kBS;      // first token of this page that is beyond the sequence
-          const bool tail = tail_from < kBS;              // warp-uniform
+          const bool tail = !full && tail_from < kBS;     // warp-uniform
           uint32_t amask[2] = {0xffffffffu, 0xffffffffu};
           if (tail) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
               amask[h] = (2 * t + 8 * h < tail_from ? 0x0000ffffu : 0u) | (2 * t + 8 * h + 1 < tail_from ? 0xffff0000u : 0u);
           }
-          uint32_t pb0, pb1;
-          if (kQuant) {
-            pb0 = pack_h2(pr[q][0] * vsc[q][0] * vnorm, pr[q][1] * vsc[q][1] * vnorm);
-            pb1 = pack_h2(pr[q][2] * vsc[q][2] * vnorm, pr[q][3] * vsc[q][3] * vnorm);
-          } else if (KV == KV_BF16) {
-            pb0 = pack_bf2(pr[q][0], pr[q][1]);
-            pb1 = pack_bf2(pr[q][2], pr[q][3]);
-          } else {
-            pb0 = pack_h2(pr[q][0], pr[q][1]);
-            pb1 = pack_h2(pr[q][2], pr[q][3]);
-          }
           if constexpr (kQuant) {
-            // lane (g,t) reads word w = g + 8*jj (4 head-dim bytes) of token rows 2t, 2t+1, 2t+8, 2t+9
-            const uint32_t rA = vbase[q] + (2 * t) * 128, rB = rA + 128, rC = rA + 8 * 128, rD = rC + 128;
-            const int xa = (2 * t) & 7, xb = (2 * t + 1) & 7;
+            // lane (g,t) reads the 16 head-dim bytes [16g, 16g + 16) of token rows 2t, 2t+1, 2t+8, 2t+9; m-tile i has
+            // dims 16g + 2i (fragment row g) and 16g + 2i + 1 (row g + 8)
+            const uint32_t xa = ((g ^ ((2 * t) & 7)) << 4), xb = ((g ^ ((2 * t + 1) & 7)) << 4);
+            const uint32_t rA = vbase[q] + (2 * t) * 128;
+            const uint4 A4 = lds128(rA + xa), B4 = lds128(rA + 128 + xb), C4 = lds128(rA + 8 * 128 + xa), D4 = lds128(rA + 9 * 128 + xb);
+            const uint32_t Aw[4] = {A4.x, A4.y, A4.z, A4.w}, Bw[4] = {B4.x, B4.y, B4.z, B4.w};
+            const uint32_t Cw[4] = {C4.x, C4.y, C4.z, C4.w}, Dw[4] = {D4.x, D4.y, D4.z, D4.w};
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
-              const int w = g + 8 * jj;
-              const int ch = w >> 2, wi = (w & 3) << 2;
-              uint32_t A = lds32(rA + ((ch ^ xa) << 4) + wi);
-              uint32_t Bw = lds32(rB + ((ch ^ xb) << 4) + wi);
-              uint32_t Cw = lds32(rC + ((ch ^ xa) << 4) + wi);
-              uint32_t Dw = lds32(rD + ((ch ^ xb) << 4) + wi);
-              if (KV == KV_I8) { A ^= 0x80808080u; Bw ^= 0x80808080u; Cw ^= 0x80808080u; Dw ^= 0x80808080u; }
-              const uint32_t ab[2] = {prmt(A, Bw, 0x5140u), prmt(A, Bw, 0x7362u)};   // [A0 B0 A1 B1], [A2 B2 A3 B3]
-              const uint32_t cd[2] = {prmt(Cw, Dw, 0x5140u), prmt(Cw, Dw, 0x7362u)};
+              const uint32_t bias = kI8 ? 0x80808080u : 0u;
+              const uint32_t A = Aw[jj] ^ bias, B = Bw[jj] ^ bias, Cc = Cw[jj] ^ bias, D = Dw[jj] ^ bias;
+              const uint32_t ab[2] = {prmt(A, B, 0x5140u), prmt(A, B, 0x7362u)};   // [A0 B0 A1 B1], [A2 B2 A3 B3]
+              const uint32_t cd[2] = {prmt(Cc, D, 0x5140u), prmt(Cc, D, 0x7362u)};
 #pragma unroll
               for (int kp = 0; kp < 2; ++kp) {
                 uint32_t af[4];
-                if (KV == KV_I8) {
+                if (kI8) {
                   af[0] = i8pair_to_h2(ab[kp], 0x4140u);   // head-dim byte 2kp   , tokens 2t, 2t+1
                   af[1] = i8pair_to_h2(ab[kp], 0x4342u);   // head-dim byte 2kp+1 , tokens 2t, 2t+1
                   af[2] = i8pair_to_h2(cd[kp], 0x4140u);   // tokens 2t+8, 2t+9
@@ -752,7 +838,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                   af[3] = e4m3pair_to_h2(cd[kp] >> 16);
                   if (tail) { af[0] &= amask[0]; af[1] &= amask[0]; af[2] &= amask[1]; af[3] &= amask[1]; }
                 }
-                mma16816<MmaT>(oacc[jj * 2 + kp], af, pb0, pb1);
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt) mma16816<MmaT>(oacc[rt][jj * 2 + kp], af, pb[rt][q][0], pb[rt][q][1]);
               }
             }
           } else {
@@ -765,7 +852,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
               // after .trans: a0 = (d 0-7, tok 0-7), a1 = (d 8-15, tok 0-7), a2 = (d 0-7, tok 8-15), a3 = (d 8-15, tok 8-15)
               ldmatrix_x4_trans(af, addr);
               if (tail) { af[0] &= amask[0]; af[1] &= amask[0]; af[2] &= amask[1]; af[3] &= amask[1]; }
-              mma16816<MmaT>(oacc[mt], af, pb0, pb1);
+#pragma unroll
+              for (int rt = 0; rt < RT; ++rt) mma16816<MmaT>(oacc[rt][mt], af, pb[rt][q][0], pb[rt][q][1]);
             }
           }
         }
@@ -783,49 +871,59 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     if (!ok) break;
 
     // ---- end of this CTA's part of sequence b ----
-    float l_row = l_run;
-    l_row += __shfl_xor_sync(0xffffffffu, l_row, 1);
-    l_row += __shfl_xor_sync(0xffffffffu, l_row, 2);
-    const float lse_row = l_row > 0.f ? m_run + log2f(l_row) : -INFINITY;
-    const float inv_row = l_row > 0.f ? vunnorm / l_row : 0.f;
-    // accumulator columns are query rows 2t and 2t+1
-    const float inv0 = __shfl_sync(0xffffffffu, inv_row, (2 * t) * 4);
-    const float inv1 = __shfl_sync(0xffffffffu, inv_row, (2 * t + 1) * 4);
-    const int r0 = 2 * t, r1 = 2 * t + 1;
     const bool direct = (n_parts == 1);
-    const int slot = c + b;
-
+    const size_t slot_row0 = static_cast<size_t>(c + b) * HqNq;
 #pragma unroll
-    for (int i = 0; i < kKS; ++i) {
+    for (int rt = 0; rt < RT; ++rt) {
+      float l_row = l_run[rt];
+      l_row += __shfl_xor_sync(0xffffffffu, l_row, 1);
+      l_row += __shfl_xor_sync(0xffffffffu, l_row, 2);
+      const float lse_row = l_row > 0.f ? m_run[rt] + log2f(l_row) - vexp : -INFINITY;
+      const float inv_row = l_row > 0.f ? 1.f / l_row : 0.f;
+      // accumulator columns are query rows 2t and 2t+1 of the tile
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        // head-dim index of accumulator register e of m-tile i
-        int d;
-        if (kQuant) d = 32 * (i >> 1) + 4 * g + 2 * (i & 1) + (e >> 1);
-        else d = 16 * i + g + ((e >> 1) << 3);
-        const int r = (e & 1) ? r1 : r0;
+      for (int h = 0; h < 2; ++h) {
+        const float inv = __shfl_sync(0xffffffffu, inv_row, (2 * t + h) * 4);
+        const int r = rbase + 8 * rt + 2 * t + h;
         if (r >= rows) continue;
-        const float val = oacc[i][e] * ((e & 1) ? inv1 : inv0);
-        const int hq = kvh * a.group + r % a.group;
-        const int qi = r / a.group;
-        if (direct) {
-          const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
-          const size_t o = orow * kD + d;
-          if (p.packed_f32) reinterpret_cast<float*>(p.out)[orow * (kD + 4) + d] = val;
-          else if (p.q_dtype == 0) reinterpret_cast<__half*>(p.out)[o] = __float2half_rn(val);
-          else reinterpret_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(val);
+        const int hq = kvh * a.group + r % a.group, qi = r / a.group;
+        const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
+        float* f32_row = direct ? (p.packed_f32 ? reinterpret_cast<float*>(p.out) + orow * (kD + 4) : nullptr)
+                                : part_o + (slot_row0 + static_cast<size_t>(hq) * p.Nq + qi) * kD;
+        uint16_t* h_row = reinterpret_cast<uint16_t*>(p.out) + orow * kD;
+        auto pack = [&](float x, float y) -> uint32_t { return p.q_dtype == 0 ? pack_h2(x, y) : pack_bf2(x, y); };
+        if constexpr (kQuant) {
+          // 16 consecutive head-dim values: tile i holds 16g + 2i (register h) and 16g + 2i + 1 (register 2 + h)
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            const float v[8] = {oacc[rt][i][h] * inv,     oacc[rt][i][2 + h] * inv,     oacc[rt][i + 1][h] * inv, oacc[rt][i + 1][2 + h] * inv,
+                                oacc[rt][i + 2][h] * inv, oacc[rt][i + 2][2 + h] * inv, oacc[rt][i + 3][h] * inv, oacc[rt][i + 3][2 + h] * inv};
+            if (f32_row != nullptr) {
+              float4* dst = reinterpret_cast<float4*>(f32_row + 16 * g + 2 * i);
+              dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+              dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+            } else {
+              *reinterpret_cast<uint4*>(h_row + 16 * g + 2 * i) = make_uint4(pack(v[0], v[1]), pack(v[2], v[3]), pack(v[4], v[5]), pack(v[6], v[7]));
+            }
+          }
         } else {
-          part_o[(static_cast<size_t>(slot) * HqNq + hq * p.Nq + qi) * kD + d] = val;
+#pragma unroll
+          for (int i = 0; i < kKS; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int d = 16 * i + g + 8 * e;
+              const float val = oacc[rt][i][2 * e + h] * inv;
+              if (f32_row != nullptr) f32_row[d] = val;
+              else if (p.q_dtype == 0) reinterpret_cast<__half*>(h_row)[d] = __float2half_rn(val);
+              else reinterpret_cast<__nv_bfloat16*>(h_row)[d] = __float2bfloat16_rn(val);
+            }
         }
       }
-    }
-    if (t == 0 && row_valid) {
-      if (direct) {
-        const size_t orow = (static_cast<size_t>(b) * p.Hq + hq_row) * p.Nq + qi_row;
-        if (p.packed_f32) reinterpret_cast<float*>(p.out)[orow * (kD + 4) + kD] = lse_row;
+      if (t == 0 && row_of[rt] < rows) {
+        const size_t orow = (static_cast<size_t>(b) * p.Hq + hq_row[rt]) * p.Nq + qi_row[rt];
+        if (!direct) part_lse[slot_row0 + static_cast<size_t>(hq_row[rt]) * p.Nq + qi_row[rt]] = lse_row;
+        else if (p.packed_f32) reinterpret_cast<float*>(p.out)[orow * (kD + 4) + kD] = lse_row;
         else if (p.lse != nullptr) p.lse[orow] = lse_row;
-      } else {
-        part_lse[static_cast<size_t>(slot) * HqNq + hq_row * p.Nq + qi_row] = lse_row;
       }
     }
 
@@ -841,7 +939,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       const int gslot = slot0 + grp * gsz;                            // the group's first slot
       const int gn = min(gsz, n_parts - grp * gsz);
       auto merge = [&](int first, int step, int n, bool final_out) {
-        for (int r = 0; r < rows; ++r) {
+        for (int r = rbase; r < rbase + my_rows; ++r) {
           const int hq = kvh * a.group + r % a.group;
           const int qi = r / a.group;
           const size_t rowi = static_cast<size_t>(hq) * p.Nq + qi;
@@ -876,9 +974,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       // true in every consumer thread of the CTA that brings `counter` to n
       auto arrive_last = [&](int* counter, int n, int* flag) -> bool {
         __threadfence();
-        named_bar_sync(1, HPC * 32);
+        named_bar_sync(1, n_cons * 32);
         if (tid == 0) *flag = atomicAdd(counter, 1) == n - 1 ? 1 : 0;
-        named_bar_sync(1, HPC * 32);
+        named_bar_sync(1, n_cons * 32);
         const bool last = *flag != 0;
         if (last) __threadfence();
         return last;
@@ -889,7 +987,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         if (n_grp > 1 && arrive_last(&counters[static_cast<size_t>(b) * a.HG + hg], n_grp, s_last + 1))
           merge(slot0, gsz, n_grp, true);
       }
-      named_bar_sync(1, HPC * 32);   // the flags are reused by the next sequence
+      named_bar_sync(1, n_cons * 32);   // the flags are reused by the next sequence
     }
 
     u = static_cast<long long>(s0) + j_hi;
@@ -948,27 +1046,25 @@ int device_sm_count() {
   return cached[dev];
 }
 
-int pick_hpc(int Hkv) {
-  if (Hkv % 8 == 0) return 8;
-  if (Hkv % 4 == 0) return 4;
-  if (Hkv % 2 == 0) return 2;
-  return 1;
+// how a launch is cut: heads per CTA, warps per head, CTAs along the units
+struct Shape {
+  int hpc, row_groups, gx;
+};
+Shape pick_shape(int Hkv, int rows, int num_splits) {
+  Shape s;
+  s.row_groups = rows > 16 ? 2 : 1;
+  s.hpc = 8 / s.row_groups;
+  while (Hkv % s.hpc != 0) s.hpc >>= 1;
+  const int hg = Hkv / s.hpc;
+  const int target = device_sm_count() * ctas_per_sm(s.hpc * s.row_groups);     // CTAs in flight over the whole grid
+  s.gx = (target + hg - 1) / hg;
+  if (num_splits > 0 && s.gx > num_splits) s.gx = num_splits;
+  return s;
 }
 
-int pick_grid_x(int Hkv, int num_splits) {
-  const int hpc = pick_hpc(Hkv);
-  const int hg = Hkv / hpc;
-  int target = device_sm_count() * (8 / hpc);     // CTAs in flight over the whole grid
-  int gx = (target + hg - 1) / hg;
-  if (gx < 1) gx = 1;
-  if (num_splits > 0 && gx > num_splits) gx = num_splits;
-  return gx;
-}
-
-template <int KV, int HPC, int D>
+template <int KV, int HPC, int D, int RT>
 cudaError_t launch_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const KernelArgs& a, int gx, size_t smem,
                      cudaStream_t stream) {
-  dim3 grid(gx, a.HG);
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
@@ -976,25 +1072,25 @@ cudaError_t launch_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const Kerne
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((HPC + 1) * 32);
+    cfg.gridDim = dim3(gx, a.HG);
+    cfg.blockDim = dim3((a.hpc * a.row_groups + 1) * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, tmK, tmV, a);
   };
-  return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true>) : go(decode_paged_kernel<KV, HPC, D, false>);
+  return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true, RT>) : go(decode_paged_kernel<KV, HPC, D, false, RT>);
 }
 
 template <int KV, int D>
-cudaError_t launch_kv(int hpc, const CUtensorMap& tmK, const CUtensorMap& tmV, const KernelArgs& a, int gx,
-                      size_t smem, cudaStream_t stream) {
-  switch (hpc) {
-    case 8: return launch_t<KV, 8, D>(tmK, tmV, a, gx, smem, stream);
-    case 4: return launch_t<KV, 4, D>(tmK, tmV, a, gx, smem, stream);
-    case 2: return launch_t<KV, 2, D>(tmK, tmV, a, gx, smem, stream);
-    default: return launch_t<KV, 1, D>(tmK, tmV, a, gx, smem, stream);
+cudaError_t launch_kv(const CUtensorMap& tmK, const CUtensorMap& tmV, const KernelArgs& a, int gx, size_t smem, cudaStream_t stream) {
+  if (a.rows > 8) return launch_t<KV, 0, D, 2>(tmK, tmV, a, gx, smem, stream);
+  switch (a.hpc) {
+    case 8: return launch_t<KV, 8, D, 1>(tmK, tmV, a, gx, smem, stream);
+    case 4: return launch_t<KV, 4, D, 1>(tmK, tmV, a, gx, smem, stream);
+    case 2: return launch_t<KV, 2, D, 1>(tmK, tmV, a, gx, smem, stream);
+    default: return launch_t<KV, 1, D, 1>(tmK, tmV, a, gx, smem, stream);
   }
 }
 
@@ -1011,15 +1107,15 @@ cudaError_t launch_combine_partials(const float* gathered, int R, long long rows
 size_t decode_workspace_bytes(int B, int Hq, int Hkv, int Nq, int D, int max_kv_len, int num_splits) {
   (void)max_kv_len;
   if (B <= 0 || Hq <= 0 || Hkv <= 0 || Nq <= 0) return 16;
-  const int hpc = pick_hpc(Hkv);
-  return make_layout(B, Hq, Nq, Hkv / hpc, pick_grid_x(Hkv, num_splits), D).total;
+  const Shape sh = pick_shape(Hkv, Hq / Hkv * Nq, num_splits);
+  return make_layout(B, Hq, Nq, Hkv / sh.hpc, sh.gx, D).total;
 }
 
 cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char* msg, size_t msg_len) {
   const bool quant = p.kv_dtype == 3 || p.kv_dtype == 4;
-  const int hpc = pick_hpc(p.Hkv);
+  const Shape sh = pick_shape(p.Hkv, p.Hq / p.Hkv * p.Nq, p.num_splits);
+  const int hpc = sh.hpc, gx = sh.gx;
   const int HG = p.Hkv / hpc;
-  const int gx = pick_grid_x(p.Hkv, p.num_splits);
   const int kD = p.D;
   const int row_bytes = quant ? kD : 2 * kD;
   if (!(kD == 128 || (kD == 64 && !quant))) {
@@ -1038,11 +1134,14 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.HG = HG;
   a.group = p.Hq / p.Hkv;
   a.rows = a.group * p.Nq;
+  a.hpc = hpc;
+  a.row_groups = sh.row_groups;
   a.stage_kv_bytes = hpc * kBS * row_bytes;
   a.scale_bytes = quant ? kBS * p.Hkv * 2 : 0;
   const size_t per_stage = 2 * static_cast<size_t>(a.stage_kv_bytes) + 2 * static_cast<size_t>(a.scale_bytes);
   // several small CTAs share an SM when a CTA holds few heads
-  const size_t budget = hpc == 8 ? 200 * 1024 : (hpc == 4 ? 100 * 1024 : (hpc == 2 ? 50 * 1024 : 26 * 1024));
+  const int per_sm = ctas_per_sm(hpc * sh.row_groups);
+  const size_t budget = per_sm == 1 ? 200 * 1024 : (per_sm == 2 ? 100 * 1024 : (per_sm == 4 ? 50 * 1024 : 33 * 1024));
   int stages = static_cast<int>(budget / per_stage);
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) {
@@ -1098,12 +1197,12 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   switch (p.kv_dtype) {
-    case 0: return kD == 64 ? launch_kv<KV_F16, 64>(hpc, tmK, tmV, a, gx, smem, stream)
-                            : launch_kv<KV_F16, 128>(hpc, tmK, tmV, a, gx, smem, stream);
-    case 1: return kD == 64 ? launch_kv<KV_BF16, 64>(hpc, tmK, tmV, a, gx, smem, stream)
-                            : launch_kv<KV_BF16, 128>(hpc, tmK, tmV, a, gx, smem, stream);
-    case 3: return launch_kv<KV_I8, 128>(hpc, tmK, tmV, a, gx, smem, stream);
-    case 4: return launch_kv<KV_E4M3, 128>(hpc, tmK, tmV, a, gx, smem, stream);
+    case 0: return kD == 64 ? launch_kv<KV_F16, 64>(tmK, tmV, a, gx, smem, stream)
+                            : launch_kv<KV_F16, 128>(tmK, tmV, a, gx, smem, stream);
+    case 1: return kD == 64 ? launch_kv<KV_BF16, 64>(tmK, tmV, a, gx, smem, stream)
+                            : launch_kv<KV_BF16, 128>(tmK, tmV, a, gx, smem, stream);
+    case 3: return launch_kv<KV_I8, 128>(tmK, tmV, a, gx, smem, stream);
+    case 4: return launch_kv<KV_E4M3, 128>(tmK, tmV, a, gx, smem, stream);
     default: snprintf(msg, msg_len, "kv_dtype %d", p.kv_dtype); return cudaErrorNotSupported;
   }
 }

@@ -52,6 +52,8 @@ extern "C" {
 #define B200FA_FLAG_FWD_PERSISTENT  8  /* tcgen05 forward: persistent CTAs (each walks many query tiles) whatever the shape */
 #define B200FA_FLAG_FWD_ONE_ITEM   16  /* tcgen05 forward: one query tile per CTA whatever the shape; without either flag the
                                           launcher chooses (persistent for large packed-sequence launches) */
+#define B200FA_FLAG_DECODE_WIDE    32  /* b200fa_decode_paged and its workspace query: (Hq/Hkv) * N up to 32 query rows per kv
+                                        * head instead of 8 */
 #define B200FA_FLAG_PACKED_F32      4  /* b200fa_decode_paged: `out` is float [B*Hq*N][D+4], the normalised row in fp32 with
                                           its base-2 lse at column D (columns D+1..D+3 pad the row to 16 bytes); `lse` is
                                           ignored.  The per-GPU partial of a sequence whose pages are spread over several
@@ -172,7 +174,8 @@ int32_t b200fa_bwd_varlen(const b200fa_desc* d, const void* q, const void* k, co
  *                  mlx_mfa/integrations/mlx_lm.py:97-110 with one group per row)
  *   block_table    int32 [B, max_blocks], -1 = no page
  *   seq_lens       int32 [B]
- *   d->N is the number of query rows per sequence, with (Hq/Hkv) * N <= 8; d->S is ignored;
+ *   d->N is the number of query rows per sequence, with (Hq/Hkv) * N <= 8, or <= 32 with B200FA_FLAG_DECODE_WIDE;
+ *   d->S is ignored;
  *   causal is per-sequence lower-right aligned.
  * `num_pages` bounds the block_table entries (larger ones are treated as holes and reported through the error word).
  * Slots of a sequence's last page beyond seq_lens[b] may hold anything, NaN patterns included: they are masked

@@ -22,6 +22,7 @@ FLAG_FORCE_MMA_SYNC = 1
 FLAG_PACKED_F32 = 4
 FLAG_FWD_PERSISTENT = 8
 FLAG_FWD_ONE_ITEM = 16
+FLAG_DECODE_WIDE = 32
 
 
 class Desc(C.Structure):

@@ -563,6 +563,12 @@ if hasattr(torch, "float8_e4m3fn"):
     _KV_CODE[torch.float8_e4m3fn] = _lib.E4M3
 
 
+# Query rows per kv head (heads of its group x query tokens) up to which a paged call runs the split-KV decode kernel:
+# it reads the pool once, 16 rows to an MMA, over all SMs, where the prefill kernel reads it once per query head into
+# 128-row tiles of which these rows fill a part.
+_MAX_DECODE_ROWS = 32
+
+
 def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, scale, causal, softcap,
                 block_size, want_lse, stream, num_splits=0, workspace=None, packed=False):
     """One decode launch.  packed=True returns (float32 [B*Hq*Nq, D+4], None): each row is the normalised output in
@@ -581,7 +587,8 @@ def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, 
     code = _DTYPE_CODE[q.dtype]
     kv_code = _KV_CODE.get(k_pages.dtype, _DTYPE_CODE.get(k_pages.dtype, -1))
     d = _desc(code, kv_code, B, Hq, Hkv, Nq, 0, D, scale, causal, softcap, -1, num_splits,
-              _FORCE_FLAGS | (_lib.FLAG_PACKED_F32 if packed else 0))
+              _FORCE_FLAGS | (_lib.FLAG_PACKED_F32 if packed else 0) |
+              (_lib.FLAG_DECODE_WIDE if (Hq // Hkv) * Nq > 8 else 0))
     with torch.cuda.device(q.device):
         need = lib.b200fa_decode_paged_workspace_bytes(C.byref(d), int(max_kv_len))
         if workspace is None or workspace.numel() < need:
@@ -635,7 +642,7 @@ def flash_attention_paged(
     ``seq_lens`` that the reference also performs (mlx_mfa/attention.py:2871-2873);
     ``num_splits`` caps how many CTAs share the page list (0 = one per SM).
 
-    Short queries ((Hq/Hkv)*Nq <= 8; D = 128, or D = 64 with 16-bit pools; block_size a multiple
+    Short queries ((Hq/Hkv)*Nq <= 32; D = 128, or D = 64 with 16-bit pools; block_size a multiple
     of 16) run the split-KV decode kernel with in-kernel combine; other shapes gather pages and attend
     per sequence like the reference (mlx_mfa/attention.py:2944-2989).  When gradients are
     wanted (q or a 16-bit pool requires grad) every shape takes the gather route, whose
@@ -682,7 +689,7 @@ def flash_attention_paged(
 
     # training: gradients flow through the gather route (gather, per-sequence attention, scatter-add into the pools)
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k_pages.requires_grad or v_pages.requires_grad)
-    decode_ok = ((Hq // Hkv) * Nq <= 8 and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
+    decode_ok = ((Hq // Hkv) * Nq <= _MAX_DECODE_ROWS and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
                  and not needs_grad)
     if decode_ok:
         out, lse = _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, float(scale),

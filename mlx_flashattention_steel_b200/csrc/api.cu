@@ -562,8 +562,9 @@ static int32_t decode_check(const b200fa_desc* d) {
     return fail(B200FA_ERR_INVALID_ARG, "bad extent");
   if (d->Hq % d->Hkv != 0)
     return fail(B200FA_ERR_INVALID_ARG, "q_heads (%d) must be divisible by kv_heads (%d)", d->Hq, d->Hkv);
-  if ((d->Hq / d->Hkv) * d->N > 8)
-    return fail(B200FA_ERR_UNSUPPORTED, "paged decode takes (Hq/Hkv)*N <= 8 query rows per kv head");
+  const int max_rows = (d->flags & B200FA_FLAG_DECODE_WIDE) ? 32 : 8;
+  if (static_cast<int64_t>(d->Hq / d->Hkv) * d->N > max_rows)
+    return fail(B200FA_ERR_UNSUPPORTED, "paged decode takes (Hq/Hkv)*N <= %d query rows per kv head", max_rows);
   const int kv = d->kv_dtype;
   if (!(kv == d->dtype || kv == B200FA_I8 || kv == B200FA_E4M3))
     return fail(B200FA_ERR_UNSUPPORTED, "kv_dtype must equal dtype or be int8 / e4m3");

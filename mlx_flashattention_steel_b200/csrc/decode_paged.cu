@@ -17,8 +17,9 @@
 //     values are widened to f16 in registers straight from the swizzled tile;
 //     k_scale multiplies the scores, v_scale is folded into P.
 //   * A CTA that covers a whole sequence writes the result; otherwise it writes a
-//     partial (normalised O, base-2 lse) and bumps a counter; the CTA that brings the
-//     counter to the number of parts combines them.  Nobody spins on anybody.
+//     partial (normalised O, base-2 lse), and a second kernel merges the partials of
+//     every row.  It is launched as a programmatic dependent, so that its blocks are
+//     in place when the last partial is written.  Nobody spins on anybody.
 //
 //   * Pages of 32, 64, ... tokens are walked as 16-token units (a unit is what one TMA box and one consumer step
 //     cover).  Dense caches [B, Hkv, S, D] (the reference's flash-decode route for N <= 4, S >= 256 on plain
@@ -27,7 +28,7 @@
 //   * head_dim 128 for every pool type; head_dim 64 for 16-bit pools and dense caches.
 //
 // Every mbarrier wait is bounded (tma.cuh); a timeout raises the error word at the
-// start of the workspace and the CTA leaves.
+// start of the workspace (through the merge kernel) and the CTA leaves.
 #include <cuda_fp8.h>
 
 #include <cstdio>
@@ -46,6 +47,7 @@ namespace {
 
 constexpr int kBS = 16;           // tokens per unit (one TMA box, one consumer step); a page is 1, 2, 4, ... units
 constexpr int kMaxStages = 8;
+constexpr int kMaxWarps = 9;      // warps of a CTA: 8 consumers and the producer
 // Up to this many sequences every CTA makes the page prefix sums itself, in shared memory (at most 4 KB): one read of
 // seq_lens and a scan, ~1 us, where a planning kernel in front and a binary search through its result in global memory
 // cost ~6 us before the first page was requested.  Beyond it decode_plan_kernel scans once for all.
@@ -58,8 +60,7 @@ enum KvKind { KV_F16 = 0, KV_BF16 = 1, KV_I8 = 2, KV_E4M3 = 3 };
 
 struct DecodeLayout {          // workspace carve-up, in bytes from the workspace base
   size_t err;                  // int[4]: [0] error word
-  size_t counters;             // int[B * HG]: parts (or groups of parts) of a sequence that have arrived
-  size_t group_counters;       // int[slots * HG]: parts of a group that have arrived, by the group's first slot
+  size_t status;               // int[gx * HG * warps of a CTA]: error bits of every warp of the main kernel
   size_t page_start;           // int[B + 1], only when B > kSmemSeqs
   size_t part_lse;             // float[slots * Hq * Nq]
   size_t part_o;               // float[slots * Hq * Nq * D]
@@ -72,10 +73,9 @@ __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a -
 __host__ __device__ inline DecodeLayout make_layout(int B, int Hq, int Nq, int HG, int G, int kD) {
   DecodeLayout L;
   L.err = 0;
-  L.counters = 16;
+  L.status = 16;
   L.slots = G + B;
-  L.group_counters = L.counters + sizeof(int) * static_cast<size_t>(B) * HG;
-  L.page_start = align_up(L.group_counters + sizeof(int) * static_cast<size_t>(L.slots) * HG, 16);
+  L.page_start = align_up(L.status + sizeof(int) * static_cast<size_t>(G) * HG * kMaxWarps, 16);
   L.part_lse = align_up(L.page_start + (B > kSmemSeqs ? sizeof(int) * (static_cast<size_t>(B) + 1) : 0), 16);
   L.part_o = align_up(L.part_lse + sizeof(float) * static_cast<size_t>(L.slots) * Hq * Nq, 16);
   L.total = align_up(L.part_o + sizeof(float) * static_cast<size_t>(L.slots) * Hq * Nq * kD, 16);
@@ -100,12 +100,8 @@ struct KernelArgs {
 };
 
 // ---------------------------------------------------------------------------
-// plan: counters and error word reset; page prefix sums when there are more than kSmemSeqs sequences
+// plan: page prefix sums of more than kSmemSeqs sequences
 // ---------------------------------------------------------------------------
-// Programmatic dependent launch: the main kernel may start as soon as this one has, and waits (pdl_wait) before it
-// touches anything that is written here.  Up to kSmemSeqs sequences that is only the counters, which it needs last, so
-// this launch costs no time of its own; it starts after everything earlier in the stream has completed, so whatever
-// the main kernel reads before its wait (pools, table, lengths, queries) is in place.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
@@ -115,17 +111,19 @@ __device__ __forceinline__ int units_of(const int32_t* seq_lens, int i, int max_
   return (len + kBS - 1) / kBS;
 }
 
-__global__ void __launch_bounds__(1024) decode_plan_kernel(const int32_t* __restrict__ seq_lens, int B,
-                                                           int max_kv_len, int n_counters,
-                                                           int* __restrict__ err, int* __restrict__ counters,
+// CTAs (of gx) that work on U units of B sequences.  With few units not every CTA does: two units (one step of the
+// consumers) each, or one sequence each when they are that short -- a CTA more to a sequence is a part more to merge, a
+// second sequence in a CTA costs it 4 us.  The CTAs that share a sequence are always consecutive.
+__device__ __forceinline__ int working_ctas(long long U, int B, int gx) {
+  const long long want = max((U + 1) / 2, min(U, static_cast<long long>(B)));
+  return want < static_cast<long long>(gx) ? static_cast<int>(want) : gx;
+}
+
+__global__ void __launch_bounds__(1024) decode_plan_kernel(const int32_t* __restrict__ seq_lens, int B, int max_kv_len,
                                                            int* __restrict__ page_start) {
-  pdl_launch_dependents();
   __shared__ int warp_sums[32];
   __shared__ int carry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 4) err[tid] = 0;
-  for (int i = tid; i < n_counters; i += blockDim.x) counters[i] = 0;
-  if (page_start == nullptr) return;
   if (tid == 0) { carry = 0; page_start[0] = 0; }
   __syncthreads();
   for (int base = 0; base < B; base += blockDim.x) {
@@ -193,9 +191,6 @@ __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
-}
 // D (16 x 8, int32) += A (16 x 32, int8) B (32 x 8, int8).  8.3 clk per instruction and scheduler, what the f16
 // m16n8k16 takes (8.4), for twice the depth.
 __device__ __forceinline__ void mma16832_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -212,53 +207,150 @@ __device__ __forceinline__ int cta_of_unit(long long u, int G, long long U) {
 }
 
 // ---------------------------------------------------------------------------
-// combine of partials
+// merge of partials
 // ---------------------------------------------------------------------------
-// One warp merges n partials of one query row: L = log2 sum_i 2^lse_i, O = sum_i 2^(lse_i - L) O_i
-// (csrc/mfa_steel_fwd.cpp:2066-2101).  lse / o point at the first partial's row, stride slots apart in units of
-// lse_step / o_step floats; lane l carries head-dim values [4l, 4l + 4).  What bounds it is the latency of L2: the
-// lanes fetch 32 log-sum-exps at once and the rows are read 16 at a time, all in flight together (one after the other,
-// the 148 partials of one 262144-token sequence took longer than half of its keys: 198 us in all).
+// L = log2 sum_i 2^lse_i, O = sum_i 2^(lse_i - L) O_i over the parts of a sequence (csrc/mfa_steel_fwd.cpp:2066-2101);
+// rows of empty sequences become zeros with lse = -inf.  A block holds kMergeWarps / W rows, W warps to a row take its
+// parts in turn; lane l carries head-dim values [4l, 4l + 4).  Bound by L2 latency: a warp fetches 32 log-sum-exps at
+// once and has 8 partial rows in flight (64 registers, so that a block fits beside a CTA of the main kernel).  The first version merged inside the main kernel, in the CTA that arrived last
+// (fences, an atomic, then one SM's eight warps for every row): 262144 tokens in 148 parts 198 us in all, 512 tokens
+// 21 us of which 13 were the merge.  Here every row has warps of its own, and the block is already resident and knows its
+// sequence's parts when the main kernel ends.
+constexpr int kMergeWarps = 8;
+
 template <int kD>
-__device__ __forceinline__ float combine_row(const float* lse, size_t lse_step, const float* o, size_t o_step, int n,
-                                             int lane, float4& out) {
+__global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const __grid_constant__ KernelArgs a, int gx, int W, int blocks_per_seq) {
+  const DecodeParams& p = a.p;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x / blocks_per_seq;
+  unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
+  __shared__ int s_sum[2][kMergeWarps];
+  __shared__ float s_part[kMergeWarps][2];
+  __shared__ float4 s_acc[kMergeWarps][32];
+
+  // units before sequence b, and of all: inputs of the launch, so nothing to wait for
+  int before = 0, all = 0;
+  for (int i = tid; i < p.B; i += blockDim.x) {
+    const int n = units_of(p.seq_lens, i, p.max_kv_len);
+    all += n;
+    if (i < b) before += n;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+    all += __shfl_xor_sync(0xffffffffu, all, o);
+  }
+  if (lane == 0) { s_sum[0][warp] = before; s_sum[1][warp] = all; }
+  __syncthreads();
+  long long s0 = 0, U = 0;
+#pragma unroll
+  for (int i = 0; i < kMergeWarps; ++i) { s0 += s_sum[0][i]; U += s_sum[1][i]; }
+  const int n_units = units_of(p.seq_lens, b, p.max_kv_len);
+  int c_first = 0, n = 0;
+  if (n_units > 0) {
+    const int G = working_ctas(U, p.B, gx);
+    c_first = cta_of_unit(s0, G, U);
+    n = cta_of_unit(s0 + n_units - 1, G, U) - c_first + 1;
+  }
+
+  pdl_wait();               // the main kernel has ended: its partials and status words can be read
+
+  if (blockIdx.x == 0) {
+    // error word = all bits that the main kernel's warps left
+    const int* status = reinterpret_cast<const int*>(ws + a.lay.status);
+    const int words = gx * a.HG * (a.hpc * a.row_groups + 1);
+    int bits = 0;
+    for (int i = tid; i < words; i += blockDim.x) bits |= __ldcg(status + i);
+    bits = __reduce_or_sync(0xffffffffu, bits);
+    __syncthreads();
+    if (lane == 0) s_sum[0][warp] = bits;
+    __syncthreads();
+    if (tid == 0) {
+      for (int i = 1; i < kMergeWarps; ++i) bits |= s_sum[0][i];
+      *reinterpret_cast<int*>(ws + a.lay.err) = bits;
+    }
+  }
+  if (n == 1) return;                                 // one CTA had the whole sequence and wrote the result
+
+  const int HqNq = p.Hq * p.Nq;
+  const int sub = warp % W;                           // which of the row's warps
+  const int row = (blockIdx.x % blocks_per_seq) * (kMergeWarps / W) + warp / W;      // hq * Nq + query token
+  const bool live = lane * 4 < kD;                    // head_dim 64: the first 16 lanes carry the row
   float m = -INFINITY, wsum = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool live = lane * 4 < kD;                  // head_dim 64: the first 16 lanes carry the row
-  for (int base = 0; base < n; base += 32) {
-    const int cn = min(32, n - base);
-    const float lv = lane < cn ? __ldcg(lse + (base + lane) * lse_step) : -INFINITY;
-    float mx = lv;
+  if (row < HqNq) {
+    const size_t slot0 = static_cast<size_t>(c_first) + b;
+    const float* lse = reinterpret_cast<const float*>(ws + a.lay.part_lse) + slot0 * HqNq + row;
+    const float* o = reinterpret_cast<const float*>(ws + a.lay.part_o) + (slot0 * HqNq + row) * kD + lane * 4;
+    const size_t o_step = static_cast<size_t>(HqNq) * kD;
+    // this warp's parts: sub, sub + W, ...; 32 of them at a time
+    for (int base = sub; base < n; base += 32 * W) {
+      const int cn = min(32, (n - base + W - 1) / W);
+      const float lv = lane < cn ? __ldcg(lse + static_cast<size_t>(base + lane * W) * HqNq) : -INFINITY;
+      float mx = lv;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-    const float m_new = fmaxf(m, mx);
-    const float ms = (m_new == -INFINITY) ? 0.f : m_new;
-    const float corr = exp2f(m - ms);               // 0 from -inf
-    acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
-    const float w = exp2f(lv - ms);
-    float ws = w;
+      for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+      const float m_new = fmaxf(m, mx);
+      const float ms = (m_new == -INFINITY) ? 0.f : m_new;
+      const float corr = exp2f(m - ms);               // 0 from -inf
+      acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
+      const float w = exp2f(lv - ms);
+      float sum = w;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, s);
-    wsum = fmaf(wsum, corr, ws);
-    m = m_new;
-    for (int i0 = 0; i0 < cn; i0 += 16) {
-      float4 v[16];
+      for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+      wsum = fmaf(wsum, corr, sum);
+      m = m_new;
+      for (int i0 = 0; i0 < cn; i0 += 8) {
+        float4 v[8];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live && i0 + k < cn) v[k] = __ldcg(reinterpret_cast<const float4*>(o + (base + i0 + k) * o_step + lane * 4));
-      }
+        for (int k = 0; k < 8; ++k) {
+          v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (live && i0 + k < cn) v[k] = __ldcg(reinterpret_cast<const float4*>(o + static_cast<size_t>(base + (i0 + k) * W) * o_step));
+        }
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const float wk = __shfl_sync(0xffffffffu, w, (i0 + k) & 31);
-        acc.x = fmaf(wk, v[k].x, acc.x); acc.y = fmaf(wk, v[k].y, acc.y);
-        acc.z = fmaf(wk, v[k].z, acc.z); acc.w = fmaf(wk, v[k].w, acc.w);
+        for (int k = 0; k < 8; ++k) {
+          const float wk = __shfl_sync(0xffffffffu, w, (i0 + k) & 31);
+          acc.x = fmaf(wk, v[k].x, acc.x); acc.y = fmaf(wk, v[k].y, acc.y);
+          acc.z = fmaf(wk, v[k].z, acc.z); acc.w = fmaf(wk, v[k].w, acc.w);
+        }
       }
     }
   }
+  if (W > 1) {
+    s_acc[warp][lane] = acc;
+    if (lane == 0) { s_part[warp][0] = m; s_part[warp][1] = wsum; }
+    __syncthreads();
+    if (sub != 0) return;
+    float mt = m;
+    for (int i = 1; i < W; ++i) mt = fmaxf(mt, s_part[warp + i][0]);
+    const float ms = (mt == -INFINITY) ? 0.f : mt;
+    const float corr = exp2f(m - ms);
+    acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
+    wsum *= corr;
+    for (int i = 1; i < W; ++i) {
+      const float c = exp2f(s_part[warp + i][0] - ms);
+      const float4 v = s_acc[warp + i][lane];
+      acc.x = fmaf(c, v.x, acc.x); acc.y = fmaf(c, v.y, acc.y); acc.z = fmaf(c, v.z, acc.z); acc.w = fmaf(c, v.w, acc.w);
+      wsum = fmaf(c, s_part[warp + i][1], wsum);
+    }
+    m = mt;
+  }
+  if (row >= HqNq) return;
   const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  out = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-  return wsum > 0.f ? m + log2f(wsum) : -INFINITY;
+  const float lse = wsum > 0.f ? m + log2f(wsum) : -INFINITY;
+  const float4 v = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+  const size_t orow = static_cast<size_t>(b) * HqNq + row;
+  if (p.packed_f32) {
+    float* pk = reinterpret_cast<float*>(p.out) + orow * (kD + 4);
+    if (live) *reinterpret_cast<float4*>(pk + lane * 4) = v;
+    if (lane == 0) pk[kD] = lse;
+  } else {
+    if (live) {
+      const uint2 pk = p.q_dtype == 0 ? make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w)) : make_uint2(pack_bf2(v.x, v.y), pack_bf2(v.z, v.w));
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out) + orow * kD + lane * 4) = pk;
+    }
+    if (p.lse != nullptr && lane == 0) p.lse[orow] = lse;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -292,8 +384,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   uint64_t* bars = reinterpret_cast<uint64_t*>(sVs + static_cast<size_t>(NS) * a.scale_bytes);  // full[NS], empty[NS]
   int* s_page = reinterpret_cast<int*>(bars + 2 * kMaxStages);
   volatile int* s_abort = s_page + kMaxStages;
-  int* s_last = const_cast<int*>(s_abort) + 1;
-  int* s_page_start = s_last + 2;                       // int[B + 1] when B <= kSmemSeqs
+  int* s_page_start = const_cast<int*>(s_abort) + 1;     // int[B + 1] when B <= kSmemSeqs
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -303,15 +394,15 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int n_cons = HPC > 0 ? HPC : a.hpc * a.row_groups;       // consumer warps; the next one is the producer
 
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
-  int* err = reinterpret_cast<int*>(ws + a.lay.err);
-  int* counters = reinterpret_cast<int*>(ws + a.lay.counters);
-  int* group_counters = reinterpret_cast<int*>(ws + a.lay.group_counters);
+  // every warp leaves its error bits (1: a bounded wait gave up, 2: a table entry beyond the pool)
+  int* status = reinterpret_cast<int*>(ws + a.lay.status) + (static_cast<size_t>(hg) * gridDim.x + c) * (n_cons + 1) + warp;
   float* part_lse = reinterpret_cast<float*>(ws + a.lay.part_lse);
   float* part_o = reinterpret_cast<float*>(ws + a.lay.part_o);
 
   const int rows = a.rows;
   const int HqNq = p.Hq * p.Nq;
 
+  pdl_launch_dependents();      // the merge kernel's blocks may take their places
   if (tid == 0) {
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
@@ -344,43 +435,16 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       if (lane == 0) s_page_start[0] = 0;
     }
   } else {
-    pdl_wait();
     page_start = reinterpret_cast<const int*>(ws + a.lay.page_start);
   }
   __syncthreads();
 
-  // Sequences of length zero have no unit: CTA 0 of each head group zero-fills them.
-  if (c == 0) {
-    for (int b = 0; b < p.B; ++b) {
-      if (page_start[b + 1] != page_start[b]) continue;
-      for (int i = tid; i < hpc * a.group * p.Nq * kD; i += blockDim.x) {
-        const int d = i % kD;
-        const int r = i / kD;                       // (head in cta, group, qi)
-        const int qi = r % p.Nq;
-        const int hq = (hg * hpc) * a.group + r / p.Nq;
-        const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
-        const size_t o = orow * kD + d;
-        if (p.packed_f32) {
-          float* pk = reinterpret_cast<float*>(p.out) + orow * (kD + 4);
-          pk[d] = 0.f;
-          if (d == 0) pk[kD] = -INFINITY;
-        } else {
-          if (p.q_dtype == 0) reinterpret_cast<__half*>(p.out)[o] = __float2half(0.f);
-          else reinterpret_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16(0.f);
-          if (p.lse != nullptr && d == 0) p.lse[orow] = -INFINITY;
-        }
-      }
-    }
-  }
-
-  // With fewer units than CTAs only the first U CTAs work, one unit each, so that the
-  // CTAs sharing a sequence are always consecutive.
   const long long U = page_start[p.B];
-  const int G = U < static_cast<long long>(gridDim.x) ? static_cast<int>(U) : static_cast<int>(gridDim.x);
+  const int G = working_ctas(U, p.B, static_cast<int>(gridDim.x));
   const long long lo = c < G ? static_cast<long long>(c) * U / G : 0;
   const long long hi = c < G ? static_cast<long long>(c + 1) * U / G : 0;
   if (lo >= hi) {
-    pdl_wait();               // the launch completes only after the plan kernel has
+    if (lane == 0) *status = 0;
     return;
   }
 
@@ -404,7 +468,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     long long u = lo;
     int b = b_first;
     bool ok = true;
-    int bad = 0;                // error bits; the error word is the plan kernel's to clear, so they go there at the end
+    int bad = 0;
     while (u < hi && ok) {
       const int s0 = page_start[b], s1 = page_start[b + 1];
       if (s1 <= u) { ++b; continue; }
@@ -455,9 +519,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       u = s0 + j_hi;
       if (u >= s1) ++b;
     }
-    if (!ok) bad |= 1;
-    pdl_wait();
-    if (bad != 0) atomicOr(err, bad);
+    bad = __reduce_or_sync(0xffffffffu, bad | (ok ? 0 : 1));
+    if (lane == 0) *status = bad;
     return;
   }
 
@@ -473,7 +536,6 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     qi_row[rt] = row_of[rt] / a.group;
     hq_row[rt] = kvh * a.group + row_of[rt] % a.group;
   }
-  const int my_rows = min(8 * RT, rows - rbase);                // may be <= 0: the warp then only keeps step
   int stage = 0;
   uint32_t phase = 0;
   long long u = lo;
@@ -927,74 +989,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
     }
 
-    if (!direct) {
-      // The part that arrives last combines.  Up to 32 parts at once; more in two steps, so that the work of a sequence
-      // spread over many CTAs is shared out: the last part of each group of 16 (64 from 512 parts on) merges its group
-      // into the group's first slot, the last group merges those.  Parts of a sequence are consecutive CTAs and their
-      // slots consecutive, so every split is the same whoever arrives last: results do not depend on the order.
-      // 262144 tokens x 8 heads over 148 CTAs: 198 us with one warp reading 148 partials a row at a time.
-      const int gsz = n_parts <= 32 ? 32 : (n_parts <= 512 ? 16 : 64);
-      const int grp = (c - c_first) / gsz, n_grp = (n_parts + gsz - 1) / gsz;
-      const int slot0 = c_first + b;                                  // the sequence's first slot
-      const int gslot = slot0 + grp * gsz;                            // the group's first slot
-      const int gn = min(gsz, n_parts - grp * gsz);
-      auto merge = [&](int first, int step, int n, bool final_out) {
-        for (int r = rbase; r < rbase + my_rows; ++r) {
-          const int hq = kvh * a.group + r % a.group;
-          const int qi = r / a.group;
-          const size_t rowi = static_cast<size_t>(hq) * p.Nq + qi;
-          const size_t row0 = static_cast<size_t>(first) * HqNq + rowi;
-          float4 v;
-          const float lse = combine_row<kD>(part_lse + row0, static_cast<size_t>(step) * HqNq, part_o + row0 * kD,
-                                            static_cast<size_t>(step) * HqNq * kD, n, lane, v);
-          const bool col_live = lane * 4 < kD;
-          if (!final_out) {
-            // in place: only this warp reads these rows, and it has
-            __syncwarp();
-            if (col_live) __stcg(reinterpret_cast<float4*>(part_o + row0 * kD + lane * 4), v);
-            if (lane == 0) __stcg(part_lse + row0, lse);
-            continue;
-          }
-          const size_t orow = (static_cast<size_t>(b) * p.Hq + hq) * p.Nq + qi;
-          const size_t o = orow * kD + lane * 4;
-          if (p.packed_f32) {
-            float* pk = reinterpret_cast<float*>(p.out) + orow * (kD + 4);
-            if (col_live) *reinterpret_cast<float4*>(pk + lane * 4) = v;
-            if (lane == 0) pk[kD] = lse;
-          } else {
-            if (col_live) {
-              const uint2 pk = p.q_dtype == 0 ? make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w))
-                                              : make_uint2(pack_bf2(v.x, v.y), pack_bf2(v.z, v.w));
-              *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out) + o) = pk;
-            }
-            if (p.lse != nullptr && lane == 0) p.lse[orow] = lse;
-          }
-        }
-      };
-      // true in every consumer thread of the CTA that brings `counter` to n
-      auto arrive_last = [&](int* counter, int n, int* flag) -> bool {
-        __threadfence();
-        named_bar_sync(1, n_cons * 32);
-        if (tid == 0) *flag = atomicAdd(counter, 1) == n - 1 ? 1 : 0;
-        named_bar_sync(1, n_cons * 32);
-        const bool last = *flag != 0;
-        if (last) __threadfence();
-        return last;
-      };
-      pdl_wait();                                                     // the counters are the plan kernel's to clear
-      if (arrive_last(&group_counters[static_cast<size_t>(gslot) * a.HG + hg], gn, s_last)) {
-        merge(gslot, 1, gn, n_grp == 1);
-        if (n_grp > 1 && arrive_last(&counters[static_cast<size_t>(b) * a.HG + hg], n_grp, s_last + 1))
-          merge(slot0, gsz, n_grp, true);
-      }
-      named_bar_sync(1, n_cons * 32);   // the flags are reused by the next sequence
-    }
-
     u = static_cast<long long>(s0) + j_hi;
     if (u >= s1) ++b;
   }
-  pdl_wait();
-  if (!ok && lane == 0) atomicOr(err, 1);
+  if (lane == 0) *status = ok ? 0 : 1;
 }
 
 // Combine of per-GPU partials: one warp per output row, lanes across the head dim.
@@ -1068,17 +1066,8 @@ cudaError_t launch_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const Kerne
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gx, a.HG);
-    cfg.blockDim = dim3((a.hpc * a.row_groups + 1) * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, tmK, tmV, a);
+    kern<<<dim3(gx, a.HG), (a.hpc * a.row_groups + 1) * 32, smem, stream>>>(tmK, tmV, a);
+    return cudaGetLastError();
   };
   return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true, RT>) : go(decode_paged_kernel<KV, HPC, D, false, RT>);
 }
@@ -1092,6 +1081,27 @@ cudaError_t launch_kv(const CUtensorMap& tmK, const CUtensorMap& tmV, const Kern
     case 2: return launch_t<KV, 2, D, 1>(tmK, tmV, a, gx, smem, stream);
     default: return launch_t<KV, 1, D, 1>(tmK, tmV, a, gx, smem, stream);
   }
+}
+
+// Warps to a row: enough that a sequence of average length has about 12 parts per warp.
+template <int D>
+cudaError_t launch_merge(const KernelArgs& a, int gx, cudaStream_t stream) {
+  int W = 1;
+  while (W < kMergeWarps && gx > 12 * a.p.B * W) W <<= 1;
+  const int rows_per_block = kMergeWarps / W;
+  const int blocks_per_seq = (a.p.Hq * a.p.Nq + rows_per_block - 1) / rows_per_block;
+  const long long blocks = static_cast<long long>(a.p.B) * blocks_per_seq;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(kMergeWarps * 32);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, decode_merge_kernel<D>, a, gx, W, blocks_per_seq);
 }
 
 }  // namespace
@@ -1190,21 +1200,23 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   }
 
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
-  decode_plan_kernel<<<1, 1024, 0, stream>>>(p.seq_lens, p.B, p.max_kv_len, (p.B + a.lay.slots) * HG,
-                                             reinterpret_cast<int*>(ws + a.lay.err),
-                                             reinterpret_cast<int*>(ws + a.lay.counters),
-                                             p.B > kSmemSeqs ? reinterpret_cast<int*>(ws + a.lay.page_start) : nullptr);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  if (p.B > kSmemSeqs) {
+    decode_plan_kernel<<<1, 1024, 0, stream>>>(p.seq_lens, p.B, p.max_kv_len, reinterpret_cast<int*>(ws + a.lay.page_start));
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
   switch (p.kv_dtype) {
-    case 0: return kD == 64 ? launch_kv<KV_F16, 64>(tmK, tmV, a, gx, smem, stream)
-                            : launch_kv<KV_F16, 128>(tmK, tmV, a, gx, smem, stream);
-    case 1: return kD == 64 ? launch_kv<KV_BF16, 64>(tmK, tmV, a, gx, smem, stream)
-                            : launch_kv<KV_BF16, 128>(tmK, tmV, a, gx, smem, stream);
-    case 3: return launch_kv<KV_I8, 128>(tmK, tmV, a, gx, smem, stream);
-    case 4: return launch_kv<KV_E4M3, 128>(tmK, tmV, a, gx, smem, stream);
+    case 0: e = kD == 64 ? launch_kv<KV_F16, 64>(tmK, tmV, a, gx, smem, stream)
+                            : launch_kv<KV_F16, 128>(tmK, tmV, a, gx, smem, stream); break;
+    case 1: e = kD == 64 ? launch_kv<KV_BF16, 64>(tmK, tmV, a, gx, smem, stream)
+                            : launch_kv<KV_BF16, 128>(tmK, tmV, a, gx, smem, stream); break;
+    case 3: e = launch_kv<KV_I8, 128>(tmK, tmV, a, gx, smem, stream); break;
+    case 4: e = launch_kv<KV_E4M3, 128>(tmK, tmV, a, gx, smem, stream); break;
     default: snprintf(msg, msg_len, "kv_dtype %d", p.kv_dtype); return cudaErrorNotSupported;
   }
+  if (e != cudaSuccess) return e;
+  return kD == 64 ? launch_merge<64>(a, gx, stream) : launch_merge<128>(a, gx, stream);
 }
 
 }  // namespace b200fa
@@ -1213,7 +1225,7 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
 // Decode without a caller-supplied workspace
 // ---------------------------------------------------------------------------
 // Scratch for b200fa_decode_paged_static: the same carve-up the workspace variant
-// uses (error word, per-sequence counters, page prefix sums, split partials), held in
+// uses (error word, status words, page prefix sums, split partials), held in
 // a fixed array that every GPU loading this library keeps until the process exits.
 #define B200FA_STATIC_SCRATCH_BYTES (16u * 1024u * 1024u)
 static __device__ __align__(256) unsigned char g_decode_static_scratch[B200FA_STATIC_SCRATCH_BYTES];
@@ -1271,8 +1283,8 @@ extern "C" int32_t b200fa_decode_paged_static(const b200fa_desc* d, const void* 
     b200fa::set_last_error(msg);
     return B200FA_ERR_CUDA;
   }
-  // Same validation, planning and kernels as the workspace variant; the plan kernel
-  // clears the counters and the error word at the start of every call.
+  // Same validation, planning and kernels as the workspace variant; the merge kernel
+  // writes the error word at the end of every call.
   return b200fa_decode_paged(d, q, k_pool, v_pool, k_scale, v_scale, block_table, seq_lens, num_pages,
                              block_size, max_blocks, max_kv_len, out, lse, scratch,
                              B200FA_STATIC_SCRATCH_BYTES, stream);

@@ -1,0 +1,96 @@
+"""Paged split-KV decode where its launch takes another form: 9 to 32 query rows per kv head (two row tiles per warp, two
+warps per head), partials merged in two steps, more sequences than a CTA scans itself, fixed-point queries of int8 pools,
+launches inside a CUDA graph.  Oracle and tolerance (2e-2 max-abs) as in test_decode_gpu.py."""
+import pytest
+import torch
+
+import mlx_flashattention_steel_b200 as fa
+from oracle import sdpa_oracle as orc
+
+from .test_decode_gpu import _run, _status_checks  # noqa: F401  (the fixture applies to this module too)
+from .util import assert_close, make_paged, randn
+
+pytestmark = pytest.mark.gpu
+
+LENS = [0, 1, 2, 16, 17, 31, 33, 500, 2100]
+
+
+@pytest.mark.parametrize("quant", [None, "int8", "e4m3"])
+@pytest.mark.parametrize("Hq,Hkv,Nq", [(6, 2, 3), (32, 8, 3), (32, 8, 4), (16, 16, 17), (8, 2, 6), (16, 2, 4), (3, 1, 11)])
+def test_more_than_eight_rows(dev, quant, Hq, Hkv, Nq):
+    # 9, 12, 16, 17, 24, 32 and 33 rows (33: the prefill route); sequences shorter than the query chunk among them
+    _run(dev, torch.bfloat16, quant, len(LENS), Hq, Hkv, Nq, LENS, 700 + Nq, softcap=30.0 if Nq == 6 else 0.0, holes=True)
+
+
+@pytest.mark.parametrize("causal,D,block_size,softcap", [(False, 128, 16, 0.0), (True, 64, 16, 0.0), (True, 64, 64, 20.0), (True, 128, 48, 100.0)])
+def test_more_than_eight_rows_options(dev, causal, D, block_size, softcap):
+    for dtype, Nq in ((torch.float16, 4), (torch.bfloat16, 7)):
+        _run(dev, dtype, None, 4, 16, 4, Nq, [700, 5, 1030, 64], 720 + Nq, causal=causal, softcap=softcap, D=D, block_size=block_size)
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+@pytest.mark.parametrize("Hq,Hkv,Nq", [(8, 2, 1), (16, 8, 1), (8, 1, 4), (4, 4, 5)])
+def test_many_parts_are_merged_in_two_steps(dev, quant, Hq, Hkv, Nq):
+    # every CTA holds a part of the one long sequence; the second one ends inside a group of parts
+    _run(dev, torch.float16, quant, 2, Hq, Hkv, Nq, [30000, 1500], 740)
+
+
+def test_more_sequences_than_a_cta_scans(dev):
+    lens = [(7 * i) % 50 for i in range(1030)]                     # every 50th is empty
+    _run(dev, torch.bfloat16, "int8", len(lens), 4, 2, 1, lens, 750)
+    _run(dev, torch.bfloat16, None, 1024, 4, 2, 1, lens[:1024], 751)
+
+
+def test_values_beyond_the_end_are_not_read_into_wide_rows(dev):
+    pg = make_paged(2, 2, 128, 16, [21, 300], torch.bfloat16, 760)
+    for name in ("k", "v"):
+        for b, n in enumerate((21, 300)):
+            pg[name][int(pg["block_table"][b, n // 16]), n % 16:] = float("nan")
+    q = randn((2, 8, 4, 128), torch.bfloat16, 761)
+    out = fa.flash_attention_paged(q.to(dev), pg["k"].to(dev), pg["v"].to(dev), pg["block_table"].to(dev), pg["seq_lens"].to(dev), causal=True)
+    clean = {n: torch.nan_to_num(pg[n].float()).to(torch.bfloat16) for n in ("k", "v")}
+    O, _ = orc.paged_attention(q, clean["k"], clean["v"], pg["block_table"], pg["seq_lens"], causal=True)
+    assert_close(out, O, torch.bfloat16)
+
+
+@pytest.mark.parametrize("Nq", [1, 4])
+def test_int8_queries_of_uneven_size(dev, Nq):
+    """A row of Q is fixed point below its largest value: rows with one value far above the others, tiny rows, zero rows.
+    The step is max|q| / 32639, so the scaled score is off by at most sum_d |k_d| * scale * max|q| / 65278: for the outlier
+    row (max|q| = 60, sum|k| ~ 128 * 0.8) 0.0083, inside the 2e-2 the outputs are held to."""
+    pg = make_paged(3, 2, 128, 16, [40, 700, 333], torch.float16, 770, quant="int8")
+    q = randn((3, 8, Nq, 128), torch.float16, 771)
+    q[0, :, :, 5] = 60.0
+    q[1, 1] = 0.0
+    q[1, 2] *= 2.0 ** -12
+    args = [x.to(dev) for x in (q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"])]
+    out = fa.flash_attention_paged(*args, causal=True, k_scale=pg["k_scale"].to(dev), v_scale=pg["v_scale"].to(dev))
+    O, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, k_scale=pg["k_scale"],
+                               v_scale=pg["v_scale"])
+    assert_close(out, O, torch.float16)
+
+
+@pytest.mark.parametrize("Nq", [1, 4])
+def test_replayed_from_a_graph(dev, Nq):
+    """The plan kernel and the main kernel are joined by a programmatic dependency: it survives capture, and replays on
+    changed inputs give what direct calls give."""
+    pg = make_paged(3, 2, 128, 16, [900, 65, 333], torch.bfloat16, 780)
+    k, v, table = (pg[n].to(dev) for n in ("k", "v", "block_table"))
+    lens, q = pg["seq_lens"].to(dev), randn((3, 8, Nq, 128), torch.bfloat16, 781).to(dev)
+
+    def call():
+        return fa.flash_attention_paged(q, k, v, table, lens, causal=True, max_kv_len=900)
+
+    from mlx_flashattention_steel_b200 import attention as A
+    A._set_check_decode_status(False)                               # the check synchronises, which a capture does not allow
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    for step in range(3):
+        q.copy_(randn(tuple(q.shape), torch.bfloat16, 790 + step).to(dev))
+        lens.copy_(torch.tensor([900 - 100 * step, 65 - step, 333], dtype=torch.int32, device=dev))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, call())

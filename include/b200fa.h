@@ -112,8 +112,9 @@ const char* b200fa_version(void);
  * Forward, dense layout.  Replaces mfa_attention_forward (csrc/bindings.cpp:21-35)
  * and mfa_forward_with_lse (csrc/bindings.cpp:38-57); host dispatch role of
  * MFAttention::eval_gpu (csrc/mfa_attention.cpp:47-409).  `lse` may be NULL.
- * The forward kernels need no scratch: both *_fwd*_workspace_bytes queries always return 0 (they exist so that a
- * binding can treat every operator alike) and the workspace arguments are ignored.
+ * No call needs the workspace: without it (NULL, or smaller than the query says) the same kernels run with less sharing
+ * between SMs.  The query is non-zero for two kinds of calls.  f16 / bf16, N <= 4, S >= 256, at most 8 query rows per kv
+ * head: with it the split-KV decode kernel runs.  f32, N > 64: with it every SM gets the same number of key tiles.
  */
 size_t  b200fa_fwd_workspace_bytes(const b200fa_desc* d);
 int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const void* v,

@@ -161,7 +161,8 @@ def _fwd_raw(q, k, v, scale, causal, softcap, window_left, want_lse, stream, out
               flags=_FORCE_FLAGS, q=q, k=k if S > 0 else None, v=v if S > 0 else None, o=out, alibi=alibi, bmask=bmask,
               kv_lens=kv_lens)
     with torch.cuda.device(q.device):
-        # non-zero only for a few query rows against a long cache (N <= 4, S >= 256): the split-KV decode route
+        # non-zero for a few query rows against a long cache (N <= 4, S >= 256: the split-KV decode route) and for
+        # float32 (partials of the query tiles that several CTAs share)
         need = lib.b200fa_fwd_workspace_bytes(C.byref(d))
         ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need > 0 else None
         st = lib.b200fa_fwd(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(ws), need,

@@ -168,8 +168,15 @@ static bool dense_decode_route(const b200fa_desc* d) {
   return contiguous(d->q_strides) && contiguous(d->o_strides);
 }
 
+// Workspace of the float32 forward, which has its CTAs share the key tiles evenly; 0 for descriptors that b200fa_fwd does
+// not run it for, and up to one tile of 64 query rows, which keeps a CTA per head.
+static size_t fwd_f32_need(const b200fa_desc* d) {
+  if (d == nullptr || d->dtype != B200FA_F32 || !(d->D == 64 || d->D == 128) || d->kv_lens != nullptr || d->N <= 64 || d->S < 0) return 0;
+  return b200fa::fwd_f32_workspace_bytes(d->B, d->Hq, d->N, d->S, d->D, d->causal ? 1 : 0, d->window_left);
+}
+
 size_t b200fa_fwd_workspace_bytes(const b200fa_desc* d) {
-  if (!dense_decode_route(d)) return 0;
+  if (!dense_decode_route(d)) return fwd_f32_need(d);
   return b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->S, d->num_splits);
 }
 
@@ -211,7 +218,9 @@ int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const voi
   if (d->kv_lens != nullptr && (d->dtype == B200FA_F32 || !b200fa::fwd_sm100_supported(p, d->dtype, d->D)))
     return fail(B200FA_ERR_UNSUPPORTED, "kv_lens takes f16 / bf16 at head_dim 64 / 128 with positive batch and head strides");
   if (d->dtype == B200FA_F32) {
-    e = b200fa::launch_fwd_f32(p, d->D, false, d->B, d->N, cs);
+    const size_t need = fwd_f32_need(d);
+    const bool given = need > 0 && workspace != nullptr && aligned16(workspace) && workspace_bytes >= need;
+    e = b200fa::launch_fwd_f32(p, d->D, false, d->B, d->N, given ? workspace : nullptr, cs);
   } else if ((d->kv_lens != nullptr || !(d->flags & B200FA_FLAG_FORCE_MMA_SYNC)) && b200fa::fwd_sm100_supported(p, d->dtype, d->D)) {
     e = b200fa::launch_fwd_sm100(p, d->dtype, d->D, d->B, d->N, cs);
   } else {
@@ -318,7 +327,7 @@ int32_t b200fa_fwd_varlen(const b200fa_desc* d, const void* q, const void* k, co
   cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e;
   if (d->dtype == B200FA_F32) {
-    e = b200fa::launch_fwd_f32(p, d->D, true, num_seqs, max_seqlen_q, cs);
+    e = b200fa::launch_fwd_f32(p, d->D, true, num_seqs, max_seqlen_q, nullptr, cs);
   } else if (!(d->flags & B200FA_FLAG_FORCE_MMA_SYNC) && b200fa::fwd_sm100_supported(p, d->dtype, d->D)) {
     e = b200fa::launch_fwd_sm100(p, d->dtype, d->D, num_seqs, max_seqlen_q, cs);
   } else {

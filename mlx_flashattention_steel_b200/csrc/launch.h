@@ -15,7 +15,9 @@ struct BwdParams;
 // dtype codes as in b200fa.h: 0 f16, 1 bf16, 2 f32.
 cudaError_t launch_fwd_mma(const FwdParams& p, int dtype, int D, bool varlen, int nbatch, int max_q,
                            cudaStream_t stream);
-cudaError_t launch_fwd_f32(const FwdParams& p, int D, bool varlen, int nbatch, int max_q,
+// workspace (dense calls; may be null): fwd_f32_workspace_bytes, which lets all SMs share the key tiles evenly
+size_t fwd_f32_workspace_bytes(int B, int Hq, int N, int S, int D, int causal, int window_left);
+cudaError_t launch_fwd_f32(const FwdParams& p, int D, bool varlen, int nbatch, int max_q, void* workspace,
                            cudaStream_t stream);
 
 // tcgen05 / TMEM / TMA forward (dense and packed-varlen layouts, D = 64 or 128, 16-bit).

@@ -492,6 +492,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   } else {
     // ============================ softmax (warps 0-3) ============================
     const int row = q0 + tid;                         // query row of this thread
+    const int w0 = q0 + warp * 32;                    // first query row of this warp
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     constexpr bool BIGCAP = CAPM == 2;
     constexpr bool use_cap = CAPM != 0;
@@ -537,6 +538,34 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int k0 = tile_of(j) * BN;
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_S_FULL + st), (g >> 1) & 1, s_abort))) { ok = false; break; }
       tc_fence_after();
+      // What a mask leaves of the tile is settled per warp (32 rows), not per CTA: of the two 64-key tiles that a causal
+      // diagonal or a window's edge crosses in 128 rows, a warp has one that it crosses, and one that is either all
+      // visible (no masking) or all hidden (P = 0, no exponentials).
+      const bool cut_hi = (k0 + BN > S) || (p.causal && (k0 + BN - 1 > w0 + off));
+      const bool cut_lo = p.window_left >= 0 && (k0 < w0 + 31 + off - p.window_left);
+      bool hidden = w0 >= N || (p.causal && k0 > w0 + 31 + off) || (p.window_left >= 0 && k0 + BN - 1 < w0 + off - p.window_left);
+      unsigned cells = 0xffffffffu;                   // FEAT: set mask cells of this row under the tile
+      bool cells_partial = false;
+      if constexpr (FEAT) {
+        if (sparse) {
+          // fetched one tile ahead, so that the mask bytes' latency hides under the previous tile's work
+          cells = cells_next;
+          cells_partial = __any_sync(0xffffffffu, cells != full_cells);
+          hidden = hidden || !__any_sync(0xffffffffu, cells != 0u);
+          if (j + 1 < n_tiles) cells_next = row_cells(tile_of(j + 1) * BN);
+        }
+      }
+      if (hidden) {
+        uint32_t zero[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) zero[i] = 0u;
+        tmem_st32(tS0 + lane_base + st * 64, zero);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BAR_P_FULL + st));
+        continue;
+      }
       uint32_t r0[32], r1[32];
       tmem_ld32(tS0 + lane_base + st * 64, r0);
       tmem_ld32(tS0 + lane_base + st * 64 + 32, r1);
@@ -545,18 +574,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
       for (int i = 0; i < 32; ++i) { x[i] = __uint_as_float(r0[i]); x[32 + i] = __uint_as_float(r1[i]); }
 
-      unsigned cells = 0xffffffffu;                   // FEAT: set mask cells of this row under the tile
-      bool cells_partial = false;
-      if constexpr (FEAT) {
-        if (sparse) {
-          // fetched one tile ahead, so that the mask bytes' latency hides under the previous tile's work
-          cells = cells_next;
-          cells_partial = __any_sync(0xffffffffu, cells != full_cells);
-          if (j + 1 < n_tiles) cells_next = row_cells(tile_of(j + 1) * BN);
-        }
-      }
-      const bool need_mask = (k0 + BN > S) || (p.causal && (k0 + BN - 1 > q0 + off)) ||
-                             (p.window_left >= 0 && (k0 < q0 + BM - 1 + off - p.window_left)) || cells_partial;
+      const bool need_mask = cut_hi || cut_lo || cells_partial;
       const bool fast = !need_mask && monotone && !(FEAT && p.alibi != nullptr);
       // mode 0: t = x*scale_log2 - m ; 1: softcap by polynomial ; 2: softcap by tanh.approx ; 3: general (masked tile)
       int mode = 3;
@@ -636,28 +654,30 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
         }
         if (need_mask) {
-          // first / last visible column of this row in tile coordinates; a tile usually crosses only one of the
-          // two edges (the diagonal or the end of the keys on the right, the window on the left)
-          const int hi_rel = (p.causal ? min(S - 1, row + off) : S - 1) - k0;
-          const int lo_rel = (p.window_left >= 0 ? row + off - p.window_left : 0) - k0;
-          const bool cut_hi = (k0 + BN > S) || (p.causal && (k0 + BN - 1 > q0 + off));
-          const bool cut_lo = p.window_left >= 0 && (k0 < q0 + BM - 1 + off - p.window_left);
+          // the row's visible columns as 64 bits: those up to the diagonal or the end of the keys, those from the
+          // window's left edge on, those of set mask cells; one select per score applies them all
+          unsigned v0 = 0xffffffffu, v1 = 0xffffffffu;
           if (cut_hi) {
-#pragma unroll
-            for (int i = 0; i < BN; ++i)
-              if (i > hi_rel) x[i] = -INFINITY;
+            const int n = min(max((p.causal ? min(S, row + off + 1) : S) - k0, 0), BN);       // visible from the left
+            v0 = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+            v1 = n >= 64 ? 0xffffffffu : (n <= 32 ? 0u : (1u << (n - 32)) - 1u);
           }
           if (cut_lo) {
-#pragma unroll
-            for (int i = 0; i < BN; ++i)
-              if (i < lo_rel) x[i] = -INFINITY;
+            const int n = min(max(row + off - p.window_left - k0, 0), BN);                    // hidden from the left
+            v0 &= n >= 32 ? 0u : 0xffffffffu << n;
+            v1 &= n >= 64 ? 0u : (n <= 32 ? 0xffffffffu : 0xffffffffu << (n - 32));
           }
           if constexpr (FEAT) {
             if (cells_partial) {
-#pragma unroll
-              for (int i = 0; i < BN; ++i)
-                if (!((cells >> (i >> cell_sh)) & 1u)) x[i] = -INFINITY;
+              auto cell = [&](int c16) -> unsigned { return (cells >> ((c16 << 4) >> cell_sh)) & 1u; };
+              v0 &= (cell(0) ? 0x0000ffffu : 0u) | (cell(1) ? 0xffff0000u : 0u);
+              v1 &= (cell(2) ? 0x0000ffffu : 0u) | (cell(3) ? 0xffff0000u : 0u);
             }
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            x[i] = (v0 & (1u << i)) != 0u ? x[i] : -INFINITY;
+            x[32 + i] = (v1 & (1u << i)) != 0u ? x[32 + i] : -INFINITY;
           }
         }
         m_tile = tree_max64(x);
@@ -673,7 +693,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float m_new = fmaxf(m_used, m_tile);
         const float corr = (m_new == -INFINITY) ? 1.f : fast_exp2(m_used - m_new);
         l_run *= corr;
-        if (j > 0) {
+        if (j > 0 && __any_sync(0xffffffffu, m_new > m_used && m_used != -INFINITY)) {   // a row that saw no key yet has O = 0
           // O is being accumulated by PV(j-1): wait for it, then scale this row in TMEM
           // P.V(j-1): completion (j-1)>>1 of its stage's barrier; the next one there needs this tile's successor's P
           if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_PV_DONE + ((g - 1) & 1)), ((g - 1) >> 1) & 1, s_abort))) { ok = false; break; }

@@ -151,6 +151,22 @@ template <int DT> __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return DT == 0 ? Elem<__half>::pack(a, b) : Elem<__nv_bfloat16>::pack(a, b);
 }
 
+// Bits c < n (n = 1, 2 or 4): mask cell cb0 + c of this mask row is set.  vec: n cells are one aligned load (the row's
+// address and cb0 are multiples of n); else byte by byte, cells from nk on counting as off.
+__device__ __forceinline__ unsigned mask_cells(const uint8_t* row, int cb0, int n, int nk, bool vec) {
+  if (vec) {
+    unsigned w = n == 4 ? __ldg(reinterpret_cast<const uint32_t*>(row + cb0))
+                        : (n == 2 ? __ldg(reinterpret_cast<const uint16_t*>(row + cb0)) : __ldg(row + cb0));
+    w |= w >> 4; w |= w >> 2; w |= w >> 1;                       // bit 0 of every byte: the byte is not zero
+    return ((w & 0x01010101u) * 0x01020408u) >> 24 & 0xfu;       // bits 0, 8, 16, 24 -> 0, 1, 2, 3
+  }
+  unsigned bits = 0u;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (c < n && cb0 + c < nk && row[cb0 + c] != 0) bits |= 1u << c;
+  return bits;
+}
+
 // ---------------------------------------------------------------------------
 // kernel
 // ---------------------------------------------------------------------------
@@ -225,17 +241,21 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (q0 >= N) return;
   }
   const bool sparse = FEAT && p.bmask != nullptr;
+  // mask cells per key tile (cells are 16, 32 or 64 keys wide), and whether those of a tile are one aligned load
+  const int cell_sh = (FEAT && sparse) ? (p.bm_bk == 16 ? 4 : (p.bm_bk == 32 ? 5 : 6)) : 6;
+  const int ncell = BN >> cell_sh;
+  const bool cells_vec = FEAT && sparse && p.bm_nk % ncell == 0 && (reinterpret_cast<uintptr_t>(p.bmask) & (ncell - 1)) == 0;
   if constexpr (FEAT) {
     if (sparse) {
-      // every thread tests key tiles (all mask bytes of a tile are fetched at once: no short-circuit, so the loads
-      // overlap), then warp 0 compacts the tiles that have a set cell under this query tile
+      // every thread tests key tiles, all mask rows of one at once so that the loads overlap; then warp 0 compacts the
+      // tiles that have a set cell under this query tile
       {
         const int rb0 = q0 / p.bm_bq, rb1 = (min(q0 + BM, N) - 1) / p.bm_bq;
         for (int kt = kt_begin + tid; kt < kt_end; kt += kThreads) {
-          const int cb0 = (kt * BN) / p.bm_bk, cb1 = (min((kt + 1) * BN, S) - 1) / p.bm_bk;
           unsigned any = 0u;
+#pragma unroll 4
           for (int rb = rb0; rb <= rb1; ++rb)
-            for (int cb = cb0; cb <= cb1; ++cb) any |= p.bmask[rb * p.bm_nk + cb];
+            any |= mask_cells(p.bmask + static_cast<int64_t>(rb) * p.bm_nk, kt << (6 - cell_sh), ncell, p.bm_nk, cells_vec);
           s_flag[kt - kt_begin] = any != 0u ? 1 : 0;
         }
       }
@@ -515,19 +535,9 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float alibi_l2 = (FEAT && p.alibi != nullptr) ? p.alibi[head] * kLog2e : 0.f;
 
     // FEAT: bit c = mask cell c of this row's block row under the key tile starting at k0
-    // (cells are 16, 32 or 64 keys wide: shifts, and the row's mask line, are worked out once)
-    const int cell_sh = (FEAT && sparse) ? (p.bm_bk == 16 ? 4 : (p.bm_bk == 32 ? 5 : 6)) : 6;
-    const int ncell = BN >> cell_sh;
     const unsigned full_cells = (1u << ncell) - 1u;
     const uint8_t* mask_row = (FEAT && sparse) ? p.bmask + static_cast<int64_t>(min(row, N - 1) / p.bm_bq) * p.bm_nk : nullptr;
-    auto row_cells = [&](int k0) -> unsigned {
-      const int cb0 = k0 >> cell_sh;
-      unsigned c4 = 0u;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (c < ncell && cb0 + c < p.bm_nk && mask_row[cb0 + c] != 0) c4 |= 1u << c;
-      return c4;
-    };
+    auto row_cells = [&](int k0) -> unsigned { return mask_cells(mask_row, k0 >> cell_sh, ncell, p.bm_nk, cells_vec); };
     unsigned cells_next = 0xffffffffu;
     if constexpr (FEAT) {
       if (sparse) cells_next = row_cells(tile_of(0) * BN);

@@ -80,6 +80,10 @@ def flash_attention_sparse(q, k, v, block_mask, scale: Optional[float] = None, c
     if k.shape[1] != H and H % k.shape[1] != 0:
         raise ValueError(f"flash_attention GQA: q_heads ({H}) must be divisible by kv_heads ({k.shape[1]}).")
     _require_cuda(q, k, v, block_mask)
-    bm = (block_mask != 0).to(torch.uint8).contiguous()
+    needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
+    if block_mask.dtype == torch.bool and not needs_grad:
+        bm = block_mask.contiguous().view(torch.uint8)       # one byte a cell already
+    else:
+        bm = (block_mask != 0).to(torch.uint8).contiguous()  # a backward reads it later: a copy that nobody writes to
     out, _ = _FlashAttnFn.apply(q, k, v, float(scale), bool(causal), 0.0, -1, False, stream, None, (bm, BQ, BK))
     return out

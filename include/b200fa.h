@@ -317,6 +317,15 @@ int32_t b200fa_rope(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, i
                     void* stream);
 
 /*
+ * The same with the positions in host memory: host_offsets [B], B at most 512, read before the call returns and sent
+ * with the launch (nothing is copied, nothing waits).  Every host_offsets[b] must be in [0, max_pos - N].
+ */
+int32_t b200fa_rope_host_offsets(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, int32_t rotary_dim,
+                                 int32_t interleaved, int32_t inverse, const void* x, const int64_t* x_strides, void* out,
+                                 const int64_t* out_strides, const float* cos_table, const float* sin_table, int32_t max_pos,
+                                 const int32_t* host_offsets, void* stream);
+
+/*
  * Reads and clears the library-wide device status word of the tcgen05 kernels
  * (forward, backward): 0 = ok, bit 0 = a bounded mbarrier wait inside a kernel
  * gave up after about a second (its outputs are then undefined).  Waits for

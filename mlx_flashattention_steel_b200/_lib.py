@@ -98,6 +98,7 @@ SIGNATURES = {
     "b200fa_paged_kv_scatter_add": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
     "b200fa_kv_append": (_I, [_I, _I, _I, _I, _I, _I, C.c_int64, _P, _P, C.c_int64, C.c_int64, _P, _P, _P, _P, _P, _P]),
     "b200fa_rope": (_I, [_I, _I, _I, _I, _I, _I, _I, _I, _P, C.POINTER(C.c_int64), _P, C.POINTER(C.c_int64), _P, _P, _I, _P, _I, _P]),
+    "b200fa_rope_host_offsets": (_I, [_I, _I, _I, _I, _I, _I, _I, _I, _P, C.POINTER(C.c_int64), _P, C.POINTER(C.c_int64), _P, _P, _I, C.POINTER(C.c_int32), _P]),
     "b200fa_kernel_status": (_I, [_P, C.POINTER(C.c_int32)]),
     "b200fa_workspace_status": (_I, [_P, _P, C.POINTER(C.c_int32)]),
     "b200fa_paged_kv_gather": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P]),

@@ -510,10 +510,10 @@ int32_t b200fa_kv_append(int32_t src_dtype, int32_t pool_dtype, int32_t T, int32
   return B200FA_OK;
 }
 
-int32_t b200fa_rope(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, int32_t rotary_dim, int32_t interleaved,
-                    int32_t inverse, const void* x, const int64_t* x_strides, void* out, const int64_t* out_strides,
-                    const float* cos_table, const float* sin_table, int32_t max_pos, const int32_t* offsets, int32_t offset,
-                    void* stream) {
+static int32_t rope_common(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, int32_t rotary_dim, int32_t interleaved,
+                           int32_t inverse, const void* x, const int64_t* x_strides, void* out, const int64_t* out_strides,
+                           const float* cos_table, const float* sin_table, int32_t max_pos, const int32_t* offsets,
+                           const int32_t* host_offsets, int32_t offset, void* stream) {
   if (dtype != B200FA_F16 && dtype != B200FA_BF16) return fail(B200FA_ERR_UNSUPPORTED, "rope: f16 / bf16 only");
   if (B < 0 || H <= 0 || N < 0 || D <= 0 || D % 8 != 0) return fail(B200FA_ERR_INVALID_ARG, "rope: bad extent (D must be a multiple of 8)");
   if (rotary_dim <= 0 || rotary_dim > D || rotary_dim % 2 != 0)
@@ -526,13 +526,36 @@ int32_t b200fa_rope(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, i
   if (!aligned16(x) || !aligned16(out)) return fail(B200FA_ERR_INVALID_ARG, "rope: x and out must be 16-byte aligned");
   for (int i = 0; i < 3; ++i)
     if (x_strides[i] % 8 != 0 || out_strides[i] % 8 != 0) return fail(B200FA_ERR_INVALID_ARG, "rope: strides must be multiples of 8 elements");
-  if (offsets == nullptr && (offset < 0 || static_cast<int64_t>(offset) + N > max_pos))
+  if (host_offsets != nullptr) {
+    if (B > b200fa::kRopeHostOffsets)
+      return fail(B200FA_ERR_UNSUPPORTED, "rope: %d offsets from the host, at most %d travel with a launch", B, b200fa::kRopeHostOffsets);
+    for (int b = 0; b < B; ++b)
+      if (host_offsets[b] < 0 || static_cast<int64_t>(host_offsets[b]) + N > max_pos)
+        return fail(B200FA_ERR_INVALID_ARG, "rope: positions [%d, %d) exceed the table's %d rows", host_offsets[b], host_offsets[b] + N, max_pos);
+  } else if (offsets == nullptr && (offset < 0 || static_cast<int64_t>(offset) + N > max_pos))
     return fail(B200FA_ERR_INVALID_ARG, "rope: positions [%d, %d) exceed the table's %d rows", offset, offset + N, max_pos);
-  cudaError_t e = b200fa::launch_rope(dtype, x, out, cos_table, sin_table, offsets, offset, B, H, N, D, rotary_dim,
+  cudaError_t e = b200fa::launch_rope(dtype, x, out, cos_table, sin_table, offsets, host_offsets, offset, B, H, N, D, rotary_dim,
                                       interleaved ? 1 : 0, inverse ? 1 : 0, x_strides, out_strides,
                                       reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "rope launch");
   return B200FA_OK;
+}
+
+int32_t b200fa_rope(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, int32_t rotary_dim, int32_t interleaved,
+                    int32_t inverse, const void* x, const int64_t* x_strides, void* out, const int64_t* out_strides,
+                    const float* cos_table, const float* sin_table, int32_t max_pos, const int32_t* offsets, int32_t offset,
+                    void* stream) {
+  return rope_common(dtype, B, H, N, D, rotary_dim, interleaved, inverse, x, x_strides, out, out_strides, cos_table, sin_table,
+                     max_pos, offsets, nullptr, offset, stream);
+}
+
+int32_t b200fa_rope_host_offsets(int32_t dtype, int32_t B, int32_t H, int32_t N, int32_t D, int32_t rotary_dim,
+                                 int32_t interleaved, int32_t inverse, const void* x, const int64_t* x_strides, void* out,
+                                 const int64_t* out_strides, const float* cos_table, const float* sin_table, int32_t max_pos,
+                                 const int32_t* host_offsets, void* stream) {
+  if (B > 0 && N > 0 && host_offsets == nullptr) return fail(B200FA_ERR_INVALID_ARG, "rope: null pointer");
+  return rope_common(dtype, B, H, N, D, rotary_dim, interleaved, inverse, x, x_strides, out, out_strides, cos_table, sin_table,
+                     max_pos, nullptr, host_offsets, 0, stream);
 }
 
 int32_t b200fa_kernel_status(void* stream, int32_t* status_out) {

@@ -58,9 +58,11 @@ cudaError_t launch_paged_scatter_add(const void* grad, const int32_t* block_tabl
                                      int D, int dtype, int block_size, int max_blocks, int max_kv_len, void* grad_pool,
                                      cudaStream_t stream);
 
-// Rotary embedding pass (rope.cu).  xs / os: batch, head, row strides in elements; offsets (device, [B]) or one offset.
+// Rotary embedding pass (rope.cu).  xs / os: batch, head, row strides in elements; offsets (device, [B]), host_offsets
+// (host, [B], B <= kRopeHostOffsets) or one offset.
+constexpr int kRopeHostOffsets = 512;
 cudaError_t launch_rope(int dtype, const void* x, void* out, const float* cosb, const float* sinb, const int* offsets,
-                        int offset, int B, int H, int N, int D, int rot, int interleaved, int inverse, const int64_t* xs,
+                        const int* host_offsets, int offset, int B, int H, int N, int D, int rot, int interleaved, int inverse, const int64_t* xs,
                         const int64_t* os, cudaStream_t stream);
 
 // Read (and clear when set) the device status word of the tcgen05 kernels of each file; they wait for `stream`.

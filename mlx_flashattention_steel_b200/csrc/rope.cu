@@ -9,8 +9,13 @@
 //   pos = offset(batch) + row;  elements d >= rot pass through;  `inverse` flips the sign of sin (the transpose of
 //   the rotation, which is what the backward pass applies to the gradients).
 //
+// Positions that the host knows (a scheduler's list) travel in the launch's parameters: copying them to the device first
+// cost a decode step of 8 sequences two synchronising 32-byte copies, more than everything else it did.
+//
 // One thread per 16-byte chunk (8 values); in split-half mode a thread owns a chunk of the first half and its
 // partner chunk, so an in-place call never reads what another thread writes.  float32 arithmetic, one rounding.
+#include <type_traits>
+
 #include "common.cuh"
 #include "launch.h"
 
@@ -18,13 +23,23 @@ namespace b200fa {
 
 namespace {
 
+struct HostOffsets {
+  int v[kRopeHostOffsets];
+};
+struct NoHostOffsets {};
+__device__ __forceinline__ int offset_of(const HostOffsets& ho, const int*, int, int b) { return ho.v[b]; }
+__device__ __forceinline__ int offset_of(const NoHostOffsets&, const int* offsets, int offset, int b) {
+  return offsets != nullptr ? offsets[b] : offset;
+}
+
+// HO: positions in the launch's parameters, or none there
 // I: index type of the flattened (batch, head, row, chunk) space: 32-bit whenever it fits, because the index is split by
 // run-time divisors for every 16-byte chunk and a 64-bit division costs several times the rest of the work
-template <typename T, typename I>
+template <typename T, typename I, typename HO>
 __global__ void __launch_bounds__(256)
 rope_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cosb, const float* __restrict__ sinb,
             const int* __restrict__ offsets, int offset, int B, int H, int N, int D, int rot, int interleaved, int inverse,
-            int64_t x_bs, int64_t x_hs, int64_t x_rs, int64_t o_bs, int64_t o_hs, int64_t o_rs) {
+            int64_t x_bs, int64_t x_hs, int64_t x_rs, int64_t o_bs, int64_t o_hs, int64_t o_rs, const __grid_constant__ HO ho) {
   const int half = rot >> 1;
   // chunks a thread may own per row: all D/8 (interleaved); first-half chunks + pass-through chunks (split halves)
   const int rot_chunks = rot >> 3, half_chunks = half >> 3, tail_chunks = (D - rot) >> 3;
@@ -39,7 +54,7 @@ rope_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restric
     const int h = static_cast<int>(r % static_cast<I>(H)), b = static_cast<int>(r / static_cast<I>(H));
     const T* xr = x + b * x_bs + h * x_hs + static_cast<int64_t>(n) * x_rs;
     T* orow = out + b * o_bs + h * o_hs + static_cast<int64_t>(n) * o_rs;
-    const int pos = (offsets != nullptr ? offsets[b] : offset) + n;
+    const int pos = offset_of(ho, offsets, offset, b) + n;
     const float* cr = cosb + static_cast<int64_t>(pos) * half;
     const float* sr = sinb + static_cast<int64_t>(pos) * half;
     const float sgn = inverse ? -1.f : 1.f;
@@ -87,23 +102,36 @@ rope_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restric
 }  // namespace
 
 cudaError_t launch_rope(int dtype, const void* x, void* out, const float* cosb, const float* sinb, const int* offsets,
-                        int offset, int B, int H, int N, int D, int rot, int interleaved, int inverse, const int64_t* xs,
-                        const int64_t* os, cudaStream_t stream) {
+                        const int* host_offsets, int offset, int B, int H, int N, int D, int rot, int interleaved, int inverse,
+                        const int64_t* xs, const int64_t* os, cudaStream_t stream) {
   const int per_row = interleaved ? D / 8 : (rot / 16 + (D - rot) / 8);
   const int64_t total = static_cast<int64_t>(B) * H * N * per_row;
   if (total <= 0) return cudaSuccess;
   const int64_t want = (total + 255) / 256;
   const unsigned grid = static_cast<unsigned>(want < 148 * 16 ? want : 148 * 16);
   const bool small = total < (1LL << 31);
-#define B200FA_ROPE_LAUNCH(T, I)                                                                                         \
-  rope_kernel<T, I><<<grid, 256, 0, stream>>>(static_cast<const T*>(x), static_cast<T*>(out), cosb, sinb, offsets, offset, B, \
-                                              H, N, D, rot, interleaved, inverse, xs[0], xs[1], xs[2], os[0], os[1], os[2])
-  if (dtype == 0) {
-    if (small) B200FA_ROPE_LAUNCH(__half, uint32_t); else B200FA_ROPE_LAUNCH(__half, int64_t);
+  auto go = [&](const auto& ho) {
+    using HO = std::decay_t<decltype(ho)>;
+    auto launch = [&](auto kern, auto* xt, auto* ot) {
+      kern<<<grid, 256, 0, stream>>>(xt, ot, cosb, sinb, offsets, offset, B, H, N, D, rot, interleaved, inverse, xs[0], xs[1],
+                                     xs[2], os[0], os[1], os[2], ho);
+    };
+    if (dtype == 0) {
+      if (small) launch(rope_kernel<__half, uint32_t, HO>, static_cast<const __half*>(x), static_cast<__half*>(out));
+      else launch(rope_kernel<__half, int64_t, HO>, static_cast<const __half*>(x), static_cast<__half*>(out));
+    } else {
+      if (small) launch(rope_kernel<__nv_bfloat16, uint32_t, HO>, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out));
+      else launch(rope_kernel<__nv_bfloat16, int64_t, HO>, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out));
+    }
+  };
+  if (host_offsets != nullptr) {
+    if (B > kRopeHostOffsets) return cudaErrorInvalidValue;
+    HostOffsets ho;
+    for (int b = 0; b < kRopeHostOffsets; ++b) ho.v[b] = b < B ? host_offsets[b] : 0;
+    go(ho);
   } else {
-    if (small) B200FA_ROPE_LAUNCH(__nv_bfloat16, uint32_t); else B200FA_ROPE_LAUNCH(__nv_bfloat16, int64_t);
+    go(NoHostOffsets{});
   }
-#undef B200FA_ROPE_LAUNCH
   return cudaGetLastError();
 }
 

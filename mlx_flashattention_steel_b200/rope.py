@@ -53,25 +53,29 @@ def make_rope_3d_tables(grid_h: int, grid_w: int, num_frames: int, d_h: Optional
     return cos, sin
 
 
+_HOST_OFFSETS = 512     # as many positions travel in the parameters of a launch
+
+
 def _rope_raw(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, offset, interleaved: bool, rot: int, inverse: bool,
               stream, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     B, H, N, D = x.shape
     if out is None:
         out = torch.empty((B, H, N, D), dtype=x.dtype, device=x.device)
-    offs_t, offs_i = None, 0
-    if isinstance(offset, torch.Tensor):
-        offs_t = offset.to(device=x.device, dtype=torch.int32).contiguous()
-        if offs_t.numel() != B:
-            raise ValueError(f"cache_seqlens length {offs_t.numel()} must equal batch size B={B}")
-    else:
-        offs_i = int(offset)
     xs = (C.c_int64 * 3)(*x.stride()[:3])
     os_ = (C.c_int64 * 3)(*out.stride()[:3])
     lib = _lib.load()
-    st = lib.b200fa_rope(_DTYPE_CODE[x.dtype], B, H, N, D, rot, 1 if interleaved else 0, 1 if inverse else 0,
-                         C.c_void_p(x.data_ptr()), xs, C.c_void_p(out.data_ptr()), os_, C.c_void_p(cos.data_ptr()),
-                         C.c_void_p(sin.data_ptr()), cos.shape[0], None if offs_t is None else C.c_void_p(offs_t.data_ptr()),
-                         offs_i, C.c_void_p(_stream_ptr(stream, x.device)))
+    head = (_DTYPE_CODE[x.dtype], B, H, N, D, rot, 1 if interleaved else 0, 1 if inverse else 0, C.c_void_p(x.data_ptr()), xs,
+            C.c_void_p(out.data_ptr()), os_, C.c_void_p(cos.data_ptr()), C.c_void_p(sin.data_ptr()), cos.shape[0])
+    sp = C.c_void_p(_stream_ptr(stream, x.device))
+    if isinstance(offset, tuple) and len(offset) <= _HOST_OFFSETS:
+        # positions the host knows go with the launch: no copy, no synchronisation
+        st = lib.b200fa_rope_host_offsets(*head, (C.c_int32 * B)(*offset), sp)
+    elif isinstance(offset, int):
+        st = lib.b200fa_rope(*head, None, offset, sp)
+    else:
+        offs = torch.tensor(offset, dtype=torch.int32) if isinstance(offset, tuple) else offset
+        offs = offs.to(device=x.device, dtype=torch.int32).contiguous()
+        st = lib.b200fa_rope(*head, C.c_void_p(offs.data_ptr()), 0, sp)
     _lib.check(st, "apply_rope")
     return out
 
@@ -114,16 +118,17 @@ def apply_rope(x, cos, sin, offset: Union[int, Sequence[int], torch.Tensor] = 0,
     N = x.shape[2]
     if isinstance(offset, torch.Tensor) and offset.ndim == 0:
         offset = int(offset)
-    if not isinstance(offset, (int, torch.Tensor)):
-        offset = [int(o) for o in offset]
+    if isinstance(offset, torch.Tensor) and offset.is_cuda:
+        if int(offset.min()) < 0 or int(offset.max()) + N > cos.shape[0]:
+            raise ValueError(f"positions exceed the rotary table's {cos.shape[0]} rows.")
+        if offset.numel() != x.shape[0]:
+            raise ValueError(f"cache_seqlens length {offset.numel()} must equal batch size B={x.shape[0]}")
+    elif not isinstance(offset, int):
+        offset = tuple(int(o) for o in (offset.reshape(-1).tolist() if isinstance(offset, torch.Tensor) else offset))
         if len(offset) != x.shape[0]:
             raise ValueError(f"cache_seqlens length {len(offset)} must equal batch size B={x.shape[0]}")
         if offset and (min(offset) < 0 or max(offset) + N > cos.shape[0]):
             raise ValueError(f"positions up to {max(offset) + N} exceed the rotary table's {cos.shape[0]} rows.")
-        offset = torch.tensor(offset, dtype=torch.int32)
-    elif isinstance(offset, torch.Tensor):
-        if int(offset.min()) < 0 or int(offset.max()) + N > cos.shape[0]:
-            raise ValueError(f"positions exceed the rotary table's {cos.shape[0]} rows.")
     ok = x.stride(-1) == 1 and all(s % 8 == 0 for s in x.stride()[:3]) and x.data_ptr() % 16 == 0
     if not ok:
         x = x.contiguous()

@@ -234,6 +234,16 @@ int32_t b200fa_paged_kv_gather_dequant(const void* pool, const void* scale, cons
                                        void* out, void* stream);
 
 /*
+ * K and V of 8-bit pools in one launch, as b200fa_fwd with desc.kv_lens reads them: k_out / v_out [B, H, max_kv_len, D]
+ * f16 / bf16.  Written are the rows up to the end of the 64-key tile in which sequence b ends (zeros beyond seq_lens[b],
+ * and for table entries that are negative or beyond num_pages); the rows after it are left as they are.
+ */
+int32_t b200fa_paged_kv_dequant_pair(const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale,
+                                     const int32_t* block_table, const int32_t* seq_lens, int32_t B, int32_t H, int32_t D,
+                                     int32_t pool_dtype, int32_t out_dtype, int32_t num_pages, int32_t block_size,
+                                     int32_t max_blocks, int32_t max_kv_len, void* k_out, void* v_out, void* stream);
+
+/*
  * Paged decode for callers that cannot give it a workspace.  Same arguments and
  * result as b200fa_decode_paged minus the workspace pair.  It has no counterpart in
  * the reference, whose primitives get their scratch from MLX's allocator.

@@ -94,6 +94,7 @@ SIGNATURES = {
     "b200fa_combine_partials": (_I, [_P, _I, C.c_int64, _I, _I, _P, _P, _P]),
     "b200fa_fwd_paged": (_I, [_DP, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "b200fa_paged_kv_gather_dequant": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
+    "b200fa_paged_kv_dequant_pair": (_I, [_P] * 6 + [_I] * 9 + [_P, _P, _P]),
     "b200fa_decode_paged_static_status": (_I, [_P, C.POINTER(C.c_int32)]),
     "b200fa_paged_kv_scatter_add": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
     "b200fa_kv_append": (_I, [_I, _I, _I, _I, _I, _I, C.c_int64, _P, _P, C.c_int64, C.c_int64, _P, _P, _P, _P, _P, _P]),

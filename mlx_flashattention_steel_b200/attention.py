@@ -549,6 +549,23 @@ def paged_kv_gather_dequant(pool, scale, block_table, seq_lens, max_kv_len: int,
     return out
 
 
+def _dequant_pair(k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, out_dtype, stream):
+    """K and V of 8-bit pools as `_fwd_raw(..., kv_lens=lens)` reads them: gathered and dequantised in one launch, rows
+    beyond the 64-key tile in which a sequence ends left uninitialised."""
+    _require_cuda(k_pages, v_pages, k_scale, v_scale, table, lens)
+    lib = _lib.load()
+    num_pages, bs, H, D = k_pages.shape
+    B, max_blocks = table.shape
+    K = torch.empty((B, H, max_kv_len, D), dtype=out_dtype, device=k_pages.device)
+    V = torch.empty_like(K)
+    with torch.cuda.device(k_pages.device):
+        st = lib.b200fa_paged_kv_dequant_pair(_ptr(k_pages), _ptr(v_pages), _ptr(k_scale), _ptr(v_scale), _ptr(table), _ptr(lens),
+                                              B, H, D, _KV_CODE[k_pages.dtype], _DTYPE_CODE[out_dtype], num_pages, bs, max_blocks,
+                                              max_kv_len, _ptr(K), _ptr(V), C.c_void_p(_stream_ptr(stream, k_pages.device)))
+    _lib.check(st, "flash_attention_paged")
+    return K, V
+
+
 _CHECK_DECODE_STATUS = False   # tests switch this on: one stream sync per call
 
 
@@ -702,8 +719,7 @@ def flash_attention_paged(
         # dtype in one pass (the reference's dense-dequant path), then the dense kernel runs with per-sequence key
         # counts -- where the reference slices and launches per sequence (mlx_mfa/attention.py:2950-2989).
         if quant:
-            K = paged_kv_gather_dequant(k_pages, k_scale, table, lens, int(max_kv_len), q.dtype, stream)
-            V = paged_kv_gather_dequant(v_pages, v_scale, table, lens, int(max_kv_len), q.dtype, stream)
+            K, V = _dequant_pair(k_pages, v_pages, k_scale, v_scale, table, lens, int(max_kv_len), q.dtype, stream)
             out, lse = _fwd_raw(q, K, V, float(scale), bool(causal), float(softcap), -1, return_lse, stream, kv_lens=lens)
         else:
             out, lse = _fwd_paged_raw(q, k_pages, v_pages, table, lens, max_kv_len, float(scale), bool(causal),

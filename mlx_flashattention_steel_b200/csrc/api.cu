@@ -299,6 +299,30 @@ int32_t b200fa_paged_kv_gather_dequant(const void* pool, const void* scale, cons
   return B200FA_OK;
 }
 
+int32_t b200fa_paged_kv_dequant_pair(const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale,
+                                     const int32_t* block_table, const int32_t* seq_lens, int32_t B, int32_t H, int32_t D,
+                                     int32_t pool_dtype, int32_t out_dtype, int32_t num_pages, int32_t block_size,
+                                     int32_t max_blocks, int32_t max_kv_len, void* k_out, void* v_out, void* stream) {
+  if (B < 0 || H <= 0 || D <= 0 || block_size <= 0 || max_blocks < 0 || max_kv_len < 0 || num_pages < 0)
+    return fail(B200FA_ERR_INVALID_ARG, "bad extent");
+  if (pool_dtype != B200FA_I8 && pool_dtype != B200FA_E4M3) return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: pools must be int8 or e4m3");
+  if (out_dtype != B200FA_F16 && out_dtype != B200FA_BF16) return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: output must be f16 or bf16");
+  if (D % 16 != 0) return fail(B200FA_ERR_INVALID_ARG, "D must be a multiple of 16");
+  if (static_cast<int64_t>(num_pages) * block_size >= (1LL << 31)) return fail(B200FA_ERR_UNSUPPORTED, "pool of 2^31 tokens or more");
+  if (B > 65535 || static_cast<int64_t>(H) * D > (1 << 24)) return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: B beyond 65535 or rows beyond 2^24 values");
+  if (B == 0 || max_kv_len == 0) return B200FA_OK;
+  if (!k_pool || !v_pool || !k_scale || !v_scale || !block_table || !seq_lens || !k_out || !v_out) return fail(B200FA_ERR_INVALID_ARG, "null pointer");
+  if (!aligned16(k_pool) || !aligned16(v_pool) || !aligned16(k_out) || !aligned16(v_out))
+    return fail(B200FA_ERR_INVALID_ARG, "pools and outputs must be 16-byte aligned");
+  if (static_cast<int64_t>(max_blocks) * block_size < max_kv_len)
+    return fail(B200FA_ERR_INVALID_ARG, "max_kv_len %d exceeds max_blocks*block_size", max_kv_len);
+  cudaError_t e = b200fa::launch_paged_dequant_pair(k_pool, v_pool, k_scale, v_scale, block_table, seq_lens, B, H, D, pool_dtype,
+                                                    out_dtype, num_pages, block_size, max_blocks, max_kv_len, k_out, v_out,
+                                                    reinterpret_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "dequant_pair launch");
+  return B200FA_OK;
+}
+
 size_t b200fa_fwd_varlen_workspace_bytes(const b200fa_desc* d, int32_t num_seqs, int32_t max_seqlen_q,
                                          int32_t max_seqlen_k) {
   (void)d; (void)num_seqs; (void)max_seqlen_q; (void)max_seqlen_k;

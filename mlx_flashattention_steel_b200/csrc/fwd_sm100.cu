@@ -236,8 +236,20 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   };
   const bool paged = p.block_table != nullptr;
   if constexpr (!PERSIST) {
-    item_geometry(static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), static_cast<int>(blockIdx.z),
-                  static_cast<int>(gridDim.x));
+    int z = static_cast<int>(blockIdx.z);
+    // Batch entries of their own key counts: the longest first, so that the last CTAs to run are short (4 entries of
+    // 1000 to 8000 keys, 512 queries, 32 heads: 169 us in the order they come).  Each warp ranks up to 32 of them.
+    if (p.kv_lens != nullptr && gridDim.z > 1 && gridDim.z <= 32) {
+      const int nz = static_cast<int>(gridDim.z);
+      const int mine = lane < nz ? p.kv_lens[lane] : -1;
+      int rank = 0;
+      for (int i = 0; i < nz; ++i) {
+        const int other = __shfl_sync(0xffffffffu, mine, i);
+        if (other > mine || (other == mine && i < lane)) ++rank;
+      }
+      z = __ffs(__ballot_sync(0xffffffffu, lane < nz && rank == z)) - 1;
+    }
+    item_geometry(static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), z, static_cast<int>(gridDim.x));
     if (q0 >= N) return;
   }
   const bool sparse = FEAT && p.bmask != nullptr;

@@ -28,6 +28,11 @@ cudaError_t launch_fwd_sm100(const FwdParams& p, int dtype, int D, int nbatch, i
 cudaError_t launch_paged_gather_dequant(const void* pool, const void* scale, const int32_t* block_table,
                                         const int32_t* seq_lens, int B, int H, int D, int pool_dtype, int out_dtype,
                                         int block_size, int max_blocks, int max_kv_len, void* out, cudaStream_t stream);
+// K and V in one launch; rows beyond the 64-key tile in which a sequence ends are left as they are
+cudaError_t launch_paged_dequant_pair(const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale,
+                                      const int32_t* block_table, const int32_t* seq_lens, int B, int H, int D, int pool_dtype,
+                                      int out_dtype, int num_pages, int block_size, int max_blocks, int max_kv_len, void* k_out,
+                                      void* v_out, cudaStream_t stream);
 cudaError_t launch_paged_gather(const void* pool, const int32_t* block_table, const int32_t* seq_lens,
                                 int B, int H, int D, int elem_bytes, int block_size, int max_blocks,
                                 int max_kv_len, void* out, cudaStream_t stream);

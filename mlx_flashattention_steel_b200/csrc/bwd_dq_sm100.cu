@@ -80,6 +80,7 @@ enum Bar {
 struct DqArgs {
   BwdParams p;
   int tma_store;
+  int gx, pairs, group;      // items (query tile, query head of a batch entry | sequence) and their order: item_of
 };
 
 template <int DT> __device__ __forceinline__ uint32_t pack16q(float a, float b) {
@@ -105,8 +106,10 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const BwdParams& p = a.p;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int head = blockIdx.y;
-  int batch = blockIdx.z;
+  int tile, pair;
+  item_of(static_cast<int>(blockIdx.x), a.gx, a.pairs, a.group, tile, pair);
+  const int head = pair % p.Hq;
+  int batch = pair / p.Hq;
   const int kvh = head / p.gqa;
   int N = p.N, S = p.S, q_begin = 0, k_begin = 0;
   if (p.cu_q != nullptr) {
@@ -116,7 +119,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     S = p.cu_k[batch + 1] - k_begin;
     batch = 0;
   }
-  const int q0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * BM;   // heavy (late) tiles first
+  const int q0 = (a.gx - 1 - tile) * BM;                    // heavy (late) tiles first
   if (q0 >= N) return;
   const int off = S - N;
   int k_hi = S;
@@ -539,7 +542,13 @@ cudaError_t launch_bwd_dq_sm100(const BwdParams& p, int dtype, int nbatch, int m
   a.p = p;
   a.tma_store = (p.cu_q == nullptr && make_map128(&tmDQ, dtype, p.dq, p.N, p.Hq, p.B, p.dq_rs, fix(p.dq_hs, 1), fix(p.dq_bs, 1), BM)) ? 1 : 0;
   if (!a.tma_store) tmDQ = tmQ;
-  dim3 grid((max_q + BM - 1) / BM, p.Hq, nbatch);
+  a.gx = (max_q + BM - 1) / BM;
+  const long long pairs = static_cast<long long>(p.Hq) * nbatch, items = pairs * a.gx;
+  if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
+  a.pairs = static_cast<int>(pairs);
+  // an item streams K and V, which the query heads of a group share
+  a.group = p.cu_q != nullptr ? 1 : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, pairs);
+  dim3 grid(static_cast<unsigned>(items), 1, 1);
   auto launch = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;

@@ -61,7 +61,8 @@ enum Bar { BAR_KV = 0, BAR_Q_FULL = 2, BAR_Q_EMPTY = 4, BAR_ST_DONE = 6 /* + hal
 struct BwdArgs {
   BwdParams p;
   int dtype;
-  int gx, gy, total_items;      // work items: (key tile, kv head, batch | sequence), key tile fastest
+  int gx, gy, total_items;      // work items: (key tile, kv head, batch | sequence)
+  int group;                    // their order: item_of
   int* counter;                 // next work item (zeroed by the preprocess kernel)
 };
 
@@ -133,7 +134,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int tries = 0; tries < (1 << 24); ++tries) {
       const int idx = atomicAdd(a.counter, 1);
       if (idx >= a.total_items) break;
-      const int kt = idx % a.gx, kvh_ = (idx / a.gx) % a.gy, z = idx / (a.gx * a.gy);
+      int kt, pair;
+      item_of(idx, a.gx, a.total_items / a.gx, a.group, kt, pair);
+      const int kvh_ = pair % a.gy, z = pair / a.gy;
       int kb = 0, S_ = p.S, qb = 0, N_ = p.N;
       if (p.cu_k != nullptr) {
         kb = p.cu_k[z];
@@ -658,6 +661,8 @@ cudaError_t launch_bwd_sm100_main(const BwdParams& p, int dtype, int nbatch, int
   const long long items = static_cast<long long>(a.gx) * a.gy * nbatch;
   if (items > 0x7fffffffLL || p.work_counter == nullptr) return cudaErrorInvalidValue;
   a.total_items = static_cast<int>(items);
+  // an item streams Q and dO of one query head at a time; packed sequences are many and short enough
+  a.group = p.cu_q != nullptr ? 1 : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.N) * HD * 4, items / a.gx);
   a.counter = p.work_counter;
   static int sm_count = 0;
   if (sm_count == 0) {

@@ -78,7 +78,8 @@ enum Bar {
 struct Sm100Args {
   FwdParams p;
   int tma_store;             // dense layout: O leaves through shared memory and TMA stores
-  int gx, gy, total_items;   // persistent CTAs: items = (query tile, head, batch | sequence), query tile fastest
+  int gx, gy, total_items;   // items = (query tile, head, batch | sequence); persistent CTAs: query tile fastest
+  int group;                 // > 1: one item per CTA, a linear grid in the order of item_of
 };
 
 // max / min of 64 values as a 3-ary tree (depth 4) instead of a 63-deep dependent chain
@@ -249,7 +250,14 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       z = __ffs(__ballot_sync(0xffffffffu, lane < nz && rank == z)) - 1;
     }
-    item_geometry(static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), z, static_cast<int>(gridDim.x));
+    int xt = static_cast<int>(blockIdx.x), h = static_cast<int>(blockIdx.y);
+    if (a.group > 1) {
+      int pair;
+      item_of(static_cast<int>(blockIdx.x), a.gx, a.total_items / a.gx, a.group, xt, pair);
+      h = pair % a.gy;
+      z = pair / a.gy;
+    }
+    item_geometry(xt, h, z, a.gx);
     if (q0 >= N) return;
   }
   const bool sparse = FEAT && p.bmask != nullptr;
@@ -1009,6 +1017,11 @@ static cudaError_t launch_hd(const FwdParams& p, int nbatch, int max_q, cudaStre
                        : (capm == 1 ? launch_p(fa_fwd_sm100_kernel<HD, DT, false, true, 1>) : launch_p(fa_fwd_sm100_kernel<HD, DT, false, true, 0>));
     }
   }
+  // dense calls with a common key count (others: longest batch entry first, see the kernel)
+  a.group = 1;
+  if (p.cu_q == nullptr && p.kv_lens == nullptr && !FEAT && items < 0x7fffffffLL)
+    a.group = order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, items / grid.x);
+  if (a.group > 1) grid = dim3(static_cast<unsigned>(items), 1, 1);
   auto launch_1 = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;

@@ -127,6 +127,8 @@ int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const voi
  * MFAVarlenAttention::eval_gpu (csrc/mfa_attention.cpp:1228-1305).
  * cu_seqlens_* are device int32 [num_seqs+1]; max_seqlen_* are host ints
  * (the reference front end passes them the same way, mlx_mfa/attention.py:2399-2400).
+ * The workspace (f16 / bf16; may be NULL) lets the CTAs take their work from a counter.  With it, and only then, rows of
+ * out and lse that belong to no sequence are set to zero; without it they are left as they are.
  */
 size_t  b200fa_fwd_varlen_workspace_bytes(const b200fa_desc* d, int32_t num_seqs,
                                           int32_t max_seqlen_q, int32_t max_seqlen_k);

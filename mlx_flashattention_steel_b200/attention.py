@@ -96,6 +96,20 @@ def _stream_ptr(stream, device) -> int:
     raise TypeError("stream must be None, a torch.cuda.Stream or a raw cudaStream_t integer")
 
 
+def _scratch(nbytes: int, device, stream) -> torch.Tensor:
+    """Scratch of one launch.  It goes back to the allocator when the call returns, so a launch on another stream than the
+    current one is recorded on it."""
+    return _used_on(torch.empty(nbytes, dtype=torch.uint8, device=device), stream)
+
+
+def _used_on(t: torch.Tensor, stream) -> torch.Tensor:
+    if stream is not None:
+        s = stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream, device=t.device)
+        if s.cuda_stream != torch.cuda.current_stream(t.device).cuda_stream:
+            t.record_stream(s)
+    return t
+
+
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else C.c_void_p(t.data_ptr())
 
@@ -164,7 +178,7 @@ def _fwd_raw(q, k, v, scale, causal, softcap, window_left, want_lse, stream, out
         # non-zero for a few query rows against a long cache (N <= 4, S >= 256: the split-KV decode route) and for
         # float32 (partials of the query tiles that several CTAs share)
         need = lib.b200fa_fwd_workspace_bytes(C.byref(d))
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need > 0 else None
+        ws = _scratch(need, q.device, stream) if need > 0 else None
         st = lib.b200fa_fwd(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(ws), need,
                             C.c_void_p(_stream_ptr(stream, q.device)))
     _lib.check(st, "flash_attention")
@@ -357,13 +371,20 @@ def _varlen_fwd_raw(q, k, v, cu_q, cu_k, nseq, max_q, max_k, scale, causal, want
     _, Hq, Tq, D = q.shape
     Hkv, Tk = k.shape[1], k.shape[2]
     q, k, v = _row_contig(q), _row_contig(k), _row_contig(v)
-    out = torch.zeros((1, Hq, Tq, D), dtype=q.dtype, device=q.device)
-    lse = torch.zeros((1, Hq, Tq), dtype=torch.float32, device=q.device) if want_lse else None
     code = _DTYPE_CODE[q.dtype]
+    out = torch.empty((1, Hq, Tq, D), dtype=q.dtype, device=q.device)
+    lse = torch.empty((1, Hq, Tq), dtype=torch.float32, device=q.device) if want_lse else None
     d = _desc(code, code, 1, Hq, Hkv, Tq, Tk, D, scale, causal, flags=_FORCE_FLAGS, q=q, k=k, v=v, o=out)
     with torch.cuda.device(q.device):
+        # with a workspace the library clears the rows that belong to no sequence, else that is done here
+        need = lib.b200fa_fwd_varlen_workspace_bytes(C.byref(d), nseq, max_q, max_k)
+        ws = _scratch(need, q.device, stream) if need > 0 else None
+        if ws is None:
+            out.zero_()
+            if lse is not None:
+                lse.zero_()
         st = lib.b200fa_fwd_varlen(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(cu_q), _ptr(cu_k), nseq,
-                                   max_q, max_k, _ptr(out), _ptr(lse), None, 0,
+                                   max_q, max_k, _ptr(out), _ptr(lse), _ptr(ws), need,
                                    C.c_void_p(_stream_ptr(stream, q.device)))
     _lib.check(st, "flash_attention_varlen")
     return out, lse
@@ -556,8 +577,8 @@ def _dequant_pair(k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, o
     lib = _lib.load()
     num_pages, bs, H, D = k_pages.shape
     B, max_blocks = table.shape
-    K = torch.empty((B, H, max_kv_len, D), dtype=out_dtype, device=k_pages.device)
-    V = torch.empty_like(K)
+    K = _used_on(torch.empty((B, H, max_kv_len, D), dtype=out_dtype, device=k_pages.device), stream)
+    V = _used_on(torch.empty_like(K), stream)
     with torch.cuda.device(k_pages.device):
         st = lib.b200fa_paged_kv_dequant_pair(_ptr(k_pages), _ptr(v_pages), _ptr(k_scale), _ptr(v_scale), _ptr(table), _ptr(lens),
                                               B, H, D, _KV_CODE[k_pages.dtype], _DTYPE_CODE[out_dtype], num_pages, bs, max_blocks,
@@ -610,7 +631,7 @@ def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, 
     with torch.cuda.device(q.device):
         need = lib.b200fa_decode_paged_workspace_bytes(C.byref(d), int(max_kv_len))
         if workspace is None or workspace.numel() < need:
-            workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
+            workspace = _scratch(max(need, 16), q.device, stream)
         st = lib.b200fa_decode_paged(C.byref(d), _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(k_scale),
                                      _ptr(v_scale), _ptr(table), _ptr(lens), num_pages, block_size,
                                      table.shape[1], int(max_kv_len), _ptr(out), _ptr(lse),

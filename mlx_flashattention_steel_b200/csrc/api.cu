@@ -325,15 +325,18 @@ int32_t b200fa_paged_kv_dequant_pair(const void* k_pool, const void* v_pool, con
 
 size_t b200fa_fwd_varlen_workspace_bytes(const b200fa_desc* d, int32_t num_seqs, int32_t max_seqlen_q,
                                          int32_t max_seqlen_k) {
-  (void)d; (void)num_seqs; (void)max_seqlen_q; (void)max_seqlen_k;
-  return 0;
+  (void)max_seqlen_k;
+  if (d == nullptr || num_seqs <= 0 || max_seqlen_q <= 0 || (d->dtype != B200FA_F16 && d->dtype != B200FA_BF16) ||
+      (d->flags & B200FA_FLAG_FORCE_MMA_SYNC))
+    return 0;
+  return b200fa::fwd_sm100_varlen_workspace_bytes();
 }
 
 int32_t b200fa_fwd_varlen(const b200fa_desc* d, const void* q, const void* k, const void* v,
                           const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int32_t num_seqs,
                           int32_t max_seqlen_q, int32_t max_seqlen_k, void* out, float* lse,
                           void* workspace, size_t workspace_bytes, void* stream) {
-  (void)workspace; (void)workspace_bytes; (void)max_seqlen_k;
+  (void)max_seqlen_k;
   int32_t st = check_common(d, true);
   if (st != B200FA_OK) return st;
   if (num_seqs < 0 || max_seqlen_q < 0) return fail(B200FA_ERR_INVALID_ARG, "negative num_seqs/max_seqlen");
@@ -350,6 +353,12 @@ int32_t b200fa_fwd_varlen(const b200fa_desc* d, const void* q, const void* k, co
   p.cu_k = cu_seqlens_k;
   cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e;
+  const size_t need = b200fa_fwd_varlen_workspace_bytes(d, num_seqs, max_seqlen_q, max_seqlen_k);
+  if (need > 0 && workspace != nullptr && aligned16(workspace) && workspace_bytes >= need) {
+    p.fwd_counter = static_cast<int*>(workspace);
+    e = b200fa::launch_fwd_sm100_varlen_prepare(p, d->D, num_seqs, max_seqlen_q, cs);
+    if (e != cudaSuccess) return cuda_fail(e, "varlen prepare launch");
+  }
   if (d->dtype == B200FA_F32) {
     e = b200fa::launch_fwd_f32(p, d->D, true, num_seqs, max_seqlen_q, nullptr, cs);
   } else if (!(d->flags & B200FA_FLAG_FORCE_MMA_SYNC) && b200fa::fwd_sm100_supported(p, d->dtype, d->D)) {

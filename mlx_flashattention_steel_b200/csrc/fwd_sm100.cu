@@ -72,14 +72,17 @@ enum Bar {
   BAR_Q_FREE = 13,           // persistent CTAs: the item's last S MMAs have read Q -- the next item's Q may land
   BAR_O_STAGED = 14,         // count 4: the softmax warps have written their O rows to shared memory
   BAR_O_FINAL = 15,          // committed once, after the last P.V: O is complete
-  BAR_COUNT = 16
+  BAR_ITEM_FULL = 16,        // +slot, persistent CTAs: the producer has put the next item's index there
+  BAR_ITEM_FREE = 18,        // +slot, count 5: the softmax warps and the MMA warp have read it
+  BAR_COUNT = 20
 };
 
 struct Sm100Args {
   FwdParams p;
   int tma_store;             // dense layout: O leaves through shared memory and TMA stores
-  int gx, gy, total_items;   // items = (query tile, head, batch | sequence); persistent CTAs: query tile fastest
-  int group;                 // > 1: one item per CTA, a linear grid in the order of item_of
+  int gx, gy, total_items;   // items = (query tile, head, batch | sequence)
+  int group;                 // their order (item_of); one item per CTA: > 1 = a linear grid in that order
+  int* counter;              // persistent CTAs: items dealt out so far beyond the first of each CTA; null = every grid-th
 };
 
 // max / min of 64 values as a 3-ary tree (depth 4) instead of a 63-deep dependent chain
@@ -174,8 +177,9 @@ __device__ __forceinline__ unsigned mask_cells(const uint8_t* row, int cb0, int 
 // FEAT adds the ALiBi bias and the block mask (reference: mlx_mfa/attention.py:1079-1216 flash_attention_sparse,
 // csrc/mfa_steel_fwd.cpp:230-262 the shader's per-tile mask test): a key tile is visited only if one of the mask
 // cells under it is set, and partially set tiles are masked by element.  The plain instantiation compiles none of it.
-// PERSIST: the CTA stays on its SM and walks items i = blockIdx.x, blockIdx.x + gridDim.x, ... (a query tile of one
-// head each) instead of one item per CTA.  TMEM, the barriers and the rings live across items: every phase is counted
+// PERSIST: the CTA stays on its SM and walks items (a query tile of one head each) instead of one item per CTA.  The
+// first is item blockIdx.x; the next ones come from a counter, one item ahead: an item is 1 to 64 key tiles, and with
+// every grid-th one dealt to each CTA the slowest of 296 CTAs had 30 % more than the average to do.  TMEM, the barriers and the rings live across items: every phase is counted
 // in tiles (g) or items (itn) since the CTA started, the producer requests the next item's Q as soon as the last S
 // MMAs of this one have read it and its K tiles as their stages free up, so set-up, launch gaps and load latency are
 // paid once per SM instead of once per query tile -- what shapes with few key tiles per query tile (a sliding
@@ -201,6 +205,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + BAR_COUNT);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   int* s_ntiles = reinterpret_cast<int*>(s_tmem + 2);
+  volatile int* s_item = reinterpret_cast<volatile int*>(s_tmem + 3);          // [2], persistent CTAs: the next items
   uint16_t* s_list = reinterpret_cast<uint16_t*>(smem + kSmemTiles + 256);     // FEAT only
   unsigned char* s_flag = reinterpret_cast<unsigned char*>(s_list + kMaxListTiles);
 
@@ -386,6 +391,10 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(bar(BAR_O_STAGED), 4);
     mbar_init(bar(BAR_O_FINAL), 1);
     mbar_init(bar(BAR_Q_FREE), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(bar(BAR_ITEM_FULL + s), 1);
+      mbar_init(bar(BAR_ITEM_FREE + s), 5);
+    }
     *s_abort = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -427,10 +436,38 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   int g0 = 0, itn = 0;       // key tiles and items this CTA has been through: every barrier phase counts from them
   int prev_q0 = 0, prev_head = 0, prev_batch = 0;
-  const int n_items = PERSIST ? a.total_items : 1;
-  for (int it = PERSIST ? static_cast<int>(blockIdx.x) : 0; it < n_items; it += PERSIST ? static_cast<int>(gridDim.x) : 1) {
-  if constexpr (PERSIST) {
-    item_geometry(it % a.gx, (it / a.gx) % a.gy, it / (a.gx * a.gy), a.gx);
+  auto locate = [&](int it) {
+    int xt, pair;
+    item_of(it, a.gx, a.total_items / a.gx, a.group, xt, pair);
+    item_geometry(xt, pair % a.gy, pair / a.gy, a.gx);
+  };
+  int it = static_cast<int>(blockIdx.x);
+  for (int n = 0;; ++n) {
+  if constexpr (!PERSIST) {
+    if (n > 0) break;
+  } else {
+    const int slot = n & 1;
+    if (n > 0) {
+      // phases: item n was put into slot n & 1 as that slot's (n - 1) / 2-th use
+      it = mbar_wait_bounded(bar(BAR_ITEM_FULL + slot), ((n - 1) >> 1) & 1, s_abort) ? s_item[slot] : -1;
+      __syncwarp();
+      if (warp != 4 && lane == 0) mbar_arrive(bar(BAR_ITEM_FREE + slot));
+    }
+    if (it < 0 || *s_abort != 0) break;
+    if (warp == 4 && lane == 0) {
+      // the next item, fetched while this one runs; cells beyond a sequence's end are passed over here
+      int next = it;
+      do {
+        next = a.counter != nullptr ? static_cast<int>(gridDim.x) + atomicAdd(a.counter, 1) : next + static_cast<int>(gridDim.x);
+        if (next >= a.total_items) { next = -1; break; }
+        locate(next);
+      } while (q0 >= N);
+      // item n + 1 goes into slot (n + 1) & 1, which item n - 1 had
+      if (n >= 2) mbar_wait_bounded(bar(BAR_ITEM_FREE + (slot ^ 1)), ((n - 2) >> 1) & 1, s_abort);
+      s_item[slot ^ 1] = next;
+      mbar_arrive(bar(BAR_ITEM_FULL + (slot ^ 1)));
+    }
+    locate(it);
     if (q0 >= N) continue;
     if (n_tiles <= 0) {
       zero_rows();
@@ -1007,6 +1044,8 @@ static cudaError_t launch_hd(const FwdParams& p, int nbatch, int max_q, cudaStre
       sm_count = 148;
     if (items < 0x7fffffffLL && want_persistent(p, nbatch, max_q, sm_count, a.p.persist_mode)) {
       const int ctas = static_cast<int>(items < 2LL * sm_count ? items : 2LL * sm_count);     // two CTAs per SM
+      a.group = p.cu_q != nullptr ? p.Hq : 1;            // a sequence's long query tiles first, its heads side by side
+      a.counter = p.fwd_counter;
       auto launch_p = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (e != cudaSuccess) return e;
@@ -1017,6 +1056,7 @@ static cudaError_t launch_hd(const FwdParams& p, int nbatch, int max_q, cudaStre
                        : (capm == 1 ? launch_p(fa_fwd_sm100_kernel<HD, DT, false, true, 1>) : launch_p(fa_fwd_sm100_kernel<HD, DT, false, true, 0>));
     }
   }
+  a.counter = nullptr;
   // dense calls with a common key count (others: longest batch entry first, see the kernel)
   a.group = 1;
   if (p.cu_q == nullptr && p.kv_lens == nullptr && !FEAT && items < 0x7fffffffLL)
@@ -1030,6 +1070,40 @@ static cudaError_t launch_hd(const FwdParams& p, int nbatch, int max_q, cudaStre
   };
   return capm == 2 ? launch_1(fa_fwd_sm100_kernel<HD, DT, FEAT, false, 2>)
                    : (capm == 1 ? launch_1(fa_fwd_sm100_kernel<HD, DT, FEAT, false, 1>) : launch_1(fa_fwd_sm100_kernel<HD, DT, FEAT, false, 0>));
+}
+
+// Rows of packed outputs that no query tile covers (before the first sequence, after the last one, beyond max_q in a
+// longer one): zeros; and the item counter of the persistent form.  One block per sequence, and kTailBlocks for the rows
+// after the last one.
+constexpr int kTailBlocks = 64;
+template <int HD>
+__global__ void __launch_bounds__(256) varlen_prepare_kernel(const FwdParams p, int nseq, int max_q) {
+  const int z = blockIdx.x;
+  if (z == 0 && threadIdx.x == 0) *p.fwd_counter = 0;
+  // block z < nseq: the uncovered end of sequence z (block 0: the rows before it too); the others: after the last sequence
+  const int covered = (max_q + BM - 1) / BM * BM;
+  auto fill = [&](int r0, int r1, int part, int parts) {
+    const long long n = static_cast<long long>(r1 - r0) * p.Hq;
+    for (long long i = part * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += static_cast<long long>(parts) * blockDim.x) {
+      const int h = static_cast<int>(i % p.Hq), r = r0 + static_cast<int>(i / p.Hq);
+      uint4* row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.o) + h * p.o_hs + static_cast<int64_t>(r) * p.o_rs);
+      for (int c = 0; c < HD / 8; ++c) row[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (p.lse != nullptr) p.lse[h * p.lse_hs + r] = 0.f;
+    }
+  };
+  if (z == 0) fill(0, min(max(p.cu_q[0], 0), p.N), 0, 1);
+  if (z >= nseq) fill(min(max(p.cu_q[nseq], 0), p.N), p.N, z - nseq, kTailBlocks);
+  else fill(min(max(p.cu_q[z] + covered, 0), p.N), min(max(p.cu_q[z + 1], 0), p.N), 0, 1);
+}
+
+size_t fwd_sm100_varlen_workspace_bytes() { return 256; }
+
+cudaError_t launch_fwd_sm100_varlen_prepare(const FwdParams& p, int D, int nseq, int max_q, cudaStream_t stream) {
+  const unsigned blocks = static_cast<unsigned>(nseq) + kTailBlocks;
+  if (D == 64) varlen_prepare_kernel<64><<<blocks, 256, 0, stream>>>(p, nseq, max_q);
+  else if (D == 128) varlen_prepare_kernel<128><<<blocks, 256, 0, stream>>>(p, nseq, max_q);
+  else varlen_prepare_kernel<256><<<blocks, 256, 0, stream>>>(p, nseq, max_q);
+  return cudaGetLastError();
 }
 
 // Dense: nbatch = B, max_q = N.  Packed varlen (p.cu_q set, B == 1, N/S = total tokens): nbatch = number of

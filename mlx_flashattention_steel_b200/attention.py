@@ -26,8 +26,10 @@ Deliberate differences from the reference, all on the side of its CPU
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
+import struct
 from typing import Optional, Sequence, Tuple, Union
 
 import torch
@@ -86,9 +88,26 @@ def _row_contig(x: torch.Tensor) -> torch.Tensor:
     return x if ok else x.contiguous()
 
 
+# A call of a few microseconds on the GPU is bound by what the host does around it, so the helpers below take the shortest
+# way there is: the raw handle of the current stream, no device guard where the device is current already, the descriptor
+# packed in one go instead of field by field (7 us of a 45 us decode call), pointers as plain integers.
+_HERE = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context in which `device` is current."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def _i32(t: torch.Tensor) -> torch.Tensor:
+    if t.dtype != torch.int32:
+        t = t.to(torch.int32)
+    return t if t.is_contiguous() else t.contiguous()
+
+
 def _stream_ptr(stream, device) -> int:
     if stream is None:
-        return torch.cuda.current_stream(device).cuda_stream
+        return torch._C._cuda_getCurrentRawStream(device.index)
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     if isinstance(stream, int):
@@ -111,32 +130,25 @@ def _used_on(t: torch.Tensor, stream) -> torch.Tensor:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+_DESC = struct.Struct("@8i12q2f4i2P3iP")      # the fields of _lib.Desc in order, with the same native alignment
+assert _DESC.size == C.sizeof(_lib.Desc)
+
+
+def _strides(t):
+    return (0, 0, 0) if t is None else t.stride()[:3]
 
 
 def _desc(dtype, kv_dtype, B, Hq, Hkv, N, S, D, scale, causal, softcap=0.0, window_left=-1,
           num_splits=0, flags=0, q=None, k=None, v=None, o=None, alibi=None, bmask=None, kv_lens=None) -> _lib.Desc:
-    d = _lib.Desc()
-    d.dtype, d.kv_dtype = dtype, kv_dtype
-    d.B, d.Hq, d.Hkv, d.N, d.S, d.D = B, Hq, Hkv, N, S, D
-    for name, t in (("q_strides", q), ("k_strides", k), ("v_strides", v), ("o_strides", o)):
-        arr = getattr(d, name)
-        if t is None:
-            arr[0] = arr[1] = arr[2] = 0
-        else:
-            arr[0], arr[1], arr[2] = t.stride(0), t.stride(1), t.stride(2)
-    d.scale = float(scale)
-    d.softcap = float(softcap)
-    d.causal = 1 if causal else 0
-    d.window_left = int(window_left)
-    d.num_splits = int(num_splits)
-    d.flags = int(flags)
-    d.alibi_slopes = None if alibi is None else alibi.data_ptr()
-    d.kv_lens = None if kv_lens is None else kv_lens.data_ptr()
-    if bmask is not None:            # (uint8 tensor [NQ, NK], block rows, block columns)
-        d.block_mask = bmask[0].data_ptr()
-        d.mask_bq, d.mask_bk, d.mask_nk = int(bmask[1]), int(bmask[2]), int(bmask[0].shape[1])
-    return d
+    # bmask: (uint8 tensor [NQ, NK], block rows, block columns)
+    mask = (0, 0, 0, 0) if bmask is None else (bmask[0].data_ptr(), int(bmask[1]), int(bmask[2]), int(bmask[0].shape[1]))
+    return _lib.Desc.from_buffer_copy(_DESC.pack(
+        dtype, kv_dtype, B, Hq, Hkv, N, S, D, *_strides(q), *_strides(k), *_strides(v), *_strides(o), float(scale),
+        float(softcap), 1 if causal else 0, int(window_left), int(num_splits), int(flags),
+        0 if alibi is None else alibi.data_ptr(), *mask, 0 if kv_lens is None else kv_lens.data_ptr()))
 
 
 _FORCE_FLAGS = 0
@@ -174,13 +186,13 @@ def _fwd_raw(q, k, v, scale, causal, softcap, window_left, want_lse, stream, out
     d = _desc(code, code, B, Hq, Hkv, N, S, D, scale, causal, softcap, window_left,
               flags=_FORCE_FLAGS, q=q, k=k if S > 0 else None, v=v if S > 0 else None, o=out, alibi=alibi, bmask=bmask,
               kv_lens=kv_lens)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         # non-zero for a few query rows against a long cache (N <= 4, S >= 256: the split-KV decode route) and for
         # float32 (partials of the query tiles that several CTAs share)
         need = lib.b200fa_fwd_workspace_bytes(C.byref(d))
         ws = _scratch(need, q.device, stream) if need > 0 else None
         st = lib.b200fa_fwd(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(ws), need,
-                            C.c_void_p(_stream_ptr(stream, q.device)))
+                            _stream_ptr(stream, q.device))
     _lib.check(st, "flash_attention")
     return out, lse
 
@@ -200,8 +212,8 @@ def _bwd_raw(q, k, v, out, lse, dout, scale, causal, stream, cu=None, alibi=None
     code = _DTYPE_CODE[q.dtype]
     d = _desc(code, code, B, Hq, Hkv, N, S, D, scale, causal, softcap, window_left, flags=_FORCE_FLAGS, q=q, k=k, v=v,
               o=out, alibi=alibi, bmask=bmask)
-    sp = C.c_void_p(_stream_ptr(stream, q.device))
-    with torch.cuda.device(q.device):
+    sp = _stream_ptr(stream, q.device)
+    with _on(q.device):
         if cu is None:
             need = lib.b200fa_bwd_workspace_bytes(C.byref(d))
             ws = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
@@ -375,7 +387,7 @@ def _varlen_fwd_raw(q, k, v, cu_q, cu_k, nseq, max_q, max_k, scale, causal, want
     out = torch.empty((1, Hq, Tq, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((1, Hq, Tq), dtype=torch.float32, device=q.device) if want_lse else None
     d = _desc(code, code, 1, Hq, Hkv, Tq, Tk, D, scale, causal, flags=_FORCE_FLAGS, q=q, k=k, v=v, o=out)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         # with a workspace the library clears the rows that belong to no sequence, else that is done here
         need = lib.b200fa_fwd_varlen_workspace_bytes(C.byref(d), nseq, max_q, max_k)
         ws = _scratch(need, q.device, stream) if need > 0 else None
@@ -385,7 +397,7 @@ def _varlen_fwd_raw(q, k, v, cu_q, cu_k, nseq, max_q, max_k, scale, causal, want
                 lse.zero_()
         st = lib.b200fa_fwd_varlen(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(cu_q), _ptr(cu_k), nseq,
                                    max_q, max_k, _ptr(out), _ptr(lse), _ptr(ws), need,
-                                   C.c_void_p(_stream_ptr(stream, q.device)))
+                                   _stream_ptr(stream, q.device))
     _lib.check(st, "flash_attention_varlen")
     return out, lse
 
@@ -466,8 +478,7 @@ def flash_attention_varlen(
     ok = (D in _SUPPORTED_HDIMS and q.dtype in _DTYPE_CODE) or (D in _FWD_ONLY_HDIMS and q.dtype in (torch.float16, torch.bfloat16))
     if not ok:
         raise NotImplementedError(f"flash_attention_varlen: head_dim={D}, dtype={q.dtype} not built.")
-    cu_q = cu_q.to(torch.int32).contiguous()
-    cu_k = cu_k.to(torch.int32).contiguous()
+    cu_q, cu_k = _i32(cu_q), _i32(cu_k)
     return _VarlenFn.apply(q, k, v, cu_q, cu_k, int(nseq), int(max_seqlen_q), int(max_seqlen_k),
                            float(scale), bool(causal), stream)
 
@@ -489,10 +500,10 @@ def paged_kv_gather(pool, block_table, seq_lens, max_kv_len: int, stream=None) -
     _, bs, H, D = pool.shape
     B, max_blocks = table.shape
     out = torch.empty((B, H, max_kv_len, D), dtype=pool.dtype, device=pool.device)
-    with torch.cuda.device(pool.device):
+    with _on(pool.device):
         st = lib.b200fa_paged_kv_gather(_ptr(pool), _ptr(table), _ptr(lens), B, H, D, pool.element_size(),
                                         bs, max_blocks, int(max_kv_len), _ptr(out),
-                                        C.c_void_p(_stream_ptr(stream, pool.device)))
+                                        _stream_ptr(stream, pool.device))
     _lib.check(st, "paged_kv_gather")
     return out
 
@@ -517,10 +528,10 @@ class _PagedGatherFn(torch.autograd.Function):
         grad_pool = torch.zeros(shape, dtype=dtype, device=g.device)
         B, H, _, D = g.shape
         lib = _lib.load()
-        with torch.cuda.device(g.device):
+        with _on(g.device):
             st = lib.b200fa_paged_kv_scatter_add(_ptr(g), _ptr(table), _ptr(lens), B, H, D, _DTYPE_CODE[dtype], shape[1],
                                                  table.shape[1], int(max_kv_len), _ptr(grad_pool),
-                                                 C.c_void_p(_stream_ptr(stream, g.device)))
+                                                 _stream_ptr(stream, g.device))
         _lib.check(st, "paged_kv_scatter_add")
         return grad_pool, None, None, None, None
 
@@ -536,10 +547,10 @@ def _fwd_paged_raw(q, k_pages, v_pages, table, lens, max_kv_len, scale, causal, 
     lse = torch.empty((B, Hq, N), dtype=torch.float32, device=q.device) if want_lse else None
     code = _DTYPE_CODE[q.dtype]
     d = _desc(code, code, B, Hq, Hkv, N, int(max_kv_len), D, scale, causal, softcap, window_left, flags=_FORCE_FLAGS, q=q, o=out)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         st = lib.b200fa_fwd_paged(C.byref(d), _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(table), _ptr(lens), num_pages,
                                   block_size, table.shape[1], int(max_kv_len), _ptr(out), _ptr(lse),
-                                  C.c_void_p(_stream_ptr(stream, q.device)))
+                                  _stream_ptr(stream, q.device))
     _lib.check(st, "flash_attention_paged")
     return out, lse
 
@@ -562,10 +573,10 @@ def paged_kv_gather_dequant(pool, scale, block_table, seq_lens, max_kv_len: int,
     _, bs, H, D = pool.shape
     B, max_blocks = table.shape
     out = torch.empty((B, H, max_kv_len, D), dtype=out_dtype, device=pool.device)
-    with torch.cuda.device(pool.device):
+    with _on(pool.device):
         st = lib.b200fa_paged_kv_gather_dequant(_ptr(pool), _ptr(scale), _ptr(table), _ptr(lens), B, H, D,
                                                 _KV_CODE[pool.dtype], _DTYPE_CODE[out_dtype], bs, max_blocks,
-                                                int(max_kv_len), _ptr(out), C.c_void_p(_stream_ptr(stream, pool.device)))
+                                                int(max_kv_len), _ptr(out), _stream_ptr(stream, pool.device))
     _lib.check(st, "paged_kv_gather_dequant")
     return out
 
@@ -579,10 +590,10 @@ def _dequant_pair(k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, o
     B, max_blocks = table.shape
     K = _used_on(torch.empty((B, H, max_kv_len, D), dtype=out_dtype, device=k_pages.device), stream)
     V = _used_on(torch.empty_like(K), stream)
-    with torch.cuda.device(k_pages.device):
+    with _on(k_pages.device):
         st = lib.b200fa_paged_kv_dequant_pair(_ptr(k_pages), _ptr(v_pages), _ptr(k_scale), _ptr(v_scale), _ptr(table), _ptr(lens),
                                               B, H, D, _KV_CODE[k_pages.dtype], _DTYPE_CODE[out_dtype], num_pages, bs, max_blocks,
-                                              max_kv_len, _ptr(K), _ptr(V), C.c_void_p(_stream_ptr(stream, k_pages.device)))
+                                              max_kv_len, _ptr(K), _ptr(V), _stream_ptr(stream, k_pages.device))
     _lib.check(st, "flash_attention_paged")
     return K, V
 
@@ -628,7 +639,7 @@ def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, 
     d = _desc(code, kv_code, B, Hq, Hkv, Nq, 0, D, scale, causal, softcap, -1, num_splits,
               _FORCE_FLAGS | (_lib.FLAG_PACKED_F32 if packed else 0) |
               (_lib.FLAG_DECODE_WIDE if (Hq // Hkv) * Nq > 8 else 0))
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         need = lib.b200fa_decode_paged_workspace_bytes(C.byref(d), int(max_kv_len))
         if workspace is None or workspace.numel() < need:
             workspace = _scratch(max(need, 16), q.device, stream)
@@ -636,11 +647,11 @@ def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, 
                                      _ptr(v_scale), _ptr(table), _ptr(lens), num_pages, block_size,
                                      table.shape[1], int(max_kv_len), _ptr(out), _ptr(lse),
                                      _ptr(workspace), workspace.numel(),
-                                     C.c_void_p(_stream_ptr(stream, q.device)))
+                                     _stream_ptr(stream, q.device))
     _lib.check(st, "flash_attention_paged")
     if _CHECK_DECODE_STATUS:
         word = C.c_int32(0)
-        _lib.check(lib.b200fa_workspace_status(_ptr(workspace), C.c_void_p(_stream_ptr(stream, q.device)),
+        _lib.check(lib.b200fa_workspace_status(_ptr(workspace), _stream_ptr(stream, q.device),
                                                C.byref(word)), "decode status")
         if word.value != 0:
             raise RuntimeError(f"flash_attention_paged: decode kernel reported status {word.value} "
@@ -703,8 +714,7 @@ def flash_attention_paged(
         raise ValueError("flash_attention_paged: block_table must be [B, max_blocks] and seq_lens [B].")
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    table = table.to(torch.int32).contiguous()
-    lens = lens.to(torch.int32).contiguous()
+    table, lens = _i32(table), _i32(lens)
     if max_kv_len is None:
         max_kv_len = int(lens.max().item()) if B > 0 else 0
     if max_kv_len == 0:
@@ -914,7 +924,7 @@ def kernel_status(stream=None) -> int:
     lib = _lib.load()
     word = C.c_int32(0)
     dev = torch.device("cuda", torch.cuda.current_device())
-    _lib.check(lib.b200fa_kernel_status(C.c_void_p(_stream_ptr(stream, dev)), C.byref(word)), "kernel_status")
+    _lib.check(lib.b200fa_kernel_status(_stream_ptr(stream, dev), C.byref(word)), "kernel_status")
     return int(word.value)
 
 

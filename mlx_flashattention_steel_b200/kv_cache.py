@@ -67,10 +67,10 @@ def kv_append(k_new, v_new, slot_mapping, k_pool, v_pool, k_scale=None, v_scale=
     lib = _lib.load()
     st = lib.b200fa_kv_append(
         _DTYPE_CODE[k_new.dtype], _POOL_CODE[k_pool.dtype], T, H, D, bs, P,
-        C.c_void_p(k_new.data_ptr()), C.c_void_p(v_new.data_ptr()), k_new.stride(0), k_new.stride(1),
-        C.c_void_p(slot_mapping.data_ptr()), C.c_void_p(k_pool.data_ptr()), C.c_void_p(v_pool.data_ptr()),
-        C.c_void_p(k_scale.data_ptr()) if quant else None, C.c_void_p(v_scale.data_ptr()) if quant else None,
-        C.c_void_p(_stream_ptr(stream, k_pool.device)))
+        k_new.data_ptr(), v_new.data_ptr(), k_new.stride(0), k_new.stride(1),
+        slot_mapping.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
+        k_scale.data_ptr() if quant else None, v_scale.data_ptr() if quant else None,
+        _stream_ptr(stream, k_pool.device))
     _lib.check(st, "kv_append")
 
 

@@ -53,6 +53,12 @@ def make_rope_3d_tables(grid_h: int, grid_w: int, num_frames: int, d_h: Optional
     return cos, sin
 
 
+def _table(t: torch.Tensor) -> torch.Tensor:
+    if t.dtype != torch.float32:
+        t = t.to(torch.float32)
+    return t if t.is_contiguous() else t.contiguous()
+
+
 _HOST_OFFSETS = 512     # as many positions travel in the parameters of a launch
 
 
@@ -64,9 +70,9 @@ def _rope_raw(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, offset, int
     xs = (C.c_int64 * 3)(*x.stride()[:3])
     os_ = (C.c_int64 * 3)(*out.stride()[:3])
     lib = _lib.load()
-    head = (_DTYPE_CODE[x.dtype], B, H, N, D, rot, 1 if interleaved else 0, 1 if inverse else 0, C.c_void_p(x.data_ptr()), xs,
-            C.c_void_p(out.data_ptr()), os_, C.c_void_p(cos.data_ptr()), C.c_void_p(sin.data_ptr()), cos.shape[0])
-    sp = C.c_void_p(_stream_ptr(stream, x.device))
+    head = (_DTYPE_CODE[x.dtype], B, H, N, D, rot, 1 if interleaved else 0, 1 if inverse else 0, x.data_ptr(), xs,
+            out.data_ptr(), os_, cos.data_ptr(), sin.data_ptr(), cos.shape[0])
+    sp = _stream_ptr(stream, x.device)
     if isinstance(offset, tuple) and len(offset) <= _HOST_OFFSETS:
         # positions the host knows go with the launch: no copy, no synchronisation
         st = lib.b200fa_rope_host_offsets(*head, (C.c_int32 * B)(*offset), sp)
@@ -75,7 +81,7 @@ def _rope_raw(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, offset, int
     else:
         offs = torch.tensor(offset, dtype=torch.int32) if isinstance(offset, tuple) else offset
         offs = offs.to(device=x.device, dtype=torch.int32).contiguous()
-        st = lib.b200fa_rope(*head, C.c_void_p(offs.data_ptr()), 0, sp)
+        st = lib.b200fa_rope(*head, offs.data_ptr(), 0, sp)
     _lib.check(st, "apply_rope")
     return out
 
@@ -114,7 +120,7 @@ def apply_rope(x, cos, sin, offset: Union[int, Sequence[int], torch.Tensor] = 0,
     if cos.ndim != 2 or cos.shape != sin.shape or cos.shape[1] != rot // 2:
         raise ValueError(f"rotary_cos / rotary_sin must both be [max_seq_len, {rot // 2}], got {tuple(cos.shape)} and {tuple(sin.shape)}.")
     _require_cuda(x, cos, sin)
-    cos, sin = cos.to(torch.float32).contiguous(), sin.to(torch.float32).contiguous()
+    cos, sin = _table(cos), _table(sin)
     N = x.shape[2]
     if isinstance(offset, torch.Tensor) and offset.ndim == 0:
         offset = int(offset)

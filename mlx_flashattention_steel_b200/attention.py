@@ -216,13 +216,13 @@ def _bwd_raw(q, k, v, out, lse, dout, scale, causal, stream, cu=None, alibi=None
     with _on(q.device):
         if cu is None:
             need = lib.b200fa_bwd_workspace_bytes(C.byref(d))
-            ws = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
+            ws = _scratch(max(need, 16), q.device, stream)
             st = lib.b200fa_bwd(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(dout),
                                 _ptr(dq), _ptr(dk), _ptr(dv), _ptr(ws), ws.numel(), sp)
         else:
             cu_q, cu_k, nseq, max_q, max_k = cu
             need = lib.b200fa_bwd_varlen_workspace_bytes(C.byref(d), nseq, max_q, max_k)
-            ws = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
+            ws = _scratch(max(need, 16), q.device, stream)
             st = lib.b200fa_bwd_varlen(C.byref(d), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse),
                                        _ptr(dout), _ptr(cu_q), _ptr(cu_k), nseq, max_q, max_k,
                                        _ptr(dq), _ptr(dk), _ptr(dv), _ptr(ws), ws.numel(), sp)

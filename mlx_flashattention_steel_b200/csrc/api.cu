@@ -404,12 +404,15 @@ static int32_t fill_bwd_params(const b200fa_desc* d, const void* q, const void* 
 static bool bwd_allow_sm100(const b200fa_desc* d) { return !(d->flags & B200FA_FLAG_FORCE_MMA_SYNC); }
 
 // The split head_dim-128 path keeps no fp32 dQ accumulator, which is most of the workspace.
-static size_t bwd_need_bytes(const b200fa_desc* d) {
+// parts: with room for the parts of dK / dV, which a call can do without
+static size_t bwd_need_bytes(const b200fa_desc* d, bool varlen, bool parts) {
   b200fa::BwdParams p;
   if (d->dtype == B200FA_F32 || d->D == 256 ||
       fill_bwd_params(d, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &p) != B200FA_OK)
     return b200fa::bwd_workspace_bytes(d->B, d->Hq, d->N, d->D, false);
-  return b200fa::bwd_workspace_bytes(d->B, d->Hq, d->N, d->D, b200fa::bwd_takes_split_path(p, d->dtype, d->D, bwd_allow_sm100(d)));
+  const bool split = b200fa::bwd_takes_split_path(p, d->dtype, d->D, bwd_allow_sm100(d));
+  return b200fa::bwd_workspace_bytes(d->B, d->Hq, d->N, d->D, split) +
+         (parts && b200fa::bwd_takes_sm100(p, d->dtype, d->D, bwd_allow_sm100(d)) ? b200fa::bwd_dkv_part_bytes(p, d->D, varlen) : 0);
 }
 
 static int32_t bwd_common(const b200fa_desc* d, const void* q, const void* k, const void* v,
@@ -427,7 +430,7 @@ static int32_t bwd_common(const b200fa_desc* d, const void* q, const void* k, co
   if (!q || !k || !v || !out || !lse || !dout || !dq || !dk || !dv)
     return fail(B200FA_ERR_INVALID_ARG, "null tensor pointer");
   if (d->D == 256) return fail(B200FA_ERR_UNSUPPORTED, "backward for head_dim 256 is not built");
-  const size_t need = bwd_need_bytes(d);
+  const size_t need = bwd_need_bytes(d, varlen, false);
   if (workspace == nullptr || workspace_bytes < need)
     return fail(B200FA_ERR_WORKSPACE, "backward needs %zu workspace bytes, got %zu", need, workspace_bytes);
   if (!aligned16(workspace)) return fail(B200FA_ERR_INVALID_ARG, "workspace must be 16-byte aligned");
@@ -439,6 +442,7 @@ static int32_t bwd_common(const b200fa_desc* d, const void* q, const void* k, co
   st = fill_bwd_params(d, q, k, v, out, lse, dout, dq, dk, dv, cu_q, cu_k, &p);
   if (st != B200FA_OK) return st;
   cudaError_t e = b200fa::launch_bwd(p, d->dtype, d->D, varlen, nbatch, max_q, max_k, workspace, bwd_allow_sm100(d),
+                                     workspace_bytes >= bwd_need_bytes(d, varlen, true),
                                      reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "backward launch");
   return B200FA_OK;
@@ -446,7 +450,7 @@ static int32_t bwd_common(const b200fa_desc* d, const void* q, const void* k, co
 
 size_t b200fa_bwd_workspace_bytes(const b200fa_desc* d) {
   if (d == nullptr) return 0;
-  return bwd_need_bytes(d);
+  return bwd_need_bytes(d, false, true);
 }
 
 int32_t b200fa_bwd(const b200fa_desc* d, const void* q, const void* k, const void* v, const void* out,
@@ -461,7 +465,7 @@ size_t b200fa_bwd_varlen_workspace_bytes(const b200fa_desc* d, int32_t num_seqs,
                                          int32_t max_seqlen_k) {
   (void)num_seqs; (void)max_seqlen_q; (void)max_seqlen_k;
   if (d == nullptr) return 0;
-  return bwd_need_bytes(d);
+  return bwd_need_bytes(d, true, true);
 }
 
 int32_t b200fa_bwd_varlen(const b200fa_desc* d, const void* q, const void* k, const void* v,

@@ -118,6 +118,30 @@ __global__ void __launch_bounds__(256) bwd_convert_kernel(const float* __restric
 }
 
 // ---------------------------------------------------------------------------
+// dK / dV parts -> dtype
+// ---------------------------------------------------------------------------
+// Sum of the parts of dK (times scale) and dV, in a fixed order, to the gradients' type.  Bound by HBM: (4 parts + 2)
+// bytes a value.  8 values per thread.
+template <typename T>
+__global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __restrict__ part, int parts, long long values, float scale,
+                                                             T* __restrict__ dk, T* __restrict__ dv) {
+  const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
+  if (i >= values) return;
+  const int which = blockIdx.y;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 4
+  for (int s = 0; s < parts; ++s) {
+    const float4* src = reinterpret_cast<const float4*>(part + (static_cast<long long>(s) * 2 + which) * values + i);
+    const float4 x = src[0], y = src[1];
+    a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+    b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+  }
+  const float f = which == 0 ? scale : 1.f;
+  *reinterpret_cast<uint4*>((which == 0 ? dk : dv) + i) =
+      make_uint4(Elem<T>::pack(a.x * f, a.y * f), Elem<T>::pack(a.z * f, a.w * f), Elem<T>::pack(b.x * f, b.y * f), Elem<T>::pack(b.z * f, b.w * f));
+}
+
+// ---------------------------------------------------------------------------
 // 2. main kernel
 // ---------------------------------------------------------------------------
 template <int ROWS, int D, typename T>
@@ -380,6 +404,16 @@ __global__ void __launch_bounds__(kThreads) bwd_main_kernel(const BwdParams p) {
   }
 }
 
+// after a tcgen05 kernel that cut its items (p.dkv_part set)
+template <typename T, int D>
+cudaError_t launch_dkv_reduce(const BwdParams& p, cudaStream_t stream) {
+  if (p.dkv_part == nullptr) return cudaSuccess;
+  const long long values = static_cast<long long>(p.B) * p.Hkv * p.S * D;
+  const dim3 grid(static_cast<unsigned>((values / 8 + 255) / 256), 2);
+  bwd_dkv_reduce_kernel<T><<<grid, 256, 0, stream>>>(p.dkv_part, bwd_dkv_parts(p, false), values, p.scale, static_cast<T*>(p.dk), static_cast<T*>(p.dv));
+  return cudaGetLastError();
+}
+
 template <typename T, int D>
 cudaError_t launch_t(const BwdParams& p, int dtype, bool varlen, int nbatch, int max_q, int max_k, bool allow_sm100,
                      cudaStream_t stream) {
@@ -404,11 +438,13 @@ cudaError_t launch_t(const BwdParams& p, int dtype, bool varlen, int nbatch, int
   if (p.dq_acc == nullptr) {
     // head_dim 128 on tcgen05: dK / dV and dQ by a kernel each, no accumulator and no conversion pass
     e = launch_bwd_dkv_sm100(p, dtype, nbatch, max_k, stream);
+    if (e == cudaSuccess) e = launch_dkv_reduce<T, D>(p, stream);
     if (e != cudaSuccess) return e;
     return launch_bwd_dq_sm100(p, dtype, nbatch, max_q, stream);
   }
   if (allow_sm100 && bwd_sm100_supported(dtype, D) && bwd_sm100_strides_ok(p)) {
     e = launch_bwd_sm100_main(p, dtype, nbatch, max_k, stream);
+    if (e == cudaSuccess) e = launch_dkv_reduce<T, D>(p, stream);
     if (e != cudaSuccess) return e;
   } else if (varlen) {
     e = cudaFuncSetAttribute(bwd_main_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -430,6 +466,27 @@ cudaError_t launch_t(const BwdParams& p, int dtype, bool varlen, int nbatch, int
 
 }  // namespace
 
+// The tcgen05 kernels: items of 128 keys of a kv head are few where heads are (22 for one kv head at S = 2800), and the
+// longest of a causal mask takes as long as all its query tiles.  They are cut until there are three per SM (148), as long
+// as a part keeps four of its 128 x 128 steps on average.  Packed sequences are not: they are many.
+int bwd_dkv_parts(const BwdParams& p, bool varlen) {
+  if (varlen || p.S <= 0) return 1;
+  const long long items = static_cast<long long>((p.S + 127) / 128) * p.Hkv * p.B;
+  long long steps = static_cast<long long>(p.gqa) * ((p.N + 127) / 128);
+  if (p.causal) steps /= 2;
+  if (p.window_left >= 0) {
+    const long long w = static_cast<long long>(p.gqa) * (p.window_left / 128 + 2);
+    if (w < steps) steps = w;
+  }
+  int parts = 1;
+  while (parts < 8 && items * parts < 3 * 148 && steps >= 8 * parts) parts *= 2;
+  return parts;
+}
+size_t bwd_dkv_part_bytes(const BwdParams& p, int D, bool varlen) {
+  const int parts = bwd_dkv_parts(p, varlen);
+  return parts == 1 ? 0 : static_cast<size_t>(parts) * 2 * p.B * p.Hkv * p.S * D * sizeof(float);
+}
+
 // delta, work counter and -- except on the split head_dim-128 path -- the fp32 dQ accumulator
 size_t bwd_workspace_bytes(int B, int Hq, int N_total, int D, bool split) {
   const size_t rows = static_cast<size_t>(B) * Hq * N_total;
@@ -440,8 +497,12 @@ bool bwd_takes_split_path(const BwdParams& p, int dtype, int D, bool allow_sm100
   return allow_sm100 && bwd_split_sm100_supported(dtype, D) && bwd_sm100_strides_ok(p);
 }
 
+bool bwd_takes_sm100(const BwdParams& p, int dtype, int D, bool allow_sm100) {
+  return bwd_takes_split_path(p, dtype, D, allow_sm100) || (allow_sm100 && bwd_sm100_supported(dtype, D) && bwd_sm100_strides_ok(p));
+}
+
 cudaError_t launch_bwd(const BwdParams& p_in, int dtype, int D, bool varlen, int nbatch, int max_q, int max_k,
-                       void* workspace, bool allow_sm100, cudaStream_t stream) {
+                       void* workspace, bool allow_sm100, bool allow_parts, cudaStream_t stream) {
   BwdParams p = p_in;
   const size_t rows = static_cast<size_t>(p.B) * p.Hq * p.N;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
@@ -449,6 +510,8 @@ cudaError_t launch_bwd(const BwdParams& p_in, int dtype, int D, bool varlen, int
   p.work_counter = reinterpret_cast<int*>(ws + bwd_align(rows * sizeof(float)));
   p.dq_acc = bwd_takes_split_path(p, dtype, D, allow_sm100) ? nullptr
                                                             : reinterpret_cast<float*>(ws + bwd_align(rows * sizeof(float)) + 256);
+  p.dkv_part = allow_parts && bwd_takes_sm100(p, dtype, D, allow_sm100) && bwd_dkv_parts(p, varlen) > 1
+                   ? reinterpret_cast<float*>(ws + bwd_workspace_bytes(p.B, p.Hq, p.N, D, p.dq_acc == nullptr)) : nullptr;
   if (rows == 0) return cudaSuccess;
   if (dtype == 0 && D == 64) return launch_t<__half, 64>(p, dtype, varlen, nbatch, max_q, max_k, allow_sm100, stream);
   if (dtype == 0 && D == 128) return launch_t<__half, 128>(p, dtype, varlen, nbatch, max_q, max_k, allow_sm100, stream);

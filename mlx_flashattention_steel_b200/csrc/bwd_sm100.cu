@@ -63,6 +63,8 @@ struct BwdArgs {
   int dtype;
   int gx, gy, total_items;      // work items: (key tile, kv head, batch | sequence)
   int group;                    // their order: item_of
+  int parts;                    // PARTS: an item's (query head, query tile) steps are cut into so many items, each leaving
+  float* part;                  // fp32 sums [part][dK, dV][B, Hkv, S][64], which launch_dkv_reduce adds up
   int* counter;                 // next work item (zeroed by the preprocess kernel)
 };
 
@@ -97,7 +99,8 @@ template <int DT> __device__ __forceinline__ uint32_t pack16b(float a, float b) 
 // FEAT: the ALiBi bias slope[h] * (key - (query + S - N)) and / or a block mask (cells of mask_bq x mask_bk, mask_bq a
 // multiple of 32 so that the 32 queries a thread handles per step share one cell), as the forward's feature
 // instantiation applies them (csrc/mfa_steel_fwd.cpp:951-970, 230-262 in the reference).  Without CAP / WIN.
-template <int DT, bool CAP, bool WIN, bool FEAT>
+// PARTS: items are cut (a.parts > 1); a variant of its own, because these kernels slow down with every register more.
+template <int DT, bool CAP, bool WIN, bool FEAT, bool PARTS>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -136,6 +139,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (idx >= a.total_items) break;
       int kt, pair;
       item_of(idx, a.gx, a.total_items / a.gx, a.group, kt, pair);
+      const int part_ = PARTS ? pair % a.parts : 0;
+      if constexpr (PARTS) pair /= a.parts;
       const int kvh_ = pair % a.gy, z = pair / a.gy;
       int kb = 0, S_ = p.S, qb = 0, N_ = p.N;
       if (p.cu_k != nullptr) {
@@ -147,7 +152,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         qb = p.cu_q[z];
         N_ = p.cu_q[z + 1] - qb;
       }
-      o[1] = kt; o[2] = kvh_; o[3] = p.cu_q != nullptr ? 0 : z; o[4] = kb; o[5] = S_; o[6] = qb; o[7] = N_;
+      o[1] = kt | (part_ << 24); o[2] = kvh_; o[3] = p.cu_q != nullptr ? 0 : z; o[4] = kb; o[5] = S_; o[6] = qb; o[7] = N_;
       o[0] = idx;
       return idx;
     }
@@ -157,11 +162,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // K / V tile of the item in slot `sl`
   auto load_k_of = [&](int sl, unsigned char* dst, uint32_t b) {
     volatile int* o = s_work + sl * 8;
-    tma_load_4d(smem_u32(dst), &tmK, b, 0, o[4] + o[1] * BK, o[2], o[3]);
+    tma_load_4d(smem_u32(dst), &tmK, b, 0, o[4] + (o[1] & 0xffffff) * BK, o[2], o[3]);
   };
   auto load_v_of = [&](int sl, uint32_t b) {
     volatile int* o = s_work + sl * 8;
-    tma_load_4d(smem_u32(sV), &tmV, b, 0, o[4] + o[1] * BK, o[2], o[3]);
+    tma_load_4d(smem_u32(sV), &tmV, b, 0, o[4] + (o[1] & 0xffffff) * BK, o[2], o[3]);
   };
   if (warp == 8 && lane == 0) {
     mbar_init(bar(BAR_KV), 1);
@@ -188,7 +193,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* wk = s_work + (w & 1) * 8;
   if (wk[0] < 0 || *s_abort != 0) break;
   const int kvh = wk[2], bb = wk[3], k_begin = wk[4], S = wk[5], q_begin = wk[6], N = wk[7];
-  const int n0 = wk[1] * BK;
+  const int n0 = (wk[1] & 0xffffff) * BK;
   const int off = S - N;
   int m_begin = 0;
   if (p.causal) m_begin = max(0, n0 - off) / BQ;
@@ -196,7 +201,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // a left window: the last row that still sees this tile's last key is i = key - off + window_left
   if constexpr (WIN) m_end = min(m_end, max(0, min(S, n0 + BK) - 1 - off + p.window_left) / BQ + 1);
   const int nm = max(0, m_end - m_begin);
-  const int n_iter = nm * p.gqa;
+  // this item's steps of (query head, query tile): it0 + it
+  const int it0 = PARTS ? nm * p.gqa * (wk[1] >> 24) / a.parts : 0;
+  const int n_iter = PARTS ? nm * p.gqa * ((wk[1] >> 24) + 1) / a.parts - it0 : nm * p.gqa;
   const int kbuf = w & 1;                              // K buffer and KV barrier of this item
   const uint32_t kv_par = (w >> 1) & 1;
   unsigned char* sKc = kbuf ? sK1 : sK;
@@ -206,7 +213,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // makes after it has staged the tile's L and delta.
   auto load_q = [&](int it) {
     const int st = it & 1;
-    const int hq = kvh * p.gqa + it / nm, m = m_begin + it % nm;
+    const int hq = kvh * p.gqa + (it0 + it) / nm, m = m_begin + (it0 + it) % nm;
     mbar_expect_tx(bar(BAR_Q_FULL + st), 2 * kTileBytes);
     tma_load_4d(smem_u32(sQ + st * kTileBytes), &tmQ, bar(BAR_Q_FULL + st), 0, q_begin + m * BQ, hq, bb);
     tma_load_4d(smem_u32(sDO + st * kTileBytes), &tmDO, bar(BAR_Q_FULL + st), 0, q_begin + m * BQ, hq, bb);
@@ -238,7 +245,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ============================ producer ============================
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
-      const int hq = kvh * p.gqa + it / nm, m = m_begin + it % nm;
+      const int hq = kvh * p.gqa + (it0 + it) / nm, m = m_begin + (it0 + it) % nm;
       // -L and -delta of the 128 query rows ride with the Q tile; rows beyond N (or without any visible key)
       // get L = +inf so that their P is exactly zero.  They are fetched before waiting for the stage so that
       // their latency does not add to the TMA's.
@@ -363,16 +370,16 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       nxt = __shfl_sync(0xffffffffu, nxt, 0);
-      if (nxt >= 0) {
+      if (nxt >= 0 || n_iter == 0) {          // without query tiles nobody else waits for this item's copies to land
         const bool pass = n_iter > 0 ? mbar_wait_bounded(bar(BAR_KV_TMEM), 0, s_abort)
                                      : mbar_wait_bounded(bar(BAR_KV + kbuf), kv_par, s_abort);
-        if (__all_sync(0xffffffffu, pass) && lane == 0) load_v_of((w + 1) & 1, bar(BAR_KV + (kbuf ^ 1)));
+        if (__all_sync(0xffffffffu, pass) && nxt >= 0 && lane == 0) load_v_of((w + 1) & 1, bar(BAR_KV + (kbuf ^ 1)));
       }
     }
     for (int it = 0; it < n_iter; ++it) {
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_DQ_DONE), it & 1, s_abort))) break;
       tc_fence_after();
-      const int hq = kvh * p.gqa + it / nm, m = m_begin + it % nm;
+      const int hq = kvh * p.gqa + (it0 + it) / nm, m = m_begin + (it0 + it) % nm;
       uint32_t r0[32], r1[32];
       tmem_ld32(tmem + lane_base + cDQ, r0);
       tmem_ld32(tmem + lane_base + cDQ + 32, r1);
@@ -410,9 +417,17 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int rloc = wq * 32 + lane;                         // key row (S^T, dK, dV) or query row (dQ) inside the tile
     const int key = n0 + rloc;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
+    auto part_row = [&](int which, int k) -> float* {
+      return a.part + ((static_cast<int64_t>((wk[1] >> 24) * 2 + which) * p.B + bb) * p.Hkv + kvh) * p.S * HD + static_cast<int64_t>(k) * HD;
+    };
     if (n_iter == 0) {
-      // no query sees these keys: dK = dV = 0
-      if (key < S) {
+      // no query sees these keys (or this part has no step): dK = dV = 0
+      if (PARTS && key < S) {
+        float4* pk = reinterpret_cast<float4*>(part_row(0, key) + hf * 32);
+        float4* pv = reinterpret_cast<float4*>(part_row(1, key) + hf * 32);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pk[i] = pv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else if (key < S) {
         const int64_t o = bb * p.dk_bs + kvh * p.dk_hs + static_cast<int64_t>(k_begin + key) * p.dk_rs + hf * 32;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -439,7 +454,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     for (int it = 0; it < n_iter && ok; ++it) {
       const int st = it & 1;
-      const int m = m_begin + it % nm;
+      const int m = m_begin + (it0 + it) % nm;
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_Q_FULL + st), (it >> 1) & 1, s_abort))) { ok = false; break; }
       const uint32_t Ls = opaque_u32(smem_u32(sL + st * BQ)), Ds = Ls + 2 * BQ * 4;
       const bool need_mask = (n0 + BK > S) || (p.causal && (n0 + BK - 1 > m * BQ + off)) ||
@@ -449,7 +464,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // key & 7: each thread stores its 32 queries as four 16-byte chunks
       const uint32_t ds_row = smem_u32(sDS) + (it & 1) * kDSBytes + rloc * 128;
       const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
-      const float alibi_l2 = (FEAT && p.alibi != nullptr) ? p.alibi[kvh * p.gqa + it / nm] * kLog2e : 0.f;
+      const float alibi_l2 = (FEAT && p.alibi != nullptr) ? p.alibi[kvh * p.gqa + (it0 + it) / nm] * kLog2e : 0.f;
       const float cap_in = CAP ? p.scale / p.softcap : 0.f, cap_out = p.softcap * kLog2e;
       const bool precise_tanh = p.softcap >= kPreciseTanhMinCap;
 
@@ -548,6 +563,18 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_ld32(tmem + lane_base + cDK + hf * 32, rk);
       tmem_ld32(tmem + lane_base + cDV + hf * 32, rv);
       tc_wait_ld();
+      if constexpr (PARTS) {
+        // fp32, straight from the registers: a row each, 128 bytes of it per tensor
+        if (n0 + rloc < S) {
+          float4* pk = reinterpret_cast<float4*>(part_row(0, n0 + rloc) + hf * 32);
+          float4* pv = reinterpret_cast<float4*>(part_row(1, n0 + rloc) + hf * 32);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            pk[i] = make_float4(__uint_as_float(rk[4 * i]), __uint_as_float(rk[4 * i + 1]), __uint_as_float(rk[4 * i + 2]), __uint_as_float(rk[4 * i + 3]));
+            pv[i] = make_float4(__uint_as_float(rv[4 * i]), __uint_as_float(rv[4 * i + 1]), __uint_as_float(rv[4 * i + 2]), __uint_as_float(rv[4 * i + 3]));
+          }
+        }
+      } else {
       const uint32_t srow = smem_u32(sQ) + rloc * 128;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -562,10 +589,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                pack16b<DT>(__uint_as_float(rv[i + 4]), __uint_as_float(rv[i + 5])),
                pack16b<DT>(__uint_as_float(rv[i + 6]), __uint_as_float(rv[i + 7])));
       }
+      }
     }
     // all eight compute warps pass here, whatever happened before (a named barrier has no time-out)
     asm volatile("bar.sync 1, 256;\n" ::: "memory");
-    if (ok) {
+    if (!PARTS && ok) {
       // warp w writes rows 16w .. 16w+15 of both tiles: lane = (row & 3, 16-byte chunk)
 #pragma unroll
       for (int r4 = 0; r4 < 4; ++r4) {
@@ -658,7 +686,9 @@ cudaError_t launch_bwd_sm100_main(const BwdParams& p, int dtype, int nbatch, int
   a.dtype = dtype;
   a.gx = (max_k + BK - 1) / BK;
   a.gy = p.Hkv;
-  const long long items = static_cast<long long>(a.gx) * a.gy * nbatch;
+  a.parts = p.dkv_part != nullptr ? bwd_dkv_parts(p, p.cu_k != nullptr) : 1;
+  a.part = p.dkv_part;
+  const long long items = static_cast<long long>(a.gx) * a.gy * nbatch * a.parts;
   if (items > 0x7fffffffLL || p.work_counter == nullptr) return cudaErrorInvalidValue;
   a.total_items = static_cast<int>(items);
   // an item streams Q and dO of one query head at a time; packed sequences are many and short enough
@@ -678,13 +708,17 @@ cudaError_t launch_bwd_sm100_main(const BwdParams& p, int dtype, int nbatch, int
     return cudaGetLastError();
   };
   const bool cap = p.softcap > 0.f, win = p.window_left >= 0, feat = p.alibi != nullptr || p.bmask != nullptr;
-  if (feat) return dtype == 0 ? launch(bwd_sm100_kernel<0, false, false, true>) : launch(bwd_sm100_kernel<1, false, false, true>);
-  if (dtype == 0) {
-    if (cap) return win ? launch(bwd_sm100_kernel<0, true, true, false>) : launch(bwd_sm100_kernel<0, true, false, false>);
-    return win ? launch(bwd_sm100_kernel<0, false, true, false>) : launch(bwd_sm100_kernel<0, false, false, false>);
-  }
-  if (cap) return win ? launch(bwd_sm100_kernel<1, true, true, false>) : launch(bwd_sm100_kernel<1, true, false, false>);
-  return win ? launch(bwd_sm100_kernel<1, false, true, false>) : launch(bwd_sm100_kernel<1, false, false, false>);
+  auto pick = [&](auto parts) -> cudaError_t {
+    constexpr bool P = decltype(parts)::value;
+    if (feat) return dtype == 0 ? launch(bwd_sm100_kernel<0, false, false, true, P>) : launch(bwd_sm100_kernel<1, false, false, true, P>);
+    if (dtype == 0) {
+      if (cap) return win ? launch(bwd_sm100_kernel<0, true, true, false, P>) : launch(bwd_sm100_kernel<0, true, false, false, P>);
+      return win ? launch(bwd_sm100_kernel<0, false, true, false, P>) : launch(bwd_sm100_kernel<0, false, false, false, P>);
+    }
+    if (cap) return win ? launch(bwd_sm100_kernel<1, true, true, false, P>) : launch(bwd_sm100_kernel<1, true, false, false, P>);
+    return win ? launch(bwd_sm100_kernel<1, false, true, false, P>) : launch(bwd_sm100_kernel<1, false, false, false, P>);
+  };
+  return a.parts > 1 ? pick(std::true_type{}) : pick(std::false_type{});
 }
 
 cudaError_t bwd_sm100_read_clear_status(cudaStream_t stream, int* out) {

@@ -57,6 +57,7 @@ struct BwdParams {
   const float* lse;
   float* delta;          // workspace [B,Hq,N_pad]
   float* dq_acc;         // workspace fp32 [B,Hq,N,D]
+  float* dkv_part;       // workspace: fp32 parts of dK / dV where a tcgen05 kernel cuts its items, or null
   int* work_counter;     // workspace: next work item of the persistent backward kernel (reset by the preprocess kernel)
   void* dq;
   void* dk;

@@ -47,13 +47,18 @@ size_t bwd_workspace_bytes(int B, int Hq, int N_total, int D, bool split);
 bool bwd_takes_split_path(const BwdParams& p, int dtype, int D, bool allow_sm100);
 // allow_sm100: let the tcgen05 kernels run where they exist (head_dim 64: one kernel plus the dQ conversion;
 // head_dim 128: a dK/dV kernel and a dQ kernel); the preprocess is common to all.
+// allow_parts: the workspace has room for bwd_dkv_part_bytes behind bwd_workspace_bytes
 cudaError_t launch_bwd(const BwdParams& p, int dtype, int D, bool varlen, int nbatch, int max_q,
-                       int max_k, void* workspace, bool allow_sm100, cudaStream_t stream);
+                       int max_k, void* workspace, bool allow_sm100, bool allow_parts, cudaStream_t stream);
 bool bwd_sm100_supported(int dtype, int D);
 bool bwd_sm100_strides_ok(const BwdParams& p);
 cudaError_t launch_bwd_sm100_main(const BwdParams& p, int dtype, int nbatch, int max_k, cudaStream_t stream);
 // head_dim 128 (bwd_dkv_sm100.cu, bwd_dq_sm100.cu): p.delta filled, *p.work_counter zero
 bool bwd_split_sm100_supported(int dtype, int D);
+// parts that an item of the tcgen05 dK / dV kernels is cut into, and the workspace for them (0 for one part)
+int bwd_dkv_parts(const BwdParams& p, bool varlen);
+size_t bwd_dkv_part_bytes(const BwdParams& p, int D, bool varlen);
+bool bwd_takes_sm100(const BwdParams& p, int dtype, int D, bool allow_sm100);
 cudaError_t launch_bwd_dkv_sm100(const BwdParams& p, int dtype, int nbatch, int max_k, cudaStream_t stream);
 cudaError_t launch_bwd_dq_sm100(const BwdParams& p, int dtype, int nbatch, int max_q, cudaStream_t stream);
 

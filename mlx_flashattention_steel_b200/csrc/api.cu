@@ -177,7 +177,7 @@ static size_t fwd_f32_need(const b200fa_desc* d) {
 
 size_t b200fa_fwd_workspace_bytes(const b200fa_desc* d) {
   if (!dense_decode_route(d)) return fwd_f32_need(d);
-  return b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->S, d->num_splits);
+  return b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->dtype, d->num_splits, false);
 }
 
 int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const void* v, void* out,
@@ -196,7 +196,7 @@ int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const voi
   // every head) instead of one 128-row tile per head.  Taken when the caller brought the workspace the query asked
   // for; without it the call runs the prefill kernel, which is correct for every shape.
   if (dense_decode_route(d) && workspace != nullptr && aligned16(workspace) &&
-      workspace_bytes >= b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->S, d->num_splits) &&
+      workspace_bytes >= b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->dtype, d->num_splits, false) &&
       !(p.B > 1 && (p.k_bs == 0 || p.v_bs == 0)) && !(p.Hkv > 1 && (p.k_hs == 0 || p.v_hs == 0))) {
     b200fa::DecodeParams dp;
     memset(&dp, 0, sizeof(dp));
@@ -642,8 +642,9 @@ static int32_t decode_check(const b200fa_desc* d) {
 }
 
 size_t b200fa_decode_paged_workspace_bytes(const b200fa_desc* d, int32_t max_kv_len) {
+  (void)max_kv_len;
   if (d == nullptr) return 0;
-  return b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, max_kv_len, d->num_splits);
+  return b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->kv_dtype, d->num_splits, true);
 }
 
 int32_t b200fa_decode_paged(const b200fa_desc* d, const void* q, const void* k_pool, const void* v_pool,
@@ -666,7 +667,7 @@ int32_t b200fa_decode_paged(const b200fa_desc* d, const void* q, const void* k_p
     return fail(B200FA_ERR_INVALID_ARG, "tensors must be 16-byte aligned");
   if (static_cast<int64_t>(max_blocks) * block_size < max_kv_len)
     return fail(B200FA_ERR_INVALID_ARG, "max_kv_len %d exceeds max_blocks*block_size", max_kv_len);
-  const size_t need = b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, max_kv_len, d->num_splits);
+  const size_t need = b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->kv_dtype, d->num_splits, false);
   if (workspace == nullptr || workspace_bytes < need)
     return fail(B200FA_ERR_WORKSPACE, "decode needs %zu workspace bytes, got %zu", need, workspace_bytes);
   if (!aligned16(workspace)) return fail(B200FA_ERR_INVALID_ARG, "workspace must be 16-byte aligned");
@@ -675,6 +676,7 @@ int32_t b200fa_decode_paged(const b200fa_desc* d, const void* q, const void* k_p
   p.q = q; p.k_pool = k_pool; p.v_pool = v_pool; p.k_scale = k_scale; p.v_scale = v_scale;
   p.block_table = block_table; p.seq_lens = seq_lens; p.out = out; p.lse = lse;
   p.workspace = workspace;
+  p.workspace_bytes = workspace_bytes;
   p.B = d->B; p.Hq = d->Hq; p.Hkv = d->Hkv; p.Nq = d->N; p.D = d->D;
   p.num_pages = num_pages; p.block_size = block_size; p.max_blocks = max_blocks; p.max_kv_len = max_kv_len;
   p.q_dtype = d->dtype; p.kv_dtype = d->kv_dtype;

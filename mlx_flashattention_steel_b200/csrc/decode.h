@@ -17,6 +17,7 @@ struct DecodeParams {
   void* out;                // [B, Hq, Nq, D] q dtype
   float* lse;               // [B, Hq, Nq] or null
   void* workspace;
+  size_t workspace_bytes;
   int B, Hq, Hkv, Nq, D;
   int num_pages, block_size, max_blocks, max_kv_len;
   int q_dtype, kv_dtype;
@@ -37,7 +38,8 @@ struct DecodeParams {
 cudaError_t launch_combine_partials(const float* gathered, int R, long long rows, int D, int out_dtype, void* out,
                                     float* lse, cudaStream_t stream);
 
-size_t decode_workspace_bytes(int B, int Hq, int Hkv, int Nq, int D, int max_kv_len, int num_splits);
+// best: with room for what the kernel can use, else what it cannot do without
+size_t decode_workspace_bytes(int B, int Hq, int Hkv, int Nq, int D, int kv_dtype, int num_splits, bool best);
 cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char* msg, size_t msg_len);
 
 }  // namespace b200fa

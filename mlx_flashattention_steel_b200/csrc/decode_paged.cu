@@ -47,7 +47,7 @@ namespace {
 
 constexpr int kBS = 16;           // tokens per unit (one TMA box, one consumer step); a page is 1, 2, 4, ... units
 constexpr int kMaxStages = 8;
-constexpr int kMaxWarps = 9;      // warps of a CTA: 8 consumers and the producer
+constexpr int kMaxWarps = 17;     // warps of a CTA: up to 16 consumers and the producer
 // Up to this many sequences every CTA makes the page prefix sums itself, in shared memory (at most 4 KB): one read of
 // seq_lens and a scan, ~1 us, where a planning kernel in front and a binary search through its result in global memory
 // cost ~6 us before the first page was requested.  Beyond it decode_plan_kernel scans once for all.
@@ -70,11 +70,11 @@ struct DecodeLayout {          // workspace carve-up, in bytes from the workspac
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-__host__ __device__ inline DecodeLayout make_layout(int B, int Hq, int Nq, int HG, int G, int kD) {
+__host__ __device__ inline DecodeLayout make_layout(int B, int Hq, int Nq, int HG, int G, int kD, int PG) {
   DecodeLayout L;
   L.err = 0;
   L.status = 16;
-  L.slots = G + B;
+  L.slots = (G + B) * PG;
   L.page_start = align_up(L.status + sizeof(int) * static_cast<size_t>(G) * HG * kMaxWarps, 16);
   L.part_lse = align_up(L.page_start + (B > kSmemSeqs ? sizeof(int) * (static_cast<size_t>(B) + 1) : 0), 16);
   L.part_o = align_up(L.part_lse + sizeof(float) * static_cast<size_t>(L.slots) * Hq * Nq, 16);
@@ -89,7 +89,8 @@ struct KernelArgs {
   int group;         // Hq / Hkv
   int rows;          // group * Nq
   int hpc;           // kv heads per CTA
-  int row_groups;    // consumer warps per kv head (1 up to 16 rows)
+  int row_groups;    // consumer warps per kv head that share its rows (1 up to 16 rows)
+  int page_groups;   // consumer warps per kv head that take its units in turn, each leaving partials of its own
   int stages;
   int upp;              // 16-token units per page = block_size / 16
   int stage_kv_bytes;   // bytes of one K (or V) stage tile = HPC * kBS * row_bytes
@@ -212,7 +213,7 @@ __device__ __forceinline__ int cta_of_unit(long long u, int G, long long U) {
 // L = log2 sum_i 2^lse_i, O = sum_i 2^(lse_i - L) O_i over the parts of a sequence (csrc/mfa_steel_fwd.cpp:2066-2101);
 // rows of empty sequences become zeros with lse = -inf.  A block holds kMergeWarps / W rows, W warps to a row take its
 // parts in turn; lane l carries head-dim values [4l, 4l + 4).  Bound by L2 latency: a warp fetches 32 log-sum-exps at
-// once and has 8 partial rows in flight (64 registers, so that a block fits beside a CTA of the main kernel).  The first version merged inside the main kernel, in the CTA that arrived last
+// once and has 6 partial rows in flight (64 registers, so that a block fits beside a CTA of the main kernel).  The first version merged inside the main kernel, in the CTA that arrived last
 // (fences, an atomic, then one SM's eight warps for every row): 262144 tokens in 148 parts 198 us in all, 512 tokens
 // 21 us of which 13 were the merge.  Here every row has warps of its own, and the block is already resident and knows its
 // sequence's parts when the main kernel ends.
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
   if (blockIdx.x == 0) {
     // error word = all bits that the main kernel's warps left
     const int* status = reinterpret_cast<const int*>(ws + a.lay.status);
-    const int words = gx * a.HG * (a.hpc * a.row_groups + 1);
+    const int words = gx * a.HG * (a.hpc * a.row_groups * a.page_groups + 1);
     int bits = 0;
     for (int i = tid; i < words; i += blockDim.x) bits |= __ldcg(status + i);
     bits = __reduce_or_sync(0xffffffffu, bits);
@@ -270,7 +271,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
       *reinterpret_cast<int*>(ws + a.lay.err) = bits;
     }
   }
-  if (n == 1) return;                                 // one CTA had the whole sequence and wrote the result
+  if (a.page_groups == 1 && n == 1) return;           // one CTA had the whole sequence and wrote the result
+  n *= a.page_groups;
 
   const int HqNq = p.Hq * p.Nq;
   const int sub = warp % W;                           // which of the row's warps
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
   float m = -INFINITY, wsum = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (row < HqNq) {
-    const size_t slot0 = static_cast<size_t>(c_first) + b;
+    const size_t slot0 = (static_cast<size_t>(c_first) + b) * a.page_groups;
     const float* lse = reinterpret_cast<const float*>(ws + a.lay.part_lse) + slot0 * HqNq + row;
     const float* o = reinterpret_cast<const float*>(ws + a.lay.part_o) + (slot0 * HqNq + row) * kD + lane * 4;
     const size_t o_step = static_cast<size_t>(HqNq) * kD;
@@ -300,15 +302,15 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
       for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
       wsum = fmaf(wsum, corr, sum);
       m = m_new;
-      for (int i0 = 0; i0 < cn; i0 += 8) {
-        float4 v[8];
+      for (int i0 = 0; i0 < cn; i0 += 6) {
+        float4 v[6];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < 6; ++k) {
           v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (live && i0 + k < cn) v[k] = __ldcg(reinterpret_cast<const float4*>(o + static_cast<size_t>(base + (i0 + k) * W) * o_step));
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < 6; ++k) {
           const float wk = __shfl_sync(0xffffffffu, w, (i0 + k) & 31);
           acc.x = fmaf(wk, v[k].x, acc.x); acc.y = fmaf(wk, v[k].y, acc.y);
           acc.z = fmaf(wk, v[k].z, acc.z); acc.w = fmaf(wk, v[k].w, acc.w);
@@ -361,8 +363,10 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
 // RT: tiles of 8 query rows (of the group's heads x query tokens) per consumer warp.  RT = 1: up to 8 rows, one warp per
 // kv head, HPC heads per CTA.  RT = 2 (HPC = 0: a.hpc heads, known at run time): up to 16 rows per warp, which fills the
 // 16 rows of the MMA, and a.row_groups warps per head share a page when there are more.
-template <int KV, int HPC, int kD, bool CAP, int RT>
-__global__ void __launch_bounds__(((HPC > 0 ? HPC : 8) + 1) * 32, HPC > 0 ? ctas_per_sm(HPC) : 1)
+// PG = 2: two warps per head take its units in turn (one each step instead of two), which doubles the warps that hide the
+// latency of a step's chain of waits, conversions and MMAs.
+template <int KV, int HPC, int kD, bool CAP, int RT, int PG>
+__global__ void __launch_bounds__(((HPC > 0 ? HPC * PG : 8) + 1) * 32, HPC > 0 ? ctas_per_sm(HPC) : 1)
 decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const KernelArgs a) {
   constexpr bool kQuant = (KV == KV_I8 || KV == KV_E4M3);
@@ -391,7 +395,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int hg = blockIdx.y;
   const int c = blockIdx.x;
   const int hpc = HPC > 0 ? HPC : a.hpc;
-  const int n_cons = HPC > 0 ? HPC : a.hpc * a.row_groups;       // consumer warps; the next one is the producer
+  const int n_cons = HPC > 0 ? HPC * PG : a.hpc * a.row_groups;       // consumer warps; the next one is the producer
 
   unsigned char* ws = reinterpret_cast<unsigned char*>(p.workspace);
   // every warp leaves its error bits (1: a bounded wait gave up, 2: a table entry beyond the pool)
@@ -408,7 +412,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     prefetch_tmap(&tmV);
     for (int i = 0; i < NS; ++i) {
       mbar_init(smem_u32(&bars[i]), 1);                 // full: producer arrive (+ tx bytes)
-      mbar_init(smem_u32(&bars[kMaxStages + i]), n_cons);  // empty: one arrive per consumer warp
+      mbar_init(smem_u32(&bars[kMaxStages + i]), n_cons / PG);  // empty: one arrive per warp that reads the stage
     }
     *s_abort = 0;
     fence_barrier_init();
@@ -525,7 +529,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   }
 
   // ======================= consumer warps =======================
-  const int wh = RT == 1 ? warp : warp / a.row_groups;          // kv head of this warp within the CTA
+  static_assert(RT == 1 || PG == 1, "wide rows split a head by rows");
+  constexpr int NPI = PG == 1 ? 2 : 1;                          // units per step
+  const int pgrp = PG == 1 ? 0 : warp % PG;
+  const int wh = RT == 1 ? warp / PG : warp / a.row_groups;          // kv head of this warp within the CTA
   const int rbase = RT == 1 ? 0 : (warp % a.row_groups) * (8 * RT);
   const int kvh = hg * hpc + wh;
   // fragment row g of row tile rt is query row rbase + 8 rt + g = (query token, head of the group)
@@ -536,7 +543,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     qi_row[rt] = row_of[rt] / a.group;
     hq_row[rt] = kvh * a.group + row_of[rt] % a.group;
   }
-  int stage = 0;
+  int stage = pgrp;             // the ring has at least two stages
   uint32_t phase = 0;
   long long u = lo;
   int b = b_first;
@@ -545,7 +552,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   while (u < hi && ok) {
     const int s0 = page_start[b], s1 = page_start[b + 1];
     if (s1 <= u) { ++b; continue; }
-    const int j_lo = static_cast<int>(u - s0);
+    // this warp's units: all, or those at its parity of the CTA's running count
+    const int j_lo = static_cast<int>(u - s0) + (PG == 1 ? 0 : static_cast<int>((u - lo + pgrp) & 1));
     const int j_hi = static_cast<int>((hi < s1 ? hi : s1) - s0);
     int len = p.seq_lens != nullptr ? p.seq_lens[b] : p.max_kv_len;
     len = len < 0 ? 0 : (len > p.max_kv_len ? p.max_kv_len : len);
@@ -659,14 +667,14 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     // Two pages per iteration: their loads, conversions and MMAs are independent, which gives the
     // scheduler twice the instruction-level parallelism, and one online-softmax step covers 32 tokens.
     for (int j = j_lo; j < j_hi; j += 2) {
-      const int np = min(2, j_hi - j);
-      int stg[2], pg[2];
+      const int np = min(NPI, j_hi - j);
+      int stg[NPI], pg[NPI];
       {
         int s2 = stage;
         uint32_t ph2 = phase;
         bool okw = true;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < NPI; ++q) {
           stg[q] = s2;
           if (q < np && okw) {
             okw = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bars[s2]), ph2, s_abort));
@@ -675,22 +683,22 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
         if (!okw) { ok = false; break; }
       }
-      uint32_t kbase[2], vbase[2];
+      uint32_t kbase[NPI], vbase[NPI];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NPI; ++q) {
         pg[q] = q < np ? s_page[stg[q]] : -2;       // -1: hole in the table, -2: no second page
         kbase[q] = smem_u32(sK + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + wh * kHeadBytes;
         vbase[q] = smem_u32(sV + static_cast<size_t>(stg[q]) * a.stage_kv_bytes) + wh * kHeadBytes;
       }
       // warp-uniform: two pages of visible tokens -- everything below that deals with edges is skipped
-      const bool full = (pg[0] | pg[1]) >= 0 && (j + 2) * kBS <= open_end;
+      const bool full = (pg[0] | pg[NPI - 1]) >= 0 && (j + NPI) * kBS <= open_end;
 
       // ---- scales: lane l fetches those of token l & 15 of page l >> 4; shuffles hand them round ----
       float ksl = 1.f, vsl = 1.f;
       if constexpr (kQuant) {
-        const int q = lane >> 4;
-        if (full || (q == 0 ? pg[0] : pg[1]) >= 0) {
-          const uint32_t off = static_cast<uint32_t>(q == 0 ? stg[0] : stg[1]) * a.scale_bytes +
+        const int q = NPI == 2 ? lane >> 4 : 0;
+        if (full || (q == 0 ? pg[0] : pg[NPI - 1]) >= 0) {
+          const uint32_t off = static_cast<uint32_t>(q == 0 ? stg[0] : stg[NPI - 1]) * a.scale_bytes +
                                static_cast<uint32_t>(((lane & 15) * p.Hkv + kvh) * 2);
           ksl = lds_half(smem_u32(sKs) + off);
           vsl = lds_half(smem_u32(sVs) + off);
@@ -706,10 +714,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
 
       // ---- S = Q K^T : per page this lane gets tokens {2t, 2t+1, 8+2t, 9+2t} of its rows ----
-      float sc[RT][2][4];
+      float sc[RT][NPI][4];
       if constexpr (kI8) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < NPI; ++q)
 #pragma unroll
           for (int jn = 0; jn < 2; ++jn) {
             int acc[RT][4];
@@ -738,13 +746,13 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             }
           }
       } else {
-        float sacc[2][2][4];
+        float sacc[NPI][2][4];
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < NPI; ++q)
 #pragma unroll
           for (int i = 0; i < 2; ++i) { sacc[q][i][0] = sacc[q][i][1] = sacc[q][i][2] = sacc[q][i][3] = 0.f; }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < NPI; ++q) {
           if (pg[q] >= 0) {
             if constexpr (kQuant) {
 #pragma unroll
@@ -777,7 +785,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
         for (int rt = 0; rt < RT; ++rt)
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
+          for (int q = 0; q < NPI; ++q)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float s = sacc[q][e >> 1][2 * rt + (e & 1)];
@@ -786,9 +794,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
 
       // ---- scale / softcap / masks ----
-      float vsc[2][4];
+      float vsc[NPI][4];
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < NPI; ++q)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int tok = ((e >> 1) << 3) + 2 * t + (e & 1);
@@ -816,8 +824,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       bool grew = false;
 #pragma unroll
       for (int rt = 0; rt < RT; ++rt) {
-        float mx = fmaxf(fmaxf(fmaxf(sc[rt][0][0], sc[rt][0][1]), fmaxf(sc[rt][0][2], sc[rt][0][3])),
-                         fmaxf(fmaxf(sc[rt][1][0], sc[rt][1][1]), fmaxf(sc[rt][1][2], sc[rt][1][3])));
+        float mx = fmaxf(fmaxf(sc[rt][0][0], sc[rt][0][1]), fmaxf(sc[rt][0][2], sc[rt][0][3]));
+        if (NPI == 2) mx = fmaxf(mx, fmaxf(fmaxf(sc[rt][NPI - 1][0], sc[rt][NPI - 1][1]), fmaxf(sc[rt][NPI - 1][2], sc[rt][NPI - 1][3])));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         m_new[rt] = fmaxf(m_run[rt], mx);
@@ -838,12 +846,12 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
           m_run[rt] = m_new[rt];
         }
       }
-      uint32_t pb[RT][2][2];
+      uint32_t pb[RT][NPI][2];
 #pragma unroll
       for (int rt = 0; rt < RT; ++rt) {
         const float sub = kQuant ? msub[rt] - vexp : msub[rt];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < NPI; ++q) {
           float pr[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -858,7 +866,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
       // ---- O^T += V^T P^T : rows = 16 head-dim values per m-tile, cols = query rows ----
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NPI; ++q) {
         if (pg[q] >= 0) {
           // Slots of the last page beyond the sequence's end hold whatever the pool's owner left there; their P is
           // zero, but 0 * NaN (or 0 * inf) would still poison the row, so their V values are cleared as they are
@@ -923,18 +931,19 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
       __syncwarp();
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NPI; ++q) {
         if (q < np) {
           if (lane == 0) mbar_arrive(smem_u32(&bars[kMaxStages + stg[q]]));
-          if (++stage == NS) { stage = 0; phase ^= 1u; }
+          stage += PG;
+          if (stage >= NS) { stage -= NS; phase ^= 1u; }
         }
       }
     }
     if (!ok) break;
 
     // ---- end of this CTA's part of sequence b ----
-    const bool direct = (n_parts == 1);
-    const size_t slot_row0 = static_cast<size_t>(c + b) * HqNq;
+    const bool direct = PG == 1 && n_parts == 1;
+    const size_t slot_row0 = (static_cast<size_t>(c + b) * PG + pgrp) * HqNq;
 #pragma unroll
     for (int rt = 0; rt < RT; ++rt) {
       float l_row = l_run[rt];
@@ -1046,7 +1055,7 @@ int device_sm_count() {
 
 // how a launch is cut: heads per CTA, warps per head, CTAs along the units
 struct Shape {
-  int hpc, row_groups, gx;
+  int hpc, row_groups, page_groups, gx;
 };
 Shape pick_shape(int Hkv, int rows, int num_splits) {
   Shape s;
@@ -1057,29 +1066,40 @@ Shape pick_shape(int Hkv, int rows, int num_splits) {
   const int target = device_sm_count() * ctas_per_sm(s.hpc * s.row_groups);     // CTAs in flight over the whole grid
   s.gx = (target + hg - 1) / hg;
   if (num_splits > 0 && s.gx > num_splits) s.gx = num_splits;
+  s.page_groups = 1;
   return s;
 }
+// int8, 8 heads to a CTA: two warps per head can take its units in turn.  At 96 registers a warp that is what keeps up
+// with HBM (128 sequences of 512 to 32768 tokens: 785 -> 638 us), but every CTA then leaves two partials per sequence, which
+// costs 3 to 6 us where there is little else (8192 tokens: 18.7 against 24.8 us); so only from 32 units per CTA on, as far
+// as the longest sequence tells, and where the workspace has room for the partials.  e4m3, whose conversions spill at 96
+// registers, gains nothing (116.9 against 115.3 us).
+bool can_take_turns(const Shape& s, int rows, int kv_dtype) { return kv_dtype == 3 && rows <= 8 && s.hpc == 8; }
 
-template <int KV, int HPC, int D, int RT>
+template <int KV, int HPC, int D, int RT, int PG>
 cudaError_t launch_t(const CUtensorMap& tmK, const CUtensorMap& tmV, const KernelArgs& a, int gx, size_t smem,
                      cudaStream_t stream) {
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    kern<<<dim3(gx, a.HG), (a.hpc * a.row_groups + 1) * 32, smem, stream>>>(tmK, tmV, a);
+    kern<<<dim3(gx, a.HG), (a.hpc * a.row_groups * a.page_groups + 1) * 32, smem, stream>>>(tmK, tmV, a);
     return cudaGetLastError();
   };
-  return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true, RT>) : go(decode_paged_kernel<KV, HPC, D, false, RT>);
+  return a.inv_cap > 0.f ? go(decode_paged_kernel<KV, HPC, D, true, RT, PG>) : go(decode_paged_kernel<KV, HPC, D, false, RT, PG>);
 }
 
 template <int KV, int D>
 cudaError_t launch_kv(const CUtensorMap& tmK, const CUtensorMap& tmV, const KernelArgs& a, int gx, size_t smem, cudaStream_t stream) {
-  if (a.rows > 8) return launch_t<KV, 0, D, 2>(tmK, tmV, a, gx, smem, stream);
+  if (a.rows > 8) return launch_t<KV, 0, D, 2, 1>(tmK, tmV, a, gx, smem, stream);
   switch (a.hpc) {
-    case 8: return launch_t<KV, 8, D, 1>(tmK, tmV, a, gx, smem, stream);
-    case 4: return launch_t<KV, 4, D, 1>(tmK, tmV, a, gx, smem, stream);
-    case 2: return launch_t<KV, 2, D, 1>(tmK, tmV, a, gx, smem, stream);
-    default: return launch_t<KV, 1, D, 1>(tmK, tmV, a, gx, smem, stream);
+    case 8:
+      if constexpr (KV == KV_I8) {
+        if (a.page_groups == 2) return launch_t<KV, 8, D, 1, 2>(tmK, tmV, a, gx, smem, stream);
+      }
+      return launch_t<KV, 8, D, 1, 1>(tmK, tmV, a, gx, smem, stream);
+    case 4: return launch_t<KV, 4, D, 1, 1>(tmK, tmV, a, gx, smem, stream);
+    case 2: return launch_t<KV, 2, D, 1, 1>(tmK, tmV, a, gx, smem, stream);
+    default: return launch_t<KV, 1, D, 1, 1>(tmK, tmV, a, gx, smem, stream);
   }
 }
 
@@ -1114,16 +1134,20 @@ cudaError_t launch_combine_partials(const float* gathered, int R, long long rows
   return cudaGetLastError();
 }
 
-size_t decode_workspace_bytes(int B, int Hq, int Hkv, int Nq, int D, int max_kv_len, int num_splits) {
-  (void)max_kv_len;
+size_t decode_workspace_bytes(int B, int Hq, int Hkv, int Nq, int D, int kv_dtype, int num_splits, bool best) {
   if (B <= 0 || Hq <= 0 || Hkv <= 0 || Nq <= 0) return 16;
-  const Shape sh = pick_shape(Hkv, Hq / Hkv * Nq, num_splits);
-  return make_layout(B, Hq, Nq, Hkv / sh.hpc, sh.gx, D).total;
+  const int rows = Hq / Hkv * Nq;
+  const Shape sh = pick_shape(Hkv, rows, num_splits);
+  return make_layout(B, Hq, Nq, Hkv / sh.hpc, sh.gx, D, best && can_take_turns(sh, rows, kv_dtype) ? 2 : 1).total;
 }
 
 cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char* msg, size_t msg_len) {
   const bool quant = p.kv_dtype == 3 || p.kv_dtype == 4;
-  const Shape sh = pick_shape(p.Hkv, p.Hq / p.Hkv * p.Nq, p.num_splits);
+  const int rows = p.Hq / p.Hkv * p.Nq;
+  Shape sh = pick_shape(p.Hkv, rows, p.num_splits);
+  if (can_take_turns(sh, rows, p.kv_dtype) && static_cast<long long>(p.B) * ((p.max_kv_len + kBS - 1) / kBS) >= 32LL * sh.gx &&
+      p.workspace_bytes >= decode_workspace_bytes(p.B, p.Hq, p.Hkv, p.Nq, p.D, p.kv_dtype, p.num_splits, true))
+    sh.page_groups = 2;
   const int hpc = sh.hpc, gx = sh.gx;
   const int HG = p.Hkv / hpc;
   const int kD = p.D;
@@ -1140,12 +1164,13 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   KernelArgs a;
   a.p = p;
   a.upp = p.dense ? 1 : p.block_size / kBS;
-  a.lay = make_layout(p.B, p.Hq, p.Nq, HG, gx, kD);
+  a.lay = make_layout(p.B, p.Hq, p.Nq, HG, gx, kD, sh.page_groups);
   a.HG = HG;
   a.group = p.Hq / p.Hkv;
   a.rows = a.group * p.Nq;
   a.hpc = hpc;
   a.row_groups = sh.row_groups;
+  a.page_groups = sh.page_groups;
   a.stage_kv_bytes = hpc * kBS * row_bytes;
   a.scale_bytes = quant ? kBS * p.Hkv * 2 : 0;
   const size_t per_stage = 2 * static_cast<size_t>(a.stage_kv_bytes) + 2 * static_cast<size_t>(a.scale_bytes);
@@ -1265,7 +1290,7 @@ extern "C" int32_t b200fa_decode_paged_static(const b200fa_desc* d, const void* 
     b200fa::set_last_error("descriptor is null");
     return B200FA_ERR_INVALID_ARG;
   }
-  const size_t need = b200fa_decode_paged_workspace_bytes(d, max_kv_len);
+  const size_t need = d->B > 0 && d->Hkv > 0 ? b200fa::decode_workspace_bytes(d->B, d->Hq, d->Hkv, d->N, d->D, d->kv_dtype, d->num_splits, false) : 16;
   if (need > B200FA_STATIC_SCRATCH_BYTES) {
     char msg[256];
     snprintf(msg, sizeof(msg),

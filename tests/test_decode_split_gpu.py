@@ -94,3 +94,12 @@ def test_replayed_from_a_graph(dev, Nq):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, call())
+
+
+@pytest.mark.parametrize("Hq,Nq,softcap", [(32, 1, 0.0), (32, 2, 0.0), (8, 1, 30.0)])
+def test_two_warps_take_a_heads_units_in_turn(dev, Hq, Nq, softcap):
+    """int8 pools, 8 kv heads, 32 or more units per CTA if all sequences were as long as the longest: every CTA leaves two
+    partials per sequence, one of them without a unit where a sequence has a single one in the CTA."""
+    lens = [2000] + [(13 * i) % 90 for i in range(39)]
+    _run(dev, torch.bfloat16, "int8", len(lens), Hq, 8, Nq, lens, 795, softcap=softcap)
+    _run(dev, torch.float16, "int8", 1, Hq, 8, Nq, [76000], 796, softcap=softcap)

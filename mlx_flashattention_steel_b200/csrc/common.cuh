@@ -84,6 +84,14 @@ struct BwdParams {
 };
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch: the dependent kernel may start once every CTA of this one has said so (or ended), and
+// waits for this one's end, and its memory, before it reads what it wrote.  Every CTA of a dependent waits, also one that
+// has nothing to do: what follows in the stream waits for the dependent alone.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // order of work items
 // ---------------------------------------------------------------------------
 // Items are (tile, pair), pair = batch entry x head, tile 0 the longest of a causal mask.  They are dealt out in groups of

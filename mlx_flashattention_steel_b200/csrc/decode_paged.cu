@@ -103,9 +103,6 @@ struct KernelArgs {
 // ---------------------------------------------------------------------------
 // plan: page prefix sums of more than kSmemSeqs sequences
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 __device__ __forceinline__ int units_of(const int32_t* seq_lens, int i, int max_kv_len) {
   int len = seq_lens != nullptr ? seq_lens[i] : max_kv_len;
   len = len < 0 ? 0 : (len > max_kv_len ? max_kv_len : len);

@@ -12,7 +12,7 @@
 //     [c U / G, (c + 1) U / G), two CTAs per SM, whatever the mask leaves of each query tile.  A query tile that two or
 //     more CTAs share leaves partials (O, row max, row sum), which fwd_f32_merge_kernel adds up.  With one CTA per query
 //     tile the longest row of tiles set the time: 16 tiles on a causal N = 1024 where an SM's share is 7.4.
-// B = 1, H = 8, N = 1024, D = 128, causal: 153 -> 87 us.
+// B = 1, H = 8, N = 1024, D = 128, causal: 153 -> 72 us.
 #include "common.cuh"
 #include "launch.h"
 
@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_fwd_f32_kernel(const 
   const int tid = threadIdx.x, lane = tid & 31;
   const int ty = tid >> 4, tx = tid & 15;       // rows ty + 8 i, score columns tx + 16 j, output columns 4 tx + 64 c
   const bool split = a.part_ml != nullptr;
+  pdl_launch_dependents();
 
   // this CTA's first query tile, the place in its key tiles, and how many units it takes
   int bh, qt, at;
@@ -301,10 +302,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_fwd_f32_kernel(const 
   }
 }
 
-// Sum of the partials of every query tile that two or more CTAs of the split launch shared: one block per query tile,
-// one warp per row at a time, lanes along the head dim.  The tiles that one CTA finished cost a look at the shares.
+// Sum of the partials of every query tile that two or more CTAs of the split launch shared: one warp per row, lanes along
+// the head dim, eight blocks to a query tile.  Bound by latency: a row is two dependent reads, so a warp has one (one block
+// per query tile, eight rows per warp in turn: 19.7 us at B = 1, H = 8, N = 1024).  The tiles that one CTA finished cost a
+// look at the shares.
+constexpr int kMergeWarps = 8;
 template <int D>
-__global__ void __launch_bounds__(256) fwd_f32_merge_kernel(const F32Args a, int G) {
+__global__ void __launch_bounds__(kMergeWarps * 32) fwd_f32_merge_kernel(const F32Args a, int G) {
   const FwdParams& p = a.p;
   const int bh = blockIdx.x / a.n_qt, qt = blockIdx.x % a.n_qt;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -320,12 +324,15 @@ __global__ void __launch_bounds__(256) fwd_f32_merge_kernel(const F32Args a, int
   const KeyTiles t = key_tiles(qt, p.N, p.S, p.causal, p.window_left);
   const long long u1 = u0 + (t.end - t.begin) - 1;
   const int c0 = static_cast<int>(((u0 + 1) * G - 1) / a.units), c1 = static_cast<int>(((u1 + 1) * G - 1) / a.units);
+  pdl_wait();
   if (c0 == c1) return;
   const int first = 2 * c0 + (c0 * a.units / G < u0 ? 1 : 0);      // slot of the first part; those of the others are even
   const int head = bh % p.Hq, bb = bh / p.Hq;
   const bool live = lane * 4 < D;
-  for (int r = warp; r < kBQ && qt * kBQ + r < p.N; r += 8) {
+  const int r = blockIdx.y * kMergeWarps + warp;
+  if (qt * kBQ + r < p.N) {
     float m = -INFINITY;
+#pragma unroll 4
     for (int c = c0; c <= c1; ++c) m = fmaxf(m, a.part_ml[(static_cast<size_t>(c == c0 ? first : 2 * c) * kBQ + r) * 2]);
     const float ms = (m == -INFINITY) ? 0.f : m;
     float sum = 0.f;
@@ -398,8 +405,16 @@ cudaError_t launch_one(const FwdParams& p, int nbatch, int max_q, void* workspac
   kern<<<s.G, kThreads, smem, stream>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  fwd_f32_merge_kernel<D><<<static_cast<unsigned>(a.n_qt) * p.Hq * p.B, 256, 0, stream>>>(a, s.G);
-  return cudaGetLastError();
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(a.n_qt) * p.Hq * p.B, kBQ / kMergeWarps);
+  cfg.blockDim = dim3(kMergeWarps * 32);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fwd_f32_merge_kernel<D>, a, s.G);
 }
 
 }  // namespace

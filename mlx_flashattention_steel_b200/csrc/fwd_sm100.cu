@@ -242,11 +242,18 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   };
   const bool paged = p.block_table != nullptr;
   if constexpr (!PERSIST) {
-    int z = static_cast<int>(blockIdx.z);
+    int xt = static_cast<int>(blockIdx.x), h = static_cast<int>(blockIdx.y), z = static_cast<int>(blockIdx.z);
+    const int pairs = a.total_items / a.gx;
+    if (a.group > 1) {
+      int pair;
+      item_of(static_cast<int>(blockIdx.x), a.gx, pairs, a.group, xt, pair);
+      h = pair % a.gy;
+      z = pair / a.gy;
+    }
     // Batch entries of their own key counts: the longest first, so that the last CTAs to run are short (4 entries of
     // 1000 to 8000 keys, 512 queries, 32 heads: 169 us in the order they come).  Each warp ranks up to 32 of them.
-    if (p.kv_lens != nullptr && gridDim.z > 1 && gridDim.z <= 32) {
-      const int nz = static_cast<int>(gridDim.z);
+    const int nz = pairs / a.gy;
+    if (p.kv_lens != nullptr && nz > 1 && nz <= 32) {
       const int mine = lane < nz ? p.kv_lens[lane] : -1;
       int rank = 0;
       for (int i = 0; i < nz; ++i) {
@@ -254,13 +261,6 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (other > mine || (other == mine && i < lane)) ++rank;
       }
       z = __ffs(__ballot_sync(0xffffffffu, lane < nz && rank == z)) - 1;
-    }
-    int xt = static_cast<int>(blockIdx.x), h = static_cast<int>(blockIdx.y);
-    if (a.group > 1) {
-      int pair;
-      item_of(static_cast<int>(blockIdx.x), a.gx, a.total_items / a.gx, a.group, xt, pair);
-      h = pair % a.gy;
-      z = pair / a.gy;
     }
     item_geometry(xt, h, z, a.gx);
     if (q0 >= N) return;
@@ -1057,10 +1057,11 @@ static cudaError_t launch_hd(const FwdParams& p, int nbatch, int max_q, cudaStre
     }
   }
   a.counter = nullptr;
-  // dense calls with a common key count (others: longest batch entry first, see the kernel)
+  // with key counts of their own: one batch entry after the other, the longest first (see the kernel), and all its heads'
+  // long query tiles before their short ones
   a.group = 1;
-  if (p.cu_q == nullptr && p.kv_lens == nullptr && !FEAT && items < 0x7fffffffLL)
-    a.group = order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, items / grid.x);
+  if (p.cu_q == nullptr && !FEAT && items < 0x7fffffffLL)
+    a.group = p.kv_lens != nullptr ? (p.causal && p.window_left < 0 ? p.Hq : 1) : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, items / grid.x);
   if (a.group > 1) grid = dim3(static_cast<unsigned>(items), 1, 1);
   auto launch_1 = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);

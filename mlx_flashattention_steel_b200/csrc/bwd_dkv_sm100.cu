@@ -638,8 +638,8 @@ cudaError_t launch_bwd_dkv_sm100(const BwdParams& p, int dtype, int nbatch, int 
   const long long items = static_cast<long long>(a.gx) * a.gy * nbatch * a.parts;
   if (items > 0x7fffffffLL || p.work_counter == nullptr) return cudaErrorInvalidValue;
   a.total_items = static_cast<int>(items);
-  // an item streams Q and dO of one query head at a time; packed sequences are many and short enough
-  a.group = p.cu_q != nullptr ? 1 : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.N) * HD * 4, items / a.gx);
+  // an item streams Q and dO of one query head at a time
+  a.group = p.cu_q != nullptr ? kPackedGroup : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.N) * HD * 4, items / a.gx);
   a.counter = p.work_counter;
   int dev = 0, sm_count = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||

@@ -547,7 +547,7 @@ cudaError_t launch_bwd_dq_sm100(const BwdParams& p, int dtype, int nbatch, int m
   if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
   a.pairs = static_cast<int>(pairs);
   // an item streams K and V, which the query heads of a group share
-  a.group = p.cu_q != nullptr ? 1 : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, pairs);
+  a.group = p.cu_q != nullptr ? kPackedGroup : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.S) * HD * 4 / p.gqa, pairs);
   dim3 grid(static_cast<unsigned>(items), 1, 1);
   auto launch = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);

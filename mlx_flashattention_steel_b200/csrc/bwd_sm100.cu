@@ -691,8 +691,8 @@ cudaError_t launch_bwd_sm100_main(const BwdParams& p, int dtype, int nbatch, int
   const long long items = static_cast<long long>(a.gx) * a.gy * nbatch * a.parts;
   if (items > 0x7fffffffLL || p.work_counter == nullptr) return cudaErrorInvalidValue;
   a.total_items = static_cast<int>(items);
-  // an item streams Q and dO of one query head at a time; packed sequences are many and short enough
-  a.group = p.cu_q != nullptr ? 1 : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.N) * HD * 4, items / a.gx);
+  // an item streams Q and dO of one query head at a time
+  a.group = p.cu_q != nullptr ? kPackedGroup : order_group(p.causal != 0, p.window_left, static_cast<long long>(p.N) * HD * 4, items / a.gx);
   a.counter = p.work_counter;
   static int sm_count = 0;
   if (sm_count == 0) {

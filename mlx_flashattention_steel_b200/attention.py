@@ -693,7 +693,7 @@ def flash_attention_paged(
     ``num_splits`` caps how many CTAs share the page list (0 = one per SM).
 
     Short queries ((Hq/Hkv)*Nq <= 32; D = 128, or D = 64 with 16-bit pools; block_size a multiple
-    of 16) run the split-KV decode kernel with in-kernel combine; other shapes gather pages and attend
+    of 16) run the split-KV decode kernel and its merge kernel; other shapes gather pages and attend
     per sequence like the reference (mlx_mfa/attention.py:2944-2989).  When gradients are
     wanted (q or a 16-bit pool requires grad) every shape takes the gather route, whose
     backward adds dK / dV back into pool-shaped gradients page by page (2878-2940, 3020-3084).
@@ -738,7 +738,9 @@ def flash_attention_paged(
 
     # training: gradients flow through the gather route (gather, per-sequence attention, scatter-add into the pools)
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k_pages.requires_grad or v_pages.requires_grad)
-    decode_ok = ((Hq // Hkv) * Nq <= _MAX_DECODE_ROWS and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
+    rows = (Hq // Hkv) * Nq
+    # beyond 128 kv heads the stage ring may not hold two stages of an 8-bit pool's scales: only short queries try
+    decode_ok = (rows <= (_MAX_DECODE_ROWS if Hkv <= 128 else 8) and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
                  and not needs_grad)
     if decode_ok:
         out, lse = _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, float(scale),

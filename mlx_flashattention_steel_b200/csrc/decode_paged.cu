@@ -226,23 +226,31 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
   __shared__ float s_part[kMergeWarps][2];
   __shared__ float4 s_acc[kMergeWarps][32];
 
-  // units before sequence b, and of all: inputs of the launch, so nothing to wait for
-  int before = 0, all = 0;
-  for (int i = tid; i < p.B; i += blockDim.x) {
-    const int n = units_of(p.seq_lens, i, p.max_kv_len);
-    all += n;
-    if (i < b) before += n;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    before += __shfl_xor_sync(0xffffffffu, before, o);
-    all += __shfl_xor_sync(0xffffffffu, all, o);
-  }
-  if (lane == 0) { s_sum[0][warp] = before; s_sum[1][warp] = all; }
-  __syncthreads();
+  // units before sequence b, and of all: up to kSmemSeqs sequences from the lengths, which are inputs of the launch, so
+  // that there is nothing to wait for; beyond from the plan kernel's sums (a scan per block would be quadratic in B)
   long long s0 = 0, U = 0;
+  if (p.B <= kSmemSeqs) {
+    int before = 0, all = 0;
+    for (int i = tid; i < p.B; i += blockDim.x) {
+      const int n = units_of(p.seq_lens, i, p.max_kv_len);
+      all += n;
+      if (i < b) before += n;
+    }
 #pragma unroll
-  for (int i = 0; i < kMergeWarps; ++i) { s0 += s_sum[0][i]; U += s_sum[1][i]; }
+    for (int o = 16; o > 0; o >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    if (lane == 0) { s_sum[0][warp] = before; s_sum[1][warp] = all; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kMergeWarps; ++i) { s0 += s_sum[0][i]; U += s_sum[1][i]; }
+  } else {
+    pdl_wait();
+    const int* page_start = reinterpret_cast<const int*>(ws + a.lay.page_start);
+    s0 = __ldcg(page_start + b);
+    U = __ldcg(page_start + p.B);
+  }
   const int n_units = units_of(p.seq_lens, b, p.max_kv_len);
   int c_first = 0, n = 0;
   if (n_units > 0) {

@@ -992,8 +992,8 @@ bool fwd_sm100_supported(const FwdParams& p, int dtype, int D) {
 }
 
 // Persistent CTAs pay off where set-up, launch gaps and the first loads' latency are a visible part of a CTA's life
-// and the items are many and short: packed sequences (config 5's forward: 0.889 -> 0.837 ms with items dealt by number, 0.755 from a counter; ten unmasked key tiles per
-// query tile: +6 %).  They do not for a sliding window (config 3: -2.5 %: its query tiles are bounded by the fill and
+// and the items are many and short: packed sequences (config 5's forward: 0.889 -> 0.837 ms with items dealt by number,
+// 0.755 from a counter; ten unmasked key tiles per query tile: +6 %).  They do not for a sliding window (config 3: -2.5 %: its query tiles are bounded by the fill and
 // drain of the S -> softmax -> P.V pipeline, which a persistent CTA pays per item just the same) and they lose where
 // items are long and uneven (config 2: 2.23 -> 2.74 ms with the static deal), which keep one CTA per item and the
 // hardware scheduler's balancing.  `mode`: 0 = choose, 1 = persistent, 2 = one item per CTA (descriptor flags).

@@ -207,6 +207,7 @@ int32_t b200fa_fwd(const b200fa_desc* d, const void* q, const void* k, const voi
     dp.scale = d->scale; dp.softcap = d->softcap; dp.causal = d->causal ? 1 : 0;
     dp.num_splits = d->num_splits;
     dp.dense = 1;
+    dp.seq_lens = d->kv_lens;          // null: all S keys of every batch entry
     dp.k_bs = p.k_bs; dp.k_hs = p.k_hs; dp.k_rs = p.k_rs;
     dp.v_bs = p.v_bs; dp.v_hs = p.v_hs; dp.v_rs = p.v_rs;
     char msg[256] = "";

@@ -245,6 +245,20 @@ def test_dense_attention_with_per_sequence_key_counts(dev):
         assert_close(lse[b:b + 1], L, dtype, "lse")
 
 
+@pytest.mark.parametrize("quant", ["int8", "e4m3"])
+@pytest.mark.parametrize("D,block_size", [(64, 16), (128, 8)])
+@pytest.mark.parametrize("Nq,Hq", [(1, 8), (4, 4)])
+def test_short_queries_over_pools_the_paged_kernel_does_not_take(dev, quant, D, block_size, Nq, Hq):
+    """8-bit pools at head_dim 64, or with pages of 8 tokens: dequantised, then dense attention over per-sequence key
+    counts.  With at most 4 query tokens that is the dense decode route, which has to stop at each sequence's own end:
+    what the dequantised buffers hold beyond it is whatever the allocation found, NaNs here."""
+    lens = [0, 5, 300, 1030]
+    poison = [torch.full((4, 2, 1030, D), float("nan"), dtype=torch.bfloat16, device=dev) for _ in range(4)]
+    del poison
+    _run(dev, torch.bfloat16, quant, 4, Hq, 2, Nq, lens, 630, D=D, block_size=block_size)
+    _run(dev, torch.bfloat16, quant, 4, Hq, 2, Nq, lens, 631, D=D, block_size=block_size, causal=False, softcap=20.0, holes=True)
+
+
 @pytest.mark.parametrize("parts", [2, 3])
 def test_packed_partials_and_combine_kernel(dev, parts):
     """What the multi-GPU long-sequence path does, on one GPU: the page list of each sequence is cut into `parts`

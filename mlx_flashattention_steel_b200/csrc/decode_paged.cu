@@ -95,6 +95,7 @@ struct KernelArgs {
   int upp;              // 16-token units per page = block_size / 16
   int stage_kv_bytes;   // bytes of one K (or V) stage tile = HPC * kBS * row_bytes
   int scale_bytes;      // bytes of one scale page = kBS * Hkv * 2 (0 when not quantized)
+  int qlo_bytes;        // int8 pools: low bytes of Q, 1 KB per consumer warp and row tile
   float q_prescale;     // folded into Q (8-bit pools) or applied to the scores (16-bit pools)
   float cap_log2;       // softcap * log2(e)
   float inv_cap;        // 1 / softcap
@@ -164,6 +165,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};\n" ::"r"(addr), "r"(x), "r"(y));
 }
 __device__ __forceinline__ float lds_half(uint32_t addr) {
   unsigned short v;
@@ -382,7 +386,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   using MmaT = typename std::conditional<KV == KV_BF16, __nv_bfloat16, __half>::type;
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // carve: [stages] K tiles, [stages] V tiles, [stages] k scales, [stages] v scales, barriers, misc
+  // carve: [stages] K tiles, [stages] V tiles, [stages] k scales, [stages] v scales, low bytes of Q, barriers, misc
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const DecodeParams& p = a.p;
   const int NS = a.stages;
@@ -390,7 +394,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   unsigned char* sV = sK + static_cast<size_t>(NS) * a.stage_kv_bytes;
   unsigned char* sKs = sV + static_cast<size_t>(NS) * a.stage_kv_bytes;
   unsigned char* sVs = sKs + static_cast<size_t>(NS) * a.scale_bytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sVs + static_cast<size_t>(NS) * a.scale_bytes);  // full[NS], empty[NS]
+  unsigned char* s_qlo = sVs + static_cast<size_t>(NS) * a.scale_bytes;      // int8: lo bytes of Q, 1 KB per consumer warp and row tile
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_qlo + a.qlo_bytes);         // full[NS], empty[NS]
   int* s_page = reinterpret_cast<int*>(bars + 2 * kMaxStages);
   volatile int* s_abort = s_page + kMaxStages;
   int* s_page_start = const_cast<int*>(s_abort) + 1;     // int[B + 1] when B <= kSmemSeqs
@@ -568,16 +573,22 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
     // ---- Q fragments (A operand) ----
     // 16-bit and e4m3 pools: qa[s][0 | 1] = row tile 0 (k low, k high), [2 | 3] = row tile 1; kKS k-steps.
-    // int8 pools: the products run on the integer tensor cores, K as it is stored.  A row of Q is fixed point with 16
-    // bits below its largest value, q = qscale * (256 hi + lo), two signed bytes; 256 * hi.k + lo.k is exact in 32 bits
-    // (|.| <= 128 * 32639 * 128).  The step is max|q| / 32639, against a relative 2^-12 per value in f16; the widening
-    // of K to f16 (3 operations per two values) and half of the MMAs fall away.  One row tile: hi in rows 0..7, lo in
-    // rows 8..15 of one MMA; two row tiles: an MMA each.
+    // int8 pools: the products run on the integer tensor cores, K as it is stored (no widening, 3 operations per two
+    // values).  A row of Q is fixed point below its largest value: 65536 hi + 256 mid + lo, three signed bytes, in steps
+    // of max|q| / 8355000.  hi and mid, whose 256 * hi.k + mid.k is exact in 32 bits (|.| <= 128 * 32639 * 128), are one
+    // MMA (one row tile: hi in rows 0..7, mid in rows 8..15) or one each (two row tiles), and their step, 256 times that,
+    // is as exact as f16 for values down to a 24th of the largest.  They are enough while at most a quarter of a row's
+    // channels lie below that (zeros are exact); else K may be small in the few channels in which Q is large, and lo,
+    // from shared memory, joins in another MMA.  128 sequences of 512 to 32768 tokens: 634 us without lo in any row, 671
+    // with lo in all.
     constexpr bool kI8 = KV == KV_I8;
     constexpr int kQA = kI8 ? 4 * RT : kKS;
     constexpr int kQR = kI8 ? 4 : 2 * RT;
     uint32_t qa[kQA][kQR];
     float qscale[RT];
+    bool fine = false;                            // int8: lo is needed in some row of this warp
+    const uint32_t qlo = smem_u32(s_qlo + warp * (RT * 1024));
+    __syncwarp();
 #pragma unroll
     for (int rt = 0; rt < RT; ++rt) {
       const bool row_valid = row_of[rt] < rows;
@@ -606,27 +617,35 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
           // below 2^-100 the reciprocal would leave the float range; such a row scores zero, as its f16 values did
-          const float inv = mx > 7.9e-31f ? 32639.f / mx : 0.f;
-          qscale[rt] = mx * (1.f / 32639.f);
+          const float inv = mx > 7.9e-31f ? 8355000.f / mx : 0.f;
+          qscale[rt] = mx * (256.f / 8355000.f);
+          int small = 0;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) small += (f[i] != 0.f && fabsf(f[i]) < mx * (1.f / 24.f)) ? 1 : 0;
+          small += __shfl_xor_sync(0xffffffffu, small, 1);
+          small += __shfl_xor_sync(0xffffffffu, small, 2);
+          fine = __any_sync(0xffffffffu, fine || small > 32);
 #pragma unroll
           for (int s = 0; s < 4; ++s) {
-            uint32_t hi4[2], lo4[2];
+            uint32_t hi4[2], mid4[2], lo4[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              hi4[h] = lo4[h] = 0u;
+              hi4[h] = mid4[h] = lo4[h] = 0u;
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const int qi = __float2int_rn(f[8 * s + 4 * h + e] * inv);
-                const int hb = (qi + 128) >> 8, lb = qi - (hb << 8);
+                const int hb = (qi + 0x8080) >> 16, r = qi - (hb << 16), mb = (r + 0x80) >> 8, lb = r - (mb << 8);
                 hi4[h] |= (static_cast<uint32_t>(hb) & 0xffu) << (8 * e);
+                mid4[h] |= (static_cast<uint32_t>(mb) & 0xffu) << (8 * e);
                 lo4[h] |= (static_cast<uint32_t>(lb) & 0xffu) << (8 * e);
               }
             }
+            sts64(qlo + rt * 1024 + (s >> 1) * 512 + lane * 16 + (s & 1) * 8, lo4[0], lo4[1]);
             if constexpr (RT == 1) {
-              qa[s][0] = hi4[0]; qa[s][1] = lo4[0]; qa[s][2] = hi4[1]; qa[s][3] = lo4[1];
+              qa[s][0] = hi4[0]; qa[s][1] = mid4[0]; qa[s][2] = hi4[1]; qa[s][3] = mid4[1];
             } else {
               qa[s][rt] = hi4[0]; qa[s][2 + rt] = hi4[1];
-              qa[4 + s][rt] = lo4[0]; qa[4 + s][2 + rt] = lo4[1];
+              qa[4 + s][rt] = mid4[0]; qa[4 + s][2 + rt] = mid4[1];
             }
           }
         } else {
@@ -647,6 +666,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
       }
     }
+
+    __syncwarp();
 
     float oacc[RT][kKS][4];
 #pragma unroll
@@ -671,6 +692,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
     // Two pages per iteration: their loads, conversions and MMAs are independent, which gives the
     // scheduler twice the instruction-level parallelism, and one online-softmax step covers 32 tokens.
+    // FINE: with lo.  The loop exists twice: lo in a branch inside it cost every call 3 to 5 %.
+    auto walk = [&](auto fine_c) __attribute__((always_inline)) {
+    constexpr bool FINE = decltype(fine_c)::value;
     for (int j = j_lo; j < j_hi; j += 2) {
       const int np = min(NPI, j_hi - j);
       int stg[NPI], pg[NPI];
@@ -725,9 +749,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         for (int q = 0; q < NPI; ++q)
 #pragma unroll
           for (int jn = 0; jn < 2; ++jn) {
-            int acc[RT][4];
+            int acc[RT + 1][4];                               // (hi | mid) or hi, mid; then lo
 #pragma unroll
-            for (int rt = 0; rt < RT; ++rt) { acc[rt][0] = acc[rt][1] = acc[rt][2] = acc[rt][3] = 0; }
+            for (int h = 0; h <= RT; ++h) { acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0; }
             if (pg[q] >= 0) {
               const uint32_t rowa = kbase[q] + (8 * jn + g) * 128;           // token 8 jn + g
               const uint4 w0 = lds128(rowa + (((2 * t) ^ g) << 4));
@@ -736,17 +760,26 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
               for (int s = 0; s < 4; ++s)
 #pragma unroll
-                for (int h = 0; h < RT; ++h)                                  // RT == 2: acc[0] = hi, acc[1] = lo
+                for (int h = 0; h < RT; ++h)                                  // RT == 2: acc[0] = hi, acc[1] = mid
                   mma16832_s8(acc[h], qa[4 * h + s], words[2 * s], words[2 * s + 1]);
+              if constexpr (FINE) {
+#pragma unroll
+                for (int s = 0; s < 4; s += 2) {
+                  const uint4 a0 = lds128(qlo + s * 256 + lane * 16);
+                  const uint4 a1 = RT == 2 ? lds128(qlo + 1024 + s * 256 + lane * 16) : make_uint4(0u, 0u, 0u, 0u);
+                  const uint32_t x[4] = {a0.x, a1.x, a0.y, a1.y}, y[4] = {a0.z, a1.z, a0.w, a1.w};
+                  mma16832_s8(acc[RT], x, words[2 * s], words[2 * s + 1]);
+                  mma16832_s8(acc[RT], y, words[2 * s + 2], words[2 * s + 3]);
+                }
+              }
             }
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              if constexpr (RT == 1) {
-                sc[0][q][2 * jn + e] = __int2float_rn((acc[0][e] << 8) + acc[0][2 + e]) * qscale[0];
-              } else {
 #pragma unroll
-                for (int rt = 0; rt < RT; ++rt)
-                  sc[rt][q][2 * jn + e] = __int2float_rn((acc[0][2 * rt + e] << 8) + acc[1][2 * rt + e]) * qscale[rt];
+              for (int rt = 0; rt < RT; ++rt) {
+                float x = __int2float_rn((acc[0][2 * rt + e] << 8) + (RT == 1 ? acc[0][2 + e] : acc[RT - 1][2 * rt + e]));
+                if constexpr (FINE) x = fmaf(__int2float_rn(acc[RT][2 * rt + e]), 1.f / 256.f, x);
+                sc[rt][q][2 * jn + e] = x * qscale[rt];
               }
             }
           }
@@ -944,6 +977,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
       }
     }
+    };
+    if (kI8 && fine) walk(std::bool_constant<kI8>{});
+    else walk(std::false_type{});
     if (!ok) break;
 
     // ---- end of this CTA's part of sequence b ----
@@ -1178,6 +1214,7 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.page_groups = sh.page_groups;
   a.stage_kv_bytes = hpc * kBS * row_bytes;
   a.scale_bytes = quant ? kBS * p.Hkv * 2 : 0;
+  a.qlo_bytes = p.kv_dtype == 3 ? hpc * sh.row_groups * sh.page_groups * (rows > 8 ? 2048 : 1024) : 0;
   const size_t per_stage = 2 * static_cast<size_t>(a.stage_kv_bytes) + 2 * static_cast<size_t>(a.scale_bytes);
   // several small CTAs share an SM when a CTA holds few heads
   const int per_sm = ctas_per_sm(hpc * sh.row_groups);
@@ -1193,7 +1230,7 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.q_prescale = sc;
   a.cap_log2 = p.softcap * kLog2e;
   a.inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
-  const size_t smem = 1024 + static_cast<size_t>(stages) * per_stage + 2 * kMaxStages * 8 + kMaxStages * 4 + 64 +
+  const size_t smem = 1024 + static_cast<size_t>(stages) * per_stage + a.qlo_bytes + 2 * kMaxStages * 8 + kMaxStages * 4 + 64 +
                       (p.B <= kSmemSeqs ? sizeof(int) * (static_cast<size_t>(p.B) + 1) : 0);
 
   // tensor maps, in bytes: (128 B, tokens, 128-byte halves of a row, heads, batch).  A pool is one "batch" of

@@ -103,3 +103,31 @@ def test_two_warps_take_a_heads_units_in_turn(dev, Hq, Nq, softcap):
     lens = [2000] + [(13 * i) % 90 for i in range(39)]
     _run(dev, torch.bfloat16, "int8", len(lens), Hq, 8, Nq, lens, 795, softcap=softcap)
     _run(dev, torch.float16, "int8", 1, Hq, 8, Nq, [76000], 796, softcap=softcap)
+
+
+@pytest.mark.parametrize("peak", [3.0, 30.0, 300.0])
+@pytest.mark.parametrize("Hkv,Nq,max_len", [(2, 1, 16), (2, 4, 16), (8, 2, 1200)])
+def test_int8_queries_keep_f16_precision(dev, Hkv, Nq, max_len, peak):
+    """Scores of int8 pools are at least as exact as with Q rounded to f16, whichever channels K weighs: one channel of Q
+    is `peak` and K has a hundredth of its usual size there.  A sequence of one token has its score as its lse.  An f16
+    rounding of q_d is off by at most 2^-11 |q_d| and by 2^-11 |q_d| / sqrt(3) in the mean, if evenly spread; the errors
+    of the channels add up as squares.  (8, 2, 1200): two warps per head."""
+    B, G = 64, 4
+    g = torch.Generator().manual_seed(799)
+    q = torch.randn((B, Hkv * G, Nq, 128), generator=g)
+    q[..., 37] = peak
+    q = q.to(torch.float16)
+    P = B * ((max_len + 15) // 16)
+    k = torch.randint(-127, 128, (P, 16, Hkv, 128), generator=g, dtype=torch.int8)
+    k[..., 37] = torch.randint(-1, 2, k.shape[:-1], generator=g, dtype=torch.int8)
+    ks = torch.full((P, 16, Hkv), 0.02, dtype=torch.float16)
+    table = torch.arange(P, dtype=torch.int32).view(B, -1)
+    lens = torch.ones(B, dtype=torch.int32)
+    _, lse = fa.flash_attention_paged(*(x.to(dev) for x in (q, k, k, table, lens)), k_scale=ks.to(dev), v_scale=ks.to(dev),
+                                      max_kv_len=max_len, return_lse=True)
+    kd = (k[table[:, 0].long(), 0].double() * ks[0, 0, 0].double()).repeat_interleave(G, dim=1)      # [B, Hq, 128]
+    c = 128 ** -0.5 * 1.4426950408889634
+    terms = q.double() * kd.unsqueeze(2) * c
+    err = lse.double().cpu() - terms.sum(-1)
+    bound = 2.0 ** -11 / 3 ** 0.5 * terms.pow(2).sum(-1).mean().sqrt()
+    assert float(err.pow(2).mean().sqrt()) <= float(bound)

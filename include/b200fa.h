@@ -182,7 +182,8 @@ int32_t b200fa_bwd_varlen(const b200fa_desc* d, const void* q, const void* k, co
  *   causal is per-sequence lower-right aligned.
  * `num_pages` bounds the block_table entries (larger ones are treated as holes and reported through the error word).
  * Slots of a sequence's last page beyond seq_lens[b] may hold anything, NaN patterns included: they are masked
- * before they reach the arithmetic.  The workspace size depends on B, Hq, Hkv, N, kv_dtype and num_splits only; max_kv_len is
+ * before they reach the arithmetic.  A NaN in a query row makes that row of `out` NaN, over 8-bit pools an infinity too.
+ * The workspace size depends on B, Hq, Hkv, N, kv_dtype and num_splits only; max_kv_len is
  * taken by the query so that the signature can stay when that changes.
  */
 size_t  b200fa_decode_paged_workspace_bytes(const b200fa_desc* d, int32_t max_kv_len);

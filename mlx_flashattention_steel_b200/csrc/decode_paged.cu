@@ -201,7 +201,7 @@ __device__ __forceinline__ void mma16832_s8(int (&c)[4], const uint32_t (&a)[4],
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ float clamp_h(float x) { return fminf(fmaxf(x, -65504.f), 65504.f); }
+__device__ __forceinline__ float clamp_h(float x) { return fabsf(x) <= 3.4028235e38f ? fminf(fmaxf(x, -65504.f), 65504.f) : NAN; }
 
 // CTA index (of G) whose unit range [c*U/G, (c+1)*U/G) holds unit u
 __device__ __forceinline__ int cta_of_unit(long long u, int G, long long U) {
@@ -579,7 +579,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     // MMA (one row tile: hi in rows 0..7, mid in rows 8..15) or one each (two row tiles), and their step, 256 times that,
     // is as exact as f16 for values down to a 24th of the largest.  They are enough while at most a quarter of a row's
     // channels lie below that (zeros are exact); else K may be small in the few channels in which Q is large, and lo,
-    // from shared memory, joins in another MMA.  128 sequences of 512 to 32768 tokens: 634 us without lo in any row, 671
+    // from shared memory, joins in another MMA.  128 sequences of 512 to 32768 tokens: 626 us without lo in any row, 687
     // with lo in all.
     constexpr bool kI8 = KV == KV_I8;
     constexpr int kQA = kI8 ? 4 * RT : kKS;
@@ -606,25 +606,31 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
           for (int e = 0; e < 4; ++e) {
             const float2 v2 = p.q_dtype == 0 ? __half22float2(*reinterpret_cast<const __half2*>(&ww[e]))
                                              : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww[e]));
-            f[i * 8 + e * 2] = clamp_h(v2.x * a.q_prescale);
-            f[i * 8 + e * 2 + 1] = clamp_h(v2.y * a.q_prescale);
+            f[i * 8 + e * 2] = v2.x * a.q_prescale;
+            f[i * 8 + e * 2 + 1] = v2.y * a.q_prescale;
           }
         }
-        if constexpr (kI8) {
-          float mx = 0.f;
+        // largest magnitude of the row, as bits: infinities and NaNs are above every number.  Such a row's scores are NaN.
+        uint32_t mb = 0u;
+        if constexpr (kI8 || RT == 2) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fabsf(f[i]));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-          // below 2^-100 the reciprocal would leave the float range; such a row scores zero, as its f16 values did
-          const float inv = mx > 7.9e-31f ? 8355000.f / mx : 0.f;
-          qscale[rt] = mx * (256.f / 8355000.f);
+          for (int i = 0; i < 32; ++i) mb = max(mb, __float_as_uint(f[i]) & 0x7fffffffu);
+          mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+          mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+        }
+        const bool finite = mb < 0x7f800000u;
+        if constexpr (kI8) {
+          const float mx = __uint_as_float(mb);
+          // below 2^-100 the reciprocal would leave the float range; such a row scores zero
+          const float inv = finite && mx > 7.9e-31f ? 8355000.f / mx : 0.f;
+          qscale[rt] = finite ? mx * (256.f / 8355000.f) : NAN;
           int small = 0;
 #pragma unroll
           for (int i = 0; i < 32; ++i) small += (f[i] != 0.f && fabsf(f[i]) < mx * (1.f / 24.f)) ? 1 : 0;
           small += __shfl_xor_sync(0xffffffffu, small, 1);
           small += __shfl_xor_sync(0xffffffffu, small, 2);
-          fine = __any_sync(0xffffffffu, fine || small > 32);
+          const bool low = finite && small > 32;            // rows that do without have lo = 0: no row's bits depend on another's
+          fine = __any_sync(0xffffffffu, fine || low);
 #pragma unroll
           for (int s = 0; s < 4; ++s) {
             uint32_t hi4[2], mid4[2], lo4[2];
@@ -634,13 +640,13 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const int qi = __float2int_rn(f[8 * s + 4 * h + e] * inv);
-                const int hb = (qi + 0x8080) >> 16, r = qi - (hb << 16), mb = (r + 0x80) >> 8, lb = r - (mb << 8);
+                const int hb = (qi + 0x8080) >> 16, r = qi - (hb << 16), mib = (r + 0x80) >> 8, lb = r - (mib << 8);
                 hi4[h] |= (static_cast<uint32_t>(hb) & 0xffu) << (8 * e);
-                mid4[h] |= (static_cast<uint32_t>(mb) & 0xffu) << (8 * e);
+                mid4[h] |= (static_cast<uint32_t>(mib) & 0xffu) << (8 * e);
                 lo4[h] |= (static_cast<uint32_t>(lb) & 0xffu) << (8 * e);
               }
             }
-            sts64(qlo + rt * 1024 + (s >> 1) * 512 + lane * 16 + (s & 1) * 8, lo4[0], lo4[1]);
+            sts64(qlo + rt * 1024 + (s >> 1) * 512 + lane * 16 + (s & 1) * 8, low ? lo4[0] : 0u, low ? lo4[1] : 0u);
             if constexpr (RT == 1) {
               qa[s][0] = hi4[0]; qa[s][1] = mid4[0]; qa[s][2] = hi4[1]; qa[s][3] = mid4[1];
             } else {
@@ -649,11 +655,20 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             }
           }
         } else {
+          // f16.  Up to 8 rows: values beyond its range become its largest.  More rows, whose calls the prefill kernel
+          // ran in the query's own type before: the row over a power of two, its largest value in [2^13, 2^14).
+          float down = 1.f;
+          if constexpr (RT == 2) {
+            const uint32_t ex = min(max(mb >> 23, 15u), 253u);
+            down = __uint_as_float((267u - ex) << 23);                          // 2^(13 - (ex - 127))
+            qscale[rt] = finite ? __uint_as_float((ex - 13u) << 23) : NAN;
+          }
+          auto h = [&](float x) { return RT == 2 ? x * down : clamp_h(x); };
           // k-step s uses d = 32t + 4s + {0,1 | 2,3}
 #pragma unroll
           for (int s = 0; s < 8; ++s) {
-            qa[s][2 * rt] = pack_h2(f[4 * s], f[4 * s + 1]);
-            qa[s][2 * rt + 1] = pack_h2(f[4 * s + 2], f[4 * s + 3]);
+            qa[s][2 * rt] = pack_h2(h(f[4 * s]), h(f[4 * s + 1]));
+            qa[s][2 * rt + 1] = pack_h2(h(f[4 * s + 2]), h(f[4 * s + 3]));
           }
         }
       } else {
@@ -827,7 +842,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float s = sacc[q][e >> 1][2 * rt + (e & 1)];
-              sc[rt][q][e] = kQuant ? s : s * a.q_prescale;
+              sc[rt][q][e] = !kQuant ? s * a.q_prescale : (RT == 2 ? s * qscale[rt] : s);
             }
       }
 

@@ -131,3 +131,36 @@ def test_int8_queries_keep_f16_precision(dev, Hkv, Nq, max_len, peak):
     err = lse.double().cpu() - terms.sum(-1)
     bound = 2.0 ** -11 / 3 ** 0.5 * terms.pow(2).sum(-1).mean().sqrt()
     assert float(err.pow(2).mean().sqrt()) <= float(bound)
+
+
+@pytest.mark.parametrize("quant", [None, "int8", "e4m3"])
+@pytest.mark.parametrize("Nq", [1, 4])
+def test_queries_that_are_not_finite(dev, quant, Nq):
+    """A NaN or an infinity in a query row makes that row NaN, as the prefill route has it, and no other."""
+    pg = make_paged(2, 2, 128, 16, [40, 3000], torch.bfloat16, 775, quant=quant)
+    q = randn((2, 8, Nq, 128), torch.bfloat16, 776)
+    bad = q.clone()
+    bad[0, 1, Nq - 1, 3], bad[1, 6, 0, 127], bad[1, 7, 0, 64] = float("nan"), float("nan"), float("inf")
+    rows = torch.zeros(q.shape[:3], dtype=torch.bool)
+    rows[0, 1, Nq - 1] = rows[1, 6, 0] = rows[1, 7, 0] = True
+    kw = {} if quant is None else dict(k_scale=pg["k_scale"].to(dev), v_scale=pg["v_scale"].to(dev))
+    args = [pg[n].to(dev) for n in ("k", "v", "block_table", "seq_lens")]
+    out = fa.flash_attention_paged(bad.to(dev), *args, **kw).cpu()
+    assert torch.isnan(out[rows]).all()
+    assert torch.equal(out[~rows], fa.flash_attention_paged(q.to(dev), *args, **kw).cpu()[~rows])
+
+
+@pytest.mark.parametrize("quant", ["int8", "e4m3"])
+def test_wide_rows_beyond_f16(dev, quant):
+    """Queries whose scaled values leave f16's range: 8-bit pools, 16 rows per kv head."""
+    pg = make_paged(2, 2, 128, 16, [40, 700], torch.bfloat16, 777, quant=quant)
+    q = randn((2, 8, 4, 128), torch.bfloat16, 778)
+    q[:, ::2] *= 3e6
+    q[:, 1] *= 1e-9
+    # a power of two, so that K is the same number in bf16: the largest score is far from the others, not from its rounding
+    pg["k_scale"] = torch.full_like(pg["k_scale"], 2.0 ** -5 if quant == "int8" else 2.0 ** -7)
+    args = [x.to(dev) for x in (q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"])]
+    kw = dict(k_scale=pg["k_scale"], v_scale=pg["v_scale"])
+    out = fa.flash_attention_paged(*args, causal=True, **{n: x.to(dev) for n, x in kw.items()})
+    O, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, **kw)
+    assert_close(out, O, torch.bfloat16)

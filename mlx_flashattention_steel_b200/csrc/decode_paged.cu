@@ -700,10 +700,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     // Tokens before this one are visible to every row and inside the sequence: steps that end before it need no masks.
     const int open_end = p.causal ? min(len, len - p.Nq + 1) : len;
     // Quantised pools: P goes into its 16-bit operand multiplied by v_scale.  Every exponent is shifted by vexp, minus
-    // the exponent of the part's first v scale, so that the product stays inside f16's normal range; the row sum
-    // carries the same power of two and it cancels.
-    float vexp = 0.f;
-    bool first_page = true;
+    // the exponent of the largest v scale of the first step, so that the product stays inside f16's normal range; the
+    // row sum carries the same power of two and it cancels.  A scale of vlimit = 2^(15 - vexp) or more moves vexp, and
+    // what has been summed with it, down.
+    float vexp = 0.f, vlimit = 0.f;
 
     // Two pages per iteration: their loads, conversions and MMAs are independent, which gives the
     // scheduler twice the instruction-level parallelism, and one online-softmax step covers 32 tokens.
@@ -738,7 +738,8 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       const bool full = (pg[0] | pg[NPI - 1]) >= 0 && (j + NPI) * kBS <= open_end;
 
       // ---- scales: lane l fetches those of token l & 15 of page l >> 4; shuffles hand them round ----
-      float ksl = 1.f, vsl = 1.f;
+      float ksl = 1.f, vsl = 0.f;
+      bool vmove = false;
       if constexpr (kQuant) {
         const int q = NPI == 2 ? lane >> 4 : 0;
         if (full || (q == 0 ? pg[0] : pg[NPI - 1]) >= 0) {
@@ -747,14 +748,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
           ksl = lds_half(smem_u32(sKs) + off);
           vsl = lds_half(smem_u32(sVs) + off);
         }
-        if (first_page) {
-          const float v0 = __shfl_sync(0xffffffffu, vsl, 0);
-          const uint32_t bits = __float_as_uint(v0) & 0x7f800000u;
-          vexp = (bits == 0u || bits == 0x7f800000u) ? 0.f : 127.f - static_cast<float>(bits >> 23);
-          first_page = false;
-        }
         // whatever the scale of a slot beyond the sequence holds (it may be a NaN pattern)
         if (!full && (j + q) * kBS + (lane & 15) >= len) vsl = 0.f;
+        vmove = vsl > vlimit && vsl < INFINITY;
       }
 
       // ---- S = Q K^T : per page this lane gets tokens {2t, 2t+1, 8+2t, 9+2t} of its rows ----
@@ -885,10 +881,17 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         msub[rt] = (m_new[rt] == -INFINITY) ? 0.f : m_new[rt];
         grew = grew || m_new[rt] > m_run[rt];
       }
-      if (__any_sync(0xffffffffu, grew)) {
+      if (__any_sync(0xffffffffu, grew || vmove)) {
+        float shift = 0.f;
+        if (kQuant && __any_sync(0xffffffffu, vmove)) {
+          const unsigned top = __reduce_max_sync(0xffffffffu, vmove ? __float_as_uint(vsl) : 0u);
+          shift = 127.f - static_cast<float>(top >> 23) - vexp;
+          vexp += shift;
+          vlimit = exp2f(15.f - vexp);
+        }
 #pragma unroll
         for (int rt = 0; rt < RT; ++rt) {
-          const float corr = fast_exp2(m_run[rt] - msub[rt]);       // 1 when unchanged, 0 from -inf
+          const float corr = fast_exp2(m_run[rt] - msub[rt] + shift);       // 1 when nothing changed, 0 from -inf
           l_run[rt] *= corr;
           const float c0 = __shfl_sync(0xffffffffu, corr, (2 * t) * 4);
           const float c1 = __shfl_sync(0xffffffffu, corr, (2 * t + 1) * 4);

@@ -164,3 +164,27 @@ def test_wide_rows_beyond_f16(dev, quant):
     out = fa.flash_attention_paged(*args, causal=True, **{n: x.to(dev) for n, x in kw.items()})
     O, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, **kw)
     assert_close(out, O, torch.bfloat16)
+
+
+@pytest.mark.parametrize("quant", ["int8", "e4m3"])
+@pytest.mark.parametrize("Nq", [1, 4])
+def test_value_scales_far_apart(dev, quant, Nq):
+    """P is multiplied by v_scale over a power of two near the first scale: later scales may be far above it (a first
+    token of zeros, stored with the smallest scale there is)."""
+    lens = [700, 37, 40]
+    pg = make_paged(3, 2, 128, 16, lens, torch.bfloat16, 785, quant=quant)
+    for b in range(3):
+        page = int(pg["block_table"][b, 0])
+        pg["v"][page, 0] = 0
+        pg["v_scale"][page, 0] = 2.0 ** -24
+    late = int(pg["block_table"][0, 20])
+    pg["v_scale"][late] *= 512.0
+    q = randn((3, 8, Nq, 128), torch.bfloat16, 786)
+    kw = dict(k_scale=pg["k_scale"], v_scale=pg["v_scale"])
+    out, lse = fa.flash_attention_paged(*(x.to(dev) for x in (q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"])), causal=True,
+                                        return_lse=True, **{n: x.to(dev) for n, x in kw.items()})
+    O, L = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, **kw)
+    assert_close(lse, L, torch.bfloat16, "lse")
+    assert_close(out[1:], O[1:], torch.bfloat16)
+    # the values of one page are 512 times the others': the same 2e-2, relative to the largest
+    assert_close(out[:1] / float(O[0].abs().max()), O[:1] / float(O[0].abs().max()), torch.bfloat16)

@@ -36,9 +36,10 @@ struct F32Args {
   float* part_o;             // [2 G][64][D], not normalised
 };
 
-// key tiles [begin, end) of query tile qt; a tile without any keeps one unit, which is masked throughout
+// key tiles [begin, end) of query tile qt; a tile without any (blind) keeps one unit, which is masked throughout
 struct KeyTiles {
   int begin, end;
+  bool blind;
 };
 __host__ __device__ inline KeyTiles key_tiles(int qt, int N, int S, int causal, int window_left) {
   const int q0 = qt * kBQ, off = S - N;
@@ -49,7 +50,8 @@ __host__ __device__ inline KeyTiles key_tiles(int qt, int N, int S, int causal, 
   KeyTiles t;
   t.begin = k_lo / kBK;
   t.end = k_hi > 0 ? (k_hi + kBK - 1) / kBK : 0;
-  if (t.end <= t.begin) t.end = t.begin + 1;
+  t.blind = t.end <= t.begin;
+  if (t.blind) t.end = t.begin + 1;
   return t;
 }
 
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_fwd_f32_kernel(const 
     const KeyTiles kts = key_tiles(qt, N, S, p.causal, p.window_left);
     const int kt_begin = kts.begin + at;
     const int kt_end = static_cast<int>(min(static_cast<long long>(kts.end), kt_begin + left));
+    const int S_read = kts.blind ? 0 : S;        // what no row sees is not read: 0 * inf would be NaN
     const bool whole = at == 0 && kt_end == kts.end;
 
     const float* qg = reinterpret_cast<const float*>(p.q) + bb * p.q_bs + head * p.q_hs + q_begin * p.q_rs;
@@ -164,9 +167,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_fwd_f32_kernel(const 
     for (int kt = kt_begin; kt < kt_end; ++kt) {
       const int k0 = kt * kBK;
       __syncthreads();  // previous tile fully consumed
-      load_rows<D, LD>(sK, kg, p.k_rs, k0, S, tid);
+      load_rows<D, LD>(sK, kg, p.k_rs, k0, S_read, tid);
       cp_async_commit();                       // Q (first tile) and K
-      load_rows<D, D>(sV, vg, p.v_rs, k0, S, tid);
+      load_rows<D, D>(sV, vg, p.v_rs, k0, S_read, tid);
       cp_async_commit();
       cp_async_wait<1>();
       __syncthreads();

@@ -46,3 +46,17 @@ def test_even_shares_with_alibi(dev):
     out = fa.flash_attention(q.to(dev), k.to(dev), v.to(dev), causal=True, alibi_slopes=slopes.to(dev))
     O, _, _ = orc.sdpa(q, k, v, causal=True, alibi_slopes=slopes)
     assert_close(out, O, torch.float32)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_query_tiles_without_a_key_read_no_values(dev, value):
+    """Causal, more queries than keys: the query tiles that see no key are zeros whatever V holds."""
+    q, k, v = randn((1, 2, 300, 64), torch.float32, 820), randn((1, 2, 100, 64), torch.float32, 821), randn((1, 2, 100, 64), torch.float32, 822)
+    k[0, 0, 0], v[0, 0, 0] = value, value
+    out, lse = fa.flash_attention(q.to(dev), k.to(dev), v.to(dev), causal=True, return_lse=True)
+    assert not out[:, :, :192].any() and torch.isneginf(lse[:, :, :192]).all()           # rows up to 199 are blind: three tiles of 64
+    O, _, _ = orc.sdpa(q[:, 1:, 200:], k[:, 1:], v[:, 1:], causal=True)
+    assert_close(out[:, 1:, 200:], O, torch.float32)
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=dev) for n in (300, 100))
+    out = fa.flash_attention_varlen(q.to(dev), k.to(dev), v.to(dev), cu_q, cu_k, 300, 100, causal=True)
+    assert not out[:, :, :192].any()

@@ -243,17 +243,16 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const bool paged = p.block_table != nullptr;
   if constexpr (!PERSIST) {
     int xt = static_cast<int>(blockIdx.x), h = static_cast<int>(blockIdx.y), z = static_cast<int>(blockIdx.z);
-    const int pairs = a.total_items / a.gx;
     if (a.group > 1) {
       int pair;
-      item_of(static_cast<int>(blockIdx.x), a.gx, pairs, a.group, xt, pair);
+      item_of(static_cast<int>(blockIdx.x), a.gx, a.total_items / a.gx, a.group, xt, pair);
       h = pair % a.gy;
       z = pair / a.gy;
     }
     // Batch entries of their own key counts: the longest first, so that the last CTAs to run are short (4 entries of
     // 1000 to 8000 keys, 512 queries, 32 heads: 169 us in the order they come).  Each warp ranks up to 32 of them.
-    const int nz = pairs / a.gy;
-    if (p.kv_lens != nullptr && nz > 1 && nz <= 32) {
+    const int nz = p.kv_lens != nullptr ? a.total_items / a.gx / a.gy : 1;
+    if (nz > 1 && nz <= 32) {
       const int mine = lane < nz ? p.kv_lens[lane] : -1;
       int rank = 0;
       for (int i = 0; i < nz; ++i) {
@@ -391,7 +390,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(bar(BAR_O_STAGED), 4);
     mbar_init(bar(BAR_O_FINAL), 1);
     mbar_init(bar(BAR_Q_FREE), 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; PERSIST && s < 2; ++s) {
       mbar_init(bar(BAR_ITEM_FULL + s), 1);
       mbar_init(bar(BAR_ITEM_FREE + s), 5);
     }

@@ -739,8 +739,10 @@ def flash_attention_paged(
     # training: gradients flow through the gather route (gather, per-sequence attention, scatter-add into the pools)
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k_pages.requires_grad or v_pages.requires_grad)
     rows = (Hq // Hkv) * Nq
-    # beyond 128 kv heads the stage ring may not hold two stages of an 8-bit pool's scales: only short queries try
-    decode_ok = (rows <= (_MAX_DECODE_ROWS if Hkv <= 128 else 8) and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
+    # Longer queries take it where the prefill route's calls all fit: beyond 128 kv heads the stage ring may not hold two
+    # stages of an 8-bit pool's scales, and the kernel's copies of the scales start on 16-byte boundaries.
+    wide = Hkv <= 128 and not (quant and (k_scale.data_ptr() | v_scale.data_ptr()) % 16)
+    decode_ok = (rows <= (_MAX_DECODE_ROWS if wide else 8) and (D == 128 or (D == 64 and not quant)) and block_size % 16 == 0
                  and not needs_grad)
     if decode_ok:
         out, lse = _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, float(scale),

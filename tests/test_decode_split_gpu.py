@@ -188,3 +188,20 @@ def test_value_scales_far_apart(dev, quant, Nq):
     assert_close(out[1:], O[1:], torch.bfloat16)
     # the values of one page are 512 times the others': the same 2e-2, relative to the largest
     assert_close(out[:1] / float(O[0].abs().max()), O[:1] / float(O[0].abs().max()), torch.bfloat16)
+
+
+def test_scales_at_any_address(dev):
+    """9 to 32 rows per kv head take the scales of 8-bit pools wherever they lie, as the prefill route does."""
+    pg = make_paged(2, 2, 128, 16, [40, 333], torch.bfloat16, 787, quant="int8")
+    q = randn((2, 8, 4, 128), torch.bfloat16, 788)
+
+    def odd(x):
+        flat = torch.empty(x.numel() + 1, dtype=x.dtype, device=dev)
+        flat[1:] = x.flatten().to(dev)
+        return flat[1:].view(x.shape)
+
+    args = [x.to(dev) for x in (q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"])]
+    out = fa.flash_attention_paged(*args, causal=True, k_scale=odd(pg["k_scale"]), v_scale=odd(pg["v_scale"]))
+    O, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, k_scale=pg["k_scale"],
+                               v_scale=pg["v_scale"])
+    assert_close(out, O, torch.bfloat16)

@@ -620,9 +620,10 @@ _MAX_DECODE_ROWS = 32
 
 
 def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, scale, causal, softcap,
-                block_size, want_lse, stream, num_splits=0, workspace=None, packed=False):
+                block_size, want_lse, stream, num_splits=0, workspace=None, packed=False, wide=False):
     """One decode launch.  packed=True returns (float32 [B*Hq*Nq, D+4], None): each row is the normalised output in
-    fp32 with its base-2 lse at column D -- the per-GPU partial that `parallel.combine_packed` merges."""
+    fp32 with its base-2 lse at column D -- the per-GPU partial that `parallel.combine_packed` merges.  wide=True: up to
+    32 query rows per kv head instead of 8."""
     _require_cuda(q, k_pages, v_pages, k_scale, v_scale, table, lens)
     lib = _lib.load()
     B, Hq, Nq, D = q.shape
@@ -638,7 +639,7 @@ def _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, 
     kv_code = _KV_CODE.get(k_pages.dtype, _DTYPE_CODE.get(k_pages.dtype, -1))
     d = _desc(code, kv_code, B, Hq, Hkv, Nq, 0, D, scale, causal, softcap, -1, num_splits,
               _FORCE_FLAGS | (_lib.FLAG_PACKED_F32 if packed else 0) |
-              (_lib.FLAG_DECODE_WIDE if (Hq // Hkv) * Nq > 8 else 0))
+              (_lib.FLAG_DECODE_WIDE if wide else 0))
     with _on(q.device):
         need = lib.b200fa_decode_paged_workspace_bytes(C.byref(d), int(max_kv_len))
         if workspace is None or workspace.numel() < need:
@@ -746,7 +747,7 @@ def flash_attention_paged(
                  and not needs_grad)
     if decode_ok:
         out, lse = _decode_raw(q, k_pages, v_pages, k_scale, v_scale, table, lens, max_kv_len, float(scale),
-                               bool(causal), float(softcap), block_size, return_lse, stream, num_splits)
+                               bool(causal), float(softcap), block_size, return_lse, stream, num_splits, wide=rows > 8)
         return (out, lse) if return_lse else out
     if not needs_grad and D in _SUPPORTED_HDIMS:
         # Prefill-sized queries (chunked prefill over the pool), one launch for all sequences.  16-bit pools: the

@@ -635,6 +635,10 @@ static int32_t decode_check(const b200fa_desc* d) {
   const int max_rows = (d->flags & B200FA_FLAG_DECODE_WIDE) ? 32 : 8;
   if (static_cast<int64_t>(d->Hq / d->Hkv) * d->N > max_rows)
     return fail(B200FA_ERR_UNSUPPORTED, "paged decode takes (Hq/Hkv)*N <= %d query rows per kv head", max_rows);
+  if (d->flags & B200FA_FLAG_DECODE_WIDE) {            // as b200fa_fwd_paged has it, which took these calls before
+    if (!(d->scale == d->scale)) return fail(B200FA_ERR_INVALID_ARG, "scale is NaN");
+    if (d->softcap < 0.f) return fail(B200FA_ERR_INVALID_ARG, "softcap must be >= 0");
+  }
   const int kv = d->kv_dtype;
   if (!(kv == d->dtype || kv == B200FA_I8 || kv == B200FA_E4M3))
     return fail(B200FA_ERR_UNSUPPORTED, "kv_dtype must equal dtype or be int8 / e4m3");

@@ -181,3 +181,13 @@ def test_kv_lens_is_refused_where_no_kernel_honours_it():
     dv = _desc(B=1)
     dv.kv_lens = 256
     assert lib.b200fa_fwd_varlen(C.byref(dv), p, p, p, p, p, 1, 16, 16, p, None, None, 0, None) == _lib.ERR_UNSUPPORTED
+
+
+def test_wide_decode_refuses_what_the_prefill_route_refuses():
+    """9 to 32 query rows per kv head came from the paged forward: a NaN scale and a negative soft cap stay refused."""
+    lib = _lib.load()
+    p = C.c_void_p(256)
+    for kw in (dict(softcap=-1.0), dict(scale=float("nan"))):
+        d = _desc(N=4, Hq=32, Hkv=8, flags=_lib.FLAG_DECODE_WIDE, **kw)
+        st = lib.b200fa_decode_paged(C.byref(d), p, p, p, None, None, p, p, 10, 16, 4, 64, p, None, None, 0, None)
+        assert st == _lib.ERR_INVALID_ARG, _lib.last_error()

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import mlx_flashattention_steel_b200 as fa
+from mlx_flashattention_steel_b200 import attention as A
 from oracle import sdpa_oracle as orc
 
 from .test_decode_gpu import _run, _status_checks  # noqa: F401  (the fixture applies to this module too)
@@ -205,3 +206,16 @@ def test_scales_at_any_address(dev):
     O, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True, k_scale=pg["k_scale"],
                                v_scale=pg["v_scale"])
     assert_close(out, O, torch.bfloat16)
+
+
+def test_what_longer_queries_refuse(dev):
+    """Only flash_attention_paged takes more than 8 rows per kv head; a NaN scale and a negative soft cap are errors there
+    as on the prefill route."""
+    pg = make_paged(1, 2, 128, 16, [40], torch.bfloat16, 789)
+    args = [x.to(dev) for x in (randn((1, 8, 4, 128), torch.bfloat16, 790), pg["k"], pg["v"], pg["block_table"], pg["seq_lens"])]
+    for kw in (dict(softcap=-1.0), dict(scale=float("nan"))):
+        with pytest.raises(ValueError):
+            fa.flash_attention_paged(*args, **kw)
+    q, k, v, table, lens = args
+    with pytest.raises(NotImplementedError):
+        A._decode_raw(q, k, v, None, None, table, lens, 40, 0.1, True, 0.0, 16, False, None, packed=True)

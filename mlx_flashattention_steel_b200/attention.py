@@ -135,6 +135,7 @@ def _ptr(t: Optional[torch.Tensor]):
 
 _DESC = struct.Struct("@8i12q2f4i2P3iP")      # the fields of _lib.Desc in order, with the same native alignment
 assert _DESC.size == C.sizeof(_lib.Desc)
+_FIELDS = [C.c_int32] * 8 + [C.c_int64] * 12 + [C.c_float] * 2 + [C.c_int32] * 4 + [C.c_void_p] * 2 + [C.c_int32] * 3 + [C.c_void_p]
 
 
 def _strides(t):
@@ -145,10 +146,16 @@ def _desc(dtype, kv_dtype, B, Hq, Hkv, N, S, D, scale, causal, softcap=0.0, wind
           num_splits=0, flags=0, q=None, k=None, v=None, o=None, alibi=None, bmask=None, kv_lens=None) -> _lib.Desc:
     # bmask: (uint8 tensor [NQ, NK], block rows, block columns)
     mask = (0, 0, 0, 0) if bmask is None else (bmask[0].data_ptr(), int(bmask[1]), int(bmask[2]), int(bmask[0].shape[1]))
-    return _lib.Desc.from_buffer_copy(_DESC.pack(
-        dtype, kv_dtype, B, Hq, Hkv, N, S, D, *_strides(q), *_strides(k), *_strides(v), *_strides(o), float(scale),
-        float(softcap), 1 if causal else 0, int(window_left), int(num_splits), int(flags),
-        0 if alibi is None else alibi.data_ptr(), *mask, 0 if kv_lens is None else kv_lens.data_ptr()))
+    fields = [dtype, kv_dtype, B, Hq, Hkv, N, S, D, *_strides(q), *_strides(k), *_strides(v), *_strides(o), float(scale),
+              float(softcap), 1 if causal else 0, int(window_left), int(num_splits), int(flags),
+              0 if alibi is None else alibi.data_ptr(), *mask, 0 if kv_lens is None else kv_lens.data_ptr()]
+    try:
+        packed = _DESC.pack(*fields)
+    except (struct.error, OverflowError):
+        # a number beyond its field (a window of sys.maxsize): as C converts it
+        fields = [t(x).value for t, x in zip(_FIELDS, fields)]
+        packed = _DESC.pack(*(0 if x is None else x for x in fields))          # c_void_p(0) reads as None
+    return _lib.Desc.from_buffer_copy(packed)
 
 
 _FORCE_FLAGS = 0

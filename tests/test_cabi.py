@@ -191,3 +191,15 @@ def test_wide_decode_refuses_what_the_prefill_route_refuses():
         d = _desc(N=4, Hq=32, Hkv=8, flags=_lib.FLAG_DECODE_WIDE, **kw)
         st = lib.b200fa_decode_paged(C.byref(d), p, p, p, None, None, p, p, 10, 16, 4, 64, p, None, None, 0, None)
         assert st == _lib.ERR_INVALID_ARG, _lib.last_error()
+
+
+def test_descriptor_fields_beyond_their_type():
+    """An unlimited window is written as the largest Python integer by some callers: fields wrap as C assigns them."""
+    from mlx_flashattention_steel_b200.attention import _desc as pack
+
+    for window, scale, cap in ((2 ** 63 - 1, 1e39, 0.0), (2 ** 32 - 1, 0.5, -1e300), (7, 0.25, 30.0)):
+        d = pack(_lib.BF16, _lib.I8, 1, 4, 2, 16, 32, 128, scale, True, cap, window, flags=5)
+        want = _desc(window_left=window, scale=scale, softcap=cap)
+        for name in ("window_left", "scale", "softcap"):
+            assert getattr(d, name) == getattr(want, name), name
+        assert (d.dtype, d.kv_dtype, d.B, d.Hq, d.Hkv, d.N, d.S, d.D, d.causal, d.flags) == (_lib.BF16, _lib.I8, 1, 4, 2, 16, 32, 128, 1, 5)

@@ -53,7 +53,8 @@ constexpr int kMaxWarps = 17;     // warps of a CTA: up to 16 consumers and the 
 // cost ~6 us before the first page was requested.  Beyond it decode_plan_kernel scans once for all.
 constexpr int kSmemSeqs = 1024;
 // CTAs that share an SM when a CTA holds few heads: as many as make 8 consumer warps (6 CTAs of one, whose registers
-// would otherwise not fit).  The grid counts on all of them being resident at once, hence the launch bounds.
+// would otherwise not fit).  The grid counts on all of them being resident at once, hence the launch bounds and the room
+// that launch_decode_paged leaves in shared memory.
 __host__ __device__ constexpr int ctas_per_sm(int warps) { return warps >= 8 ? 1 : (warps >= 4 ? 2 : (warps >= 2 ? 4 : 6)); }
 
 enum KvKind { KV_F16 = 0, KV_BF16 = 1, KV_I8 = 2, KV_E4M3 = 3 };
@@ -374,8 +375,10 @@ __global__ void __launch_bounds__(kMergeWarps * 32, 4) decode_merge_kernel(const
 // 16 rows of the MMA, and a.row_groups warps per head share a page when there are more.
 // PG = 2: two warps per head take its units in turn (one each step instead of two), which doubles the warps that hide the
 // latency of a step's chain of waits, conversions and MMAs.
+// Launch bounds: those of the CTA's own width, or for RT = 2, whose width is known at run time, 384 threads (168
+// registers a thread: 2 CTAs of 5 warps, 4 of 3 or 6 of 2 fit an SM's 65536).
 template <int KV, int HPC, int kD, bool CAP, int RT, int PG>
-__global__ void __launch_bounds__(((HPC > 0 ? HPC * PG : 8) + 1) * 32, HPC > 0 ? ctas_per_sm(HPC) : 1)
+__global__ void __launch_bounds__(HPC > 0 ? (HPC * PG + 1) * 32 : 384, HPC > 0 ? ctas_per_sm(HPC) : 1)
 decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const KernelArgs a) {
   constexpr bool kQuant = (KV == KV_I8 || KV == KV_E4M3);
@@ -1237,8 +1240,14 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   // several small CTAs share an SM when a CTA holds few heads
   const int per_sm = ctas_per_sm(hpc * sh.row_groups);
   const size_t budget = per_sm == 1 ? 200 * 1024 : (per_sm == 2 ? 100 * 1024 : (per_sm == 4 ? 50 * 1024 : 33 * 1024));
+  // what a CTA takes beside its stages, the 1 KB that the hardware keeps per CTA included
+  const size_t beside = 1024 + 1024 + a.qlo_bytes + 2 * kMaxStages * 8 + kMaxStages * 4 + 64 +
+                        (p.B <= kSmemSeqs ? sizeof(int) * (static_cast<size_t>(p.B) + 1) : 0);
   int stages = static_cast<int>(budget / per_stage);
   if (stages > kMaxStages) stages = kMaxStages;
+  // all per_sm of them at once, as the grid counts on: one stage less where the prefix sums of many sequences or the low
+  // bytes of Q would be in the way
+  while (stages > 2 && per_sm * (beside + stages * per_stage) > 228 * 1024) --stages;
   if (stages < 2) {
     snprintf(msg, msg_len, "Hkv=%d needs %zu bytes per stage; too large for the stage ring", p.Hkv, per_stage);
     return cudaErrorNotSupported;
@@ -1248,8 +1257,7 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.q_prescale = sc;
   a.cap_log2 = p.softcap * kLog2e;
   a.inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
-  const size_t smem = 1024 + static_cast<size_t>(stages) * per_stage + a.qlo_bytes + 2 * kMaxStages * 8 + kMaxStages * 4 + 64 +
-                      (p.B <= kSmemSeqs ? sizeof(int) * (static_cast<size_t>(p.B) + 1) : 0);
+  const size_t smem = beside - 1024 + static_cast<size_t>(stages) * per_stage;
 
   // tensor maps, in bytes: (128 B, tokens, 128-byte halves of a row, heads, batch).  A pool is one "batch" of
   // num_pages * block_size tokens with the heads of a token side by side; a dense cache has its own strides.

@@ -310,7 +310,8 @@ int32_t b200fa_paged_kv_dequant_pair(const void* k_pool, const void* v_pool, con
   if (out_dtype != B200FA_F16 && out_dtype != B200FA_BF16) return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: output must be f16 or bf16");
   if (D % 16 != 0) return fail(B200FA_ERR_INVALID_ARG, "D must be a multiple of 16");
   if (static_cast<int64_t>(num_pages) * block_size >= (1LL << 31)) return fail(B200FA_ERR_UNSUPPORTED, "pool of 2^31 tokens or more");
-  if (B > 65535 || static_cast<int64_t>(H) * D > (1 << 24)) return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: B beyond 65535 or rows beyond 2^24 values");
+  if (static_cast<int64_t>(H) * D > (1 << 30) || (static_cast<int64_t>(max_kv_len) + 31) / 32 * B >= (1LL << 31))
+    return fail(B200FA_ERR_UNSUPPORTED, "dequant_pair: rows beyond 2^30 values, or 2^31 blocks of 32 tokens");
   if (B == 0 || max_kv_len == 0) return B200FA_OK;
   if (!k_pool || !v_pool || !k_scale || !v_scale || !block_table || !seq_lens || !k_out || !v_out) return fail(B200FA_ERR_INVALID_ARG, "null pointer");
   if (!aligned16(k_pool) || !aligned16(v_pool) || !aligned16(k_out) || !aligned16(v_out))

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) paged_kv_gather_dequant_kernel(
   }
 }
 
-// The same for K and V in one launch, for the forward over per-sequence key counts (blockIdx.z: 0 = K, 1 = V): rows up to
+// The same for K and V in one launch, for the forward over per-sequence key counts (blockIdx.y: 0 = K, 1 = V): rows up to
 // the end of a sequence's last 64-key tile are written (zeros beyond its length, for the tensor core multiplies them all
 // the same), the rest of the padded output is not, since nothing reads it.  Bound by HBM: 386 bytes per token and head.  A
 // block takes kDqTokens tokens of one sequence and all heads, a thread 16 values at a time, four in flight; whole blocks
@@ -102,15 +102,16 @@ template <typename T, bool E4M3>
 __global__ void __launch_bounds__(256) paged_kv_dequant_pair_kernel(
     const uint4* __restrict__ k_pool, const uint4* __restrict__ v_pool, const __half* __restrict__ k_scale,
     const __half* __restrict__ v_scale, const int32_t* __restrict__ block_table, const int32_t* __restrict__ seq_lens, int H,
-    unsigned cpr, int block_size, int max_blocks, int max_kv_len, int num_pages, uint4* __restrict__ k_out, uint4* __restrict__ v_out) {
+    unsigned cpr, int block_size, int max_blocks, int max_kv_len, int num_pages, int tiles, uint4* __restrict__ k_out,
+    uint4* __restrict__ v_out) {
   __shared__ int s_row[kDqTokens];       // token's row in the pool, -1: zeros
-  const int b = blockIdx.y, t0 = blockIdx.x * kDqTokens;
+  const int b = blockIdx.x / tiles, t0 = (blockIdx.x % tiles) * kDqTokens;
   const int len = min(max(seq_lens[b], 0), max_kv_len);
   const int end = min((len + kKeyTile - 1) / kKeyTile * kKeyTile, max_kv_len);
   if (t0 >= end) return;
-  const uint4* pool = blockIdx.z == 0 ? k_pool : v_pool;
-  const __half* scale = blockIdx.z == 0 ? k_scale : v_scale;
-  uint4* out = blockIdx.z == 0 ? k_out : v_out;
+  const uint4* pool = blockIdx.y == 0 ? k_pool : v_pool;
+  const __half* scale = blockIdx.y == 0 ? k_scale : v_scale;
+  uint4* out = blockIdx.y == 0 ? k_out : v_out;
   if (threadIdx.x < kDqTokens) {
     const int t = t0 + threadIdx.x;
     int row = -1;
@@ -251,11 +252,12 @@ cudaError_t launch_paged_dequant_pair(const void* k_pool, const void* v_pool, co
                                       int out_dtype, int num_pages, int block_size, int max_blocks, int max_kv_len, void* k_out,
                                       void* v_out, cudaStream_t stream) {
   if (B <= 0 || max_kv_len <= 0) return cudaSuccess;
-  const dim3 grid((max_kv_len + kDqTokens - 1) / kDqTokens, B, 2);
+  const int tiles = static_cast<int>((static_cast<long long>(max_kv_len) + kDqTokens - 1) / kDqTokens);
+  const dim3 grid(static_cast<unsigned>(tiles) * B, 2);
   auto go = [&](auto kern) {
     kern<<<grid, 256, 0, stream>>>(static_cast<const uint4*>(k_pool), static_cast<const uint4*>(v_pool),
                                    static_cast<const __half*>(k_scale), static_cast<const __half*>(v_scale), block_table, seq_lens, H,
-                                   static_cast<unsigned>(D / 16), block_size, max_blocks, max_kv_len, num_pages,
+                                   static_cast<unsigned>(D / 16), block_size, max_blocks, max_kv_len, num_pages, tiles,
                                    static_cast<uint4*>(k_out), static_cast<uint4*>(v_out));
   };
   if (out_dtype == 0) {

@@ -203,3 +203,11 @@ def test_descriptor_fields_beyond_their_type():
         for name in ("window_left", "scale", "softcap"):
             assert getattr(d, name) == getattr(want, name), name
         assert (d.dtype, d.kv_dtype, d.B, d.Hq, d.Hkv, d.N, d.S, d.D, d.causal, d.flags) == (_lib.BF16, _lib.I8, 1, 4, 2, 16, 32, 128, 1, 5)
+
+
+def test_dequantising_takes_any_number_of_sequences():
+    lib = _lib.load()
+    dp = lib.b200fa_paged_kv_dequant_pair
+    assert dp(*[None] * 6, 70000, 2, 64, _lib.I8, _lib.BF16, 10, 16, 4, 0, None, None, None) == _lib.OK      # nothing to do
+    assert dp(*[None] * 6, 70000, 2, 64, _lib.I8, _lib.BF16, 10, 16, 4, 1 << 25, None, None, None) == _lib.ERR_UNSUPPORTED
+    assert dp(*[None] * 6, 1, 2, 64, _lib.BF16, _lib.BF16, 10, 16, 4, 64, None, None, None) == _lib.ERR_UNSUPPORTED

@@ -228,6 +228,41 @@ def test_gather_dequant_is_bit_exact(dev, quant, out_dtype):
     assert np.array_equal(got.cpu().view(torch.int16).numpy(), ref)
 
 
+@pytest.mark.parametrize("quant", ["int8", "e4m3"])
+@pytest.mark.parametrize("block_size,D", [(16, 128), (64, 64), (8, 128)])
+def test_dequantised_pair_is_bit_exact_up_to_the_last_key_tile(dev, quant, block_size, D):
+    """What a chunk of a prefill over 8-bit pools reads: K and V in one launch, written up to the end of the 64-key tile in
+    which a sequence ends, zeros beyond its length and for holes; the rows after that stay as they are."""
+    from mlx_flashattention_steel_b200 import _lib
+
+    lens = [5, 0, 200, 64, 65, 130]
+    pg = make_paged(len(lens), 3, D, block_size, lens, torch.bfloat16, 640, quant=quant)
+    table = pg["block_table"].clone()
+    table[2, 1] = -1
+    table[5, 0] = pg["num_pages"] + 3                  # beyond the pool: a hole
+    args = [x.to(dev) for x in (pg["k"], pg["v"], pg["k_scale"], pg["v_scale"], table, pg["seq_lens"])]
+    got = [torch.full((len(lens), 3, 200, D), float("nan"), dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    st = _lib.load().b200fa_paged_kv_dequant_pair(*(x.data_ptr() for x in args), len(lens), 3, D, A._KV_CODE[pg["k"].dtype], _lib.BF16,
+                                                  pg["num_pages"], block_size, table.shape[1], 200, *(x.data_ptr() for x in got),
+                                                  torch.cuda.current_stream().cuda_stream)
+    assert st == _lib.OK, _lib.last_error()
+    table[5, 0] = -1
+    for out, name in zip(got, ("k", "v")):
+        deq = orc.dequant(pg[name], pg[name + "_scale"], torch.bfloat16)
+        ref = orc.paged_gather(deq.view(torch.int16).numpy(), table.numpy(), pg["seq_lens"].numpy(), 200)
+        bits = out.cpu().view(torch.int16).numpy()
+        for b, n in enumerate(lens):
+            end = min((n + 63) // 64 * 64, 200)
+            assert np.array_equal(bits[b, :, :end], ref[b, :, :end])
+            assert torch.isnan(out[b, :, end:]).all()
+    # and the forward over these buffers reads no row that was not written
+    q = randn((len(lens), 6, 70, D), torch.bfloat16, 641)
+    for causal in (True, False):
+        out, _ = A._fwd_raw(q.to(dev), *got, D ** -0.5, causal, 0.0, -1, False, None, kv_lens=args[5])
+        O, _ = orc.paged_attention(q, pg["k"], pg["v"], table, pg["seq_lens"], causal=causal, k_scale=pg["k_scale"], v_scale=pg["v_scale"])
+        assert_close(out, O, torch.bfloat16)
+
+
 def test_dense_attention_with_per_sequence_key_counts(dev):
     """kv_lens through the raw forward: each batch entry attends to its own number of keys of a padded dense cache."""
     dtype = torch.float16
@@ -257,6 +292,25 @@ def test_short_queries_over_pools_the_paged_kernel_does_not_take(dev, quant, D, 
     del poison
     _run(dev, torch.bfloat16, quant, 4, Hq, 2, Nq, lens, 630, D=D, block_size=block_size)
     _run(dev, torch.bfloat16, quant, 4, Hq, 2, Nq, lens, 631, D=D, block_size=block_size, causal=False, softcap=20.0, holes=True)
+
+
+@pytest.mark.parametrize("B", [2, 32, 33])
+@pytest.mark.parametrize("causal", [False, True])
+def test_key_counts_in_any_order(dev, B, causal):
+    """Up to 32 batch entries run with the longest key count first, more in the order they come: every entry is done, equal
+    counts and counts beyond the cache or below zero among them."""
+    dtype = torch.bfloat16
+    lens = [(37 * i) % 150 for i in range(B)]
+    lens[0], lens[1], lens[-1] = 400, -3, lens[0]
+    q = randn((B, 2, 140, 64), dtype, 650)
+    k, v = randn((B, 1, 300, 64), dtype, 651), randn((B, 1, 300, 64), dtype, 652)
+    lt = torch.tensor(lens, dtype=torch.int32, device=dev)
+    out, lse = A._fwd_raw(q.to(dev), k.to(dev), v.to(dev), 0.125, causal, 0.0, -1, True, None, kv_lens=lt)
+    for b, n in enumerate(lens):
+        n = max(0, min(n, 300))
+        O, L, _ = orc.sdpa(q[b:b + 1], k[b:b + 1, :, :n], v[b:b + 1, :, :n], causal=causal)
+        assert_close(out[b:b + 1], O, dtype)
+        assert_close(lse[b:b + 1], L, dtype, "lse")
 
 
 @pytest.mark.parametrize("parts", [2, 3])

@@ -219,3 +219,30 @@ def test_what_longer_queries_refuse(dev):
     q, k, v, table, lens = args
     with pytest.raises(NotImplementedError):
         A._decode_raw(q, k, v, None, None, table, lens, 40, 0.1, True, 0.0, 16, False, None, packed=True)
+
+
+def test_more_than_1024_sequences_from_a_graph(dev):
+    """Beyond 1024 sequences the merge kernel reads the plan kernel's sums: replays whose lengths change between them."""
+    B = 1100
+    lens0 = [(11 * i) % 70 for i in range(B)]
+    pg = make_paged(B, 2, 128, 16, [69] * B, torch.bfloat16, 782)
+    k, v, table = (pg[n].to(dev) for n in ("k", "v", "block_table"))
+    lens, q = torch.tensor(lens0, dtype=torch.int32, device=dev), randn((B, 4, 1, 128), torch.bfloat16, 783).to(dev)
+
+    def call():
+        return fa.flash_attention_paged(q, k, v, table, lens, causal=True, max_kv_len=69)
+
+    A._set_check_decode_status(False)                               # the check synchronises, which a capture does not allow
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    for step in range(3):
+        now = torch.tensor([(n * (step + 3) + 5 * step) % 70 for n in lens0], dtype=torch.int32)
+        lens.copy_(now.to(dev))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, call())
+        O, _ = orc.paged_attention(q.cpu()[:40], pg["k"], pg["v"], pg["block_table"][:40], now[:40], causal=True)
+        assert_close(out[:40], O, torch.bfloat16)

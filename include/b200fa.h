@@ -165,8 +165,9 @@ int32_t b200fa_bwd_varlen(const b200fa_desc* d, const void* q, const void* k, co
                           void* workspace, size_t workspace_bytes, void* stream);
 
 /*
- * Paged-KV attention for short queries (decode), split-KV with the
- * log-sum-exp combine done inside the same launch.  Replaces
+ * Paged-KV attention for short queries (decode), split-KV: the main kernel and,
+ * as its programmatic dependent, a kernel that merges the partials by their
+ * log-sum-exp; beyond 1024 sequences a planning kernel in front.  Replaces
  * mfa_paged_steel_forward (csrc/bindings.cpp:367-407) and the gather +
  * per-sequence flash-decode route of flash_attention_paged
  * (mlx_mfa/attention.py:3008-3017, csrc/mfa_attention.cpp:150-288).
@@ -255,22 +256,23 @@ int32_t b200fa_paged_kv_dequant_pair(const void* k_pool, const void* v_pool, con
  * page pool at start-up and has no allocator left to ask at decode time; a host
  * binding (cgo, JNI, a plugin ABI) that only passes the operator its input and output
  * buffers; a latency-bound step that must not run into the device-wide stall a
- * cudaMalloc/cudaFree can cause.  The split-KV partials, counters and page prefix
+ * cudaMalloc/cudaFree can cause.  The split-KV partials, status words and page prefix
  * sums live instead in a 16 MiB array inside the library's device image, which every
  * GPU that loads the library holds until the process exits.
  *
  * Limits and rules:
- *   - the problem must fit: b200fa_decode_paged_workspace_bytes(d, max_kv_len) <= 16 MiB
- *     (config-4-sized decode, B=128 Hq=32 D=128, needs 4.6 MB); larger problems get
- *     B200FA_ERR_WORKSPACE with an explanatory message and run nothing;
+ *   - the problem must fit: what b200fa_decode_paged cannot do without <= 16 MiB (about
+ *     (SMs + B) * Hq * N * (D + 1) floats; config-4-sized decode, B=128 Hq=32 D=128, needs
+ *     4.6 MB).  b200fa_decode_paged_workspace_bytes also counts what it can only use (int8,
+ *     kv heads in eights: twice that).  Larger problems get B200FA_ERR_WORKSPACE with an
+ *     explanatory message and run nothing;
  *   - the first call on each device looks up the array's device address (a host-side
  *     query, no allocation); make that first call outside any stream capture;
  *   - all calls on a device share the one array: two calls whose kernels can overlap
  *     on the GPU (different streams, no ordering between them) race on it — serialise
  *     them, or give the second one its own workspace through b200fa_decode_paged;
- *   - what must start from zero (counters, error word) is cleared by the call itself;
- *     the rest of the array keeps the previous call's partials and is overwritten
- *     before it is read;
+ *   - the error word is written at the end of every call; the rest of the array keeps the
+ *     previous call's partials and is overwritten before it is read;
  *   - it calls no cudaMalloc, cudaFree or allocating library routine.
  */
 int32_t b200fa_decode_paged_static(const b200fa_desc* d, const void* q,

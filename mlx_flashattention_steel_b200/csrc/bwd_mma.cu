@@ -467,8 +467,9 @@ cudaError_t launch_t(const BwdParams& p, int dtype, bool varlen, int nbatch, int
 }  // namespace
 
 // The tcgen05 kernels: items of 128 keys of a kv head are few where heads are (22 for one kv head at S = 2800), and the
-// longest of a causal mask takes as long as all its query tiles.  They are cut until there are three per SM (148), as long
-// as a part keeps four of its 128 x 128 steps on average.  Packed sequences are not: they are many.
+// longest of a causal mask takes as long as all its query tiles.  They are cut until there are three per SM, as long as a
+// part keeps four of its 128 x 128 steps on average.  Packed sequences are not: they are many.  The SMs are a B200's 148
+// whatever the device has free: the parts are summed in float32, and a gradient's bits are the shape's alone.
 int bwd_dkv_parts(const BwdParams& p, bool varlen) {
   if (varlen || p.S <= 0) return 1;
   const long long items = static_cast<long long>((p.S + 127) / 128) * p.Hkv * p.B;

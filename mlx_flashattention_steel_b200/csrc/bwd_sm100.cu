@@ -127,8 +127,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   auto bar = [&](int i) -> uint32_t { return smem_u32(&bars[i]); };
 
   // Persistent CTA, one per SM: work items (128 keys of one kv head of one batch entry or sequence) come from a global
-  // counter in grid order, which puts the key tiles with the most query tiles of each sequence first.  While an item
-  // runs, the producer thread fetches the next one and starts its K load (second buffer) and, once this item's V sits
+  // counter in the order of item_of, a group of heads' key tiles with the most query tiles first.  While an item runs,
+  // the producer thread fetches the next one and starts its K load (second buffer) and, once this item's V sits
   // in TMEM, its V load; set-up, K/V latency and the gap between CTAs are paid once per SM instead of once per item.
   // Next item that has keys (grid cells beyond a sequence's end are skipped), decoded into slot `sl` of s_work for
   // every role to read; index -1 when the list is exhausted.  Run by one thread, with global latency per try.

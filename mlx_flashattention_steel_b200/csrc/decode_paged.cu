@@ -1,5 +1,5 @@
-// Paged-KV decode: split-KV flash-decoding with the log-sum-exp combine inside the
-// same launch.  Replaces the reference's gather + per-sequence two-kernel flash-decode
+// Paged-KV decode: split-KV flash-decoding, its partials merged by their log-sum-exp in
+// a dependent kernel.  Replaces the reference's gather + per-sequence two-kernel flash-decode
 // route (mlx_mfa/attention.py:3008-3017; csrc/mfa_attention.cpp:150-288; kernels
 // csrc/mfa_steel_fwd.cpp:1541-1991, 2008-2105) and its paged forward
 // (csrc/mfa_steel_fwd.cpp:2462-3121).
@@ -13,9 +13,10 @@
 //     contiguous 16 KB of HBM for 8 int8 heads), 128B-swizzled by token, plus one
 //     bulk copy per scale array, into a ring of stages guarded by mbarriers.
 //   * A consumer warp computes S = Q.K^T (rows = the GQA group x query tokens, padded
-//     to the 16 rows of mma.m16n8k16) and O^T += V^T.P^T for its head.  int8 / e4m3
-//     values are widened to f16 in registers straight from the swizzled tile;
-//     k_scale multiplies the scores, v_scale is folded into P.
+//     to the 16 rows of mma.m16n8k16) and O^T += V^T.P^T for its head.  8-bit values
+//     are widened to f16 in registers straight from the swizzled tile, except for int8
+//     K, which meets fixed-point queries on the integer tensor cores; k_scale
+//     multiplies the scores, v_scale is folded into P.
 //   * A CTA that covers a whole sequence writes the result; otherwise it writes a
 //     partial (normalised O, base-2 lse), and a second kernel merges the partials of
 //     every row.  It is launched as a programmatic dependent, so that its blocks are
@@ -1131,11 +1132,12 @@ Shape pick_shape(int Hkv, int rows, int num_splits) {
   s.page_groups = 1;
   return s;
 }
-// int8, 8 heads to a CTA: two warps per head can take its units in turn.  At 96 registers a warp that is what keeps up
-// with HBM (128 sequences of 512 to 32768 tokens: 785 -> 638 us), but every CTA then leaves two partials per sequence, which
-// costs 3 to 6 us where there is little else (8192 tokens: 18.7 against 24.8 us); so only from 32 units per CTA on, as far
-// as the longest sequence tells, and where the workspace has room for the partials.  e4m3, whose conversions spill at 96
-// registers, gains nothing (116.9 against 115.3 us).
+// int8, 8 heads to a CTA: two warps per head can take its units in turn.  At 96 registers a warp (a dozen values spilled)
+// that is what keeps up with HBM (128 sequences of 512 to 32768 tokens: 785 -> 638 us), but every CTA then leaves two
+// partials per sequence, which costs 3 to 6 us where there is little else (8192 tokens: 18.7 against 24.8 us); so only from
+// 32 units per CTA on, as far as the longest sequence tells, and where the workspace has room for the partials.  e4m3, with
+// more conversions to do at 96 registers, gains nothing (116.9 against 115.3 us).  CTAs of 4, 2 or 1 heads, two to six of
+// them on an SM, are not built in that form; whether they would gain has not been measured.
 bool can_take_turns(const Shape& s, int rows, int kv_dtype) { return kv_dtype == 3 && rows <= 8 && s.hpc == 8; }
 
 template <int KV, int HPC, int D, int RT, int PG>

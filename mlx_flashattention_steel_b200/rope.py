@@ -106,8 +106,10 @@ class _RopeFn(torch.autograd.Function):
 def apply_rope(x, cos, sin, offset: Union[int, Sequence[int], torch.Tensor] = 0, interleaved: bool = True,
                rotary_dim: Optional[int] = None, stream=None) -> torch.Tensor:
     """Rotate ``x`` ``[B, H, N, D]`` (f16 / bf16) with tables ``cos`` / ``sin`` float32 ``[max_seq_len, rotary_dim/2]``;
-    row n of batch b takes position ``offset[b] + n`` (one int for all batches, or one per batch).  Role of
-    ``_apply_rope_mlx`` (mlx_mfa/attention.py:2128-2210).  Differentiable with respect to ``x``."""
+    row n of batch b takes position ``offset[b] + n`` (one int for all batches, or one per batch).  Up
+    to 512 positions that the host holds travel with the launch, so that a captured graph keeps them; a device tensor's are
+    checked on the host, which a capture does not allow.  Role of ``_apply_rope_mlx``
+    (mlx_mfa/attention.py:2128-2210).  Differentiable with respect to ``x``."""
     x, cos, sin = _as_tensor(x, "x"), _as_tensor(cos, "rotary_cos"), _as_tensor(sin, "rotary_sin")
     if x.ndim != 4:
         raise ValueError(f"apply_rope expects [B, H, N, D], got {x.ndim}D.")

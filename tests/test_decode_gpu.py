@@ -177,7 +177,7 @@ def test_decode_via_kvcache_entry(dev):
 
 
 def test_gather_route_for_long_queries(dev):
-    # (Hq/Hkv)*Nq > 8 -> gather + per-sequence attention, as the reference routes it
+    # (Hq/Hkv)*Nq > 32 -> the prefill route, where the reference gathers and attends per sequence
     pg = make_paged(2, 2, 128, 16, [48, 100], torch.bfloat16, 460)
     q = randn((2, 8, 16, 128), torch.bfloat16, 461)
     out = fa.flash_attention_paged(q.to(dev), pg["k"].to(dev), pg["v"].to(dev), pg["block_table"].to(dev),

@@ -1,5 +1,5 @@
 """Paged split-KV decode where its launch takes another form: 9 to 32 query rows per kv head (two row tiles per warp, two
-warps per head), partials merged in two steps, more sequences than a CTA scans itself, fixed-point queries of int8 pools,
+warps per head), many partials to merge, more sequences than a CTA scans itself, fixed-point queries of int8 pools,
 launches inside a CUDA graph.  Oracle and tolerance (2e-2 max-abs) as in test_decode_gpu.py."""
 import pytest
 import torch
@@ -32,7 +32,7 @@ def test_more_than_eight_rows_options(dev, causal, D, block_size, softcap):
 @pytest.mark.parametrize("quant", [None, "int8"])
 @pytest.mark.parametrize("Hq,Hkv,Nq", [(8, 2, 1), (16, 8, 1), (8, 1, 4), (4, 4, 5)])
 def test_many_parts_are_merged_in_two_steps(dev, quant, Hq, Hkv, Nq):
-    # every CTA holds a part of the one long sequence; the second one ends inside a group of parts
+    # every CTA holds a part of the long sequence, and a merge block's warps share each row's parts
     _run(dev, torch.float16, quant, 2, Hq, Hkv, Nq, [30000, 1500], 740)
 
 
@@ -57,7 +57,7 @@ def test_values_beyond_the_end_are_not_read_into_wide_rows(dev):
 @pytest.mark.parametrize("Nq", [1, 4])
 def test_int8_queries_of_uneven_size(dev, Nq):
     """A row of Q is fixed point below its largest value: rows with one value far above the others, tiny rows, zero rows.
-    The step is max|q| / 32639, so the scaled score is off by at most sum_d |k_d| * scale * max|q| / 65278: for the outlier
+    The step is at most max|q| / 32637, so the scaled score is off by at most sum_d |k_d| * scale * max|q| / 65278: for the outlier
     row (max|q| = 60, sum|k| ~ 128 * 0.8) 0.0083, inside the 2e-2 the outputs are held to."""
     pg = make_paged(3, 2, 128, 16, [40, 700, 333], torch.float16, 770, quant="int8")
     q = randn((3, 8, Nq, 128), torch.float16, 771)
@@ -73,7 +73,7 @@ def test_int8_queries_of_uneven_size(dev, Nq):
 
 @pytest.mark.parametrize("Nq", [1, 4])
 def test_replayed_from_a_graph(dev, Nq):
-    """The plan kernel and the main kernel are joined by a programmatic dependency: it survives capture, and replays on
+    """The main kernel and the merge kernel are joined by a programmatic dependency: it survives capture, and replays on
     changed inputs give what direct calls give."""
     pg = make_paged(3, 2, 128, 16, [900, 65, 333], torch.bfloat16, 780)
     k, v, table = (pg[n].to(dev) for n in ("k", "v", "block_table"))

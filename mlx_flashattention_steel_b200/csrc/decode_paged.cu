@@ -754,7 +754,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
         // whatever the scale of a slot beyond the sequence holds (it may be a NaN pattern)
         if (!full && (j + q) * kBS + (lane & 15) >= len) vsl = 0.f;
-        vmove = vsl > vlimit && vsl < INFINITY;
+        vmove = fabsf(vsl) > vlimit && fabsf(vsl) < INFINITY;
       }
 
       // ---- S = Q K^T : per page this lane gets tokens {2t, 2t+1, 8+2t, 9+2t} of its rows ----
@@ -888,7 +888,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       if (__any_sync(0xffffffffu, grew || vmove)) {
         float shift = 0.f;
         if (kQuant && __any_sync(0xffffffffu, vmove)) {
-          const unsigned top = __reduce_max_sync(0xffffffffu, vmove ? __float_as_uint(vsl) : 0u);
+          const unsigned top = __reduce_max_sync(0xffffffffu, vmove ? __float_as_uint(fabsf(vsl)) : 0u);
           shift = 127.f - static_cast<float>(top >> 23) - vexp;
           vexp += shift;
           vlimit = exp2f(15.f - vexp);

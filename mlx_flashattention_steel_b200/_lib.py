@@ -6,6 +6,7 @@ operators raise, they never fall back to another implementation.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libb200fa.so"
@@ -109,15 +110,38 @@ _lib = None
 
 
 class _NotBuilt:
-    """Stands for the extension before a build: takes no call, so that each one reaches load(), which says so."""
+    """The host calls without the extension: take no call, so that the Python code has each one."""
 
     fwd = bwd = decode = rope = append = staticmethod(lambda *args: None)
 
 
-try:
-    from . import _host_calls as host_calls     # csrc/host_calls.cpp
-except ImportError as _e:
-    host_calls, _host_error = _NotBuilt, _e
+class _HostCalls:
+    """The native forms of the plain calls (csrc/host_calls.cpp).  The extension is imported when one of them is first asked
+    for, or by load(), not with the package: the build is a module of the package, and a program that builds the library has
+    to be able to call it afterwards.  Everybody who calls them keeps this one object."""
+
+    error = None        # why the extension could not be imported
+
+    def bind(self) -> bool:
+        """Imports the extension if that has not happened yet; True if it is there."""
+        if "fwd" in self.__dict__:
+            return True
+        importlib.invalidate_caches()       # it may have been built a moment ago
+        try:
+            ext = importlib.import_module(f"{__package__}._host_calls")
+        except ImportError as e:
+            self.error = e
+            return False
+        self.error = None
+        self.__dict__.update({name: getattr(ext, name) for name in ("fwd", "bwd", "decode", "rope", "append")})
+        return True
+
+    def __getattr__(self, name):            # reached only for what bind() has not set
+        none = getattr(_NotBuilt, name)
+        return self.__dict__[name] if self.error is None and self.bind() else none
+
+
+host_calls = _HostCalls()
 
 
 def load() -> C.CDLL:
@@ -125,8 +149,8 @@ def load() -> C.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    if LIB_PATH.exists() and host_calls is _NotBuilt:
-        raise RuntimeError(f"the host extension beside {LIB_PATH} does not load ({_host_error}). Run: python -m "
+    if LIB_PATH.exists() and not host_calls.bind():
+        raise RuntimeError(f"the host extension beside {LIB_PATH} does not load ({host_calls.error}). Run: python -m "
                            "mlx_flashattention_steel_b200.build")
     if not LIB_PATH.exists():
         raise RuntimeError(

@@ -1,0 +1,49 @@
+"""A build and what follows it in the same process, in a copy of the tree that has the compiled kernels and no more."""
+import shutil
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+PKG = "mlx_flashattention_steel_b200"
+
+# the extension is what every front-end module calls, and takes or gives back calls
+BOUND = f"""
+import {PKG} as fa
+from {PKG} import _lib, attention, kv_cache, rope
+assert attention._H is kv_cache._H is rope._H is _lib.host_calls
+for name in ("fwd", "bwd", "decode", "rope", "append"):
+    assert getattr(_lib.host_calls, name) is getattr(sys.modules["{PKG}._host_calls"], name), name
+assert _lib.host_calls.fwd() is None
+"""
+
+
+@pytest.fixture
+def tree(tmp_path):
+    """The sources, libb200fa.so and the objects, as a copy keeps them; no host extension."""
+    for d in (f"{PKG}/csrc", f"{PKG}/build", f"{PKG}/integrations", "include", "oracle"):
+        shutil.copytree(ROOT / d, tmp_path / d, ignore=shutil.ignore_patterns("__pycache__"))
+    for f in [*(ROOT / PKG).glob("*.py"), ROOT / PKG / "libb200fa.so", ROOT / "__graft_entry__.py"]:
+        shutil.copy2(f, tmp_path / f.relative_to(ROOT))
+    return tmp_path
+
+
+def _python(tree, code):
+    r = subprocess.run([sys.executable, "-c", "import sys\n" + code], cwd=tree, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r
+
+
+def test_first_build_and_use_in_one_process(tree):
+    _python(tree, f"""
+import {PKG} as fa, torch
+q = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
+try:
+    fa.flash_attention(q, q, q)             # before the build: the Python code has the call
+except RuntimeError as e:
+    assert "no CPU path" in str(e)
+import __graft_entry__
+__graft_entry__.build()
+""" + BOUND)

@@ -7,6 +7,8 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib
+import sysconfig
+import warnings
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libb200fa.so"
@@ -115,12 +117,19 @@ class _NotBuilt:
     fwd = bwd = decode = rope = append = staticmethod(lambda *args: None)
 
 
+def host_abi() -> str:
+    """What the host extension depends on beside its sources: this torch, its C++ ABI, this Python."""
+    import torch
+
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, {sysconfig.get_config_var('SOABI')}"
+
+
 class _HostCalls:
     """The native forms of the plain calls (csrc/host_calls.cpp).  The extension is imported when one of them is first asked
     for, or by load(), not with the package: the build is a module of the package, and a program that builds the library has
     to be able to call it afterwards.  Everybody who calls them keeps this one object."""
 
-    error = None        # why the extension could not be imported
+    error = None        # why the extension is not bound, if that was tried
 
     def bind(self) -> bool:
         """Imports the extension if that has not happened yet; True if it is there."""
@@ -130,7 +139,10 @@ class _HostCalls:
         try:
             ext = importlib.import_module(f"{__package__}._host_calls")
         except ImportError as e:
-            self.error = e
+            self.error = str(e)
+            return False
+        if getattr(ext, "built_for", None) != host_abi():     # it may load and read tensors wrongly all the same
+            self.error = f"built for {getattr(ext, 'built_for', None)}, this is {host_abi()}"
             return False
         self.error = None
         self.__dict__.update({name: getattr(ext, name) for name in ("fwd", "bwd", "decode", "rope", "append")})
@@ -149,14 +161,15 @@ def load() -> C.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    if LIB_PATH.exists() and not host_calls.bind():
-        raise RuntimeError(f"the host extension beside {LIB_PATH} does not load ({host_calls.error}). Run: python -m "
-                           "mlx_flashattention_steel_b200.build")
     if not LIB_PATH.exists():
         raise RuntimeError(
             f"{LIB_PATH} is not built. Run: python -m mlx_flashattention_steel_b200.build "
             "(needs nvcc). There is no fallback implementation."
         )
+    if not host_calls.bind():
+        # the kernels do not need it: every call goes through the Python code, 10 to 20 us later
+        warnings.warn(f"the host extension beside {LIB_PATH} does not load ({host_calls.error}); small calls are slower without it. "
+                      "Run: python -m mlx_flashattention_steel_b200.build", RuntimeWarning, stacklevel=2)
     lib = C.CDLL(str(LIB_PATH))
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)

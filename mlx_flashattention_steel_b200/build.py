@@ -9,16 +9,20 @@ from __future__ import annotations
 
 import concurrent.futures
 import os
+import shlex
 import shutil
 import subprocess
 import sys
 from pathlib import Path
+
+from . import _lib
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libb200fa.so"
 HOST = PKG / "_host_calls.so"
+HOST_ABI = OBJ / "_host_calls.abi"      # what the extension beside the library was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -58,25 +62,35 @@ def _compile(src: Path, verbose: bool) -> Path:
 
 
 def _build_host_calls(force: bool) -> None:
-    """The native half of the Python front end: an extension module against the installed torch, beside the library."""
+    """The native half of the Python front end: an extension module against the installed torch, beside the library.  Built again
+    when its sources, that torch or that Python are others than it was built with, or when it does not load."""
     import sysconfig
 
     import torch
 
     src = CSRC / "host_calls.cpp"
     newest = max(src.stat().st_mtime, (PKG.parent / "include" / "b200fa.h").stat().st_mtime)
-    if HOST.exists() and not force and HOST.stat().st_mtime > newest:
+    built_for = _lib.host_abi()
+    if (HOST.exists() and not force and HOST.stat().st_mtime > newest and HOST_ABI.exists() and HOST_ABI.read_text() == built_for
+            and _lib.host_calls.bind()):
         return
     root = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parent.parent
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    new = HOST.with_suffix(f".{os.getpid()}.tmp")
+    cmd = [*shlex.split(os.environ.get("CXX", "g++")), "-O2", "-std=c++17", "-shared", "-fPIC",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DB200FA_HOST_ABI="{built_for}"',
            f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
-           f"-I{cuda}/include", str(src), "-o", str(HOST), f"-L{PKG}", "-lb200fa", f"-L{root}/lib", "-ltorch_python",
+           f"-I{cuda}/include", str(src), "-o", str(new), f"-L{PKG}", "-lb200fa", f"-L{root}/lib", "-ltorch_python",
            "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"building {HOST.name} failed:\n{res.stdout}\n{res.stderr}")
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"building {HOST.name} failed:\n{res.stdout}\n{res.stderr}")
+        os.replace(new, HOST)
+    finally:
+        new.unlink(missing_ok=True)
+    HOST_ABI.write_text(built_for)
+    _lib.host_calls.error = None        # if importing it failed in this process: try again
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:

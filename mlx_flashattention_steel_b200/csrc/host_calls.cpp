@@ -375,4 +375,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_calls", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host_calls() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host_calls() {
+  PyObject* m = PyModule_Create(&module);
+  // the torch and Python this was built for (build.py), for the importer to compare
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", B200FA_HOST_ABI) != 0) Py_CLEAR(m);
+  return m;
+}

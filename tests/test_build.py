@@ -5,6 +5,9 @@ import sys
 from pathlib import Path
 
 import pytest
+import torch
+
+from mlx_flashattention_steel_b200 import _lib
 
 ROOT = Path(__file__).resolve().parent.parent
 PKG = "mlx_flashattention_steel_b200"
@@ -47,3 +50,28 @@ except RuntimeError as e:
 import __graft_entry__
 __graft_entry__.build()
 """ + BOUND)
+
+
+BUILD = f"from {PKG} import build\nbuild.build()\n"
+
+
+@pytest.mark.parametrize("what", ["does not load", "built for another torch"])
+def test_a_build_replaces_an_extension_that_is_not_for_this_torch(tree, what):
+    """Newer than its sources in both cases, so that its age does not show it; the compiler has arguments of its own."""
+    so, abi = tree / PKG / "_host_calls.so", tree / PKG / "build" / "_host_calls.abi"
+    if what == "does not load":
+        so.write_bytes(b"\x7fELF of another machine")
+        abi.write_text(_lib.host_abi())
+    else:
+        ours, other = torch.__version__, "9" * len(torch.__version__)
+        so.write_bytes((ROOT / PKG / "_host_calls.so").read_bytes().replace(b"torch " + ours.encode(), b"torch " + other.encode()))
+        abi.write_text(_lib.host_abi().replace(ours, other))
+    # the Python code has the calls until then, and says what is wrong
+    r = _python(tree, f"from {PKG} import _lib\nlib = _lib.load()\nassert lib.b200fa_version() and _lib.host_calls.fwd() is None")
+    assert "does not load" in r.stderr and f"python -m {PKG}.build" in r.stderr
+    assert what == "does not load" or "built for torch 9" in r.stderr
+    build = f"import os\nos.environ['CXX'] = 'env LANG=C g++'\nfrom {PKG} import build\nbuild.build()\n"
+    _python(tree, build + BOUND)
+    before = so.stat().st_mtime_ns
+    _python(tree, build + BOUND)            # and once is enough
+    assert so.stat().st_mtime_ns == before

@@ -6,7 +6,7 @@
 // which the CTA walks the query heads of the GQA group and the 128-row query tiles that can see those keys.  Per query tile, five GEMMs, all M = 128:
 //   S^T  = K . Q^T      (A = K rows in TMEM, per half of 64 queries, K = 64)   -> TMEM [0,64) and [128,192)
 //   dP^T = V . dO^T     (A = V rows in TMEM, per half)                          -> TMEM [64,128) and [192,256)
-//   and a fifth k-step each, a constant operand against three 16-bit parts of the query's -L / (scale*log2e) or -delta
+//   and a fifth k-step each, constants against three 16-bit parts of the query's -L / (scale*log2e) or -delta
 //   (Parts3): the compute warps read neither from shared memory, which was 400 of 1480 clk of a half's arithmetic (with a
 //   soft cap L is subtracted after the cap, from shared memory)
 //   8 compute warps (thread = key row, four warps per query half) turn these into
@@ -58,15 +58,16 @@ constexpr uint32_t cKA = 448, cVA = 480;
 
 constexpr int kTileBytes = 128 * HD * 2;                 // 16384: one [128 rows][64] tile
 constexpr int kDSBytes = BQ * BK * 2;                    // 32768: dS as two 64-key halves [half][query][128 B]
-// Behind the tiles: the two constant A operands (128 rows x 16) and, per stage and half, the B operand (64 queries x 16) of
-// the k-step that subtracts L and delta; -L in fp32 for a soft cap, which is applied to the score before L is subtracted
-constexpr int kConstBytes = BK * 32, kAugBytes = 64 * 32;
-constexpr int kStatBytes = 2 * kConstBytes + 4 * kAugBytes + 2 * BQ * 4;
+// In front of the tiles, for the k-steps that subtract L and delta: the constant A operand (128 rows x 8 values), the B operands
+// of L and of delta per stage and half (64 queries x 8) and zeros, the other 8 of a k-step's 16 for all of them; then -L in
+// fp32 for a soft cap, which is applied to the score before L is subtracted
+constexpr int kConstBytes = BK * 16, kAugBytes = 64 * 16, kZeroBytes = BK * 16;
+constexpr int kStatBytes = kConstBytes + 8 * kAugBytes + kZeroBytes + 2 * BQ * 4;
 constexpr int kDQStageBytes = BQ * HD * 4;               // 32768: dQ tile in fp32, two 32-column halves [half][query][128 B]
 // K, V, Q x2, dO x2, dS x2, dQ, second K buffer (the next work item's keys) = 212992
 constexpr int kSmemTiles = 2 * kTileBytes + 4 * kTileBytes + 2 * kDSBytes + kDQStageBytes + kTileBytes;
 constexpr int kSmemBytes = kSmemTiles + kStatBytes + 256 + 1024;
-static_assert(kSmemTiles % 1024 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
+static_assert(kStatBytes % 1024 == 0 && kSmemTiles % 1024 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
 
 // BAR_KV (+ K buffer) live for the whole kernel; the others are set up again for every work item
 enum Bar {
@@ -133,8 +134,6 @@ template <int DT> struct Parts3 {
     return make_uint4(pack16b<DT>(a, b), pack16b<DT>(c, 0.f), 0u, 0u);
   }
 };
-// Row r, 16-byte chunk c of an operand of 32-byte rows in the 32B-swizzled layout
-__device__ __forceinline__ uint32_t aug_off(int r, int c) { return static_cast<uint32_t>(r * 32 + ((c ^ ((r >> 2) & 1)) << 4)); }
 
 // CAP: the forward capped the scores (cap * tanh(s / cap)); P is rebuilt from the capped score and dS carries the
 // factor 1 - tanh^2.  WIN: a left window (fewer query tiles per key tile, one more test in the masked tiles).  Both are
@@ -151,7 +150,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmDQ, const BwdArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sK = smem;
+  unsigned char* sConst = smem;                        // [128][16 B]: the parts' constants in every row
+  unsigned char* sAug = sConst + kConstBytes;          // [2 stages][2 halves][64][16 B]: parts of -L / scale_log2; the same of -delta
+  unsigned char* sZero = sAug + 8 * kAugBytes;
+  float* sL = reinterpret_cast<float*>(sZero + kZeroBytes);    // [2][BQ], soft cap only
+  unsigned char* sK = smem + kStatBytes;
   unsigned char* sV = sK + kTileBytes;
   unsigned char* sQ = sV + kTileBytes;                 // [2][128][128 B]
   unsigned char* sDO = sQ + 2 * kTileBytes;            // [2][128][128 B]
@@ -161,9 +164,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSmemTiles + kStatBytes);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + BAR_COUNT);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
-  unsigned char* sConst = smem + kSmemTiles;           // [2][128][32 B]: the parts' constants in chunk 0 (L), in chunk 1 (delta)
-  float* sL = reinterpret_cast<float*>(smem + kSmemTiles + 2 * kConstBytes + 4 * kAugBytes);    // [2][BQ], soft cap only
-  unsigned char* sAug = sConst + 2 * kConstBytes;      // [2 stages][2 halves][64][32 B]: parts of -L / scale_log2 and of -delta
   // [2][8]: this item and the next one as {index or -1, key tile, kv head, batch, k_begin, S, q_begin, N}
   volatile int* s_work = reinterpret_cast<volatile int*>(s_tmem + 2);
 
@@ -227,12 +227,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   {
     // the k-step that subtracts L and delta: S^T -= L / scale_log2, dP^T -= delta, each query's value in every key row
-    for (int i = tid; i < 4 * BK; i += kThreads) {
-      const int which = i / (2 * BK), r = (i >> 1) & (BK - 1), c = i & 1;
-      using P3 = Parts3<DT>;
-      const uint4 v = c == which ? make_uint4(pack16b<DT>(P3::c0, P3::c1), pack16b<DT>(P3::c2, 0.f), 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(sConst + which * kConstBytes + aug_off(r, c)) = v;
-    }
+    using P3 = Parts3<DT>;
+    for (int i = tid; i < 2 * BK; i += kThreads)
+      *reinterpret_cast<uint4*>(i < BK ? sConst + i * 16 : sZero + (i - BK) * 16) =
+          i < BK ? make_uint4(pack16b<DT>(P3::c0, P3::c1), pack16b<DT>(P3::c2, 0.f), 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async();
   }
   if (warp == kMmaWarp) {
@@ -334,25 +332,26 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (it >= 2 && !__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_Q_EMPTY + 2 * st + x), ((it >> 1) & 1) ^ 1, s_abort))) break;
       const float L0 = Ln[0], L1 = Ln[1], d0 = dn[0], d1 = dn[1];
       if (u + 1 < 2 * n_iter) load_stat(u + 1);
-      // finite for every row that is not NaN: the other value's constants are zeros in this k-step, and 0 x infinity is not
       auto l_part = [&](float L) {
         const float v = (L == -INFINITY ? -1e25f : -L) * inv_scale;
         return Parts3<DT>::split(v > 1e30f ? 1e30f : (v < -1e30f ? -1e30f : v));
       };
-      // a delta that is not finite makes its query's column NaN, in S^T as in dP^T
       auto d_part = [&](float d) { return Parts3<DT>::split(fabsf(d) < INFINITY ? -d : NAN); };
       if constexpr (CAP) {
         // stored negated: the compute loop adds it
         *reinterpret_cast<float2*>(sL + st * BQ + x * 64 + lane * 2) = make_float2(L0 == -INFINITY ? -INFINITY : -L0, L1 == -INFINITY ? -INFINITY : -L1);
       }
-      {
-        unsigned char* t = sAug + (2 * st + x) * kAugBytes;
-        *reinterpret_cast<uint4*>(t + aug_off(lane * 2, 0)) = CAP ? make_uint4(0u, 0u, 0u, 0u) : l_part(L0);
-        *reinterpret_cast<uint4*>(t + aug_off(lane * 2, 1)) = d_part(d0);
-        *reinterpret_cast<uint4*>(t + aug_off(lane * 2 + 1, 0)) = CAP ? make_uint4(0u, 0u, 0u, 0u) : l_part(L1);
-        *reinterpret_cast<uint4*>(t + aug_off(lane * 2 + 1, 1)) = d_part(d1);
-        fence_proxy_async();         // written with ordinary stores, read by the MMAs
+      // L and delta have operands of their own: a delta that is not finite makes its query's dP^T NaN and leaves S^T, and so dV,
+      // alone (0 x NaN is NaN, so a shared row of parts would not)
+      uint4* t = reinterpret_cast<uint4*>(sAug + (2 * st + x) * kAugBytes) + lane * 2;
+      if constexpr (!CAP) {
+        t[0] = l_part(L0);
+        t[1] = l_part(L1);
       }
+      t += 4 * kAugBytes / 16;
+      t[0] = d_part(d0);
+      t[1] = d_part(d1);
+      fence_proxy_async();           // written with ordinary stores, read by the MMAs
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(BAR_Q_FULL + 2 * st + x));
       __syncwarp();
@@ -373,7 +372,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint64_t dsd0 = smem_desc(smem_u32(sDS), kTileBytes, 1024);
     const uint64_t qd0 = smem_desc(smem_u32(sQ), 16, 1024), dod0 = smem_desc(smem_u32(sDO), 16, 1024);
     const uint64_t qmn0 = smem_desc(smem_u32(sQ), kTileBytes, 1024), domn0 = smem_desc(smem_u32(sDO), kTileBytes, 1024);
-    const uint64_t constd = smem_desc32(smem_u32(sConst)), augd0 = smem_desc32(smem_u32(sAug));
+    const uint64_t constd = smem_desc_plain(smem_u32(sConst), static_cast<uint32_t>(sZero - sConst), 128);
+    const uint64_t augd0 = smem_desc_plain(smem_u32(sAug), static_cast<uint32_t>(sZero - sAug), 128);
+    constexpr uint64_t kAugU = (kAugBytes >> 4) - (static_cast<uint64_t>(kAugBytes >> 4) << 16);     // the next one, as much nearer to the zeros
     constexpr uint64_t kTileU = kTileBytes >> 4, kHalfRowsU = (64 * 128) >> 4, kDSU = kDSBytes >> 4;
     bool ok = wait(BAR_KV_TMEM, 0);
     tc_fence_after();
@@ -389,12 +390,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
       for (int k = 0; k < HD / 16; ++k)
         mma_ts(tmem + cST + 128 * x, tmem + cKA + k * 8, qd + k * 2, id_st, k > 0 ? 1u : 0u);
-      const uint64_t aug = augd0 + (2 * st + x) * (kAugBytes >> 4);
+      const uint64_t aug = augd0 + (2 * st + x) * kAugU;
       if constexpr (!CAP) mma_ss(tmem + cST + 128 * x, constd, aug, id_st, 1u);
 #pragma unroll
       for (int k = 0; k < HD / 16; ++k)
         mma_ts(tmem + cDPT + 128 * x, tmem + cVA + k * 8, dod + k * 2, id_st, k > 0 ? 1u : 0u);
-      mma_ss(tmem + cDPT + 128 * x, constd + (kConstBytes >> 4), aug, id_st, 1u);
+      mma_ss(tmem + cDPT + 128 * x, constd, aug + 4 * kAugU, id_st, 1u);
       tc_commit(bar(BAR_ST_DONE + x));
     };
     for (int x = 0; x < 2 && ok; ++x) {

@@ -118,15 +118,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
   return d;
 }
 
-// The same for K-major operands of one k-step, 16 elements (32 bytes) a row: 32B swizzle (layout 6), 8-row groups 256 B apart.
-__device__ __forceinline__ uint64_t smem_desc32(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr >> 4) & 0x3fffu);
-  d |= static_cast<uint64_t>(1) << 16;
-  d |= static_cast<uint64_t>(256 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(6) << 61;
-  return d;
+// The same without a swizzle, for K-major operands of one k-step: 8 rows x 16 bytes are 128 contiguous bytes, the next 8 rows
+// sbo_bytes on, the other 8 of a row's 16 elements lbo_bytes on.
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return smem_desc(saddr, lbo_bytes, sbo_bytes) & ~(static_cast<uint64_t>(7) << 61);
 }
 
 // Instruction descriptor for kind::f16: f32 accumulate, A/B format (0 f16, 1 bf16),

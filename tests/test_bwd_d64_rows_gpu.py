@@ -66,3 +66,41 @@ def test_a_row_that_is_not_finite_stays_a_row(dev, dtype, bad):
     assert torch.isfinite(dq[0, 0]).all() and torch.isfinite(dk[0, 0]).all() and torch.isfinite(dv[0, 0]).all()
     assert torch.isfinite(dq[0, 1, rows]).all() and not torch.isfinite(dq[0, 1, 150]).any()
     assert not torch.isfinite(dk[0, 1]).all()
+
+
+_FORMS = [dict(), dict(causal=True), dict(causal=True, window_size=(70, 0)), dict(alibi_slopes="4 heads"), dict(softcap=20.0)]
+
+
+@pytest.mark.parametrize("form", range(len(_FORMS)))
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_a_channel_of_do_that_is_not_finite_stays_a_channel_of_dv(dev, dtype, form):
+    """dV = P^T dO: of a dO row with one infinite channel, that channel of dV has it, and no other."""
+    kw = dict(_FORMS[form])
+    if "alibi_slopes" in kw:
+        kw["alibi_slopes"] = torch.tensor([0.1, 0.2, 0.3, 0.4], device=dev)
+    q, k, v, do = randn((1, 4, 200, 64), dtype, 50), randn((1, 2, 200, 64), dtype, 51), randn((1, 2, 200, 64), dtype, 52), randn((1, 4, 200, 64), dtype, 53)
+    bad = do.clone()
+    bad[0, 1, 150, 7] = float("inf")
+    got, base = _grads(dev, q, k, v, bad, **kw), _grads(dev, q, k, v, do, **kw)
+    other = [d for d in range(64) if d != 7]
+    assert not torch.isfinite(got[2][0, 0, 100:150, 7]).any()
+    assert torch.equal(got[2][..., other], base[2][..., other]) and torch.equal(got[2][0, 1], base[2][0, 1])
+    assert not torch.isfinite(got[0][0, 1, 150]).any()
+
+
+@pytest.mark.parametrize("softcap", [0.0, 20.0])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_delta_that_is_not_finite_by_itself(dev, bad, softcap):
+    """delta = sum(dO o O) not finite where dO is: dV does not depend on it, that row's dS and what is made of it do."""
+    dtype = torch.bfloat16
+    q, k, v, do = (randn((1, 2, 150, 64), dtype, 70 + i).to(dev) for i in range(4))
+    out, lse = fa.flash_attention(q, k, v, softcap=softcap, return_lse=True)
+    base = A._bwd_raw(q, k, v, out, lse, do, 0.125, False, None, softcap=softcap)
+    out[0, 1, 77, 3] = bad
+    dq, dk, dv = A._bwd_raw(q, k, v, out, lse, do, 0.125, False, None, softcap=softcap)
+    assert torch.equal(dv, base[2]) and torch.equal(dk[0, 0], base[1][0, 0])
+    assert not torch.isfinite(dk[0, 1]).any() and not torch.isfinite(dq[0, 1, 77]).any()
+    rows = torch.ones(150, dtype=torch.bool)
+    rows[77] = False
+    # dQ is summed over the key tiles in any order
+    assert torch.allclose(dq[0, 1, rows].float(), base[0][0, 1, rows].float(), rtol=2.0 ** -7, atol=1e-6)

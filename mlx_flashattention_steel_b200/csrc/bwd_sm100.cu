@@ -118,19 +118,18 @@ template <int DT> __device__ __forceinline__ uint32_t pack16b(float a, float b) 
 }
 
 // A float as a sum of three 16-bit values times constants (that the A operand of the k-step has): exact to 2^-24 of it or
-// better.  bfloat16 has float's range.  float16 does not: its constants spread the three parts over 2^31 .. 2^-36; what is
-// larger still (a row that no key of the tile sees, scores beyond 2e9) is cut off there.
+// better.  bfloat16 has float's range.  float16 does not: its constants spread the three parts over 2^31 .. 2^-33 (dS, which is
+// rounded to float16, has no bits below 2^-24).  What is larger than kMax, or not a number, becomes NaN.
 template <int DT> struct Parts3 {
-  static constexpr float c0 = DT == 0 ? 32768.f : 1.f, c1 = 1.f, c2 = DT == 0 ? 1.f / 4096.f : 1.f;
-  // the parts of v as the first 16 bytes of a row of the B operand
+  static constexpr float c0 = DT == 0 ? 32768.f : 1.f, c1 = DT == 0 ? 16.f : 1.f, c2 = DT == 0 ? 1.f / 256.f : 1.f;
+  static constexpr float kMax = DT == 0 ? 65504.f * 32768.f : 1.7014118e38f;
+  // the parts of v as a row of the B operand
   static __device__ __forceinline__ uint4 split(float v) {
-    auto round16 = [](float x) -> float {
-      if (DT == 0) return __half2float(__float2half_rn(x > 65504.f ? 65504.f : (x < -65504.f ? -65504.f : x)));
-      return __bfloat162float(__float2bfloat16_rn(x));
-    };
+    auto round16 = [](float x) -> float { return DT == 0 ? __half2float(__float2half_rn(x)) : __bfloat162float(__float2bfloat16_rn(x)); };
+    if (!(fabsf(v) <= kMax)) v = NAN;
     const float a = round16(v * (1.f / c0));
-    const float r1 = v - a * c0, b = round16(r1);
-    const float r2 = r1 - b, c = round16(r2 * (1.f / c2));
+    const float r1 = v - a * c0, b = round16(r1 * (1.f / c1));
+    const float r2 = r1 - b * c1, c = round16(r2 * (1.f / c2));
     return make_uint4(pack16b<DT>(a, b), pack16b<DT>(c, 0.f), 0u, 0u);
   }
 };
@@ -332,11 +331,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (it >= 2 && !__all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_Q_EMPTY + 2 * st + x), ((it >> 1) & 1) ^ 1, s_abort))) break;
       const float L0 = Ln[0], L1 = Ln[1], d0 = dn[0], d1 = dn[1];
       if (u + 1 < 2 * n_iter) load_stat(u + 1);
-      auto l_part = [&](float L) {
-        const float v = (L == -INFINITY ? -1e25f : -L) * inv_scale;
-        return Parts3<DT>::split(v > 1e30f ? 1e30f : (v < -1e30f ? -1e30f : v));
-      };
-      auto d_part = [&](float d) { return Parts3<DT>::split(fabsf(d) < INFINITY ? -d : NAN); };
+      // A row that sees no key, or is not there, gets the largest value: its P is zero
+      auto l_part = [&](float L) { return Parts3<DT>::split(fabsf(L) == INFINITY ? -copysignf(Parts3<DT>::kMax, inv_scale) : -L * inv_scale); };
       if constexpr (CAP) {
         // stored negated: the compute loop adds it
         *reinterpret_cast<float2*>(sL + st * BQ + x * 64 + lane * 2) = make_float2(L0 == -INFINITY ? -INFINITY : -L0, L1 == -INFINITY ? -INFINITY : -L1);
@@ -349,8 +345,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         t[1] = l_part(L1);
       }
       t += 4 * kAugBytes / 16;
-      t[0] = d_part(d0);
-      t[1] = d_part(d1);
+      t[0] = Parts3<DT>::split(-d0);
+      t[1] = Parts3<DT>::split(-d1);
       fence_proxy_async();           // written with ordinary stores, read by the MMAs
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(BAR_Q_FULL + 2 * st + x));
@@ -749,11 +745,13 @@ bool bwd_sm100_strides_ok(const BwdParams& p) {
            (p.Hkv > 1 && (p.k_hs == 0 || p.v_hs == 0)));
 }
 
-// The kernel of this file also divides L by the scale (see l_part), which has to leave it a float: what is not an ordinary
-// scale takes the portable kernel.
+// The kernel of this file also divides L by the scale (see l_part), which has to leave it a float, and in float16 a number of
+// at most 2^31 (Parts3).  What is not an ordinary scale takes the portable kernel.  In float16 that is one below 2^-7 in the log2
+// domain: from there on a score of 2^31 times the scale is 2^24 or more, where float32 rounds it by up to 1 and P is off by a
+// factor of two in any kernel; below, such scores (rows of a few thousand under a small scale) still have exact gradients.
 bool bwd_sm100_takes(const BwdParams& p, int dtype, int D) {
   const float c = fabsf(p.scale_log2);
-  return bwd_sm100_supported(dtype, D) && bwd_sm100_strides_ok(p) && (p.softcap > 0.f || (c >= 1e-6f && c <= 1e6f));
+  return bwd_sm100_supported(dtype, D) && bwd_sm100_strides_ok(p) && (p.softcap > 0.f || (c >= (dtype == 0 ? 0x1p-7f : 1e-6f) && c <= 1e6f));
 }
 
 // Main backward step only: p.delta and p.dq_acc must already hold delta and zeros.

@@ -104,3 +104,61 @@ def test_a_delta_that_is_not_finite_by_itself(dev, bad, softcap):
     rows[77] = False
     # dQ is summed over the key tiles in any order
     assert torch.allclose(dq[0, 1, rows].float(), base[0][0, 1, rows].float(), rtol=2.0 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype,size,scale", [(torch.float16, 2e4, 1e-6), (torch.float16, 2e4, -1e-6), (torch.float16, 5e3, 2e-5),
+                                              (torch.bfloat16, 2e4, 1e-6)])
+def test_large_rows_under_a_small_scale(dev, dtype, size, scale):
+    """Dot products of 2^28 and beyond 2^31 whose scores are ordinary (up to 2^14 in the log2 domain).  The tensor cores sum them to
+    2^-21 of sum |q_d k_d| (four steps of 2^-23), forward and backward apart, and L is rounded: a relative error of each P that the
+    gradients inherit.  That bound is added to 1.5 times the portable kernel's error, as in test_scores_of_every_size."""
+    q, k, v, do = (randn((1, 4, n, 64), torch.float32, 90 + i).clamp(-3, 3) for i, n in enumerate((200, 333, 333, 200)))
+    q, k, v, do = (q * size).to(dtype), (k * size).to(dtype), v.to(dtype), do.to(dtype)
+    refs = [r.double() for r in orc.backward(q, k, v, do, causal=True, scale=scale)]
+    got = _grads(dev, q, k, v, do, causal=True, scale=scale)
+    base = _grads(dev, q, k, v, do, flags=_lib.FLAG_FORCE_MMA_SYNC, causal=True, scale=scale)
+    Q, K, V, G = (x.double() for x in (q, k, v, do))
+    S = (scale * Q @ K.mT).masked_fill(torch.ones(200, 333).triu(134).bool(), -torch.inf)
+    P, dP = S.softmax(-1), G @ V.mT
+    eP = P * (2 * abs(scale) * 2.0 ** -21 * (Q.abs() @ K.abs().mT) + 2.0 ** -23 * S.logsumexp(-1, keepdim=True).abs())
+    eS = eP * (dP - (P * dP).sum(-1, keepdim=True)).abs() + P * (eP * dP.abs()).sum(-1, keepdim=True)
+    bounds = abs(scale) * (eS @ K.abs()), abs(scale) * (eS.mT @ Q.abs()), eP.mT @ G.abs()
+    for name, g, b, r, bound in zip(("dQ", "dK", "dV"), got, base, refs, bounds):
+        assert torch.isfinite(g).all(), name
+        e, eb = float((g - r).norm()), float((b - r).norm())
+        assert e <= 1.5 * eb + float(bound.norm()), (name, e, eb, float(bound.norm()), float(r.norm()))
+
+
+def test_float16_scores_up_to_the_largest_that_are_taken(dev):
+    """One key per query, q.k = 38016^2 = 1.4e9 (of 2^31; exact), the smallest scale the tcgen05 kernel takes: L is 1.1e7, rounded by up
+    to 1/2, and L / scale by 2^-23 of 1.4e9, a score of 1.4: P between 2^-2 and 2^2."""
+    eye = torch.eye(64, dtype=torch.float16)[None, None] * 38016
+    v, do = randn((1, 1, 64, 64), torch.float16, 20), torch.full((1, 1, 64, 64), 4.0, dtype=torch.float16)
+    dv = _grads(dev, eye, eye, v, do, scale=0.0055)[2]
+    assert (dv.log2() - 2).abs().max() <= 2.0
+
+
+def test_float16_parts_keep_float_precision(dev):
+    """The same with q.k = 17456^2 = 3.05e8, whose second part is beyond 65504: L is 2.4e6, rounded by up to 1/8, and L / scale by
+    2^-23 of 3.05e8, a score of 0.29."""
+    eye = torch.eye(64, dtype=torch.float16)[None, None] * 17456
+    v, do = randn((1, 1, 64, 64), torch.float16, 20), torch.full((1, 1, 64, 64), 4.0, dtype=torch.float16)
+    dv = _grads(dev, eye, eye, v, do, scale=0.0055)[2]
+    assert (dv.log2() - 2).abs().max() <= 0.5
+
+
+@pytest.mark.parametrize("dtype,size", [(torch.bfloat16, 1e34), (torch.float16, 2e3)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_rows_behind_a_sequence_do_not_matter(dev, dtype, size, causal):
+    """Query tiles reach beyond a sequence's end into the next one (or into what pads the packed rows): however large those rows
+    are, the gradients of the sequence in front are those it has alone."""
+    q, k, v, do = (randn((1, 2, 130, 64), dtype, 30 + i).to(dev) for i in range(4))
+    q[:, :, 70:] = (q[:, :, 70:].float() * size).to(dtype)
+    cu = torch.tensor([0, 70], dtype=torch.int32, device=dev)
+    t = [x.clone().requires_grad_(True) for x in (q, k, v)]
+    out = fa.flash_attention_varlen(*t, cu, cu, 70, 70, causal=causal)
+    got = torch.autograd.grad(out, t, do)
+    t = [x[:, :, :70].contiguous().requires_grad_(True) for x in (q, k, v)]
+    want = torch.autograd.grad(fa.flash_attention(*t, causal=causal), t, do[:, :, :70].contiguous())
+    for name, g, w in zip(("dQ", "dK", "dV"), got, want):
+        assert torch.allclose(g[:, :, :70].double(), w.double(), rtol=2.0 ** -7, atol=2.0 ** -10), name

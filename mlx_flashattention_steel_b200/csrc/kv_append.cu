@@ -23,6 +23,15 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 
+// 16 bytes of a row.  Volatile, so that the load stays where it is written, ahead of its use and behind pdl_wait: an ordinary load,
+// which the compiler may move down to it, made the e4m3 kernel, whose conversions are long, slower (262144 tokens x 8 x 128 358 us
+// instead of 348; int8 278.5 either way; with the no-allocate hint for L1 284.5).
+__device__ __forceinline__ uint4 ld16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // SrcT: __half or __nv_bfloat16.  POOL: 0 f16, 1 bf16, 3 int8, 4 e4m3 (the library's dtype codes).
 // No pointer is __restrict__: the launch is a programmatic dependent, and loads of the read-only kind could be served by lines
 // from before the wait.
@@ -75,7 +84,7 @@ kv_append_kernel(const SrcT* k_new, const SrcT* v_new, int64_t token_stride, int
       r.slot = slots[t];
 #pragma unroll
       for (int j = 0; j < VPL / 8; ++j)
-        r.raw[j] = *reinterpret_cast<const uint4*>(new_base + t * token_stride + r.h * head_stride + l * VPL + j * 8);
+        r.raw[j] = ld16(new_base + t * token_stride + r.h * head_stride + l * VPL + j * 8);
     }
     r.write = r.slot >= 0 && r.slot < total_slots;      // padding entries and slots outside the pool write nothing
     f_row += step;

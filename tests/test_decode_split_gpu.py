@@ -327,3 +327,43 @@ def test_ctas_of_one_sequence_each(dev, quant, lens):
     # of units on both sides of the rule
     _run(dev, torch.bfloat16, quant, len(lens), 8, 2, 1, lens, 820)
     _run(dev, torch.bfloat16, quant, len(lens), 32, 8, 3 if len(lens) < 32 else 1, lens, 821)
+
+
+@pytest.mark.parametrize("Hq,Nq,softcap", [(32, 1, 0.0), (16, 4, 30.0)])
+@pytest.mark.parametrize("lens", [[60000, 40000], [60000, 0, 40000], [38000, 1, 0, 17, 30001], [3344 - 150 * (i % 20) for i in range(23)]])
+def test_two_warps_per_head_in_ctas_of_one_sequence_each(dev, lens, Hq, Nq, softcap):
+    # int8, 8 kv heads: 32 or more units per CTA (two warps take them in turn) of so few sequences that no CTA has two; a
+    # sequence of one unit leaves the second warp without any
+    _run(dev, torch.bfloat16, "int8", len(lens), Hq, 8, Nq, lens, 830, softcap=softcap)
+
+
+def test_lengths_written_by_the_launch_directly_in_front(dev):
+    """The merge kernel reads the lengths before it waits for the main kernel, which therefore lets it in only after its own wait:
+    the append in front, which lets its successor in at once, writes them here (16-bit rows are copied bit for bit)."""
+    lens = [700, 16, 0, 333, 1]
+    pg = make_paged(len(lens), 2, 128, 16, lens, torch.bfloat16, 840)
+    q = randn((len(lens), 8, 1, 128), torch.bfloat16, 841)
+    want, _ = orc.paged_attention(q, pg["k"], pg["v"], pg["block_table"], pg["seq_lens"], causal=True)
+    buf, other = (torch.zeros(32, dtype=torch.int32, device=dev) for _ in range(2))
+    now = torch.zeros(32, dtype=torch.int32)
+    now[:len(lens)] = pg["seq_lens"]
+    rows = [x.to(dev).view(torch.float16).view(1, 1, 64) for x in (torch.zeros_like(now), now)]
+    pools = [x.view(torch.float16).view(1, 1, 1, 64) for x in (buf, other)]
+    slot = torch.zeros(1, dtype=torch.int64, device=dev)
+    qd, kp, vp, table = q.to(dev), pg["k"].to(dev), pg["v"].to(dev), pg["block_table"].to(dev)
+    A._set_check_decode_status(False)
+
+    def call():
+        for r in rows:
+            fa.kv_append(r, r, slot, *pools)
+        return fa.flash_attention_paged(qd, kp, vp, table, buf[:len(lens)], causal=True, max_kv_len=700)
+
+    for _ in range(20):
+        assert_close(call(), want, torch.bfloat16)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    for _ in range(20):
+        out.fill_(1.0)
+        graph.replay()
+        assert_close(out, want, torch.bfloat16)

@@ -199,3 +199,81 @@ def test_capture(dev):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.gpu
+def test_which_calls_are_taken(dev):
+    """The comparisons above hold as well where the extension takes nothing: here each plain call has to be taken, once and by the
+    form in front of the Python code, and each other one given back."""
+    taken = []
+
+    class Named:
+        def __getattr__(self, name):
+            def call(*a):
+                r = getattr(H, name)(*a)
+                if r is not None:
+                    taken.append(name if name != "fwd" or a[9] else "fwd, behind the checks")
+                return r
+            return call
+
+    def check(want, fn):
+        taken.clear()
+        old = A._H
+        A._H = R._H = K._H = Named()
+        try:
+            fn()
+        finally:
+            A._H = R._H = K._H = old
+        assert taken == want, (taken, want)
+
+    for dt in (torch.float16, torch.bfloat16, torch.float32):
+        for D in (64, 128):
+            q, k = _r(2, 4, 70, D, dt=dt), _r(2, 2, 133, D, dt=dt)
+            for kw in (dict(), dict(causal=True, return_lse=True), dict(scale=2, window_size=(20, 0), causal=True), dict(softcap=20)):
+                check(["fwd"], lambda: fa.flash_attention(q, k, k, **kw))
+            bshd = _r(2, 133, 2, D, dt=dt).transpose(1, 2)
+            check(["fwd"], lambda: fa.flash_attention(q, bshd, bshd))
+            check(["fwd"], lambda: fa.flash_attention(q[:1].expand(2, 4, 70, D), k, k))
+            check(["fwd, behind the checks"], lambda: fa.flash_attention(q, k, k, causal=1))
+            check(["fwd, behind the checks"], lambda: fa.flash_attention(q, k, k, window_size=[10, -1]))
+            odd, one = _r(2, 2, 133, D + 1, dt=dt)[..., :D], k[:, :1].expand(2, 2, 133, D)
+            for x in (odd, one):
+                check([], lambda: fa.flash_attention(q, x, x))
+            check([], lambda: fa.flash_attention(q, k, k, stream=torch.cuda.current_stream()))
+
+            def train(g):
+                t = [x.clone().requires_grad_(True) for x in (q, k, k)]
+                torch.autograd.grad(fa.flash_attention(*t), t, g)
+            if dt != torch.float32:
+                check(["fwd, behind the checks", "bwd"], lambda: train(q))
+                check(["fwd, behind the checks"], lambda: train(q[:, :, :1].expand(q.shape)))
+
+    B, P = 3, 40
+    table, lens = torch.randperm(P, device=dev)[:B * 12].view(B, 12).int(), torch.tensor([1, 100, 190], dtype=torch.int32, device=dev)
+    for pool in (torch.float16, torch.int8, torch.float8_e4m3fn):
+        kp = _r(P, 16, 2, 128).mul(20).to(pool)
+        s = None if pool == torch.float16 else torch.rand(P, 16, 2, device=dev).half() * 0.05
+        for Nq, rows_ok in ((1, True), (4, True), (8, True), (9, False)):        # 4, 16, 32 and 36 query rows per kv head
+            q = _r(B, 8, Nq, 128)
+
+            def paged(q=q, table=table, lens=lens, **kw):
+                return fa.flash_attention_paged(q, kp, kp, table, lens, k_scale=s, v_scale=s, **kw)
+            for kw in (dict(), dict(causal=True, return_lse=True, softcap=30.0), dict(scale=0.2, num_splits=2)):
+                check(["decode"] if rows_ok else [], lambda: paged(max_kv_len=190, **kw))
+        check([], lambda: paged(q=q[:, :, :2]))
+        check([], lambda: paged(q=q[:, :, :2], max_kv_len=190))                  # q strided
+        q = _r(B, 8, 1, 128)
+        check([], lambda: paged(q=q))
+        check([], lambda: paged(q=q, table=table.long(), max_kv_len=190))
+        check([], lambda: paged(q=q, lens=lens.long(), max_kv_len=190))
+        kn, slots, pools = _r(B, 2, 1, 128)[:, :, 0], torch.tensor([5, -1, 77], device=dev), [kp.clone(), kp.clone(), s, s]
+        check(["append"], lambda: fa.kv_append(kn, kn, slots, *pools))
+        check([], lambda: fa.kv_append(kn, kn.transpose(0, 1).contiguous().transpose(0, 1), slots, *pools))
+    x, cos = _r(B, 8, 1, 128), torch.rand(300, 64, device=dev)
+    for off in (0, 7, [1, 2, 290], (1, 2, 3)):
+        check(["rope"], lambda: fa.apply_rope(x, cos, cos, off))
+        check(["rope"], lambda: fa.apply_rope(x, cos[:, :16].contiguous(), cos[:, :16].contiguous(), off, interleaved=False, rotary_dim=32))
+        check([], lambda: fa.apply_rope(x, cos[:, :16], cos[:, :16], off, rotary_dim=32))
+    for off in (torch.tensor([4, 5, 6]), torch.tensor([4, 5, 6], device=dev), [True, 1, 2]):
+        check([], lambda: fa.apply_rope(x, cos, cos, off))
+    check([], lambda: fa.apply_rope(x.requires_grad_(True), cos, cos, 0))

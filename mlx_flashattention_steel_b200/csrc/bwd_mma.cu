@@ -33,6 +33,23 @@ constexpr int kThreads = 256;
 
 __host__ __device__ inline size_t bwd_align(size_t x) { return (x + 255) / 256 * 256; }
 
+// Packed rows of no sequence (in front of the first, behind the last) have no gradient, and the kernels that follow do not
+// visit them: zeros in chunk c (8 values) of dK, dV and, where no accumulator stands behind it, dQ, by the threads of row i of
+// query head h.
+template <int D> __device__ __forceinline__ void clear_rows_of_no_sequence(const BwdParams& p, int h, int i, int c) {
+  if (p.cu_k == nullptr) return;
+  auto clear = [&](void* t, int64_t row) { reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(t) + row)[c] = make_uint4(0u, 0u, 0u, 0u); };
+  if (h < p.Hkv) {
+    const int first = p.cu_k[0], last = p.cu_k[p.nseq];
+    for (int64_t k = i; k < p.S; k += p.N) {
+      if (k >= first && k < last) continue;
+      clear(p.dk, h * p.dk_hs + k * p.dk_rs);
+      clear(p.dv, h * p.dk_hs + k * p.dk_rs);
+    }
+  }
+  if (p.dq_acc == nullptr && (i < p.cu_q[0] || i >= p.cu_q[p.nseq])) clear(p.dq, h * p.dq_hs + i * p.dq_rs);
+}
+
 // ---------------------------------------------------------------------------
 // 1. delta and dQ-accumulator reset.  One warp per (b, h, row).
 // ---------------------------------------------------------------------------
@@ -60,6 +77,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const BwdParams p, 
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
   if (lane == 0) p.delta[warp] = acc;
+  if (lane < D / 8) clear_rows_of_no_sequence<D>(p, h, i, lane);
   if (p.dq_acc != nullptr) {          // the split head_dim-128 path has no accumulator
     float* dq = p.dq_acc + static_cast<int64_t>(warp) * D;
 #pragma unroll
@@ -102,6 +120,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_vec_kernel(const BwdParams
 #pragma unroll
   for (int sft = LPR / 2; sft > 0; sft >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sft);
   if (live && c == 0) p.delta[row] = acc;
+  if (live) clear_rows_of_no_sequence<D>(p, h, i, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -507,6 +526,7 @@ cudaError_t launch_bwd(const BwdParams& p_in, int dtype, int D, bool varlen, int
   BwdParams p = p_in;
   const size_t rows = static_cast<size_t>(p.B) * p.Hq * p.N;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+  p.nseq = varlen ? nbatch : 0;
   p.delta = reinterpret_cast<float*>(ws);
   p.work_counter = reinterpret_cast<int*>(ws + bwd_align(rows * sizeof(float)));
   p.dq_acc = bwd_takes_split_path(p, dtype, D, allow_sm100) ? nullptr

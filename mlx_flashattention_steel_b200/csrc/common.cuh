@@ -78,6 +78,7 @@ struct BwdParams {
   int window_left;       // -1 = off
   const int* cu_q;
   const int* cu_k;
+  int nseq;              // cu_q, cu_k: number of sequences
   const float* alibi;    // per q-head slopes, or null
   const unsigned char* bmask;  // block mask bytes [rows / bm_bq][bm_nk], or null
   int bm_bq, bm_bk, bm_nk;

@@ -92,6 +92,7 @@ struct KernelArgs {
   int group;         // Hq / Hkv
   int rows;          // group * Nq
   int hpc;           // kv heads per CTA
+  int merge_lets_in; // the merge kernel lets its successor in before it has ended
   int aligned;       // CTAs of one sequence each (take_aligned)
   int row_groups;    // consumer warps per kv head that share its rows (1 up to 16 rows)
   int page_groups;   // consumer warps per kv head that take its units in turn, each leaving partials of its own
@@ -316,7 +317,7 @@ decode_merge_kernel(const __grid_constant__ KernelArgs a, int gx, int W_, int bl
   }
 
   pdl_wait();               // the main kernel has ended: its partials and status words can be read
-  pdl_launch_dependents();
+  if (a.merge_lets_in) pdl_launch_dependents();
 
   if (blockIdx.x == 0) {
     // error word = all bits that the main kernel's warps left
@@ -1304,6 +1305,11 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.row_groups = sh.row_groups;
   a.aligned = take_aligned(p.B, p.max_kv_len, gx) ? 1 : 0;
   a.page_groups = sh.page_groups;
+  // Not where four or six CTAs share an SM: they are 12 warps of 168 registers, which is all of its registers, and the next
+  // call's, placed while merge blocks still run, came up one short on some SMs (presumably because those leave the four register
+  // files unevenly free) and waited there for another's end.  100 sequences up to 12000 tokens, 3 queries, 2 kv heads, back to
+  // back: int8 156 -> 102.5 us, f16 136 -> 112; 1 kv head, 2 queries, int8 101 -> 85.5.  Elsewhere it gains up to 1 us.
+  a.merge_lets_in = ctas_per_sm(hpc * sh.row_groups) < 4 ? 1 : 0;
   a.stage_kv_bytes = hpc * kBS * row_bytes;
   a.scale_bytes = quant ? kBS * p.Hkv * 2 : 0;
   a.qlo_bytes = p.kv_dtype == 3 ? hpc * sh.row_groups * sh.page_groups * (rows > 8 ? 2048 : 1024) : 0;

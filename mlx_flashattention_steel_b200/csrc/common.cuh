@@ -93,7 +93,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Host side: launches `kern` as such a dependent of what is in front of it in the stream.  Every kernel launched so waits
 // (pdl_wait) before it touches global memory, reads included, so that "the kernel before it has ended" implies the same of
 // all kernels before that one; and it reads what others may have written with loads that are not of the read-only
-// kind, which may be served by lines fetched before the wait.
+// kind, which may be served by lines fetched before the wait.  One exception: decode_merge_kernel reads the lengths
+// before it waits, which holds because decode_paged_kernel, always in front of it, lets it in behind its own wait.
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr;

@@ -403,3 +403,11 @@ def test_full_size_properties(dev):
     vsc.fill_(0.02)
     outc = fa.flash_attention_paged(q, kq, vq, tt, lt, causal=True, k_scale=ksc, v_scale=vsc, max_kv_len=int(lens.max()))
     assert float((outc.float() - 1.0).abs().max()) <= 1e-2
+
+
+@pytest.mark.parametrize("D,block_size", [(64, 16), (64, 32), (128, 16), (128, 48), (128, 64)])
+def test_paged_prefill_of_a_few_tiles(dev, D, block_size):
+    # one to four key tiles of 64, on both sides of a tile's end and of the two that are asked for before the loop, with holes
+    lens = [1, 16, 63, 64, 65, 127, 128, 129, 191, 193, 250]
+    _run(dev, torch.bfloat16, None, len(lens), 8, 2, 20, lens, 640, D=D, block_size=block_size, holes=True)
+    _run(dev, torch.float16, None, len(lens), 2, 2, 140, lens, 641, D=D, block_size=block_size, causal=False)

@@ -106,6 +106,12 @@ def _i32(t: torch.Tensor) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _f16(t: torch.Tensor) -> torch.Tensor:
+    if t.dtype != torch.float16:
+        t = t.to(torch.float16)
+    return t if t.is_contiguous() else t.contiguous()
+
+
 def _stream_ptr(stream, device) -> int:
     if stream is None:
         return torch._C._cuda_getCurrentRawStream(device.index)
@@ -761,9 +767,8 @@ def flash_attention_paged(
     if quant:
         if k_scale is None or v_scale is None:
             raise ValueError("flash_attention_paged: int8/fp8 pools need k_scale and v_scale.")
-        k_scale = _as_tensor(k_scale, "k_scale").to(torch.float16).contiguous()
-        v_scale = _as_tensor(v_scale, "v_scale").to(torch.float16).contiguous()
-        if tuple(k_scale.shape) != tuple(k_pages.shape[:3]) or tuple(v_scale.shape) != tuple(v_pages.shape[:3]):
+        k_scale, v_scale = _f16(_as_tensor(k_scale, "k_scale")), _f16(_as_tensor(v_scale, "v_scale"))
+        if not (k_scale.shape == v_scale.shape == k_pages.shape[:3]):
             raise ValueError("flash_attention_paged: scales must be [num_pages, block_size, Hkv].")
     elif k_pages.dtype != q.dtype:
         raise ValueError(f"flash_attention_paged: pool dtype {k_pages.dtype} must equal q dtype or be int8/fp8.")

@@ -214,15 +214,20 @@ PyObject* decode_impl(PyObject* const* a, Py_ssize_t n) {
   double scale = 0., softcap;
   bool given, causal, want_lse;
   int64_t block_size, max_kv_len, num_splits, flags, max_rows;
-  if (n != 16 || !get_scale(a[7], &scale, &given) || !get_bool(a[8], &causal) || !get_float(a[9], &softcap) || !get_int(a[10], &block_size) ||
-      !get_int(a[11], &max_kv_len) || !get_bool(a[12], &want_lse) || !get_int(a[13], &num_splits) || !get_int(a[14], &flags) ||
-      !get_int(a[15], &max_rows) || !plain_mode())
-    NOT_HERE;
+  if (n != 16) NOT_HERE;
+  // First what gives back the chunks of a prefill, the other calls that come this way: too many query rows per kv head
   const Tensor* t[5];
-  for (int i = 0; i < 5; ++i)
+  if ((t[0] = plain(a[0])) == nullptr || (t[1] = plain(a[1])) == nullptr || t[0]->dim() != 4 || t[1]->dim() != 4 || !get_int(a[15], &max_rows) ||
+      t[0]->size(1) * t[0]->size(2) > max_rows * t[1]->size(2))
+    NOT_HERE;
+  if (!get_scale(a[7], &scale, &given) || !get_bool(a[8], &causal) || !get_float(a[9], &softcap) || !get_int(a[10], &block_size) ||
+      !get_int(a[11], &max_kv_len) || !get_bool(a[12], &want_lse) || !get_int(a[13], &num_splits) || !get_int(a[14], &flags) ||
+      !plain_mode())
+    NOT_HERE;
+  for (int i = 2; i < 5; ++i)
     if ((t[i] = plain(a[i])) == nullptr) NOT_HERE;
   const Tensor &q = *t[0], &kp = *t[1], &vp = *t[2], &table = *t[3], &lens = *t[4];
-  if (wants_grad(q) || wants_grad(kp) || wants_grad(vp) || q.dim() != 4 || kp.dim() != 4 || vp.dim() != 4 || !current_device(q)) NOT_HERE;
+  if (wants_grad(q) || wants_grad(kp) || wants_grad(vp) || vp.dim() != 4 || !current_device(q)) NOT_HERE;
   const int64_t B = q.size(0), Hq = q.size(1), Nq = q.size(2), D = q.size(3), Hkv = kp.size(2);
   const int code = half_code(q.scalar_type()), kv = pool_code(kp.scalar_type());
   const bool quant = kv == B200FA_I8 || kv == B200FA_E4M3;

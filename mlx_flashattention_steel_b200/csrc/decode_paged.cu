@@ -92,7 +92,6 @@ struct KernelArgs {
   int group;         // Hq / Hkv
   int rows;          // group * Nq
   int hpc;           // kv heads per CTA
-  int merge_lets_in; // the merge kernel lets its successor in before it has ended
   int aligned;       // CTAs of one sequence each (take_aligned)
   int row_groups;    // consumer warps per kv head that share its rows (1 up to 16 rows)
   int page_groups;   // consumer warps per kv head that take its units in turn, each leaving partials of its own
@@ -118,8 +117,8 @@ __device__ __forceinline__ int units_of(const int32_t* seq_lens, int i, int max_
 // CTAs (of gx) that work on U units of B sequences.  With few units not every CTA does: two units (one step of the
 // consumers) each, or one sequence each when they are that short -- a CTA more to a sequence is a part more to merge, a
 // second sequence in a CTA costs it 4 us.  The CTAs that share a sequence are always consecutive.
-__device__ __forceinline__ int working_ctas(long long U, int B, int gx) {
-  const long long want = max((U + 1) / 2, min(U, static_cast<long long>(B)));
+__host__ __device__ inline int working_ctas(long long U, int B, int gx) {
+  const long long pairs = (U + 1) / 2, seqs = U < B ? U : B, want = pairs > seqs ? pairs : seqs;
   return want < static_cast<long long>(gx) ? static_cast<int>(want) : gx;
 }
 
@@ -268,7 +267,7 @@ constexpr int kMaxMergeWarps = 32;
 // AL: the main kernel's CTAs have one sequence each.  MANY: W > 1.  One warp to a row has few parts: 6 at a time, and four blocks to an SM.
 template <int kD, bool MANY, bool AL>
 __global__ void __launch_bounds__(MANY ? kMaxMergeWarps * 32 : kMergeWarps * 32, MANY ? 1 : 4)
-decode_merge_kernel(const __grid_constant__ KernelArgs a, int gx, int W_, int blocks_per_seq) {
+decode_merge_kernel(const __grid_constant__ KernelArgs a, int gx, int W_, int blocks_per_seq, int let_in) {
   constexpr int kBatch = MANY ? 8 : 6;                // partial rows in flight per warp
   const int W = MANY ? W_ : 1;
   const DecodeParams& p = a.p;
@@ -317,7 +316,7 @@ decode_merge_kernel(const __grid_constant__ KernelArgs a, int gx, int W_, int bl
   }
 
   pdl_wait();               // the main kernel has ended: its partials and status words can be read
-  if (a.merge_lets_in) pdl_launch_dependents();
+  if (let_in) pdl_launch_dependents();
 
   if (blockIdx.x == 0) {
     // error word = all bits that the main kernel's warps left
@@ -490,10 +489,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     fence_barrier_init();
     fence_proxy_async();
   }
-  // The kernel before this one has ended: its outputs (lengths, tables, queries, the rows just appended) can be read.  Only behind
-  // this (in the producer warp) may the merge kernel's blocks take their places, since they read the lengths without a wait of
-  // their own.
+  // The kernel before this one has ended: its outputs (lengths, tables, queries, the rows just appended) can be read.  Only now
+  // may the merge kernel's blocks take their places, since they read the lengths without a wait of their own.
   pdl_wait();
+  pdl_launch_dependents();
   // page prefix sums
   const int* page_start = s_page_start;
   if (p.B <= kSmemSeqs) {
@@ -557,9 +556,6 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
   if (warp == n_cons) {
     // ======================= producer warp =======================
-    // The merge kernel may come in.  Here and not behind the wait, where the int8 kernel of 9 to 32 rows, at its limit of 168
-    // registers, was compiled into one 3 % slower (100 sequences up to 12000 tokens, 12 rows, 4 kv heads 182 -> 177 us).
-    pdl_launch_dependents();
     int stage = 0;
     uint32_t phase = 0;
     long long u = lo;
@@ -1249,13 +1245,23 @@ template <int D>
 cudaError_t launch_merge(const KernelArgs& a, int gx, cudaStream_t stream) {
   int W = 1;
   while (W < kMaxMergeWarps && static_cast<long long>(gx) * a.page_groups > 8LL * a.p.B * W) W <<= 1;
+  // The successor may come in before the merge kernel has ended, but not where four or six CTAs share an SM and most of them
+  // have work: they are 12 warps of 168 registers, which is all of its registers, and the next call's, placed while merge
+  // blocks still run, came up one short on some SMs (presumably because those leave the four register files unevenly free)
+  // and waited there for another's end.  100 sequences up to 12000 tokens, 3 queries, 2 kv heads, back to back: int8 156
+  // -> 102.5 us, f16 136 -> 112; 1 kv head, 2 queries, int8 101 -> 85.5.  Elsewhere it gains up to 1 us (1 sequence of 576 tokens,
+  // 2 kv heads, 4 queries 11.2 -> 10.6); a CTA without work, as far as the longest length tells, ends at once and makes room.
+  // (A parameter of its own: the main kernels for 9 to 32 rows, at their limit of 168 registers, come out of the compiler
+  // differently with every member of KernelArgs; one more made int8 182 -> 177 us and e4m3 186 -> 188.)
+  const int let_in = ctas_per_sm(a.hpc * a.row_groups) < 4 ||
+                     2 * working_ctas(static_cast<long long>(a.p.B) * ((a.p.max_kv_len + kBS - 1) / kBS), a.p.B, gx) <= gx;
   const int warps = W > kMergeWarps ? W : kMergeWarps, rows_per_block = warps / W;
   const int blocks_per_seq = (a.p.Hq * a.p.Nq + rows_per_block - 1) / rows_per_block;
   const long long blocks = static_cast<long long>(a.p.B) * blocks_per_seq;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   const size_t smem = W > 1 ? static_cast<size_t>(warps) * 32 * sizeof(float4) : 0;
   const dim3 grid(static_cast<unsigned>(blocks)), block(warps * 32);
-  auto go = [&](auto kern) { return launch_dependent(kern, grid, block, smem, stream, a, gx, W, blocks_per_seq); };
+  auto go = [&](auto kern) { return launch_dependent(kern, grid, block, smem, stream, a, gx, W, blocks_per_seq, let_in); };
   if (a.aligned) return W > 1 ? go(decode_merge_kernel<D, true, true>) : go(decode_merge_kernel<D, false, true>);
   return W > 1 ? go(decode_merge_kernel<D, true, false>) : go(decode_merge_kernel<D, false, false>);
 }
@@ -1308,11 +1314,6 @@ cudaError_t launch_decode_paged(const DecodeParams& p, cudaStream_t stream, char
   a.row_groups = sh.row_groups;
   a.aligned = take_aligned(p.B, p.max_kv_len, gx) ? 1 : 0;
   a.page_groups = sh.page_groups;
-  // Not where four or six CTAs share an SM: they are 12 warps of 168 registers, which is all of its registers, and the next
-  // call's, placed while merge blocks still run, came up one short on some SMs (presumably because those leave the four register
-  // files unevenly free) and waited there for another's end.  100 sequences up to 12000 tokens, 3 queries, 2 kv heads, back to
-  // back: int8 156 -> 102.5 us, f16 136 -> 112; 1 kv head, 2 queries, int8 101 -> 85.5.  Elsewhere it gains up to 1 us.
-  a.merge_lets_in = ctas_per_sm(hpc * sh.row_groups) < 4 ? 1 : 0;
   a.stage_kv_bytes = hpc * kBS * row_bytes;
   a.scale_bytes = quant ? kBS * p.Hkv * 2 : 0;
   a.qlo_bytes = p.kv_dtype == 3 ? hpc * sh.row_groups * sh.page_groups * (rows > 8 ? 2048 : 1024) : 0;

@@ -153,7 +153,8 @@ int32_t b200fa_bwd(const b200fa_desc* d, const void* q, const void* k, const voi
 /*
  * Backward, packed variable-length sequences, one launch sequence for all
  * sequences.  Replaces the per-sequence Python loop of _varlen_bwd
- * (mlx_mfa/attention.py:2492-2521).
+ * (mlx_mfa/attention.py:2492-2521).  Rows of dq, dk and dv in front of the first or behind the last sequence are set
+ * to zero.
  */
 size_t  b200fa_bwd_varlen_workspace_bytes(const b200fa_desc* d, int32_t num_seqs,
                                           int32_t max_seqlen_q, int32_t max_seqlen_k);

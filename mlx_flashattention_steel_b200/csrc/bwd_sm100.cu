@@ -406,8 +406,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (!wait(BAR_PD_READY + x, it & 1)) { ok = false; break; }
         tc_fence_after();
         const uint64_t qmn = qmn0 + st * kTileU + x * kHalfRowsU, domn = domn0 + st * kTileU + x * kHalfRowsU;
-        // A in TMEM: 8 columns per 16 queries; queries 0-31 of the half at +0, 32-63 at +32 (where the two warps of a
-        // row wrote them); B rows = queries, 16 rows = 128 units
+        // A in TMEM: 8 columns per 16 queries; queries 0-31 of the half at +0, 32-63 at +32 (each part over the scores
+        // it was made from); B rows = queries, 16 rows = 128 units
         if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -614,7 +614,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
         // P^T and dS^T go back as 16-bit pairs along the query index, inside the 32 columns this warp has just read
-        // (the other warp of these rows may still be reading its own 32)
+        // (it reads the half's other 32 after these)
         tmem_st16(tmem + lane_base + cST + 128 * x + hf * 32, pp);
         tmem_st16(tmem + lane_base + cDPT + 128 * x + hf * 32, pd);
 #pragma unroll
@@ -647,7 +647,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     // every MMA of the item is complete (a barrier of its own: half a's warps can be two completions ahead of DQ_DONE)
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar(BAR_ACC_DONE), 0, s_abort));
-    // dK, dV: rows = keys, this warp's 32 of the 64 columns.  The tiles go through shared memory (the Q stages, which
+    // dK, dV: rows = keys, all 64 columns of one of them per warp.  The tiles go through shared memory (the Q stages, which
     // nothing reads any more) so that each store instruction writes four whole 128-byte rows: straight from the TMEM
     // layout a warp would touch 32 different rows per instruction, which took 3600 clk per CTA.
     if (ok) {
